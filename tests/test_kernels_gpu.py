@@ -248,6 +248,28 @@ def test_gemm_rows_do_not_depend_on_the_batch():
     assert torch.equal(one[0], full[97])
 
 
+@pytest.mark.parametrize("N, K", [(1, 4), (77, 300), (1024, 1024), (2500, 132)])
+def test_gemm_simt_forms_agree_bit_for_bit(N, K):
+    """The streaming form (up to 4, 8, 16 rows) and every tile form the same sum, one chain of FMAs over k."""
+    g = torch.Generator(device=DEV).manual_seed(9)
+    a = torch.randn(513, K, device=DEV, generator=g)
+    w = torch.randn(N, K, device=DEV, generator=g)
+    full = torch.empty(513, N, device=DEV)
+    ops().gemm_tn_simt(a, w, full)
+    # K FMAs of N(0, 1) products: each rounds a partial sum of at most a few sqrt(K) by 2^-24 of it
+    ref = a.double() @ w.double().T
+    assert (full.double() - ref).abs().max() <= 4 * K * 2.0 ** -24 * math.sqrt(K) + 1e-6
+    for M in (1, 4, 5, 8, 9, 16, 17, 32, 33, 65, 129, 305):
+        some = torch.full((M, N), 7.0, device=DEV)
+        ops().gemm_tn_simt(a[:M].contiguous(), w, some)
+        assert torch.equal(some, full[:M]), M
+    shifted = torch.empty(1 + 5 * K, device=DEV)[1:].view(5, K)          # rows that 16-byte copies do not take
+    shifted.copy_(a[:5])
+    some = torch.empty(5, N, device=DEV)
+    ops().gemm_tn_simt(shifted, w, some)
+    assert torch.equal(some, full[:5])
+
+
 def test_argmax_ties_go_to_the_lowest_id():
     logits = torch.zeros(4, 1000, device=DEV)
     logits[0, [5, 700]] = 3.0
