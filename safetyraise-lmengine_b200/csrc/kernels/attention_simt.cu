@@ -1,113 +1,319 @@
-// Paged causal attention for a ragged batch, plain SIMT arithmetic in float32.
+// Paged causal attention for a ragged batch, plain FMA arithmetic in float32.
 //
-// One warp per (token, query head).  The warp walks the request's keys in
-// blocks of 32 aligned to multiples of 32 from the start of the sequence, so
-// the order of every sum depends only on the token's position: the result is
-// the same however the tokens were cut into steps or batched.  This is the
-// attention of the float32 path, and the reference the tensor-core kernels are
-// tested against.  Formula: src/model/math.rs:102-155 (scale 1/sqrt(hd) or the
-// given one, query head h reads KV head h / (nq/nkv), online softmax).
+// A row (token, query head) walks its request's keys in blocks of 32 aligned to
+// multiples of 32 from the start of the sequence, one running softmax, a score one
+// chain of FMAs over the head, an output one chain over the keys: the order of
+// every sum depends only on the token's position, so the result is the same however
+// the tokens were cut into steps or batched.  This is the attention of the float32
+// path, and the reference the tensor-core kernels are tested against.  Formula:
+// src/model/math.rs:102-155 (scale 1/sqrt(hd) or the given one, query head h reads
+// KV head h / (nq/nkv), online softmax).
+//
+// A block serves up to 32 rows that read the same KV head: the query heads of a run of tokens of one request.  Keys and
+// values of a span of 128 / 64 / 32 keys (heads up to 64 / 128 / 256) are copied to shared memory once for all rows, the
+// next span in flight under the current one.  Eight warps form the scores, a lane a key; then each warp owns up to four
+// rows, a lane the dimensions lane + 32 i.  Bound by the FMA and shared-memory pipes for prompts (2,048 tokens, 32 heads of
+// 128: 2.8 ms; 34.2 with a warp a row that read its keys from global memory), by the chain of spans of the longest request
+// for decode steps (8 requests of 2,048: 0.19 ms; 2.75).
 #include <math_constants.h>
 
 #include "common.cuh"
 
 namespace srlm {
 
-constexpr int kMaxDimsPerLane = 8;   // head_dim <= 256
+constexpr int SA_THREADS = 256, SA_WARPS = 8, SA_ROWS = 32, SA_OWN = SA_ROWS / SA_WARPS;
 
-template <typename TA, typename TC>
-__global__ void paged_attention_simt_kernel(
-    const TA* __restrict__ q, const TC* __restrict__ k_cache, const TC* __restrict__ v_cache,
-    TA* __restrict__ out, const int* __restrict__ block_table, int table_stride,
-    const int* __restrict__ entry_of_token, const int* __restrict__ positions, int T, int nq, int nkv,
-    int hd, int page_size, float scale, int window) {
-  extern __shared__ float q_sh[];      // [warps per block][hd]
-  const int warp_in_block = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + warp_in_block;
-  if (warp >= (long long)T * nq) return;
-  const int t = (int)(warp / nq), h = (int)(warp % nq);
-  const int kvh = h / (nq / nkv);
-  const int pos = positions[t];
-  const int* table = block_table + (size_t)entry_of_token[t] * table_stride;
+template <int DIMS>                  // dimensions a lane owns: heads up to 32 * DIMS
+struct SimtSpan {
+  static constexpr int KEYS = DIMS <= 2 ? 128 : DIMS <= 4 ? 64 : 32;
+};
 
-  float* qv = q_sh + warp_in_block * hd;
-  const TA* qsrc = q + ((size_t)t * nq + h) * hd;
-  for (int d = lane; d < hd; d += 32) qv[d] = to_float(qsrc[d]);
-  __syncwarp();
+// Floats from a staged key to the next: an odd number of 16-byte pieces, so that lanes on neighbouring keys share no bank.
+__host__ __device__ __forceinline__ int simt_key_ld(int hd) { return 4 * (((hd + 3) / 4) | 1); }
+__host__ __device__ __forceinline__ int simt_row_ld(int hd) { return (hd + 3) / 4 * 4; }
 
-  float acc[kMaxDimsPerLane];
+static size_t simt_smem(int hd, int keys) {
+  return sizeof(float) * (2ull * keys * (simt_key_ld(hd) + simt_row_ld(hd)) + (size_t)SA_ROWS * simt_row_ld(hd) +
+                          (size_t)SA_ROWS * keys) + sizeof(long long) * 2 * keys;
+}
+
+// Scores of `NR` neighbouring rows against a lane's key.
+template <int NR>
+__device__ __forceinline__ void simt_scores(const float* __restrict__ kp, const float* __restrict__ qs, int ldq, int pieces,
+                                            float (&dot)[NR]) {
 #pragma unroll
-  for (int i = 0; i < kMaxDimsPerLane; ++i) acc[i] = 0.f;
-  float m = -CUDART_INF_F, z = 0.f;
-
-  const int first_key = window > 0 ? max(0, pos - window + 1) : 0;
-  for (int jb = (first_key / 32) * 32; jb <= pos; jb += 32) {
-    const int j = jb + lane;
-    const bool valid = j >= first_key && j <= pos;
-    float s = -CUDART_INF_F;
-    size_t row = 0;
-    if (valid) {
-      const int page = table[j / page_size];
-      row = ((size_t)page * nkv + kvh) * page_size + (j % page_size);
-      const TC* kp = k_cache + row * hd;
-      float dot = 0.f;
-      for (int d = 0; d < hd; ++d) dot += qv[d] * to_float(kp[d]);
-      s = dot * scale;
+  for (int r = 0; r < NR; ++r) dot[r] = 0.f;
+#pragma unroll 4
+  for (int c = 0; c < pieces; ++c) {
+    const float4 k = *reinterpret_cast<const float4*>(kp + 4 * c);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      const float4 x = *reinterpret_cast<const float4*>(qs + r * ldq + 4 * c);
+      dot[r] = fmaf(x.x, k.x, dot[r]);
+      dot[r] = fmaf(x.y, k.y, dot[r]);
+      dot[r] = fmaf(x.z, k.z, dot[r]);
+      dot[r] = fmaf(x.w, k.w, dot[r]);
     }
-    const float m_new = fmaxf(m, warp_max(s));
-    const float alpha = expf(m - m_new);          // m = -inf at first: exp(-inf) = 0
-    const float p = valid ? expf(s - m_new) : 0.f;
-    z = z * alpha + warp_sum(p);
+  }
+}
+
+struct SimtYes { static constexpr bool value = true; };
+struct SimtNo { static constexpr bool value = false; };
+
+// The rows of tokens t0 .. t0 + tokens - 1 (one request) and heads h_lo .. h_lo + heads - 1 of KV head kvh.
+template <typename TA, int DIMS, bool COPY>       // COPY: float32 rows of whole 16-byte pieces, fetched asynchronously
+__device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cache, const TA* __restrict__ v_cache,
+                          TA* __restrict__ out, const int* __restrict__ table, const int* __restrict__ positions, int t0,
+                          int tokens, int nq, int nkv, int kvh, int h_lo, int heads, int hd, int page_size, float scale,
+                          int window) {
+  constexpr int KEYS = SimtSpan<DIMS>::KEYS;
+  extern __shared__ __align__(16) float simt_sh[];
+  const int g = nq / nkv;
+  const int rows = tokens * heads;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ldk = simt_key_ld(hd), ldv = simt_row_ld(hd), pieces = ldv / 4;
+  float* k_sh = simt_sh;                                     // [2][KEYS][ldk]
+  float* v_sh = k_sh + 2 * KEYS * ldk;                       // [2][KEYS][ldv]
+  float* q_sh = v_sh + 2 * KEYS * ldv;                       // [SA_ROWS][ldv]
+  float* s_sh = q_sh + SA_ROWS * ldv;                        // [SA_ROWS][KEYS]: scores, then weights
+  long long* at_sh = reinterpret_cast<long long*>(s_sh + SA_ROWS * KEYS);      // [2][KEYS]: cache row of a key, or -1
+
+  for (int i = tid; i < SA_ROWS * ldv; i += SA_THREADS) {
+    const int r = i / ldv, d = i % ldv;
+    const bool there = r < rows && d < hd;
+    q_sh[i] = there ? to_float(q[((size_t)(t0 + r / heads) * nq + kvh * g + h_lo + r % heads) * hd + d]) : 0.f;
+  }
+  int first = 0x7fffffff, last = -1;                         // keys that some row of the block sees
+  for (int i = 0; i < tokens; ++i) {
+    const int p = positions[t0 + i];
+    first = min(first, window > 0 ? max(0, p - window + 1) : 0);
+    last = max(last, p);
+  }
+  first = first / KEYS * KEYS;
+  const int spans = last / KEYS - first / KEYS + 1;
+  auto locate = [&](int span) {
+    if (tid < KEYS) {
+      const int j = first + span * KEYS + tid;
+      at_sh[(span & 1) * KEYS + tid] =
+          j <= last ? (((long long)table[j / page_size] * nkv + kvh) * page_size + j % page_size) * hd : -1;
+    }
+  };
+  auto fetch = [&](int span) {
+    if (span < spans) {
+      float* kd = k_sh + (span & 1) * KEYS * ldk;
+      float* vd = v_sh + (span & 1) * KEYS * ldv;
+      const long long* at = at_sh + (span & 1) * KEYS;
+      for (int i = tid; i < KEYS * pieces; i += SA_THREADS) {
+        const int key = i / pieces, c = (i % pieces) * 4;
+        const long long row = at[key];
+        if (row < 0) continue;                               // nobody uses what this place holds
+        if constexpr (COPY) {
+          const unsigned int ka = (unsigned int)__cvta_generic_to_shared(kd + key * ldk + c);
+          const unsigned int va = (unsigned int)__cvta_generic_to_shared(vd + key * ldv + c);
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ka), "l"(k_cache + row + c) : "memory");
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(va), "l"(v_cache + row + c) : "memory");
+        } else {
 #pragma unroll
-    for (int i = 0; i < kMaxDimsPerLane; ++i) acc[i] *= alpha;
-    const int n_here = min(32, pos - jb + 1);
-    for (int jj = 0; jj < n_here; ++jj) {
-      const float pj = __shfl_sync(0xffffffffu, p, jj);
-      const size_t rj = __shfl_sync(0xffffffffu, (unsigned long long)row, jj);
-      if (pj == 0.f) continue;                    // masked by the window (uniform over the warp)
-      const TC* vp = v_cache + rj * hd;
-#pragma unroll
-      for (int i = 0; i < kMaxDimsPerLane; ++i) {
-        const int d = lane + 32 * i;
-        if (d < hd) acc[i] += pj * to_float(vp[d]);
+          for (int e = 0; e < 4; ++e) {
+            kd[key * ldk + c + e] = c + e < hd ? to_float(k_cache[row + c + e]) : 0.f;
+            vd[key * ldv + c + e] = c + e < hd ? to_float(v_cache[row + c + e]) : 0.f;
+          }
+        }
       }
     }
-    m = m_new;
-  }
-  TA* o = out + ((size_t)t * nq + h) * hd;
-  const float inv = 1.f / z;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  // the rows that this warp owns behind the scores: warp, warp + 8, ...
+  float acc[SA_OWN][DIMS], m[SA_OWN], z[SA_OWN];
+  int low[SA_OWN], high[SA_OWN];
 #pragma unroll
-  for (int i = 0; i < kMaxDimsPerLane; ++i) {
-    const int d = lane + 32 * i;
-    if (d < hd) o[d] = from_float<TA>(acc[i] * inv);
+  for (int o = 0; o < SA_OWN; ++o) {
+    const int r = warp + o * SA_WARPS;
+    const int p = r < rows ? positions[t0 + r / heads] : -1;
+    low[o] = r < rows ? (window > 0 ? max(0, p - window + 1) : 0) : 0x7fffffff;
+    high[o] = p;
+    m[o] = -CUDART_INF_F;
+    z[o] = 0.f;
+#pragma unroll
+    for (int i = 0; i < DIMS; ++i) acc[o][i] = 0.f;
   }
+
+  locate(0);
+  __syncthreads();
+  fetch(0);
+  locate(1);
+  __syncthreads();
+  for (int span = 0; span < spans; ++span) {
+    fetch(span + 1);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();                                         // the span has arrived, the places of the next are read
+    const int j0 = first + span * KEYS;
+    {
+      const float* ks = k_sh + (span & 1) * KEYS * ldk;
+      const bool few = rows <= 2;
+      const int groups = few ? 1 : (rows + 7) / 8;
+      for (int task = warp; task < groups * (KEYS / 32); task += SA_WARPS) {
+        const int kb = task % (KEYS / 32) * 32, r0 = task / (KEYS / 32) * 8;
+        const float* kp = ks + (kb + lane) * ldk;
+        if (few) {
+          float dot[2];
+          simt_scores<2>(kp, q_sh, ldv, pieces, dot);
+#pragma unroll
+          for (int r = 0; r < 2; ++r) s_sh[r * KEYS + kb + lane] = dot[r] * scale;
+        } else {
+          float dot[8];
+          simt_scores<8>(kp, q_sh + r0 * ldv, ldv, pieces, dot);
+#pragma unroll
+          for (int r = 0; r < 8; ++r) s_sh[(r0 + r) * KEYS + kb + lane] = dot[r] * scale;
+        }
+      }
+    }
+    locate(span + 2);
+    __syncthreads();
+    const float* vs = v_sh + (span & 1) * KEYS * ldv;
+#pragma unroll 1
+    for (int kb = 0; kb < KEYS; kb += 32) {
+      const int jb = j0 + kb, j = jb + lane;
+      bool any = false, all = true;                          // (uniform over the warp)
+#pragma unroll
+      for (int o = 0; o < SA_OWN; ++o) {
+        if (warp + o * SA_WARPS >= rows) continue;
+        float* sp = s_sh + (warp + o * SA_WARPS) * KEYS + kb + lane;
+        const bool valid = j >= low[o] && j <= high[o];
+        float p = 0.f;
+        if (__any_sync(0xffffffffu, valid)) {                // else the row does not see this block: nothing changes
+          const float s = valid ? *sp : -CUDART_INF_F;
+          const float m_new = fmaxf(m[o], warp_max(s));
+          const float alpha = expf(m[o] - m_new);            // m = -inf at first: exp(-inf) = 0
+          p = valid ? expf(s - m_new) : 0.f;
+          z[o] = z[o] * alpha + warp_sum(p);
+          m[o] = m_new;
+#pragma unroll
+          for (int i = 0; i < DIMS; ++i) acc[o][i] *= alpha;
+          any = true;
+        }
+        all &= __all_sync(0xffffffffu, p != 0.f);
+        *sp = p;
+      }
+      if (!any) continue;
+      __syncwarp();
+      const float* vp = vs + (size_t)kb * ldv + lane;
+      // a weight of zero (a key out of the row's sight, or one far below the maximum) leaves its value unread
+      auto add = [&](auto tested) {
+#pragma unroll 2
+        for (int jj = 0; jj < 32; jj += 4) {
+          float v[4][DIMS];
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int i = 0; i < DIMS; ++i) v[e][i] = lane + 32 * i < ldv ? vp[(jj + e) * ldv + 32 * i] : 0.f;
+#pragma unroll
+          for (int o = 0; o < SA_OWN; ++o) {
+            if (warp + o * SA_WARPS >= rows) continue;
+            const float4 w = *reinterpret_cast<const float4*>(s_sh + (warp + o * SA_WARPS) * KEYS + kb + jj);
+            const float ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (!decltype(tested)::value || ws[e] != 0.f)
+#pragma unroll
+                for (int i = 0; i < DIMS; ++i) acc[o][i] = fmaf(ws[e], v[e][i], acc[o][i]);
+          }
+        }
+      };
+      if (all) add(SimtNo{}); else add(SimtYes{});
+    }
+    __syncthreads();                                         // the span's buffers and scores are free
+  }
+#pragma unroll
+  for (int o = 0; o < SA_OWN; ++o) {
+    const int r = warp + o * SA_WARPS;
+    if (r >= rows) continue;
+    TA* dst = out + ((size_t)(t0 + r / heads) * nq + kvh * g + h_lo + r % heads) * hd;
+    const float inv = 1.f / z[o];
+#pragma unroll
+    for (int i = 0; i < DIMS; ++i) {
+      const int d = lane + 32 * i;
+      if (d < hd) dst[d] = from_float<TA>(acc[o][i] * inv);
+    }
+  }
+}
+
+// Blocks (tile of tokens, KV head, z): of the runs of tokens of one request within the tile, the block serves the z-th and
+// every gridDim.z-th behind it.
+template <typename TA, int DIMS, bool COPY>
+__global__ void __launch_bounds__(SA_THREADS, 1)
+paged_attention_simt_kernel(const TA* __restrict__ q, const TA* __restrict__ k_cache, const TA* __restrict__ v_cache,
+                            TA* __restrict__ out, const int* __restrict__ block_table, int table_stride,
+                            const int* __restrict__ entry_of_token, const int* __restrict__ positions, int T, int nq,
+                            int nkv, int hd, int page_size, float scale, int window, int tile_tokens, int head_groups) {
+  const int g = nq / nkv, kvh = blockIdx.y / head_groups, h_lo = (blockIdx.y % head_groups) * SA_ROWS;
+  const int heads = min(g - h_lo, SA_ROWS);                  // (tile_tokens is 1 where a group has more heads than rows)
+  const int t_end = min(((int)blockIdx.x + 1) * tile_tokens, T);
+  int run = 0;
+  for (int t = blockIdx.x * tile_tokens; t < t_end; ++run) {
+    const int entry = entry_of_token[t];
+    int tokens = 1;
+    while (t + tokens < t_end && entry_of_token[t + tokens] == entry) ++tokens;
+    if (run % gridDim.z == blockIdx.z)
+      simt_rows<TA, DIMS, COPY>(q, k_cache, v_cache, out, block_table + (size_t)entry * table_stride, positions, t, tokens, nq,
+                                nkv, kvh, h_lo, heads, hd, page_size, scale, window);
+    t += tokens;
+  }
+}
+
+template <typename TA, int DIMS, bool COPY>
+static int run_simt(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
+                    int table_stride, const int* entry_of_token, const int* positions, int T, int nq, int nkv, int hd,
+                    int page_size, float scale, int window, int runs, cudaStream_t stream) {
+  const size_t smem = simt_smem(hd, SimtSpan<DIMS>::KEYS);
+  const auto kernel = paged_attention_simt_kernel<TA, DIMS, COPY>;
+  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return (int)e;
+  const int g = nq / nkv, head_groups = (g + SA_ROWS - 1) / SA_ROWS;
+  const int tile_tokens = g >= SA_ROWS ? 1 : SA_ROWS / g;
+  const int z = runs < 1 ? 1 : runs < tile_tokens ? runs : tile_tokens;
+  kernel<<<dim3((T + tile_tokens - 1) / tile_tokens, nkv * head_groups, z), SA_THREADS, smem, stream>>>(
+      (const TA*)q, (const TA*)k_cache, (const TA*)v_cache, (TA*)out, block_table, table_stride, entry_of_token, positions, T,
+      nq, nkv, hd, page_size, scale, window, tile_tokens, head_groups);
+  return launched();
+}
+
+template <typename TA, bool COPY, typename... Args>
+static int run_simt_dims(int hd, Args... args) {
+  if (hd <= 64) return run_simt<TA, 2, COPY>(args...);
+  if (hd <= 128) return run_simt<TA, 4, COPY>(args...);
+  return run_simt<TA, 8, COPY>(args...);
 }
 
 }  // namespace srlm
 
 using namespace srlm;
 
+// runs: how many requests' tokens may stand beside each other in a tile of tokens (a hint: it spreads them over blocks).
 extern "C" int srlm_paged_attention_simt(const void* q, const void* k_cache, const void* v_cache,
                                          void* out, int act_dtype, int cache_dtype,
                                          const int* block_table, int table_stride,
                                          const int* entry_of_token, const int* positions, int T, int nq,
-                                         int nkv, int hd, int page_size, float scale, int window,
+                                         int nkv, int hd, int page_size, float scale, int window, int runs,
                                          cudaStream_t stream) {
   if (T <= 0) return ST_OK;
-  if (nq <= 0 || nkv <= 0 || nq % nkv || hd <= 0 || hd > 32 * kMaxDimsPerLane || page_size <= 0)
+  if (nq <= 0 || nkv <= 0 || nq % nkv || hd <= 0 || hd > 256 || page_size <= 0 ||
+      nkv * ((nq / nkv + SA_ROWS - 1) / SA_ROWS) > 65535)
     return refuse(ST_BAD_SIZE,
                   "paged_attention_simt: nq=%d nkv=%d hd=%d page_size=%d (needs nq %% nkv == 0, hd <= %d)",
-                  nq, nkv, hd, page_size, 32 * kMaxDimsPerLane);
+                  nq, nkv, hd, page_size, 256);
   if (act_dtype != cache_dtype)
     return refuse(ST_BAD_DTYPE, "paged_attention_simt: cache dtype %d differs from activations %d",
                   cache_dtype, act_dtype);
-  const int warps_per_block = 4;
-  const long long warps = (long long)T * nq;
-  const long long grid = (warps + warps_per_block - 1) / warps_per_block;
-  const size_t smem = (size_t)warps_per_block * hd * sizeof(float);
-  SRLM_DISPATCH_ACT(act_dtype, TA, (paged_attention_simt_kernel<TA, TA>
-      <<<(unsigned)grid, warps_per_block * 32, smem, stream>>>(
-          (const TA*)q, (const TA*)k_cache, (const TA*)v_cache, (TA*)out, block_table, table_stride,
-          entry_of_token, positions, T, nq, nkv, hd, page_size, scale, window)));
-  return launched();
+  if (act_dtype == DT_F32) {
+    if (hd % 4 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0)
+      return run_simt_dims<float, true>(hd, q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T,
+                                        nq, nkv, hd, page_size, scale, window, runs, stream);
+    return run_simt_dims<float, false>(hd, q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T,
+                                       nq, nkv, hd, page_size, scale, window, runs, stream);
+  }
+  if (act_dtype != DT_BF16) return refuse(ST_BAD_DTYPE, "dtype code %d is not known", act_dtype);
+  return run_simt_dims<bf16, false>(hd, q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T, nq,
+                                    nkv, hd, page_size, scale, window, runs, stream);
 }

@@ -270,6 +270,28 @@ def test_gemm_simt_forms_agree_bit_for_bit(N, K):
     assert torch.equal(some, full[:5])
 
 
+@pytest.mark.parametrize("nq, nkv, hd, ps", [(40, 1, 64, 16), (33, 1, 20, 3), (3, 1, 18, 5), (2, 2, 7, 16), (64, 8, 128, 16),
+                                             (8, 1, 130, 7)])
+@pytest.mark.parametrize("dt", ACT)
+@pytest.mark.parametrize("window", [0, 70])
+def test_paged_attention_simt_spans_and_runs(nq, nkv, hd, ps, dt, window):
+    """Spans' edges, more heads a group than a block has rows, sizes without whole 16-byte pieces; tokens of several requests
+    within a tile, in order and mixed: a row's result does not depend on its neighbours."""
+    lens_q, lens_kv = [1, 1, 90, 3, 2], [129, 128, 260, 3, 65]
+    q, kc, vc, tables, bt, eot, pos = make_paged_case(nq, nkv, hd, ps, dt, lens_q, lens_kv, pages=max(64, 800 // ps))
+    out = torch.empty_like(q)
+    scale = 1 / math.sqrt(hd)
+    ops().paged_attention_simt(q, kc, vc, out, bt, eot, pos, nq, nkv, hd, ps, scale, window)
+    ref = ref_paged_attention(q, kc, vc, tables, eot.cpu(), pos.cpu(), nq, nkv, hd, ps, scale, window)
+    t = dict(rtol=1e-4, atol=1e-5) if dt == torch.float32 else dict(rtol=2e-2, atol=2e-2)
+    assert torch.allclose(out.float().cpu().view(-1, nq, hd).double(), ref, **t)
+    order = torch.randperm(q.shape[0], generator=torch.Generator().manual_seed(1)).to(DEV)
+    mixed = torch.empty_like(q)
+    ops().paged_attention_simt(q[order].contiguous(), kc, vc, mixed, bt, eot[order].contiguous(), pos[order].contiguous(), nq,
+                               nkv, hd, ps, scale, window)
+    assert torch.equal(mixed, out[order])
+
+
 def test_argmax_ties_go_to_the_lowest_id():
     logits = torch.zeros(4, 1000, device=DEV)
     logits[0, [5, 700]] = 3.0
