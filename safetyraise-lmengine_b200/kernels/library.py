@@ -1463,6 +1463,56 @@ class KernelLibrary:
             C.c_int(rank), C.c_int(v_off), C.c_int(pages.shape[2]), C.c_float(scale), C.c_int(window or 0), _stream()),
             "latent_prefill_attention")
 
+    def latent_prefill_tcgen05_takes(self, q, dim, rot, dv, rank, page_size) -> bool:
+        """Whether latent_prefill_tcgen05 serves these sizes (q: the projected queries, float32 rows)."""
+        return bool(q.dtype == torch.float32 and q.stride(1) == 1 and self.lib.srlm_latent_prefill_tcgen05_takes(
+            C.c_int(dim), C.c_int(rot), C.c_int(dv), C.c_int(rank), C.c_int(page_size)))
+
+    def latent_prefill_plan(self, q_lens, kv_lens, heads: int, sms: int) -> int:
+        """Row tiles a block (1 or 2) of latent_prefill_tcgen05, by a model of its time in microseconds fitted to
+        measurements on B200: a block of one row tile takes 9 + 1.9 a key tile, a block of two 13 + 2.9 a key tile;
+        blocks run in rounds of one per SM."""
+        key_tiles = (max(kv_lens) + 127) // 128
+        blocks = lambda rows: sum((n + rows - 1) // rows for n in q_lens) * heads
+        rounds = lambda n: -(-n // max(1, sms))
+        return 2 if rounds(blocks(256)) * (13 + 2.9 * key_tiles) < rounds(blocks(128)) * (9 + 1.9 * key_tiles) else 1
+
+    def latent_prefill_tcgen05(self, ctx, q, rotation, pages, kv_rows, cu_kv, out, block_table, heads, dim, rot, dv, rank,
+                               v_off, scale, window=0, gate=None):
+        """latent_prefill_attention on tcgen05 tensor cores (sizes: latent_prefill_tcgen05_takes): q float32, heads x
+        (dim + rot) leading each row, not yet rotated; out bfloat16; gate: (float32 rows, column of head 0's logit), whose
+        logistic multiplies a head's output, or None."""
+        pairs = rotation.pairs if rotation is not None else 0
+        if q.dtype != torch.float32 or not q.is_cuda or q.stride(1) != 1 or q.shape[1] < heads * (dim + rot):
+            raise ShapeError("latent_prefill_tcgen05: the queries are float32 rows that begin with the heads")
+        if out.dtype != torch.bfloat16 or pages.dtype != torch.bfloat16 or kv_rows.dtype != torch.bfloat16:
+            raise ShapeError("latent_prefill_tcgen05: pages, keys and values and the output are bfloat16")
+        if pages.shape[3] != rank + rot or pages.shape[1] != 1:
+            raise ShapeError("latent_prefill_tcgen05: a page row is the latent and the rotated key part")
+        gate_ptr, gate_ld = C.c_void_p(0), 0
+        if gate is not None:
+            logits, column = gate
+            if logits.dtype != torch.float32 or not logits.is_cuda or logits.stride(1) != 1 or logits.shape[1] < column + heads:
+                raise ShapeError("latent_prefill_tcgen05: the gate's logits are float32 columns of a row-major tensor")
+            gate_ptr, gate_ld = C.c_void_p(logits.data_ptr() + 4 * column), logits.stride(0)
+        q_lens = ctx.host["q_lens"]
+        tiles = self.latent_prefill_plan(q_lens, ctx.host["kv_lens"], heads, self.sm_count(q.device))
+        key = ("latent_prefill_work", tiles)
+        work = ctx.tables.get(key)
+        if work is None:           # blocks of an entry's last tokens see the most keys: they go first
+            pairs_of = [(e, b) for e, n in enumerate(q_lens) for b in range((n + 128 * tiles - 1) // (128 * tiles))]
+            pairs_of.sort(key=lambda eb: -(ctx.host["starts"][eb[0]] + min((eb[1] + 1) * 128 * tiles, q_lens[eb[0]])))
+            work = ctx.tables[key] = torch.tensor(pairs_of, dtype=torch.int32).pin_memory().to(q.device, non_blocking=True)
+        self._check(self.lib.srlm_latent_prefill_tcgen05(
+            C.c_void_p(q.data_ptr()), C.c_longlong(q.stride(0)), _ptr(rotation.cos if pairs else None),
+            _ptr(rotation.sin if pairs else None), C.c_int(pairs), C.c_int(int(bool(pairs and not rotation.interleaved))),
+            _ptr(pages), C.c_longlong(pages.shape[0]), _ptr(kv_rows), C.c_longlong(kv_rows.shape[0]),
+            C.c_longlong(kv_rows.stride(0)), _ptr(cu_kv), gate_ptr, C.c_longlong(gate_ld), _ptr(out), _ptr(block_table),
+            C.c_int(block_table.stride(0)), _ptr(ctx.cu_q), _ptr(ctx.kv_lens), _ptr(work), C.c_int(work.shape[0]),
+            C.c_int(tiles), C.c_int(heads), C.c_int(dim), C.c_int(rot), C.c_int(dv), C.c_int(rank), C.c_int(v_off),
+            C.c_int(pages.shape[2]), C.c_float(scale), C.c_int(window or 0), _ptr(self._gemm_state(q.device)[1]), _stream()),
+            "latent_prefill_tcgen05")
+
     def head_gate(self, x, proj, g_off, out, heads, dv):
         """out[t, h, :] = x[t, h, :] * sigmoid(proj[t, g_off + h]); x float32, or bfloat16 (out may then be x itself);
         g_off < 0: no gate."""

@@ -150,6 +150,12 @@ class LatentAttention(Part):
         ops.latent_gather(ctx, cache, latents, ctx.block_tables[group], cu_kv, s.kv_rank, kv_first)
         kv_rows = ctx.workspace.get("latent.kv_rows", keys, s.heads * (s.head_dim + s.v_head_dim), ctx.dtype)
         ops.gemm(latents, self.up_kv, kv_rows)
+        if ops.latent_prefill_tcgen05_takes(q_heads, s.head_dim, s.rot_dim, s.v_head_dim, s.kv_rank, cache.shape[2]):
+            # rotates the queries as it reads them and gates the heads as it writes them
+            ops.latent_prefill_tcgen05(ctx, q_heads, rot, cache, kv_rows, cu_kv, gated, ctx.block_tables[group], s.heads,
+                                       s.head_dim, s.rot_dim, s.v_head_dim, s.kv_rank, s.heads * s.head_dim, s.softmax_scale,
+                                       s.window or 0, gate=(proj, self.g_off) if s.output_gate else None)
+            return
         q = ctx.workspace.get("latent.q_heads", T, s.heads * (s.head_dim + s.rot_dim), torch.float32)
         ops.latent_rotate_q(q_heads, rot, q, s.heads, s.head_dim, s.rot_dim)
         # without a gate the attention writes the output projection's input itself

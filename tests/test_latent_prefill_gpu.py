@@ -1,0 +1,100 @@
+"""Prompts of a latent attention on the tensor-memory kernel: rows and keys at the edges of its tiles, pages of every form it
+takes, windows with pages given back, both pairings of the rotation, the gate, operands whose rows are no whole 16-byte
+pieces, and neighbours that must not be read."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+DIM, ROT, DV, RANK = 128, 64, 128, 40
+
+
+class Ctx:
+    def __init__(self, q_lens, kv_lens):
+        starts = [k - q for q, k in zip(q_lens, kv_lens)]
+        cu = [0]
+        for q in q_lens:
+            cu.append(cu[-1] + q)
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+        self.cu_q, self.kv_lens, self.tables = i32(cu), i32(kv_lens), {}
+        self.host = {"q_lens": q_lens, "kv_lens": kv_lens, "starts": starts}
+
+
+@pytest.mark.parametrize("page", [8, 16, 64, 256])
+@pytest.mark.parametrize("window", [0, 70, 300])
+@pytest.mark.parametrize("heads, pairs, interleaved, gated", [(2, 32, True, True), (3, 16, False, False), (1, 0, True, True)])
+def test_prompts_against_float64(page, window, heads, pairs, interleaved, gated):
+    from safetyraise_lmengine_b200.kernels import ops
+    from safetyraise_lmengine_b200.parts.base import Rotation
+    g = torch.Generator().manual_seed(page + window + heads)
+    q_lens, kv_lens = [1, 128, 5, 257, 130], [1, 128, 300, 384, 515]
+    T, scale = sum(q_lens), 0.5 * (DIM + ROT) ** -0.5
+    ctx = Ctx(q_lens, kv_lens)
+    wide = heads * (DIM + ROT) + 1 + heads                                       # the gate's columns behind the queries'
+    q = torch.randn(T, wide, generator=g)
+    first = [max(0, k - n - window + 1) if window else 0 for n, k in zip(q_lens, kv_lens)]
+    cu_kv, keys = [], 0
+    for f, k in zip(first, kv_lens):
+        cu_kv.append(keys - f)
+        keys += k - f
+    rows = torch.randn(keys, heads * (DIM + DV), generator=g).bfloat16()
+    n_pages = sum(-(-k // page) for k in kv_lens)
+    order = torch.randperm(n_pages, generator=g).tolist()
+    pages = torch.full((n_pages, 1, page, RANK + ROT), float("nan"), dtype=torch.bfloat16)
+    shared = [torch.randn(k, ROT, generator=g).bfloat16() for k in kv_lens]
+    table = torch.zeros(len(kv_lens), max(-(-k // page) for k in kv_lens) + 1, dtype=torch.int32)
+    at = 0
+    for e, k in enumerate(kv_lens):
+        for b in range(-(-k // page)):
+            if (b + 1) * page <= first[e]:
+                table[e, b] = -1                                                 # behind the window: given back
+                continue
+            table[e, b] = order[at]
+            lo, hi = b * page, min((b + 1) * page, k)
+            pages[order[at], 0, :hi - lo, RANK:] = shared[e][lo:hi]
+            at += 1
+    cos = sin = rotation = None
+    if pairs:
+        angle = torch.randn(T, pairs, generator=g)
+        cos, sin = angle.cos(), angle.sin()
+        rotation = Rotation(cos.to(DEV), sin.to(DEV), pairs, interleaved)
+    # the reference: queries rounded to bfloat16 once turned, as the kernel's operands are
+    x = q[:, :heads * (DIM + ROT)].reshape(T, heads, DIM + ROT).clone()
+    if pairs:
+        c, s, tail = cos[:, None], sin[:, None], x[..., DIM:DIM + 2 * pairs].clone()
+        a, b = (tail[..., 0::2], tail[..., 1::2]) if interleaved else (tail[..., :pairs], tail[..., pairs:])
+        turned = (a * c - b * s, b * c + a * s)
+        x[..., DIM:DIM + 2 * pairs] = torch.stack(turned, -1).flatten(-2) if interleaved else torch.cat(turned, -1)
+    x = x.bfloat16().double()
+    ref = torch.zeros(T, heads, DV, dtype=torch.float64)
+    t = 0
+    for e, (n, k) in enumerate(zip(q_lens, kv_lens)):
+        mine = rows[cu_kv[e] + first[e]:cu_kv[e] + k].double()
+        j = torch.arange(first[e], k)
+        i = torch.arange(k - n, k)[:, None]
+        seen = (j <= i) & (j > i - window if window else j >= 0)
+        for h in range(heads):
+            key = torch.cat([mine[:, h * DIM:(h + 1) * DIM], shared[e][first[e]:].double()], -1)
+            p = torch.softmax((x[t:t + n, h] @ key.T * scale).masked_fill(~seen, -math.inf), -1)
+            ref[t:t + n, h] = p @ mine[:, heads * DIM + h * DV:heads * DIM + (h + 1) * DV]
+        t += n
+    gate = None
+    if gated:
+        gate = (q.to(DEV), heads * (DIM + ROT) + 1)
+        ref *= torch.sigmoid(q[:, -heads:].double())[:, :, None]
+    out = torch.full((T, heads * DV), 7.0, dtype=torch.bfloat16, device=DEV)
+    assert ops.latent_prefill_tcgen05_takes(q.to(DEV), DIM, ROT, DV, RANK, page)
+    flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.bind_error_flag(flag)
+    try:
+        ops.latent_prefill_tcgen05(ctx, q.to(DEV), rotation, pages.to(DEV), rows.to(DEV), torch.tensor(cu_kv, dtype=torch.int32, device=DEV),
+                                   out, table.to(DEV), heads, DIM, ROT, DV, RANK, heads * DIM, scale, window, gate=gate)
+        got = out.double().cpu().view(T, heads, DV)
+    finally:
+        ops.bind_error_flag(None)
+    assert int(flag) == 0
+    # weights and the result are rounded to 8 bits of mantissa (2^-9 each way): a value is a mean of N(0, 1) values under weights
+    # that are off by 2^-9 of themselves, then off by 2^-9 of itself
+    assert (got - ref).abs().max() <= 2.0 ** -8 * (1.0 + ref.abs().max())
