@@ -12,7 +12,8 @@
 //
 // Shared memory holds 96 KB of queries, two K tiles (96 KB) and one V tile (32 KB): a V tile is fetched under the S product
 // and the softmax that follow the product that freed it.  Bound by the softmax (one exponential and about eight other
-// instructions a score) and the MMA issue of the longest block.  1,800 tokens behind 200, 16 heads: see launch rule below.
+// instructions a score) and the MMA issue of the longest block: 2.1 us a tile of 128 keys for two row tiles, 10 us before and
+// after them.  1,800 tokens behind 200, 16 heads: 53 us (485 on mma.sync, plus 30 for the rotation and the gate by themselves).
 #include "attention_tcgen05.cuh"
 
 namespace srlm {
@@ -32,7 +33,7 @@ static_assert(SMEM <= 227 * 1024, "");
 struct Args {
   const float* q;            // heads x (128 | 64) lead a token's row of ldq floats
   long long ldq;
-  bool q_vec;                // rows of whole 16-byte pieces
+  bool q_vec;                // see load_queries
   const float* cos_t;        // [T, pairs]
   const float* sin_t;
   int pairs;
@@ -51,35 +52,110 @@ struct Args {
   int* err_flag;
 };
 
-// Elements d .. d + 7 of a query head (d a multiple of 8), its last 64 rotated.
-__device__ __forceinline__ void query_piece(const Args& a, int token, int head, int d, float (&x)[8]) {
-  const float* src = a.q + (size_t)token * a.ldq + (size_t)head * (DIM + ROT);
-  if (a.q_vec) {
-    const float4 lo = __ldg(reinterpret_cast<const float4*>(src + d)), hi = __ldg(reinterpret_cast<const float4*>(src + d + 4));
-    x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w;
-    x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
-  } else {
+__device__ __forceinline__ void load8(const float* src, float (&x)[8]) {
+  const float4 lo = __ldg(reinterpret_cast<const float4*>(src)), hi = __ldg(reinterpret_cast<const float4*>(src + 4));
+  x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w;
+  x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+}
+// Element r of a query's rotated part: x, partner, cosine and sine -> the turned element.
+__device__ __forceinline__ float turned(float x, float partner, float c, float s, bool second) {
+  return second ? x * c + partner * s : x * c - partner * s;
+}
+__device__ __forceinline__ void put8(uint32_t at, const float (&x)[8]) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(at), "r"(pack2(x[0], x[1])), "r"(pack2(x[2], x[3])),
+               "r"(pack2(x[4], x[5])), "r"(pack2(x[6], x[7])) : "memory");
+}
+
+// `rows` query rows of a head -> shared memory, turned and rounded, in the swizzled K-major layout (zeros beyond the entry's
+// rows).  A thread has four pieces (of eight elements) in flight, two of the rotated part, whose cosines and sines come
+// with them (with scalar reads of the tables a tile of 128 rows took 12 us instead of 4); more pieces unrolled make code that
+// every block fetches cold: with eight and four, a block of 5 rows took 12.3 us instead of 10.3.
+template <bool VEC>              // whole 16-byte pieces everywhere: rows, tables, and pairs that do not straddle a piece
+__device__ __forceinline__ void load_queries(const Args& a, uint32_t q_tiles, int rows, bool two, int first_token, int left,
+                                             int head, int tid, int threads) {
+  auto place = [&](int row, int c) {       // a block of one row tile keeps it in slot 1
+    return tile_addr(q_tiles + (two ? row >> 7 : 1) * QK_BYTES, row & 127, c);
+  };
+  auto source = [&](int row) { return a.q + (size_t)(first_token + row) * a.ldq + (size_t)head * (DIM + ROT); };
+  constexpr int PLAIN = DIM / 8, TURNED = ROT / 8, QB = 4, RB = 2;
+#pragma unroll 1
+  for (int base = tid; base < rows * PLAIN; base += threads * QB) {
+    float x[QB][8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) x[j] = __ldg(src + d + j);
-  }
-  const int r0 = d - DIM;
-  if (r0 < 0 || r0 >= 2 * a.pairs) return;
-  const float* c = a.cos_t + (size_t)token * a.pairs;
-  const float* s = a.sin_t + (size_t)token * a.pairs;
-  float y[8];
+    for (int j = 0; j < QB; ++j) {
+      const int idx = base + j * threads, row = idx / PLAIN, d = (idx % PLAIN) * 8;
+      const bool there = idx < rows * PLAIN && row < left;
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const int r = r0 + j;
-    y[j] = x[j];
-    if (r < 2 * a.pairs) {
-      const bool second = a.halves ? r >= a.pairs : r & 1;
-      const int i = a.halves ? (second ? r - a.pairs : r) : r >> 1;
-      const float partner = a.halves ? __ldg(src + DIM + (second ? r - a.pairs : r + a.pairs)) : x[j ^ 1];
-      y[j] = second ? x[j] * c[i] + partner * s[i] : x[j] * c[i] - partner * s[i];
+      for (int i = 0; i < 8; ++i) x[j][i] = 0.f;
+      if (there) {
+        if constexpr (VEC) {
+          load8(source(row) + d, x[j]);
+        } else {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[j][i] = __ldg(source(row) + d + i);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < QB; ++j) {
+      const int idx = base + j * threads;
+      if (idx < rows * PLAIN) put8(place(idx / PLAIN, idx % PLAIN), x[j]);
     }
   }
+#pragma unroll 1
+  for (int base = tid; base < rows * TURNED; base += threads * RB) {
+    float x[RB][8], y[RB][8], c[RB][8], s[RB][8];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) x[j] = y[j];
+    for (int j = 0; j < RB; ++j) {
+      const int idx = base + j * threads, row = idx / TURNED, r0 = (idx % TURNED) * 8;
+      const bool there = idx < rows * TURNED && row < left;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[j][i] = y[j][i] = s[j][i] = 0.f, c[j][i] = 1.f;
+      if (!there) continue;
+      const float* src = source(row) + DIM;
+      const float* ct = a.cos_t + (size_t)(first_token + row) * a.pairs;
+      const float* st = a.sin_t + (size_t)(first_token + row) * a.pairs;
+      if constexpr (VEC) {
+        load8(src + r0, x[j]);
+        if (r0 < 2 * a.pairs) {
+          if (a.halves) {
+            const bool second = r0 >= a.pairs;
+            load8(src + (second ? r0 - a.pairs : r0 + a.pairs), y[j]);
+            load8(ct + (second ? r0 - a.pairs : r0), c[j]);
+            load8(st + (second ? r0 - a.pairs : r0), s[j]);
+          } else {
+            const float4 c4 = __ldg(reinterpret_cast<const float4*>(ct + r0 / 2)), s4 = __ldg(reinterpret_cast<const float4*>(st + r0 / 2));
+            c[j][0] = c[j][1] = c4.x; c[j][2] = c[j][3] = c4.y; c[j][4] = c[j][5] = c4.z; c[j][6] = c[j][7] = c4.w;
+            s[j][0] = s[j][1] = s4.x; s[j][2] = s[j][3] = s4.y; s[j][4] = s[j][5] = s4.z; s[j][6] = s[j][7] = s4.w;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[j][i] = x[j][i ^ 1];
+          }
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = r0 + i;
+          x[j][i] = __ldg(src + r);
+          if (r < 2 * a.pairs) {
+            const bool second = a.halves ? r >= a.pairs : r & 1;
+            const int pair = a.halves ? (second ? r - a.pairs : r) : r >> 1;
+            y[j][i] = __ldg(src + (a.halves ? (second ? r - a.pairs : r + a.pairs) : r ^ 1));
+            c[j][i] = __ldg(ct + pair);
+            s[j][i] = __ldg(st + pair);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < RB; ++j) {
+      const int idx = base + j * threads, r0 = (idx % TURNED) * 8;
+      if (idx < rows * TURNED) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[j][i] = turned(x[j][i], y[j][i], c[j][i], s[j][i], a.halves ? r0 + i >= a.pairs : i & 1);
+        put8(place(idx / TURNED, PLAIN + idx % TURNED), x[j]);
+      }
+    }
+  }
 }
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -152,29 +228,10 @@ latent_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_rows, cons
   const bool dirty_last = jb0 + n_tiles1 * KT > kv_len;
 
   if (warp != 0) {
-    // Q rows -> shared memory, rotated and rounded, in the swizzled K-major layout (zeros beyond the entry's rows), while
-    // warp 0 already fetches the first keys
-    constexpr int PIECES = (DIM + ROT) / 8, QB = 4;
-    const int total = (two ? 2 : 1) * BR * PIECES;
-    for (int base = threadIdx.x - 32; base < total; base += (THREADS - 32) * QB) {
-      float x[QB][8];
-#pragma unroll
-      for (int j = 0; j < QB; ++j) {
-        const int idx = base + j * (THREADS - 32), row = idx / PIECES, r = r_block + row;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) x[j][i] = 0.f;
-        if (idx < total && r < q_len) query_piece(a, q0 + r, head, (idx % PIECES) * 8, x[j]);
-      }
-#pragma unroll
-      for (int j = 0; j < QB; ++j) {
-        const int idx = base + j * (THREADS - 32), row = idx / PIECES, c = idx % PIECES;
-        if (idx < total) {
-          const uint32_t tile = s32(q_t) + (two ? row >> 7 : 1) * QK_BYTES;     // a block of one row tile keeps it in slot 1
-          asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(tile_addr(tile, row & 127, c)), "r"(pack2(x[j][0], x[j][1])),
-                       "r"(pack2(x[j][2], x[j][3])), "r"(pack2(x[j][4], x[j][5])), "r"(pack2(x[j][6], x[j][7])) : "memory");
-        }
-      }
-    }
+    // while warp 0 already fetches the first keys
+    const int rows = (two ? 2 : 1) * BR, threads = THREADS - 32;
+    if (a.q_vec) load_queries<true>(a, s32(q_t), rows, two, q0 + r_block, q_len - r_block, head, threadIdx.x - 32, threads);
+    else load_queries<false>(a, s32(q_t), rows, two, q0 + r_block, q_len - r_block, head, threadIdx.x - 32, threads);
     fence_async_smem();
     __syncwarp();
     if (lane == 0) mbar_arrive(q_full);
@@ -426,7 +483,8 @@ extern "C" int srlm_latent_prefill_tcgen05(const float* q, long long ldq, const 
   const cudaError_t e = cudaFuncSetAttribute(lfmha::latent_prefill_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              lfmha::SMEM);
   if (e != cudaSuccess) return refuse((int)e, "latent_prefill_tcgen05: cannot get %d bytes of shared memory", lfmha::SMEM);
-  lfmha::Args a{q, ldq, ldq % 4 == 0 && (uintptr_t)q % 16 == 0, cos_t, sin_t, pairs, halves != 0, gate, ld_gate, (bf16*)out,
+  const bool q_vec = ldq % 4 == 0 && pairs % (halves ? 8 : 4) == 0 && (((uintptr_t)q | (uintptr_t)cos_t | (uintptr_t)sin_t) & 15) == 0;
+  lfmha::Args a{q, ldq, q_vec, cos_t, sin_t, pairs, halves != 0, gate, ld_gate, (bf16*)out,
                 block_table, table_stride, cu_q, kv_lens, cu_kv, work, heads, page_size, rank, v_off, tiles_per_block, window,
                 scale * 1.4426950408889634f, err_flag};
   launch_pdl(lfmha::latent_prefill_tcgen05_kernel, dim3(n_work * heads), dim3(lfmha::THREADS), lfmha::SMEM, stream, rows_map,

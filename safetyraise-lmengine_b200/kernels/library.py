@@ -1470,12 +1470,12 @@ class KernelLibrary:
 
     def latent_prefill_plan(self, q_lens, kv_lens, heads: int, sms: int) -> int:
         """Row tiles a block (1 or 2) of latent_prefill_tcgen05, by a model of its time in microseconds fitted to
-        measurements on B200: a block of one row tile takes 9 + 1.9 a key tile, a block of two 13 + 2.9 a key tile;
+        measurements on B200: a block of one row tile takes 10 + 1.9 a key tile, a block of two 13 + 2.1 a key tile;
         blocks run in rounds of one per SM."""
         key_tiles = (max(kv_lens) + 127) // 128
         blocks = lambda rows: sum((n + rows - 1) // rows for n in q_lens) * heads
         rounds = lambda n: -(-n // max(1, sms))
-        return 2 if rounds(blocks(256)) * (13 + 2.9 * key_tiles) < rounds(blocks(128)) * (9 + 1.9 * key_tiles) else 1
+        return 2 if rounds(blocks(256)) * (13 + 2.1 * key_tiles) < rounds(blocks(128)) * (10 + 1.9 * key_tiles) else 1
 
     def latent_prefill_tcgen05(self, ctx, q, rotation, pages, kv_rows, cu_kv, out, block_table, heads, dim, rot, dv, rank,
                                v_off, scale, window=0, gate=None):

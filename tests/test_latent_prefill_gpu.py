@@ -24,7 +24,8 @@ class Ctx:
 
 @pytest.mark.parametrize("page", [8, 16, 64, 256])
 @pytest.mark.parametrize("window", [0, 70, 300])
-@pytest.mark.parametrize("heads, pairs, interleaved, gated", [(2, 32, True, True), (3, 16, False, False), (1, 0, True, True)])
+@pytest.mark.parametrize("heads, pairs, interleaved, gated", [(2, 32, True, True), (2, 32, False, False), (3, 16, False, False), (1, 0, True, True),
+                                                               (2, 6, True, False)])
 def test_prompts_against_float64(page, window, heads, pairs, interleaved, gated):
     from safetyraise_lmengine_b200.kernels import ops
     from safetyraise_lmengine_b200.parts.base import Rotation
@@ -32,7 +33,7 @@ def test_prompts_against_float64(page, window, heads, pairs, interleaved, gated)
     q_lens, kv_lens = [1, 128, 5, 257, 130], [1, 128, 300, 384, 515]
     T, scale = sum(q_lens), 0.5 * (DIM + ROT) ** -0.5
     ctx = Ctx(q_lens, kv_lens)
-    wide = heads * (DIM + ROT) + 1 + heads                                       # the gate's columns behind the queries'
+    wide = heads * (DIM + ROT) + (4 if heads == 2 else 1) + heads + heads % 2    # the gate's columns, behind the queries'
     q = torch.randn(T, wide, generator=g)
     first = [max(0, k - n - window + 1) if window else 0 for n, k in zip(q_lens, kv_lens)]
     cu_kv, keys = [], 0
@@ -82,7 +83,7 @@ def test_prompts_against_float64(page, window, heads, pairs, interleaved, gated)
         t += n
     gate = None
     if gated:
-        gate = (q.to(DEV), heads * (DIM + ROT) + 1)
+        gate = (q.to(DEV), wide - heads)
         ref *= torch.sigmoid(q[:, -heads:].double())[:, :, None]
     out = torch.full((T, heads * DV), 7.0, dtype=torch.bfloat16, device=DEV)
     assert ops.latent_prefill_tcgen05_takes(q.to(DEV), DIM, ROT, DV, RANK, page)
