@@ -13,6 +13,7 @@
 //   delta_conv_carry   -- the slot's last taps-1 inputs after this step;
 //   delta_recurrence   -- the recurrence, token by token within an entry, entries / heads / columns of S in parallel;
 //   delta_output       -- per head o / rms(o) * w * silu(gate) in the activation dtype.
+// Steps with longer portions in bfloat16 go by chunks of tokens instead of the first and the third (delta_chunks.cu).
 // Projection row (proj, [T, ldp]): q (G dk) | k (G dk) | v (H dv) | b (H) | a (H) | gate (H dv).
 #include "common.cuh"
 
@@ -249,6 +250,23 @@ static int delta_sizes_ok(int H, int G, int dk, int dv, int taps) {
   return H > 0 && G > 0 && H % G == 0 && dk > 0 && dk <= 512 && dv > 0 && taps >= 1 && taps <= kMaxTaps;
 }
 
+// The slots' carried inputs after a step, behind the kernels that read them.
+extern "C" int srlm_delta_conv_carry(const void* proj, int proj_dtype, long long ldp, float* state, long long state_stride,
+                                     const int* cu_q, const int* slots, int n_entries, int H, int G, int dk, int dv, int taps,
+                                     cudaStream_t stream) {
+  if (n_entries <= 0 || taps <= 1) return ST_OK;
+  const long long C = 2LL * G * dk + (long long)H * dv;
+  if (!delta_sizes_ok(H, G, dk, dv, taps) || ldp < C || state_stride < (long long)H * dk * dv + C * (taps - 1))
+    return refuse(ST_BAD_SIZE, "delta_conv_carry: H=%d G=%d dk=%d dv=%d taps=%d ldp=%lld state=%lld", H, G, dk, dv, taps, ldp,
+                  state_stride);
+  SRLM_DISPATCH_ACT(proj_dtype, TP, {
+    const long long n = (long long)n_entries * C;
+    launch_pdl(delta_conv_carry_kernel<TP>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, (const TP*)proj, ldp, state,
+               state_stride, (long long)H * dk * dv, cu_q, slots, n_entries, (int)C, taps);
+  });
+  return launched();
+}
+
 extern "C" int srlm_delta_prepare(const void* proj, int proj_dtype, long long ldp, const float* conv_w,
                                   const float* a_log, const float* dt_bias, float* state, long long state_stride,
                                   const int* entry_of_token, const int* cu_q, const int* slots, int n_entries,
@@ -267,13 +285,9 @@ extern "C" int srlm_delta_prepare(const void* proj, int proj_dtype, long long ld
     launch_pdl(delta_prepare_kernel<TP>, dim3(T), dim3(256), smem, stream, (const TP*)proj, ldp, conv_w, a_log, dt_bias, state, state_stride,
                                                        entry_of_token, cu_q, slots, qkv_out, beta_out, decay_out, qk_out,
                                                        H, G, dk, dv, taps, unit_eps);
-    if (taps > 1) {
-      const long long n = (long long)n_entries * C;
-      launch_pdl(delta_conv_carry_kernel<TP>, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, stream, 
-          (const TP*)proj, ldp, state, state_stride, (long long)H * dk * dv, cu_q, slots, n_entries, (int)C, taps);
-    }
   });
-  return launched();
+  if (int r = launched()) return r;
+  return srlm_delta_conv_carry(proj, proj_dtype, ldp, state, state_stride, cu_q, slots, n_entries, H, G, dk, dv, taps, stream);
 }
 
 extern "C" int srlm_delta_recurrence(const float* qkv, const float* beta, const float* decay, const float* qk, float* state,

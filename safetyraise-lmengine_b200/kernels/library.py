@@ -1540,6 +1540,41 @@ class KernelLibrary:
             _ptr(ctx.slots), C.c_int(ctx.n_entries), _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv),
             _stream()), "delta_recurrence")
 
+    DELTA_CHUNK = 16         # tokens of a chunk
+    DELTA_CHUNKS_FROM = 16   # steps with an entry of at least this many tokens go by chunks
+
+    def delta_by_chunks(self, ctx, state, dk, dv, taps) -> int:
+        """How many chunks of 16 tokens the step's entries make, 0 where the step goes token by token: decode steps and
+        short portions, sizes that the chunked kernels do not take, and the float32 path, whose results do not depend on
+        where a request is cut."""
+        if ctx.dtype != torch.bfloat16 or ctx.max_q_len < self.DELTA_CHUNKS_FROM:
+            return 0
+        if not self.lib.srlm_delta_chunk_record(C.c_int(dk), C.c_int(dv), C.c_int(taps)):
+            return 0
+        if state.stride(0) % 2 or state.data_ptr() % 8:        # the walk moves two rows of a column at a time
+            return 0
+        return sum(-(-n // self.DELTA_CHUNK) for n in ctx.host["q_lens"])
+
+    def delta_chunks(self, ctx, proj, conv_w, a_log, dt_bias, state, o_out, n_chunks, H, G, dk, dv, taps, unit_eps):
+        """o_out float32 [T, H dv] = the gated delta rule of the step's tokens from the projection (float32 rows: q | k | v |
+        beta | decay ..), by chunks of 16 tokens, as csrc/kernels/delta_chunks.cu says; S and the convolution's carried
+        inputs in ``state`` are renewed."""
+        if proj.dtype != torch.float32:
+            raise ShapeError("delta_chunks: the projection is float32")
+        record = int(self.lib.srlm_delta_chunk_record(C.c_int(dk), C.c_int(dv), C.c_int(taps)))
+        records = ctx.workspace.get("delta.records", n_chunks * H, max(record, 1), torch.float32, reserve=0)
+        self._check(self.lib.srlm_delta_chunks(
+            _ptr(proj), C.c_longlong(proj.stride(0)), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias), _ptr(state),
+            C.c_longlong(state.stride(0)), _ptr(ctx.cu_q), _ptr(ctx.slots), C.c_int(ctx.n_entries), _ptr(records),
+            C.c_int(n_chunks), _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps),
+            _stream()), "delta_chunks")
+        self.launches += 1
+        if taps > 1:
+            self._check(self.lib.srlm_delta_conv_carry(
+                _ptr(proj), dtype_code(proj.dtype), C.c_longlong(proj.stride(0)), _ptr(state), C.c_longlong(state.stride(0)),
+                _ptr(ctx.cu_q), _ptr(ctx.slots), C.c_int(ctx.n_entries), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv),
+                C.c_int(taps), _stream()), "delta_conv_carry")
+
     def delta_output(self, o, norm_w, eps, proj, gate_off, out, H, dv, logistic=False):
         """out = per head o / sqrt(mean(o^2) + eps) * norm_w * silu(gate) (``logistic``: logistic(gate) in silu's place),
         the gate in the columns of proj from gate_off."""

@@ -1,0 +1,100 @@
+"""The gated delta rule by chunks of 16 tokens: against the recurrence in float64, outputs and the whole state behind them, on
+portions around whole chunks, several entries a step, states that are not zero, tokens that continue a portion (carried
+convolution inputs), grouped heads, values of other sizes, fewer taps, decays that underflow and decays of nearly one."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+DK, EPS = 128, 1e-6
+
+
+class Ctx:
+    dtype = torch.bfloat16
+
+    def __init__(self, lens, slots):
+        cu = [0]
+        for n in lens:
+            cu.append(cu[-1] + n)
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+        self.cu_q, self.slots, self.n_entries, self.max_q_len = i32(cu), i32(slots), len(lens), max(lens)
+        self.entry_of_token = i32([e for e, n in enumerate(lens) for _ in range(n)])
+        self.host = {"q_lens": lens}
+        from safetyraise_lmengine_b200.parts.base import Workspace
+        self.workspace = Workspace(torch.device(DEV), cu[-1])
+
+
+def recurrence(proj, conv_w, a_log, dt_bias, state, H, G, dv, taps):
+    """One entry in float64 -> (o [n, H, dv], the state row behind it)."""
+    n, C = proj.shape[0], 2 * G * DK + H * dv
+    S = state[:H * DK * dv].view(H, dv, DK).transpose(1, 2).clone()
+    carry = state[H * DK * dv:].view(C, taps - 1).T
+    x = torch.cat([carry, proj[:, :C]])
+    y = sum(x[j:j + n] * conv_w[:, j] for j in range(taps))
+    y = y * torch.sigmoid(y)
+    unit = lambda a: a / torch.sqrt((a * a).sum(-1, keepdim=True) + EPS)
+    q, k = unit(y[:, :G * DK].view(n, G, DK)) * DK ** -0.5, unit(y[:, G * DK:2 * G * DK].view(n, G, DK))
+    q, k = q.repeat_interleave(H // G, 1), k.repeat_interleave(H // G, 1)
+    v = y[:, 2 * G * DK:].view(n, H, dv)
+    beta = torch.sigmoid(proj[:, C:C + H])
+    g = torch.exp(-torch.exp(a_log) * torch.nn.functional.softplus(proj[:, C + H:C + 2 * H] + dt_bias))
+    o = torch.empty(n, H, dv, dtype=torch.float64, device=proj.device)
+    for t in range(n):
+        S = S * g[t][:, None, None]
+        u = beta[t][:, None] * (v[t] - torch.einsum("hkv,hk->hv", S, k[t]))
+        S = S + k[t][:, :, None] * u[:, None]
+        o[t] = torch.einsum("hkv,hk->hv", S, q[t])
+    return o, torch.cat([S.transpose(1, 2).reshape(-1), x[n:].T.reshape(-1)])
+
+
+@pytest.mark.parametrize("H, G, dv, taps", [(2, 2, 128, 4), (4, 2, 48, 4), (3, 1, 16, 2), (2, 1, 144, 1), (1, 1, 128, 3)])
+@pytest.mark.parametrize("lens", [[16], [1, 17, 2, 33], [15, 31, 48], [130]])
+def test_against_float64(H, G, dv, taps, lens):
+    from safetyraise_lmengine_b200.kernels import ops
+    gen = torch.Generator(device=DEV).manual_seed(H + dv + taps + len(lens))
+    rand = lambda *s: torch.randn(*s, generator=gen, device=DEV)
+    C, T = 2 * G * DK + H * dv, sum(lens)
+    row = H * DK * dv + C * (taps - 1)
+    row += row % 2
+    state = rand(6, row)
+    slots = [4, 1, 5, 2][:len(lens)]
+    proj = rand(T, C + 2 * H + 3)
+    proj[T // 2:, C + H:C + 2 * H] += 8.0            # decays that underflow within a chunk, behind decays of nearly one
+    conv_w, dt_bias = rand(C, taps) * 0.5, rand(H) - 4.0
+    a_log = torch.log(1.0 + 15.0 * torch.rand(H, generator=gen, device=DEV))
+    before = state.double().clone()
+    ctx = Ctx(lens, slots)
+    o = torch.empty(T, H * dv, device=DEV)
+    n = ops.delta_by_chunks(ctx, state, DK, dv, taps)
+    if max(lens) < ops.DELTA_CHUNKS_FROM:
+        assert n == 0
+        return
+    assert n == sum(-(-x // 16) for x in lens)
+    ops.delta_chunks(ctx, proj, conv_w, a_log, dt_bias, state, o, n, H, G, DK, dv, taps, EPS)
+    want_o, want_state, t = [], before.clone(), 0
+    for x, slot in zip(lens, slots):
+        used = H * DK * dv + C * (taps - 1)
+        a, b = recurrence(proj[t:t + x].double(), conv_w.double(), a_log.double(), dt_bias.double(), before[slot, :used], H, G, dv, taps)
+        want_o.append(a.reshape(x, -1))
+        want_state[slot, :used] = b
+        t += x
+    want_o = torch.cat(want_o)
+    # float32 sums over 128 rows and 16 tokens of terms of about one: a few hundred roundings of 2^-24
+    assert (o.double() - want_o).abs().max() <= 2e-5 * want_o.abs().max()
+    assert (state.double() - want_state).abs().max() <= 2e-5 * want_state.abs().max()
+    untouched = [s for s in range(6) if s not in slots]
+    assert torch.equal(state[untouched].double(), before[untouched])
+
+
+def test_the_float32_path_and_short_steps_go_token_by_token():
+    from safetyraise_lmengine_b200.kernels import ops
+    state = torch.zeros(1, 128 * 128 + 3 * 384, device=DEV)
+    ctx = Ctx([64], [0])
+    assert ops.delta_by_chunks(ctx, state, 128, 128, 4) == 4
+    ctx.dtype = torch.float32
+    assert ops.delta_by_chunks(ctx, state, 128, 128, 4) == 0
+    assert ops.delta_by_chunks(Ctx([15, 4], [0, 0]), state, 128, 128, 4) == 0
+    assert ops.delta_by_chunks(Ctx([64], [0]), state, 64, 128, 4) == 0
+    assert ops.delta_by_chunks(Ctx([64], [0]), state[:, 1:], 128, 128, 4) == 0
