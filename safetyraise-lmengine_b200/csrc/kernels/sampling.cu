@@ -6,6 +6,8 @@
 
 namespace srlm {
 
+constexpr uint32_t kMaxCluster = 8;
+
 // A row may be shared by the blocks of a thread-block cluster: block `rank` of `nranks` takes the
 // elements [lo, hi) of the row, lo a multiple of 4.
 struct Slice {
@@ -102,8 +104,10 @@ __device__ unsigned long long cluster_best(const float* row, int V, Slice sl, un
   }
   cluster_sync();
   best = 0;
-  for (uint32_t r = 0; r < cluster_size(); ++r) {
-    const unsigned long long other = peer_u64(slot, r);
+  const uint32_t n = cluster_size();
+#pragma unroll
+  for (uint32_t r = 0; r < kMaxCluster; ++r) {
+    const unsigned long long other = r < n ? peer_u64(slot, r) : 0;
     best = other > best ? other : best;
   }
   cluster_sync();                       // nobody rewrites its slot while another block still reads it
@@ -177,11 +181,14 @@ extern "C" int srlm_argmax(const float* logits, long long row_stride, int n, int
 // element at which a running total in sorted order reaches a target" is then found
 // by a radix search over the 32 bits of the order key, 8 bits a pass: a pass adds
 // the elements that match the prefix found so far into 256 bins, and a scan of the
-// bins from the top gives the next 8 bits.  Counts (top-k) and masses are integers
+// bins from the top (by one warp) gives the next 8 bits.  Counts (top-k) and masses are integers
 // (a mass is exp(v - max) in units of 2^-31), so the sums do not depend on the
 // order of the additions: the same token on every run.  Elements with equal keys
 // are ordered by id; a tie on a boundary is resolved by a search over the ids.
-// About a dozen passes over the row instead of a hundred.
+// About a dozen passes over the row instead of a hundred; a block's slice of the row lies in shared memory where it fits.
+// A top-k of a few hundred ends after the search for its boundary: the kept elements are collected and ordered.
+// 8 rows of 151,936, top-k 50, top-p 0.9, penalty: 154 us with 64-bit additions and the bins scanned by one thread, 85 us
+// without either, 42 us with the collected list; without a top-k 114 -> 64 us.
 // ---------------------------------------------------------------------------
 namespace srlm {
 
@@ -222,15 +229,21 @@ struct Kept {
 
 constexpr int REPLICAS = 32;          // one copy of the bins per lane: the lanes of a warp never meet
 constexpr int REPLICA_STRIDE = 257;   // in bins: the copies of a bin fall on different banks
+// A bin's copy is two 32-bit sums, of the masses' lower 16 bits and of the rest (a 64-bit addition in shared memory is a loop
+// of compare-and-swap).  A lane adds at most 2^16 elements of a part of a slice, so the lower sums stay below 2^32.
+constexpr int COPY_WORDS = REPLICAS * REPLICA_STRIDE;
+constexpr int MAX_PART = 32 << 15;
 
 struct Shared {
   u64 bins[256];          // the pass in progress: the sums over the whole row
-  u64 mine[256];          // ... and over this block's slice (read by the other blocks of the cluster)
+  u64 mine[2][256];       // ... and over this block's slice (read by the other blocks of the cluster), by turns: a pass
+                          // writes one while slower blocks may still read the other
   u64 first[256];         // masses of the kept set by the top 8 bits of the key (reused by both searches)
   u64 found[3];           // digit, sum above it, its own bin
   u64 low_id[256];        // smallest id of this block's slice that fell into each bin (kept for shift == 0)
   u64 low_all[256];       // ... and of the whole row
   u64 word;               // one word for the other blocks to read
+  u64 total;
   unsigned long long warp_best[32];
   int is[32];
 };
@@ -241,9 +254,44 @@ __device__ u64 cluster_sum(u64 mine, Shared& sh) {
   if (threadIdx.x == 0) sh.word = mine;
   cluster_sync();
   u64 sum = 0;
-  for (uint32_t r = 0; r < cluster_size(); ++r) sum += peer_u64(&sh.word, r);
+  const uint32_t n = cluster_size();
+#pragma unroll
+  for (uint32_t r = 0; r < kMaxCluster; ++r) sum += r < n ? peer_u64(&sh.word, r) : 0;
   cluster_sync();
   return sum;
+}
+
+// By one warp: the digit, from the top, at which `above + bins` first reaches `target` (0 if none does), the sum above that
+// digit, and the digit's own bin.
+__device__ __forceinline__ void scan_bins(const u64* bins, u64 above, u64 target, u64* found) {
+  const int lane = threadIdx.x;
+  u64 b[8], own = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    b[j] = bins[255 - 8 * lane - j];
+    own += b[j];
+  }
+  u64 through = own;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u64 up = __shfl_up_sync(0xffffffffu, through, o);
+    if (lane >= o) through += up;
+  }
+  const unsigned hits = __ballot_sync(0xffffffffu, above + through >= target);
+  if (lane == (hits ? __ffs(hits) - 1 : 31)) {
+    u64 acc = above + through - own, bin = b[7];
+    int at = 7;
+    bool hit = false;
+#pragma unroll
+    for (int j = 0; j < 7; ++j) {
+      if (hit) continue;
+      if (acc + b[j] >= target) hit = true, at = j, bin = b[j];
+      else acc += b[j];
+    }
+    found[0] = (u64)(255 - 8 * lane - at);
+    found[1] = acc;
+    found[2] = bin;
+  }
 }
 
 // One radix pass: adds `weight(v)` of every element for which `match(key, i)` holds into the bin of its
@@ -251,55 +299,66 @@ __device__ u64 cluster_sum(u64 mine, Shared& sh) {
 // `target`, the sum above that digit, and the digit's own bin go to sh.found.  The keys of a row share
 // few leading digits, so every lane adds into a copy of the bins of its own (`copies`, in dynamic shared
 // memory); the copies are summed before the scan.  Integer additions: any order gives the same sums.
-template <typename Match, typename Weight>
-__device__ __forceinline__ void radix_pass(const float* v, int V, Slice sl, int shift, u64 above, u64 target,
-                                           Shared& sh, u64* copies, Match match, Weight weight, bool fill) {
+// COUNT: every weight is 1.  turn: passes that fill alternate between 0 and 1.
+template <bool COUNT, typename Match, typename Weight>
+__device__ __forceinline__ void radix_pass(const float* v, int V, Slice sl, int shift, u64 above, u64 target, int& turn,
+                                           Shared& sh, uint32_t* copies, Match match, Weight weight, bool fill) {
   if (fill) {
-    for (int i = threadIdx.x; i < REPLICAS * REPLICA_STRIDE; i += blockDim.x) copies[i] = 0;
+    u64* mine = sh.mine[turn];
+    turn ^= 1;
     if (shift == 0)
       for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.low_id[i] = 0x7fffffffull;
-    __syncthreads();
-    u64* lane_copy = copies + (threadIdx.x & (REPLICAS - 1)) * REPLICA_STRIDE;
-    for_each_of_row(v, V, sl, [&](int i, float x) {
-      const uint32_t key = order_key(x);
-      if (match(key, i)) {
-        const u64 w = weight(x);
-        const uint32_t d = (key >> shift) & 255u;
-        if (w) atomicAdd(&lane_copy[d], w);
-        if (shift == 0) atomicMin(&sh.low_id[d], (u64)i);
-      }
-    });
-    __syncthreads();
-    for (int d = threadIdx.x; d < 256; d += blockDim.x) {
+    uint32_t* lane_copy = copies + (threadIdx.x & (REPLICAS - 1)) * REPLICA_STRIDE;
+    for (int lo = sl.lo; lo == sl.lo || lo < sl.hi; lo += MAX_PART) {      // one part, for every vocabulary that there is
+      const Slice part{lo, min(sl.hi, lo + MAX_PART)};
+      for (int i = threadIdx.x; i < (COUNT ? 1 : 2) * COPY_WORDS; i += blockDim.x) copies[i] = 0;
+      __syncthreads();
+      for_each_of_row(v, V, part, [&](int i, float x) {
+        const uint32_t key = order_key(x);
+        if (match(key, i)) {
+          const uint32_t d = (key >> shift) & 255u;
+          if (COUNT) {
+            atomicAdd(&lane_copy[d], 1u);
+          } else {
+            const uint32_t w = weight(x);
+            if (w) {
+              atomicAdd(&lane_copy[d], w & 0xffffu);
+              atomicAdd(&lane_copy[COPY_WORDS + d], w >> 16);
+            }
+          }
+          if (shift == 0) atomicMin(&sh.low_id[d], (u64)i);
+        }
+      });
+      __syncthreads();
+      const int d = threadIdx.x >> 2, quarter = threadIdx.x & 3;          // 1024 threads: four a bin, eight copies each
       u64 sum = 0;
-#pragma unroll 8
-      for (int c = 0; c < REPLICAS; ++c) sum += copies[c * REPLICA_STRIDE + d];
-      sh.mine[d] = sum;
+#pragma unroll
+      for (int c = 0; c < REPLICAS / 4; ++c) {
+        const int at = (4 * c + quarter) * REPLICA_STRIDE + d;
+        sum += copies[at];
+        if (!COUNT) sum += (u64)copies[COPY_WORDS + at] << 16;
+      }
+      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      if (quarter == 0) mine[d] = lo == sl.lo ? sum : mine[d] + sum;
+      __syncthreads();
     }
     cluster_sync();                       // every block's slice is in its `mine`
     const uint32_t n = cluster_size();
     for (int d = threadIdx.x; d < 256; d += blockDim.x) {
       u64 sum = 0, low = 0x7fffffffull;
-      for (uint32_t r = 0; r < n; ++r) {
-        sum += peer_u64(&sh.mine[d], r);
+#pragma unroll
+      for (uint32_t r = 0; r < kMaxCluster; ++r) {
+        if (r >= n) break;
+        sum += peer_u64(&mine[d], r);
         if (shift == 0) { const u64 other = peer_u64(&sh.low_id[d], r); low = other < low ? other : low; }
       }
       sh.bins[d] = sum;
       if (shift == 0) sh.low_all[d] = low;
     }
-    cluster_sync();                       // nobody rewrites `mine` or `low_id` while another block reads them
+    __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    u64 acc = above;
-    int d = 255;
-    for (; d > 0; --d) {
-      if (acc + sh.bins[d] >= target) break;
-      acc += sh.bins[d];
-    }
-    sh.found[0] = (u64)d;
-    sh.found[1] = acc;
-    sh.found[2] = sh.bins[d];
-  }
+  if (threadIdx.x < 32) scan_bins(sh.bins, above, target, sh.found);
   __syncthreads();
 }
 
@@ -359,7 +418,7 @@ __device__ int nth_holder(const float* v, int V, Slice sl, uint32_t key, const K
 // ascending, first reaches `target` (1 <= target <= total mass).  sh.first must hold the kept set's
 // masses by the top 8 bits of the key.
 __device__ void select_by_mass(const float* v, int V, Slice sl, const Kept& kept, float vmax, u64 target, Shared& sh,
-                               u64* copies, uint32_t* key_sel, int* id_sel, u64* mass_through) {
+                               uint32_t* copies, int& turn, uint32_t* key_sel, int* id_sel, u64* mass_through) {
   uint32_t prefix = 0;
   u64 above = 0;
   for (int level = 0; level < 4; ++level) {
@@ -369,9 +428,9 @@ __device__ void select_by_mass(const float* v, int V, Slice sl, const Kept& kept
       __syncthreads();
     }
     const uint32_t pre = prefix;
-    radix_pass(v, V, sl, shift, above, target, sh, copies,
-               [&](uint32_t key, int i) { return kept.has(key, i) && (key >> (shift + 8)) == pre; },
-               [&](float x) { return (u64)mass_of(x, vmax); }, level != 0);
+    radix_pass<false>(v, V, sl, shift, above, target, turn, sh, copies,
+                      [&](uint32_t key, int i) { return kept.has(key, i) && (key >> (shift + 8)) == pre; },
+                      [&](float x) { return mass_of(x, vmax); }, level != 0);
     prefix = (prefix << 8) | (uint32_t)sh.found[0];
     above = sh.found[1];
   }
@@ -388,6 +447,81 @@ __device__ void select_by_mass(const float* v, int V, Slice sl, const Kept& kept
   *mass_through = above + need * w;
 }
 
+// The choice among few kept elements (top-k of at most kList): block 0 of the cluster collects them, orders them by key
+// descending and id ascending, and reads the cutoff and the draw off their running masses: the element that the searches
+// above would find.  -> its id in block 0's thread 0; the other blocks return at once.  lists: 3 * kList words of shared
+// memory, at the same place in every block.
+constexpr int kList = 512;
+__device__ int select_from_list(const float* v, int V, Slice sl, const Kept& kept, float vmax, float tp, float uniform,
+                                Shared& sh, u64* lists) {
+  u64 *own = lists, *all = lists + kList, *sorted = lists + 2 * kList;
+  __syncthreads();
+  if (threadIdx.x == 0) sh.is[0] = 0;
+  __syncthreads();
+  for_each_of_row(v, V, sl, [&](int i, float x) {
+    const uint32_t key = order_key(x);
+    if (kept.has(key, i)) {
+      const int at = atomicAdd(&sh.is[0], 1);
+      if (at < kList) own[at] = ((u64)key << 32) | (uint32_t)(0x7fffffff - i);
+    }
+  });
+  __syncthreads();
+  if (threadIdx.x == 0) sh.word = (u64)min(sh.is[0], kList);
+  cluster_sync();
+  int n = 0;
+  if (cluster_rank() == 0) {
+    for (uint32_t r = 0; r < cluster_size(); ++r) {
+      const int count = min((int)peer_u64(&sh.word, r), kList - n);
+      for (int j = threadIdx.x; j < count; j += blockDim.x) all[n + j] = peer_u64(&own[j], r);
+      n += count;
+    }
+  }
+  cluster_sync();
+  if (cluster_rank() != 0) return 0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const u64 mine = all[i];
+    int before = 0;
+    for (int j = 0; j < n; ++j) before += all[j] > mine;
+    sorted[before] = mine;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return 0;
+  const int lane = threadIdx.x, per = (n + 31) / 32, lo = min(n, lane * per), hi = min(n, lo + per);
+  auto mass = [&](int i) { return (u64)mass_of(key_value((uint32_t)(sorted[i] >> 32)), vmax); };
+  u64 own_mass = 0;
+  for (int i = lo; i < hi; ++i) own_mass += mass(i);
+  u64 through = own_mass;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const u64 up = __shfl_up_sync(0xffffffffu, through, o);
+    if (lane >= o) through += up;
+  }
+  const u64 total = __shfl_sync(0xffffffffu, through, 31);
+  // the first element whose running mass reaches `target` (1 .. total), and that mass
+  auto reach = [&](u64 target, u64* mass_through) {
+    const int lane_of = __ffs(__ballot_sync(0xffffffffu, through >= target)) - 1;
+    u64 acc = through - own_mass;
+    int at = lo;
+    if (lane == lane_of)
+      for (; at < hi; ++at) {
+        acc += mass(at);
+        if (acc >= target) break;
+      }
+    *mass_through = __shfl_sync(0xffffffffu, acc, lane_of);
+    return __shfl_sync(0xffffffffu, at, lane_of);
+  };
+  u64 kept_mass = total, unused;
+  int cut = n - 1;
+  if (tp < 1.f) {
+    u64 target = (u64)ceil((double)tp * (double)total);
+    target = target < 1 ? 1 : (target > total ? total : target);
+    cut = reach(target, &kept_mass);
+  }
+  u64 draw = (u64)ceil((double)uniform * (double)kept_mass);
+  draw = draw < 1 ? 1 : (draw > kept_mass ? kept_mass : draw);
+  return 0x7fffffff - (int)(uint32_t)sorted[min(reach(draw, &unused), cut)];
+}
+
 // One block per row.  hist_offsets[row]..hist_offsets[row+1] index `history` (ids for the penalty).
 // scratch: one row of V floats per row of logits.
 __global__ void __launch_bounds__(1024)
@@ -395,16 +529,19 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
               const float* __restrict__ temperature, const int* __restrict__ top_k,
               const float* __restrict__ top_p, const float* __restrict__ penalty,
               const float* __restrict__ uniform, const int* __restrict__ history,
-              const int* __restrict__ hist_offsets, float* __restrict__ scratch, int* __restrict__ out_token,
-              int* __restrict__ bad) {
-  extern __shared__ u64 dyn_smem[];                 // the copies of the bins, then the penalty's bitmap
-  u64* copies = dyn_smem;
-  uint32_t* seen_bits = reinterpret_cast<uint32_t*>(dyn_smem + REPLICAS * REPLICA_STRIDE);   // ceil(V / 32) words
+              const int* __restrict__ hist_offsets, float* __restrict__ scratch, int slice_room,
+              int* __restrict__ out_token, int* __restrict__ bad) {
+  extern __shared__ __align__(16) float dyn_smem[];  // [the slice's adjusted values], the copies of the bins, the penalty's bitmap
   __shared__ Shared sh;
   const int r = blockIdx.x / cluster_size();
   const Slice sl = slice_of(V);
   const float* row = logits + (size_t)r * row_stride;
-  float* v = scratch + (size_t)r * V;
+  // the adjusted values: in shared memory where the slice fits, else in the scratch row.  (Indexed like the row; slices
+  // begin on a multiple of 4, so a slice in shared memory keeps the row's alignment of 16 bytes.)
+  float* v = slice_room ? dyn_smem - sl.lo : scratch + (size_t)r * V;
+  uint32_t* copies = reinterpret_cast<uint32_t*>(dyn_smem + slice_room);
+  uint32_t* seen_bits = copies + 2 * COPY_WORDS;                                   // ceil(V / 32) words
+  int turn = 0;
   const float temp = temperature[r];
   const float pen = penalty ? penalty[r] : 1.f;
   const bool use_pen = pen != 1.f && history;
@@ -447,9 +584,9 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
     for (int level = 0; level < 4; ++level) {
       const int shift = 24 - 8 * level;
       const uint32_t pre = prefix;
-      radix_pass(v, V, sl, shift, above, (u64)k, sh, copies,
-                 [&](uint32_t key, int) { return level == 0 || (key >> (shift + 8)) == pre; },
-                 [](float) { return (u64)1; }, true);
+      radix_pass<true>(v, V, sl, shift, above, (u64)k, turn, sh, copies,
+                       [&](uint32_t key, int) { return level == 0 || (key >> (shift + 8)) == pre; },
+                       [](float) { return 1u; }, true);
       prefix = (prefix << 8) | (uint32_t)sh.found[0];
       above = sh.found[1];
     }
@@ -461,15 +598,21 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
       kept.id_cut = nth_holder(v, V, sl, prefix, Kept{0u, 0x7fffffff}, (u64)k - above, ties,
                                first_id == 0x7fffffff ? -1 : first_id, sh);
   }
+  if (k > 0 && k < V && k <= kList) {
+    const int id = select_from_list(v, V, sl, kept, bv, top_p[r], uniform[r], sh, reinterpret_cast<u64*>(copies));
+    if (writer) out_token[r] = id;
+    return;
+  }
   // the kept set's masses by the top 8 bits of the key; their sum is the softmax denominator
-  radix_pass(v, V, sl, 24, 0, ~(u64)0, sh, copies, [&](uint32_t key, int i) { return kept.has(key, i); },
-             [&](float x) { return (u64)mass_of(x, bv); }, true);
+  radix_pass<false>(v, V, sl, 24, 0, ~(u64)0, turn, sh, copies, [&](uint32_t key, int i) { return kept.has(key, i); },
+                    [&](float x) { return mass_of(x, bv); }, true);
   for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.first[i] = sh.bins[i];
+  if (threadIdx.x == 0) sh.total = sh.found[1] + sh.found[2];      // no bin reaches the target: all above bin 0, and bin 0
   __syncthreads();
-  u64 total = 0;
-  for (int i = 0; i < 256; ++i) total += sh.first[i];
+  const u64 total = sh.total;
   if (total == 0) {                       // the same in every block: the bins hold the whole row
     if (writer) { atomicExch(bad, 1); out_token[r] = bi; }
+    cluster_sync();                     // no block leaves while another reads its shared memory
     return;
   }
   // top-p cutoff: the shortest prefix whose mass >= top_p
@@ -480,7 +623,7 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
   if (tp < 1.f) {
     u64 target = (u64)ceil((double)tp * (double)total);
     target = target < 1 ? 1 : (target > total ? total : target);
-    select_by_mass(v, V, sl, kept, bv, target, sh, copies, &key_cut, &id_cut, &kept_mass);
+    select_by_mass(v, V, sl, kept, bv, target, sh, copies, turn, &key_cut, &id_cut, &kept_mass);
   }
   // the draw
   u64 draw = (u64)ceil((double)uniform[r] * (double)kept_mass);
@@ -488,10 +631,11 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
   uint32_t key_sel;
   int id_sel;
   u64 through;
-  select_by_mass(v, V, sl, kept, bv, draw, sh, copies, &key_sel, &id_sel, &through);
+  select_by_mass(v, V, sl, kept, bv, draw, sh, copies, turn, &key_sel, &id_sel, &through);
   // never beyond the cutoff element (the reference falls back to the last kept element)
   if (key_sel < key_cut || (key_sel == key_cut && id_sel > id_cut)) id_sel = id_cut;
   if (writer) out_token[r] = id_sel;
+  cluster_sync();                       // no block leaves while another reads its shared memory
 }
 
 }  // namespace srlm
@@ -504,14 +648,15 @@ extern "C" int srlm_sample(const float* logits, long long row_stride, int n, int
   if (n <= 0) return ST_OK;
   if (V <= 0 || row_stride < V) return refuse(ST_BAD_SIZE, "sample: V=%d stride=%lld", V, row_stride);
   if (!scratch) return refuse(ST_BAD_SIZE, "sample: a scratch row of V floats per row of logits is needed");
-  const size_t smem = (size_t)REPLICAS * REPLICA_STRIDE * 8 + (history ? (size_t)((V + 31) / 32) * 4 : 0);
-  if (smem > 190 * 1024) return refuse(ST_BAD_SIZE, "sample: vocabulary %d is too large for the penalty bitmap", V);
-  static bool raised = false;
-  if (!raised) {
-    cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 190 * 1024);
-    raised = true;
-  }
-  launch_rows(sample_kernel, n, blocks_per_row(V, n), 1024, smem, stream, logits, row_stride, V, temperature, top_k, top_p,
-              penalty, uniform, history, hist_offsets, scratch, out_token, bad_flag);
+  const int cluster = blocks_per_row(V, n);
+  const int slice = ((V + cluster - 1) / cluster + 3) & ~3;
+  const size_t fixed = (size_t)2 * COPY_WORDS * 4 + (history ? (size_t)((V + 31) / 32) * 4 : 0);
+  if (fixed > 190 * 1024) return refuse(ST_BAD_SIZE, "sample: vocabulary %d is too large for the penalty bitmap", V);
+  const int room = fixed + (size_t)slice * 4 <= 190 * 1024 ? slice : 0;
+  const size_t smem = fixed + (size_t)room * 4;
+  const cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 190 * 1024);
+  if (e != cudaSuccess) return refuse((int)e, "sample: cannot get 190 KB of shared memory");
+  launch_rows(sample_kernel, n, cluster, 1024, smem, stream, logits, row_stride, V, temperature, top_k, top_p,
+              penalty, uniform, history, hist_offsets, scratch, room, out_token, bad_flag);
   return launched();
 }

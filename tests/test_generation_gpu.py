@@ -316,6 +316,24 @@ def test_sampling_rows_shared_by_clusters_of_blocks(V, n):
     assert out.tolist() == [int(np.argmax(r)) for r in logits]
 
 
+@pytest.mark.parametrize("V, k", [(700, 1), (700, 699), (8192, 512), (8192, 513), (40004, 511), (40004, 512)])
+def test_sampling_around_the_longest_collected_list(V, k):
+    """A top-k of up to 512 collects and orders what it keeps, a larger one searches by mass: both follow the plain sampler,
+    with ties on the boundary and with all values equal."""
+    from safetyraise_lmengine_b200.sampling.params import SamplingParams
+    from safetyraise_lmengine_b200.sampling.sampler import Sampler, uniform_for
+    rng = np.random.default_rng(V + k)
+    n = 6
+    logits = rng.normal(0, 2.0, size=(n, V)).astype(np.float32)
+    logits[1] = np.round(logits[1])
+    logits[2] = 1.0
+    params = [SamplingParams(temperature=1.0, top_p=[1.0, 0.9][i % 2], top_k=k) for i in range(n)]
+    seeds, idx = [50 + i for i in range(n)], list(range(n))
+    got = Sampler(DEV, V, n).sample(torch.tensor(logits, device=DEV), params, seeds, idx, [[]] * n)
+    for i, p in enumerate(params):
+        assert consistent_with_plain(got[i], logits[i], [], 1.0, k, p.top_p, 1.0, uniform_for(seeds[i], idx[i])), (i, got[i])
+
+
 def test_sampling_statistics():
     """Frequencies over many draws follow the truncated distribution."""
     from safetyraise_lmengine_b200.sampling.params import SamplingParams
