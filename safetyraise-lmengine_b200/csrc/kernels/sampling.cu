@@ -154,9 +154,11 @@ static void launch_rows(void (*kernel)(KArgs...), int rows, int cluster, int blo
 }
 // Blocks per row: a long row is shared by a cluster of up to 8 (the portable size), each block a slice,
 // as long as the clusters of all rows find room on the GPU at once.
-static int blocks_per_row(int V, int rows) {
+// whole_sms: a block fills an SM, and the GPU's clusters of SMs hold 15 clusters of 8 such blocks or 36 of 4 at a time
+// (16 rows: 128 us in clusters of 8, which take two rounds, 85 us in clusters of 4).
+static int blocks_per_row(int V, int rows, bool whole_sms = false) {
   int c = V >= 32768 ? 8 : V >= 8192 ? 2 : 1;
-  while (c > 1 && rows * c > 148) c >>= 1;
+  while (c > 1 && (rows * c > 148 || (whole_sms && rows > (c == 8 ? 15 : c == 4 ? 36 : 74)))) c >>= 1;
   return c;
 }
 
@@ -648,7 +650,7 @@ extern "C" int srlm_sample(const float* logits, long long row_stride, int n, int
   if (n <= 0) return ST_OK;
   if (V <= 0 || row_stride < V) return refuse(ST_BAD_SIZE, "sample: V=%d stride=%lld", V, row_stride);
   if (!scratch) return refuse(ST_BAD_SIZE, "sample: a scratch row of V floats per row of logits is needed");
-  const int cluster = blocks_per_row(V, n);
+  const int cluster = blocks_per_row(V, n, true);
   const int slice = ((V + cluster - 1) / cluster + 3) & ~3;
   const size_t fixed = (size_t)2 * COPY_WORDS * 4 + (history ? (size_t)((V + 31) / 32) * 4 : 0);
   if (fixed > 190 * 1024) return refuse(ST_BAD_SIZE, "sample: vocabulary %d is too large for the penalty bitmap", V);
