@@ -11,6 +11,7 @@ import ctypes as C
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
+import numpy as np
 import torch
 
 from ..errors import ConfigError, ResourceExhausted
@@ -82,6 +83,15 @@ def runtime():
                                                         "free_pages": 1}.get(name, 2)
         lib.srlm_cache_table.restype = C.c_int
         lib.srlm_cache_table.argtypes = [C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_int32), C.c_int]
+        # a whole step at once: addresses of int32 arrays, taken as plain numbers
+        at = C.c_void_p
+        lib.srlm_cache_look.argtypes = [C.c_void_p, C.c_int, at, at, at]
+        lib.srlm_cache_look.restype = None
+        lib.srlm_cache_reserve_many.argtypes = [C.c_void_p, C.c_int, at, at, at]
+        lib.srlm_cache_commit_many.argtypes = [C.c_void_p, C.c_int, at, at]
+        lib.srlm_lay_out_tokens.argtypes = [C.c_int, at, at, at, at, at, at]
+        lib.srlm_lay_out_tokens.restype = None
+        lib.srlm_cache_lay_out_pages.argtypes = [C.c_void_p, C.c_int, C.c_int, at, at, at, C.c_int, C.c_int, at, at]
         lib.srlm_cache_destroy.argtypes = [C.c_void_p]
         lib.srlm_cache_reuse_counts.argtypes = [C.c_void_p, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
         lib.srlm_sched_destroy.argtypes = [C.c_void_p]
@@ -210,6 +220,39 @@ class CacheManager:
         if n < 0:
             raise ValueError(f"slot {slot} is not open")
         return n
+
+    # ---- a step's entries at once (int32 arrays; one call into the runtime instead of several an entry) ----
+    def look(self, slots: np.ndarray) -> Tuple[List[int], List[int]]:
+        """(lengths, generations) of the slots; a length of -1 for a slot that is not open."""
+        n = len(slots)
+        out = np.empty((2, n), dtype=np.int32)
+        self._lib.srlm_cache_look(self._h, n, slots.ctypes.data, out.ctypes.data, out[1:].ctypes.data)
+        return out[0].tolist(), out[1].tolist()
+
+    def reserve_many(self, slots: np.ndarray, starts: np.ndarray, new_lens: np.ndarray) -> int:
+        """reserve() for every entry, all or nothing: the number of entries, or the index of the first without pages (the
+        others then hold what they held)."""
+        r = self._lib.srlm_cache_reserve_many(self._h, len(slots), slots.ctypes.data, starts.ctypes.data, new_lens.ctypes.data)
+        if r < 0:
+            raise ValueError(f"reserve(slot={slots[-1 - r]}, new_len={new_lens[-1 - r]}) is invalid")
+        return r
+
+    def commit_many(self, slots: np.ndarray, new_lens: np.ndarray) -> None:
+        r = self._lib.srlm_cache_commit_many(self._h, len(slots), slots.ctypes.data, new_lens.ctypes.data)
+        if r != len(slots):
+            raise ValueError(f"commit(slot={slots[r]}, new_len={new_lens[r]}) is invalid")
+
+    def lay_out_tokens(self, starts, q_lens, positions, entry_of_token, cu_q, kv_lens) -> None:
+        """Positions and entry of every token, offsets of the entries' tokens, context lengths, into int32 arrays."""
+        self._lib.srlm_lay_out_tokens(len(starts), starts.ctypes.data, q_lens.ctypes.data, positions.ctypes.data,
+                                      entry_of_token.ctypes.data, cu_q.ctypes.data, kv_lens.ctypes.data)
+
+    def lay_out_pages(self, group: str, slots, starts, q_lens, pages: int, tables, kv_slot) -> int:
+        """The entries' block tables in ``group`` ([entries, pages], zeros behind what a slot holds) and the flat cache row of
+        every token, into int32 arrays; 0, or 1 + the entry whose slot holds more pages."""
+        return self._lib.srlm_cache_lay_out_pages(self._h, self._paged_index[group], len(slots), slots.ctypes.data,
+                                                  starts.ctypes.data, q_lens.ctypes.data, self.page_size, pages,
+                                                  tables.ctypes.data, kv_slot.ctypes.data)
 
     def free_pages(self, group: Optional[str] = None) -> int:
         return self._lib.srlm_cache_free_pages(self._h, self._paged_index[group] if group else 0)

@@ -41,6 +41,58 @@ void srlm_cache_reuse_counts(void* c, int64_t* taken, int64_t* reused) {
   *reused = static_cast<CacheManager*>(c)->pages_reused_total();
 }
 
+void srlm_cache_look(void* c, int n, const int32_t* slots, int32_t* lengths, int32_t* generations) {
+  const CacheManager* m = static_cast<CacheManager*>(c);
+  for (int i = 0; i < n; ++i) {
+    lengths[i] = m->length(slots[i]);
+    generations[i] = m->generation(slots[i]);
+  }
+}
+int srlm_cache_reserve_many(void* c, int n, const int32_t* slots, const int32_t* starts, const int32_t* new_lens) {
+  CacheManager* m = static_cast<CacheManager*>(c);
+  for (int i = 0; i < n; ++i) {
+    const int r = m->reserve(slots[i], new_lens[i]);
+    if (r == 1) continue;
+    for (int j = 0; j < i; ++j) m->truncate(slots[j], starts[j]);
+    return r == 0 ? i : -1 - i;
+  }
+  return n;
+}
+int srlm_cache_commit_many(void* c, int n, const int32_t* slots, const int32_t* new_lens) {
+  for (int i = 0; i < n; ++i)
+    if (static_cast<CacheManager*>(c)->commit(slots[i], new_lens[i]) != 0) return i;
+  return n;
+}
+void srlm_lay_out_tokens(int n, const int32_t* starts, const int32_t* q_lens, int32_t* positions, int32_t* entry_of_token,
+                         int32_t* cu_q, int32_t* kv_lens) {
+  int t = 0;
+  cu_q[0] = 0;
+  for (int e = 0; e < n; ++e) {
+    for (int j = 0; j < q_lens[e]; ++j, ++t) {
+      positions[t] = starts[e] + j;
+      entry_of_token[t] = e;
+    }
+    cu_q[e + 1] = t;
+    kv_lens[e] = starts[e] + q_lens[e];
+  }
+}
+int srlm_cache_lay_out_pages(void* c, int group, int n, const int32_t* slots, const int32_t* starts,
+                             const int32_t* q_lens, int page_size, int pages, int32_t* tables, int32_t* kv_slot) {
+  const CacheManager* m = static_cast<CacheManager*>(c);
+  int t = 0;
+  for (int e = 0; e < n; ++e) {
+    int32_t* row = tables + static_cast<int64_t>(e) * pages;
+    const int held = m->table(group, slots[e], row, pages);
+    if (held < 0 || held > pages) return 1 + e;
+    for (int i = held; i < pages; ++i) row[i] = 0;
+    for (int j = 0; j < q_lens[e]; ++j, ++t) {
+      const int p = starts[e] + j;
+      kv_slot[t] = row[p / page_size] * page_size + p % page_size;
+    }
+  }
+  return 0;
+}
+
 void* srlm_sched_create(void* cache, int max_active, int queue_capacity, int prefill_chunk,
                         int max_batch_tokens, int max_context) {
   if (!cache || max_active <= 0 || queue_capacity <= 0 || prefill_chunk <= 0 ||

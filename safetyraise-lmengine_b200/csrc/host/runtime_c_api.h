@@ -23,6 +23,19 @@ int srlm_cache_generation(void* cache, int slot);
 int srlm_cache_table(void* cache, int group, int slot, int32_t* out, int cap);
 int srlm_cache_free_pages(void* cache, int group);
 int srlm_cache_audit(void* cache);
+/* The same for the n entries of a step at once.  look: lengths and generations (-1 where there is none).
+ * reserve_many: n, all or nothing; else the first entry without pages, as its index, or as -1 - index where the
+ * arguments are invalid (what the call took is given back).  commit_many: n, or the index of the first invalid entry. */
+void srlm_cache_look(void* cache, int n, const int32_t* slots, int32_t* lengths, int32_t* generations);
+int srlm_cache_reserve_many(void* cache, int n, const int32_t* slots, const int32_t* starts, const int32_t* new_lens);
+int srlm_cache_commit_many(void* cache, int n, const int32_t* slots, const int32_t* new_lens);
+/* A step's layout: positions, entry of every token, offsets of the entries' tokens, context lengths; and for a group the
+ * entries' block tables (`pages` columns, zeros behind what a slot holds) and the flat cache row of every token.
+ * lay_out_pages: 0, or 1 + the entry whose slot holds more than `pages` pages or is not open. */
+void srlm_lay_out_tokens(int n, const int32_t* starts, const int32_t* q_lens, int32_t* positions, int32_t* entry_of_token,
+                         int32_t* cu_q, int32_t* kv_lens);
+int srlm_cache_lay_out_pages(void* cache, int group, int n, const int32_t* slots, const int32_t* starts,
+                             const int32_t* q_lens, int page_size, int pages, int32_t* tables, int32_t* kv_slot);
 void srlm_cache_reuse_counts(void* cache, int64_t* taken, int64_t* reused);
 
 void* srlm_sched_create(void* cache, int max_active, int queue_capacity, int prefill_chunk,

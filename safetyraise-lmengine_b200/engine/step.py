@@ -60,6 +60,7 @@ class PreparedStep:
     missing: int                      # token ids still to be set
     state_snapshot: Optional[dict] = None   # fixed-size state of the step's slots before the forward
     host: Optional[np.ndarray] = None       # the pinned buffer as an array (made once: set_token is called per token)
+    arrays: Optional[tuple] = None          # (slots, lengths behind the step) as int32 arrays
 
     def set_token(self, entry: int, index: int, token: int) -> None:
         h = self.host if self.host is not None else self.pair[0].numpy()
@@ -147,24 +148,26 @@ class Engine:
 
     # ---- the step -------------------------------------------------------------
     def _validate(self, entries: Sequence[StepEntry]):
+        """Checks the entries; -> (slots as an int32 array, lengths, generations) of their slots."""
         if not entries:
             raise ShapeError("a step needs at least one entry")
+        slots = np.array([e.slot for e in entries], dtype=np.int32)
+        lengths, generations = self.cache.look(slots)
         seen = set()
         total = 0
         vocab = self.spec.vocab_size
-        for e in entries:
+        for e, start, generation in zip(entries, lengths, generations):
             if e.slot in seen:
                 raise ShapeError(f"slot {e.slot} appears twice in one step")
             seen.add(e.slot)
             n = len(e.tokens)
             if n == 0:
                 raise ShapeError("an entry without tokens")
-            start = self.cache.length(e.slot)
             if start < 0:
                 raise ShapeError(f"slot {e.slot} is not open")
-            if e.generation is not None and e.generation != self.cache.generation(e.slot):
+            if e.generation is not None and e.generation != generation:
                 raise ShapeError(f"slot {e.slot} was given to another request since this one opened it "
-                                 f"(generation {self.cache.generation(e.slot)}, the entry holds {e.generation})")
+                                 f"(generation {generation}, the entry holds {e.generation})")
             if start + n > self.max_context:
                 raise ShapeError(f"slot {e.slot}: {start}+{n} tokens exceed the context of {self.max_context}")
             if n == 1:                               # a decoded token: no array for one number
@@ -182,6 +185,7 @@ class Engine:
             total += n
         if total > self.mctx.max_batch_tokens:
             raise ShapeError(f"{total} tokens in one step exceed max_batch_tokens={self.mctx.max_batch_tokens}")
+        return slots, lengths, generations
 
     def _meta_buffers(self, words: int):
         """A pinned host buffer that no copy in flight still reads, and the device buffer."""
@@ -198,7 +202,7 @@ class Engine:
             pair[1].synchronize()
         return pair, self._meta_dev
 
-    def _lay_out(self, entries: Sequence[StepEntry], starts: List[int]) -> PreparedStep:
+    def _lay_out(self, entries: Sequence[StepEntry], starts: List[int], slots: Optional[np.ndarray] = None) -> PreparedStep:
         """Flattens the batch into a pinned host buffer (no device work)."""
         n = len(entries)
         q_lens = [len(e.tokens) for e in entries]
@@ -208,7 +212,7 @@ class Engine:
         kv_lens = [s + q for s, q in zip(starts, q_lens)]
         # decode-only steps round the table width coarsely: its value is part of a graph's identity
         decode_only = max(q_lens) == 1
-        pages = _round_up(max(1, max((l + ps - 1) // ps for l in kv_lens)), 16 if decode_only else 8)
+        pages = _round_up(max(1, (max(kv_lens) + ps - 1) // ps), 16 if decode_only else 8)
         R = sum(len(e.want) for e in entries)
         # layout, in int32 words; every section starts on a 16-byte boundary
         sections, off = {}, 0
@@ -229,58 +233,58 @@ class Engine:
         pair, _ = self._meta_buffers(off)
         h = pair[0].numpy()
         view = lambda name: h[sections[name][0]:sections[name][0] + sections[name][1]]
-        tok, posv, eot = view("token_ids"), view("positions"), view("entry_of_token")
-        cu = view("cu_q")
-        rows = view("logit_rows")
-        cu[0] = 0
-        t0 = r0 = 0
-        token_at, missing = [], 0
-        slot_views = [(view("kv_slot:" + g.name), view("table:" + g.name), g.name) for g in groups]
-        for i, e in enumerate(entries):
-            q = q_lens[i]
-            token_at.append(sections["token_ids"][0] + t0)
-            if q == 1:                               # a decoded token: plain numbers
-                t = int(e.tokens[0])
-                missing += t == LATER
-                tok[t0] = t
-                posv[t0] = starts[i]
-                eot[t0] = i
-            else:
-                ids = np.asarray(e.tokens, dtype=np.int32)
-                missing += int((ids == LATER).sum())
-                tok[t0:t0 + q] = ids
-                posv[t0:t0 + q] = np.arange(starts[i], starts[i] + q, dtype=np.int32)
-                eot[t0:t0 + q] = i
-            for w in e.want:
-                rows[r0] = t0 + int(w)
-                r0 += 1
-            for kvs, tabs, name in slot_views:
-                tv = tabs[i * pages:(i + 1) * pages]
-                held = self.cache.table_into(name, e.slot, tv)      # the block table, straight into its row
-                if held > pages:
-                    raise ShapeError(f"slot {e.slot} holds {held} pages, the step laid out {pages}")
-                tv[held:] = 0
+        if slots is None:
+            slots = np.array([e.slot for e in entries], dtype=np.int32)
+        starts_a, q_a = np.array(starts, dtype=np.int32), np.array(q_lens, dtype=np.int32)
+        view("slots")[:] = slots
+        self.cache.lay_out_tokens(starts_a, q_a, view("positions"), view("entry_of_token"), view("cu_q"), view("kv_lens"))
+        for g in groups:
+            over = self.cache.lay_out_pages(g.name, slots, starts_a, q_a, pages, view("table:" + g.name),
+                                            view("kv_slot:" + g.name))
+            if over:
+                raise ShapeError(f"slot {entries[over - 1].slot} holds more pages than the {pages} that the step laid out")
+        tok, first = view("token_ids"), sections["token_ids"][0]
+        if decode_only:                              # decoded tokens: plain numbers
+            ids = [int(e.tokens[0]) for e in entries]
+            tok[:] = ids
+            missing = ids.count(LATER)
+            token_at = list(range(first, first + n))
+            rows = [t for t, e in enumerate(entries) for _ in e.want]
+        else:
+            rows, token_at, missing, t0 = [], [], 0, 0
+            for q, e in zip(q_lens, entries):
+                token_at.append(first + t0)
                 if q == 1:
-                    p = starts[i]
-                    kvs[t0] = int(tv[p // ps]) * ps + p % ps
+                    t = int(e.tokens[0])
+                    missing += t == LATER
+                    tok[t0] = t
                 else:
-                    p = posv[t0:t0 + q]
-                    kvs[t0:t0 + q] = tv[p // ps] * ps + p % ps
-            t0 += q
-            cu[i + 1] = t0
-        view("slots")[:] = [e.slot for e in entries]
-        view("kv_lens")[:] = kv_lens
+                    ids = np.asarray(e.tokens, dtype=np.int32)
+                    missing += int((ids == LATER).sum())
+                    tok[t0:t0 + q] = ids
+                rows += [t0 + int(w) for w in e.want]
+                t0 += q
+        if R:
+            view("logit_rows")[:] = rows
         return PreparedStep(entries=entries, starts=starts, q_lens=q_lens, kv_lens=kv_lens, sections=sections,
-                            words=off, pair=pair, pages=pages, wanted=R, token_at=token_at, missing=missing, host=h)
+                            words=off, pair=pair, pages=pages, wanted=R, token_at=token_at, missing=missing, host=h,
+                            arrays=(slots, starts_a + q_a))
 
     def _upload(self, prep: PreparedStep) -> StepContext:
         """Copies the laid-out batch to the device in one copy and returns the device views."""
-        sections, off, pair = prep.sections, prep.words, prep.pair
-        dev = self._meta_dev
-        dev[:off].copy_(pair[0][:off], non_blocking=True)
+        self._send(prep)
+        return self._context(prep)
+
+    def _send(self, prep: PreparedStep) -> None:
+        off, pair = prep.words, prep.pair
+        self._meta_dev[:off].copy_(pair[0][:off], non_blocking=True)
         self.last_h2d_bytes = off * 4
         pair[1] = torch.cuda.Event()
         pair[1].record()
+
+    def _context(self, prep: PreparedStep) -> StepContext:
+        """The device views of a batch that was sent."""
+        sections, dev = prep.sections, self._meta_dev
         groups = self.cache.paged_groups
         n, pages = len(prep.entries), prep.pages
         d = lambda name: dev[sections[name][0]:sections[name][0] + sections[name][1]]
@@ -299,6 +303,22 @@ class Engine:
     def build_context(self, entries: Sequence[StepEntry], starts: List[int]) -> StepContext:
         """Flattens the batch, uploads it in one copy and returns the device views."""
         return self._upload(self._lay_out(entries, starts))
+
+    def _recorded(self, prep: PreparedStep) -> Optional[torch.Tensor]:
+        """Replays the CUDA graph of this kind of step, if there is one (its kernels read the batch from where it was sent:
+        no views are needed); else None."""
+        if not self.use_graphs or max(prep.q_lens) != 1 or self._graph_generation != self.workspace.generation:
+            return None
+        hit = self._graphs.get((len(prep.entries), len(prep.entries), prep.wanted, prep.pages * self.cache.page_size))
+        return self._replay(hit) if hit is not None else None
+
+    def _replay(self, hit) -> torch.Tensor:
+        from ..kernels import ops
+        graph, logits, launches = hit
+        graph.replay()
+        ops.launches += launches
+        self.graph_replays += 1
+        return logits
 
     def _forward(self, ctx: StepContext) -> torch.Tensor:
         """Runs the model on the batch: eagerly, or by replaying the CUDA graph of this kind of step."""
@@ -323,39 +343,31 @@ class Engine:
                 logits = self.model.forward(ctx)
             hit = self._graphs[key] = (graph, logits, ops.launches - before)
             ops.launches = before
-        graph, logits, launches = hit
-        graph.replay()
-        ops.launches += launches
-        self.graph_replays += 1
-        return logits
+        return self._replay(hit)
 
     def prepare(self, entries: Sequence[StepEntry]) -> PreparedStep:
         """The host half of a step: checks, page reservation, batch layout.  Token ids given as LATER
         may be supplied afterwards (``PreparedStep.set_token``).  Between prepare() and run() or
         discard() of a step no other step may be prepared or run."""
-        self._validate(entries)
-        starts = [self.cache.length(e.slot) for e in entries]
-        self._greet_new_occupants(entries)
-        done = []
-        for e, s in zip(entries, starts):
-            if not self.cache.reserve(e.slot, s + len(e.tokens)):
-                for e2, s2 in done:                     # give back what this step took
-                    self.cache.truncate(e2.slot, s2)
-                raise ResourceExhausted(f"no free cache pages for slot {e.slot} "
-                                        f"({s}+{len(e.tokens)} tokens); nothing was run")
-            done.append((e, s))
+        slots, starts, generations = self._validate(entries)
+        self._greet_new_occupants(entries, generations)
+        starts_a = np.array(starts, dtype=np.int32)
+        got = self.cache.reserve_many(slots, starts_a, starts_a + np.array([len(e.tokens) for e in entries], dtype=np.int32))
+        if got < len(entries):                          # what the step took has been given back
+            e, s = entries[got], starts[got]
+            raise ResourceExhausted(f"no free cache pages for slot {e.slot} "
+                                    f"({s}+{len(e.tokens)} tokens); nothing was run")
         try:
             with torch.cuda.device(self.mctx.device):
-                return self._lay_out(entries, starts)
+                return self._lay_out(entries, starts, slots)
         except Exception:
             self.discard_reservation(entries, starts)
             raise
 
-    def _greet_new_occupants(self, entries) -> None:
+    def _greet_new_occupants(self, entries, generations) -> None:
         """A slot that changed hands since this engine last ran it starts from a zero fixed-size state,
         whoever opened it (this engine, or the scheduler when it admits or re-admits a request)."""
-        for e in entries:
-            g = self.cache.generation(e.slot)
+        for e, g in zip(entries, generations):
             if g != self._slot_generation[e.slot]:
                 self._slot_generation[e.slot] = g
                 for pool in self.cache.state_pools.values():
@@ -397,11 +409,16 @@ class Engine:
                             raise ShapeError(f"token {index} of entry {entry} is not open, or row {row} does not exist")
                         h[at + 2 * k], h[at + 2 * k + 1] = word, row
                     layout_words, prep.words = prep.words, at + 2 * len(patch)
-                ctx = self._upload(prep)
+                self._send(prep)
                 if patch:
                     prep.words = layout_words
                     ops.patch_words(self._meta_dev, self._meta_dev[at:at + 2 * len(patch)],
                                     self.status[STATUS_WORDS:], len(patch), self.status[FAULT_TOKEN:FAULT_TOKEN + 1])
+                if not self.cache.state_pools:
+                    logits = self._recorded(prep)
+                    if logits is not None:
+                        return logits
+                ctx = self._context(prep)
                 if self.cache.state_pools:
                     # fixed-size state cannot be truncated: keep what the step's slots held
                     # (src/engine/state.rs:222-224 clones the whole state for the same reason)
@@ -414,8 +431,7 @@ class Engine:
             raise
 
     def commit(self, prep: PreparedStep) -> None:
-        for e, s in zip(prep.entries, prep.starts):
-            self.cache.commit(e.slot, s + len(e.tokens))
+        self.cache.commit_many(*prep.arrays)
         self.steps_run += 1
 
     def revoke(self, prep: PreparedStep) -> None:

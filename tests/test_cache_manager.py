@@ -1,6 +1,7 @@
 """The cache manager's accounting (no GPU): no page lost, held twice or freed twice."""
 import random
 
+import numpy as np
 import pytest
 
 from safetyraise_lmengine_b200.cache.manager import (FIXED_STATE, PAGED_ALL, PAGED_WINDOW, CacheGroupSpec,
@@ -114,3 +115,64 @@ def test_random_orders_lose_nothing(seed):
     for s in list(live):
         m.close_request(s)
     assert m.audit() == 0 and all(m.free_pages(g.name) == m.num_pages for g in m.paged_groups)
+
+
+@pytest.mark.parametrize("groups", [[(PAGED_ALL, None)], [(PAGED_WINDOW, 9)], [(PAGED_ALL, None), (PAGED_WINDOW, 6)], []])
+def test_a_step_at_once_is_its_entries_one_by_one(groups):
+    """look, reserve_many, lay_out_tokens, lay_out_pages and commit_many against the calls for one entry each."""
+    make = lambda: CacheManager([CacheGroupSpec(f"g{i}", k, (i,), 1, 8, window=w) for i, (k, w) in enumerate(groups)], 4, 20, 5)
+    one, many = make(), make()
+    rng = np.random.default_rng(len(groups))
+    for c in (one, many):
+        for _ in range(4):
+            c.open_request()
+    i32 = lambda v: np.array(v, dtype=np.int32)
+    for step in range(40):
+        slots = [int(s) for s in rng.permutation(4)[:rng.integers(1, 5)]]
+        q = [int(rng.integers(1, 8)) for _ in slots]
+        starts, generations = many.look(i32(slots + [4, -1, 99]))
+        assert starts == [one.length(s) for s in slots] + [-1, -1, -1]
+        assert generations == [one.generation(s) for s in slots] + [one.generation(4), -1, -1]
+        starts = starts[:len(slots)]
+        done = 0
+        for s, a, n in zip(slots, starts, q):
+            if not one.reserve(s, a + n):
+                break
+            done += 1
+        got = many.reserve_many(i32(slots), i32(starts), i32(starts) + i32(q))
+        assert got == done
+        if done < len(slots):
+            for s, a in list(zip(slots, starts))[:done]:
+                one.truncate(s, a)
+        assert [many.free_pages(g.name) for g in many.paged_groups] == [one.free_pages(g.name) for g in one.paged_groups]
+        if done < len(slots) or max(a + n for a, n in zip(starts, q)) > 60:
+            for c in (one, many):
+                c.truncate(slots[-1], c.length(slots[-1]))
+                longest = max(slots, key=c.length)
+                c.close_request(longest)
+                assert c.open_request() == longest
+            continue
+        T = sum(q)
+        pos, eot, cu, kv = (np.full(n, -7, np.int32) for n in (T, T, len(q) + 1, len(q)))
+        many.lay_out_tokens(i32(starts), i32(q), pos, eot, cu, kv)
+        assert pos.tolist() == [a + j for a, n in zip(starts, q) for j in range(n)]
+        assert eot.tolist() == [e for e, n in enumerate(q) for _ in range(n)]
+        assert cu.tolist() == [0] + np.cumsum(q).tolist() and kv.tolist() == [a + n for a, n in zip(starts, q)]
+        for g in many.paged_groups:
+            tables = [one.table(g.name, s) for s in slots]
+            pages = max(len(t) for t in tables) + 2
+            out, rows = np.full(len(q) * pages, -7, np.int32), np.full(T, -7, np.int32)
+            assert many.lay_out_pages(g.name, i32(slots), i32(starts), i32(q), pages, out, rows) == 0
+            assert out.reshape(len(q), pages).tolist() == [t + [0] * (pages - len(t)) for t in tables]
+            assert rows.tolist() == [tables[e][p // 4] * 4 + p % 4 for e, p in zip(eot.tolist(), pos.tolist())]
+            longest = max(len(t) for t in tables)
+            assert many.lay_out_pages(g.name, i32(slots), i32(starts), i32(q), longest - 1, out, rows) == 1 + [
+                len(t) for t in tables].index(longest)
+        for s, a, n in zip(slots, starts, q):
+            one.commit(s, a + n)
+        many.commit_many(i32(slots), i32(starts) + i32(q))
+        assert many.audit() == one.audit() == 0
+    with pytest.raises(ValueError):
+        many.commit_many(i32([0]), i32([10 ** 6]))
+    with pytest.raises(ValueError):
+        many.reserve_many(i32([0, 77]), i32([many.length(0), 0]), i32([many.length(0), 1]))
