@@ -355,9 +355,11 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, cons
     const int pos_min = start + r_first[i] / g;
     const int pos_max = start + (min(r_first[i] + BR, r_end) - 1) / g;
     const int lo_max = a.window > 0 ? max(0, pos_max - a.window + 1) : 0;
+    // the row whose head's numbers the thread takes: of a block with one row tile the other tile's rows end at the block's
+    // first one, and the row in front of that may be no row at all
+    const int rs = max(0, min(r, r_end - 1));
     float m_run = -CUDART_INF_F, l_run = 0.f;
     if (a.sinks && (!sliced || blockIdx.y == 0)) {
-      const int rs = min(r, r_end - 1);
       m_run = a.sinks[kvh * g + rs % g] * 1.4426950408889634f;      // in log2 units, like the scaled scores
       l_run = 1.f;
     }
@@ -365,7 +367,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_k, cons
     const bool modified = a.mods.pen_weight || (a.mods.head_scale && !capped);
     float factor = 1.f, weight_q = 0.f, rate = 0.f;
     if (a.mods.head_scale || a.mods.pen_weight) {
-      const int h = kvh * g + min(r, r_end - 1) % g;
+      const int h = kvh * g + rs % g;
       if (a.mods.head_scale) factor = a.mods.head_scale[h];
       if (a.mods.pen_weight) {
         weight_q = a.mods.pen_weight[h] / a.scale_log2;
