@@ -224,6 +224,31 @@ __global__ void attention_merge_kernel(const float* __restrict__ part_o, const f
   }
   __syncthreads();
   TO* o = out + ((size_t)(t0 + r / G) * nq + kvh * G + r % G) * dv;
+  if (dv % 4 == 0 && (reinterpret_cast<uintptr_t>(part_o) & 15) == 0) {      // four columns a thread, eight slices in flight
+    constexpr int AHEAD = 8;
+    const size_t step = (size_t)rows_padded * dv;
+    for (int col = 4 * threadIdx.x; col < dv; col += 4 * blockDim.x) {
+      const float* at = part_o + first * dv + col;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int s = 0; s < nsplit; s += AHEAD) {
+        float4 v[AHEAD];
+#pragma unroll
+        for (int x = 0; x < AHEAD; ++x)
+          if (s + x < nsplit) v[x] = *reinterpret_cast<const float4*>(at + (size_t)(s + x) * step);
+#pragma unroll
+        for (int x = 0; x < AHEAD; ++x)
+          if (s + x < nsplit) {
+            a.x += v[x].x * w[s + x]; a.y += v[x].y * w[s + x];
+            a.z += v[x].z * w[s + x]; a.w += v[x].w * w[s + x];
+          }
+      }
+      o[col] = from_float<TO>(a.x * inv_l);
+      o[col + 1] = from_float<TO>(a.y * inv_l);
+      o[col + 2] = from_float<TO>(a.z * inv_l);
+      o[col + 3] = from_float<TO>(a.w * inv_l);
+    }
+    return;
+  }
   for (int col = threadIdx.x; col < dv; col += blockDim.x) {
     float a = 0.f;
     for (int s = 0; s < nsplit; ++s) a += part_o[(first + (size_t)s * rows_padded) * dv + col] * w[s];

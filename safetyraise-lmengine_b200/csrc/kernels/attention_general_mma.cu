@@ -266,7 +266,7 @@ paged_attention_general_decode_kernel(const float* __restrict__ q, const bf16* _
                                       const float* __restrict__ sinks, int nq, int nkv, int dk, int dv,
                                       int page_size, float scale, int window, int nsplit, int kv_chunk,
                                       float* __restrict__ part_o, float* __restrict__ part_ml, int row_tiles,
-                                      ScoreMods mods, HeadGate gate) {
+                                      ScoreMods mods, HeadGate gate, bool q_vec) {
   pdl_wait();        // launched as a dependent of the kernel ahead: nothing is read before it has finished
   pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -285,10 +285,19 @@ paged_attention_general_decode_kernel(const float* __restrict__ q, const bf16* _
   const int start = kv_len - q_len;
   const int* table = block_table + (size_t)e * table_stride;
 
-  for (int idx = tid; idx < 16 * dk; idx += blockDim.x) {
-    const int r = idx / dk, d = idx - r * dk, row = r0 + r;
-    const float v = row < rows ? q[((size_t)(t0 + row / G) * nq + kvh * G + row % G) * dk + d] : 0.f;
-    q_s[r * ks + d] = __float2bfloat16_rn(v);
+  // the queries, a warp a row (rows of 576 element by element, with a division each, took a third of a short slice's time)
+#pragma unroll
+  for (int r = warp; r < 16; r += kMmaWarps) {
+    const int row = r0 + r;
+    const float* src = q + ((size_t)(t0 + min(row, rows - 1) / G) * nq + kvh * G + min(row, rows - 1) % G) * dk;
+    if (q_vec) {                                            // dk is a multiple of 16: rows of whole pieces of 4
+      for (int d = 4 * lane; d < dk; d += 128) {
+        const float4 v = row < rows ? *reinterpret_cast<const float4*>(src + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<uint2*>(q_s + r * ks + d) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+      }
+    } else {
+      for (int d = lane; d < dk; d += 32) q_s[r * ks + d] = __float2bfloat16_rn(row < rows ? src[d] : 0.f);
+    }
   }
   float m[2], l[2], row_scale[2], pen_w[2], pen_r[2];
   int pos[2], first[2];
@@ -323,21 +332,17 @@ paged_attention_general_decode_kernel(const float* __restrict__ q, const bf16* _
     last_key = min(last_key, base + (slice + 1) * kv_chunk - 1);
   }
   const int jb0 = (first_key / kDecKeys) * kDecKeys;
-  const int kvec = dk / 8, vvec = dv / 8;
+  // a warp fetches every fourth key of a tile, its lanes the pieces of the key (and of its value): one look into the block
+  // table a key, no divisions a piece
   auto fetch = [&](int jb, int buf) {
-    for (int idx = tid; idx < kDecKeys * kvec; idx += blockDim.x) {
-      const int jj = idx / kvec, c = idx - jj * kvec, j = jb + jj;
+#pragma unroll
+    for (int jj = warp; jj < kDecKeys; jj += kMmaWarps) {
+      const int j = jb + jj;
       const bool there = j >= first_key && j <= last_key;
       const size_t rowi = there ? ((size_t)table[j / page_size] * nkv + kvh) * page_size + (j % page_size) : 0;
-      cp_async_16(k_s + buf * k_tile + jj * ks + c * 8, k_cache + rowi * dk + c * 8, there);
-    }
-    if (v_cache) {
-      for (int idx = tid; idx < kDecKeys * vvec; idx += blockDim.x) {
-        const int jj = idx / vvec, c = idx - jj * vvec, j = jb + jj;
-        const bool there = j >= first_key && j <= last_key;
-        const size_t rowi = there ? ((size_t)table[j / page_size] * nkv + kvh) * page_size + (j % page_size) : 0;
-        cp_async_16(v_s + buf * v_tile + jj * vs + c * 8, v_cache + rowi * dv + c * 8, there);
-      }
+      for (int c = 8 * lane; c < dk; c += 256) cp_async_16(k_s + buf * k_tile + jj * ks + c, k_cache + rowi * dk + c, there);
+      if (v_cache)
+        for (int c = 8 * lane; c < dv; c += 256) cp_async_16(v_s + buf * v_tile + jj * vs + c, v_cache + rowi * dv + c, there);
     }
     cp_async_commit();
   };
@@ -568,7 +573,7 @@ extern "C" int srlm_paged_attention_general_decode(const float* q, const void* k
     launch_pdl(kern, dim3(grid), dim3(kMmaWarps * 32), smem, stream, q, (const bf16*)k_cache, (const bf16*)v_cache, (TO*)out,          \
                                                  block_table, table_stride, cu_q, kv_lens, sinks, nq, nkv, dk, dv, \
                                                  page_size, scale, window, nsplit, kv_chunk, part_o, part_ml,      \
-                                                 row_tiles, mods, gate);                                           \
+                                                 row_tiles, mods, gate, ((uintptr_t)q & 15) == 0);                 \
   } while (0)
 #define SRLM_DEC_SIZES(TO)                                \
   do {                                                    \

@@ -27,8 +27,6 @@ __device__ __forceinline__ float rotated_element(const TP* __restrict__ src, int
   return second ? v * c + other * s : v * c - other * s;
 }
 
-constexpr int kTokTile = 16;
-
 // One block per token.  proj row: [.. | c_raw (rank) | kr_raw (rot) | ..] starting at column c_off.  q_out != null: the
 // same block also norms the q_width columns from q_col (a latent of the queries in the same stacked projection) with
 // q_norm_w into q_out [T, q_width].
@@ -68,68 +66,83 @@ __global__ void latent_append_kernel(const TP* __restrict__ proj, long long ldp,
   }
 }
 
-// The two per-head products: out[t, h, c] = sum_k in[t, h, k] * W[h, k, c].  A block takes 16 tokens, one head
-// and 32 columns; its four warps each take a quarter of k (a lane owns a column, so a warp reads 32
-// consecutive weights) and their partial sums are added in warp order through shared memory: the order of
-// every sum depends on the sizes alone.  Decode steps launch heads x columns / 32 blocks, not one per head.
-constexpr int kColTile = 32, kProductWarps = 4;
+// The two per-head products: out[t, h, c] = sum_k in[t, h, k] * W[h, k, c].  A block takes TOK = 8 or 16 tokens, one head
+// and 32 columns; its 16 warps each take a sixteenth of k (a lane owns a column, so a warp reads 32 consecutive weights) and
+// their partial sums are added in warp order through shared memory: the order of every sum depends on the sizes alone.
+// Decode steps launch heads x columns / 32 blocks, not one per head.  Bound by the trips to memory of a warp's weights (16
+// are in flight at a time) and by its reads of the tokens (a piece of four k's is read at once): four warps, weight by
+// weight and k by k, took 26 us (512 x 128, 16 heads, 8 tokens), these 8 us.
+constexpr int kColTile = 32, kProductWarps = 16;
+// Floats from a token's row of K inputs to the next in shared memory: whole 16-byte pieces.
+__host__ __device__ constexpr int product_ld(int K) { return (K + 3) / 4 * 4; }
+static size_t product_smem(int tok, int K) {
+  return ((size_t)tok * product_ld(K) + (size_t)kProductWarps * tok * kColTile) * sizeof(float);
+}
 
-template <typename TW>
+// sum: what the lane finishes, its column of token `warp` (warps beyond the tokens: nothing).
+template <int TOK, typename TW>
 __device__ __forceinline__ void head_product(const float* __restrict__ in_s, int K, const TW* __restrict__ w, int cols,
-                                             int col, float* __restrict__ red, float (&sum)[kTokTile / kProductWarps]) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int per = (K + kProductWarps - 1) / kProductWarps, k0 = warp * per, k1 = min(K, k0 + per);
-  float acc[kTokTile];
+                                             int col, float* __restrict__ red, float& sum) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ld = product_ld(K);
+  const int per = ((K + kProductWarps - 1) / kProductWarps + 3) / 4 * 4, k0 = min(K, warp * per), k1 = min(K, k0 + per);
+  float acc[TOK];
 #pragma unroll
-  for (int tt = 0; tt < kTokTile; ++tt) acc[tt] = 0.f;
+  for (int tt = 0; tt < TOK; ++tt) acc[tt] = 0.f;
   if (col < cols) {
-    for (int k = k0; k < k1; ++k) {
-      const float wv = to_float(w[(size_t)k * cols + col]);
+    constexpr int AHEAD = 16;
+    for (int k = k0; k < k1; k += AHEAD) {
+      float wv[AHEAD];
 #pragma unroll
-      for (int tt = 0; tt < kTokTile; ++tt) acc[tt] += in_s[tt * K + k] * wv;
+      for (int x = 0; x < AHEAD; ++x) wv[x] = k + x < k1 ? to_float(w[(size_t)(k + x) * cols + col]) : 0.f;
+#pragma unroll
+      for (int x = 0; x < AHEAD; x += 4) {
+        if (k + x >= k1) break;                             // (the inputs behind K are zero)
+#pragma unroll
+        for (int tt = 0; tt < TOK; ++tt) {
+          const float4 v = *reinterpret_cast<const float4*>(in_s + tt * ld + k + x);
+          acc[tt] += v.x * wv[x];
+          acc[tt] += v.y * wv[x + 1];
+          acc[tt] += v.z * wv[x + 2];
+          acc[tt] += v.w * wv[x + 3];
+        }
+      }
     }
   }
 #pragma unroll
-  for (int tt = 0; tt < kTokTile; ++tt) red[(warp * kTokTile + tt) * kColTile + lane] = acc[tt];
+  for (int tt = 0; tt < TOK; ++tt) red[(warp * TOK + tt) * kColTile + lane] = acc[tt];
   __syncthreads();
+  sum = 0.f;
+  if (warp < TOK) {
 #pragma unroll
-  for (int i = 0; i < kTokTile / kProductWarps; ++i) {      // this warp finishes four of the sixteen tokens
-    const int tt = warp * (kTokTile / kProductWarps) + i;
-    float v = 0.f;
-#pragma unroll
-    for (int ww = 0; ww < kProductWarps; ++ww) v += red[(ww * kTokTile + tt) * kColTile + lane];
-    sum[i] = v;
+    for (int ww = 0; ww < kProductWarps; ++ww) sum += red[(ww * TOK + warp) * kColTile + lane];
   }
 }
 
 // Block (token tile, head, 32 columns of the latent).  q row: heads x [dim unrotated | rot rotated].
 // uk: [heads, dim, rank].  q_out: float32 [T, heads, rank + rot]; the blocks of the first columns also rotate.
-template <typename TP, typename TW>
+template <int TOK, typename TP, typename TW>
 __global__ void __launch_bounds__(kProductWarps * 32)
 latent_absorb_kernel(const TP* __restrict__ proj, long long ldp, const TW* __restrict__ uk,
                      const float* __restrict__ cos_t, const float* __restrict__ sin_t, int pairs, int halves,
                      float* __restrict__ q_out, int T, int heads, int dim, int rot, int rank) {
   pdl_wait();        // launched as a dependent of the kernel ahead: nothing is read before it has finished
   pdl_trigger();
-  extern __shared__ float sh[];                              // [kTokTile][dim] | [warps][kTokTile][32]
+  extern __shared__ __align__(16) float sh[];                // [TOK][ld] | [warps][TOK][32]
+  const int ld = product_ld(dim);
   float* q_s = sh;
-  float* red = sh + kTokTile * dim;
-  const int t0 = blockIdx.x * kTokTile, h = blockIdx.y;
-  const int n = min(kTokTile, T - t0);
-  for (int idx = threadIdx.x; idx < kTokTile * dim; idx += blockDim.x) {
-    const int tt = idx / dim, d = idx - tt * dim;
-    q_s[idx] = tt < n ? to_float(proj[(size_t)(t0 + tt) * ldp + (size_t)h * (dim + rot) + d]) : 0.f;
+  float* red = sh + TOK * ld;
+  const int t0 = blockIdx.x * TOK, h = blockIdx.y;
+  const int n = min(TOK, T - t0);
+  for (int idx = threadIdx.x; idx < TOK * ld; idx += blockDim.x) {
+    const int tt = idx / ld, d = idx - tt * ld;
+    q_s[idx] = tt < n && d < dim ? to_float(proj[(size_t)(t0 + tt) * ldp + (size_t)h * (dim + rot) + d]) : 0.f;
   }
   __syncthreads();
   const int qd = rank + rot, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.z * kColTile + lane;
-  float sum[kTokTile / kProductWarps];
-  head_product(q_s, dim, uk + (size_t)h * dim * rank, rank, col, red, sum);
-#pragma unroll
-  for (int i = 0; i < kTokTile / kProductWarps; ++i) {
-    const int tt = warp * (kTokTile / kProductWarps) + i;
-    if (tt < n && col < rank) q_out[((size_t)(t0 + tt) * heads + h) * qd + col] = sum[i];
-  }
+  float sum;
+  head_product<TOK>(q_s, dim, uk + (size_t)h * dim * rank, rank, col, red, sum);
+  if (warp < n && col < rank) q_out[((size_t)(t0 + warp) * heads + h) * qd + col] = sum;
   if (blockIdx.z != 0) return;
   for (int idx = threadIdx.x; idx < n * rot; idx += blockDim.x) {
     const int tt = idx / rot, i = idx - tt * rot, t = t0 + tt;
@@ -141,43 +154,41 @@ latent_absorb_kernel(const TP* __restrict__ proj, long long ldp, const TW* __res
 
 // Block (token tile, head, 32 value columns).  o_lat: float32 [T, heads, rank]; uv_t: [heads, rank, dv] (the up
 // projection of the values, transposed per head); gate: column g_off + h of the projection row, or none.
-template <typename TP, typename TW, typename TA>
+template <int TOK, typename TP, typename TW, typename TA>
 __global__ void __launch_bounds__(kProductWarps * 32)
 latent_expand_kernel(const float* __restrict__ o_lat, const TW* __restrict__ uv_t, const TP* __restrict__ proj,
                      long long ldp, int g_off, TA* __restrict__ out, int T, int heads, int rank, int dv) {
   pdl_wait();        // launched as a dependent of the kernel ahead: nothing is read before it has finished
   pdl_trigger();
-  extern __shared__ __align__(16) float sh[];                // [kTokTile][rank] | [warps][kTokTile][32]
+  extern __shared__ __align__(16) float sh[];                // [TOK][ld] | [warps][TOK][32]
+  const int ld = product_ld(rank);
   float* o_s = sh;
-  float* red = sh + kTokTile * rank;
-  const int t0 = blockIdx.x * kTokTile, h = blockIdx.y;
-  const int n = min(kTokTile, T - t0);
+  float* red = sh + TOK * ld;
+  const int t0 = blockIdx.x * TOK, h = blockIdx.y;
+  const int n = min(TOK, T - t0);
   if (rank % 4 == 0) {          // 16-byte pieces: a quarter of the trips to memory
     const int r4 = rank / 4;
-    for (int idx = threadIdx.x; idx < kTokTile * r4; idx += blockDim.x) {
+    for (int idx = threadIdx.x; idx < TOK * r4; idx += blockDim.x) {
       const int tt = idx / r4, r = (idx - tt * r4) * 4;
       const float4 v = tt < n ? *reinterpret_cast<const float4*>(o_lat + ((size_t)(t0 + tt) * heads + h) * rank + r)
                               : make_float4(0.f, 0.f, 0.f, 0.f);
       *reinterpret_cast<float4*>(o_s + tt * rank + r) = v;
     }
   } else {
-    for (int idx = threadIdx.x; idx < kTokTile * rank; idx += blockDim.x) {
-      const int tt = idx / rank, r = idx - tt * rank;
-      o_s[idx] = tt < n ? o_lat[((size_t)(t0 + tt) * heads + h) * rank + r] : 0.f;
+    for (int idx = threadIdx.x; idx < TOK * ld; idx += blockDim.x) {
+      const int tt = idx / ld, r = idx - tt * ld;
+      o_s[idx] = tt < n && r < rank ? o_lat[((size_t)(t0 + tt) * heads + h) * rank + r] : 0.f;
     }
   }
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int col = blockIdx.z * kColTile + lane;
-  float sum[kTokTile / kProductWarps];
-  head_product(o_s, rank, uv_t + (size_t)h * rank * dv, dv, col, red, sum);
-#pragma unroll
-  for (int i = 0; i < kTokTile / kProductWarps; ++i) {
-    const int tt = warp * (kTokTile / kProductWarps) + i;
-    if (tt >= n || col >= dv) continue;
+  float sum;
+  head_product<TOK>(o_s, rank, uv_t + (size_t)h * rank * dv, dv, col, red, sum);
+  if (warp < n && col < dv) {
     float g = 1.f;
-    if (g_off >= 0) g = 1.f / (1.f + expf(-to_float(proj[(size_t)(t0 + tt) * ldp + g_off + h])));
-    out[((size_t)(t0 + tt) * heads + h) * dv + col] = from_float<TA>(sum[i] * g);
+    if (g_off >= 0) g = 1.f / (1.f + expf(-to_float(proj[(size_t)(t0 + warp) * ldp + g_off + h])));
+    out[((size_t)(t0 + warp) * heads + h) * dv + col] = from_float<TA>(sum * g);
   }
 }
 
@@ -294,14 +305,23 @@ extern "C" int srlm_latent_absorb(const void* proj, int proj_dtype, long long ld
                                   const float* cos_t, const float* sin_t, int pairs, int halves, float* q_out, int T, int heads,
                                   int dim, int rot, int rank, cudaStream_t stream) {
   if (T <= 0) return ST_OK;
-  const size_t smem = ((size_t)kTokTile * dim + (size_t)kProductWarps * kTokTile * kColTile) * sizeof(float);
-  if (heads <= 0 || heads > 65535 || dim <= 0 || rank <= 0 || rot < 0 || 2 * pairs > rot || smem > 48 * 1024 ||
+  if (heads <= 0 || heads > 65535 || dim <= 0 || dim > 640 || rank <= 0 || rot < 0 || 2 * pairs > rot ||
       ldp < (long long)heads * (dim + rot) || (pairs > 0 && (!cos_t || !sin_t)))
     return refuse(ST_BAD_SIZE, "latent_absorb: heads=%d dim=%d rot=%d rank=%d pairs=%d ldp=%lld", heads, dim, rot, rank,
                   pairs, ldp);
-  dim3 grid((T + kTokTile - 1) / kTokTile, heads, (rank + kColTile - 1) / kColTile);
-  SRLM_LATENT_TYPES(proj_dtype, w_dtype, (launch_pdl(latent_absorb_kernel<TP, TW>, dim3(grid), dim3(kProductWarps * 32), smem, stream, 
-      (const TP*)proj, ldp, (const TW*)uk, cos_t, sin_t, pairs, halves, q_out, T, heads, dim, rot, rank)));
+  const int tok = T <= 8 ? 8 : 16;
+  const size_t smem = product_smem(tok, dim);
+  dim3 grid((T + tok - 1) / tok, heads, (rank + kColTile - 1) / kColTile);
+#define SRLM_ABSORB(TOK)                                                                                         \
+  do {                                                                                                           \
+    auto kern = latent_absorb_kernel<TOK, TP, TW>;                                                               \
+    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+    launch_pdl(kern, grid, dim3(kProductWarps * 32), smem, stream, (const TP*)proj, ldp, (const TW*)uk, cos_t, sin_t, pairs,  \
+               halves, q_out, T, heads, dim, rot, rank);                                                         \
+  } while (0)
+  if (tok == 8) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_ABSORB(8));
+  else SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_ABSORB(16));
+#undef SRLM_ABSORB
   return launched();
 }
 
@@ -309,19 +329,22 @@ extern "C" int srlm_latent_expand(const float* o_lat, const void* uv_t, int w_dt
                                   long long ldp, int g_off, void* out, int out_dtype, int T, int heads, int rank,
                                   int dv, cudaStream_t stream) {
   if (T <= 0) return ST_OK;
-  const size_t smem = ((size_t)kTokTile * rank + (size_t)kProductWarps * kTokTile * kColTile) * sizeof(float);
-  if (heads <= 0 || heads > 65535 || rank <= 0 || dv <= 0 || smem > 200 * 1024 || (g_off >= 0 && ldp < g_off + heads))
+  if (heads <= 0 || heads > 65535 || rank <= 0 || rank > 3072 || dv <= 0 || (g_off >= 0 && ldp < g_off + heads))
     return refuse(ST_BAD_SIZE, "latent_expand: heads=%d rank=%d dv=%d g_off=%d ldp=%lld", heads, rank, dv, g_off, ldp);
-  dim3 grid((T + kTokTile - 1) / kTokTile, heads, (dv + kColTile - 1) / kColTile);
-#define SRLM_EXPAND(TA)                                                                                          \
+  const int tok = T <= 8 ? 8 : 16;
+  const size_t smem = product_smem(tok, rank);
+  dim3 grid((T + tok - 1) / tok, heads, (dv + kColTile - 1) / kColTile);
+#define SRLM_EXPAND(TOK, TA)                                                                                     \
   do {                                                                                                           \
-    auto kern = latent_expand_kernel<TP, TW, TA>;                                                                \
+    auto kern = latent_expand_kernel<TOK, TP, TW, TA>;                                                              \
     if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
     launch_pdl(kern, dim3(grid), dim3(kProductWarps * 32), smem, stream, o_lat, (const TW*)uv_t, (const TP*)proj, ldp, g_off, (TA*)out, T, heads,   \
                                       rank, dv);                                                                 \
   } while (0)
-  if (out_dtype == DT_F32) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_EXPAND(float));
-  else if (out_dtype == DT_BF16) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_EXPAND(bf16));
+  if (out_dtype == DT_F32 && tok == 8) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_EXPAND(8, float));
+  else if (out_dtype == DT_F32) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_EXPAND(16, float));
+  else if (out_dtype == DT_BF16 && tok == 8) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_EXPAND(8, bf16));
+  else if (out_dtype == DT_BF16) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_EXPAND(16, bf16));
   else return refuse(ST_BAD_DTYPE, "latent_expand: output dtype %d", out_dtype);
 #undef SRLM_EXPAND
   return launched();

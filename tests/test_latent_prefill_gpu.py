@@ -99,3 +99,28 @@ def test_prompts_against_float64(page, window, heads, pairs, interleaved, gated)
     # weights and the result are rounded to 8 bits of mantissa (2^-9 each way): a value is a mean of N(0, 1) values under weights
     # that are off by 2^-9 of themselves, then off by 2^-9 of itself
     assert (got - ref).abs().max() <= 2.0 ** -8 * (1.0 + ref.abs().max())
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 40])
+@pytest.mark.parametrize("dim, rot, rank, dv", [(128, 64, 512, 128), (12, 6, 20, 9), (64, 0, 130, 33), (3, 2, 5, 1)])
+def test_the_per_head_products(T, dim, rot, rank, dv):
+    """The up projections folded into the queries and applied behind the attention: token tiles of 8 and 16, sizes that are no
+    whole pieces, columns beyond a block's 32; a token's result does not depend on its neighbours."""
+    from safetyraise_lmengine_b200.kernels import ops
+    g = torch.Generator().manual_seed(T + dim)
+    heads = 3
+    q = torch.randn(T, heads * (dim + rot) + heads, generator=g)
+    uk, uv = torch.randn(heads, dim, rank, generator=g).bfloat16(), torch.randn(heads, rank, dv, generator=g).bfloat16()
+    out = torch.empty(T, heads * (rank + rot), device=DEV)
+    ops.latent_absorb(q.to(DEV), uk.to(DEV), None, out, heads, dim, rot, rank)
+    x = q[:, :heads * (dim + rot)].view(T, heads, dim + rot).double()
+    ref = torch.cat([torch.einsum("thd,hdr->thr", x[..., :dim], uk.double()), x[..., dim:]], -1)
+    assert (out.cpu().double().view(ref.shape) - ref).abs().max() <= 1e-5 * ref.abs().max()
+    o = torch.randn(T, heads * rank, generator=g)
+    got = torch.empty(T, heads * dv, device=DEV)
+    ops.latent_expand(o.to(DEV), uv.to(DEV), q.to(DEV), heads * (dim + rot), got, heads, rank, dv)
+    ref = torch.einsum("thr,hrc->thc", o.view(T, heads, rank).double(), uv.double()) * torch.sigmoid(q[:, -heads:].double())[:, :, None]
+    assert (got.cpu().double().view(ref.shape) - ref).abs().max() <= 1e-5 * ref.abs().max()
+    one = torch.empty(1, heads * dv, device=DEV)
+    ops.latent_expand(o[T - 1:].contiguous().to(DEV), uv.to(DEV), q[T - 1:].contiguous().to(DEV), heads * (dim + rot), one, heads, rank, dv)
+    assert torch.equal(one[0], got[T - 1])
