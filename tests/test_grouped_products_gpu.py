@@ -1,0 +1,58 @@
+"""The grouped products of few rows an expert (mma.sync), the gather, the combination and the clamped GLU at the edges of
+their tiles and vectors, against float64 loops."""
+import pytest
+import torch
+
+from safetyraise_lmengine_b200.kernels import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("K", [8, 56, 64, 72, 264])          # around a slab of 64 and past the ring of four
+@pytest.mark.parametrize("counts", [(1, 0, 16, 17), (32, 33, 48, 63), (64, 65, 0, 81)])
+def test_rows_around_the_groups_of_sixteen(counts, K):
+    g = torch.Generator().manual_seed(K + counts[0])
+    E, N, n = len(counts), 136, sum(counts)
+    choice = torch.cat([torch.full((c,), e, dtype=torch.int32) for e, c in enumerate(counts)])[torch.randperm(n, generator=g)]
+    x = torch.randn(n, K, generator=g).bfloat16()
+    w = torch.randn(E, N, K, generator=g).bfloat16()
+    heads = torch.zeros(2, E + 1, dtype=torch.int32, device=DEV)
+    por, rop = (torch.zeros(n, dtype=torch.int32, device=DEV) for _ in range(2))
+    ops.moe_sort(choice[:, None].to(DEV), E, heads[0], heads[1], por, rop)
+    out = torch.full((n, N), float("nan"), device=DEV)
+    ops.moe_grouped(x.to(DEV), por, 1, w.to(DEV), out, heads[0], heads[1])
+    got = out[rop.long()].cpu().double()
+    for i in range(n):
+        a, b = x[i].double(), w[int(choice[i])].double()
+        # float32 sums of exact products: at most K roundings of the sum of the products' sizes
+        assert ((got[i] - b @ a).abs() <= K * 2.0 ** -23 * (b.abs() @ a.abs())).all(), i
+
+
+@pytest.mark.parametrize("act", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,H,top", [(1, 4, 1), (3, 508, 4), (2, 512, 5), (5, 516, 9), (3, 515, 2)])
+def test_combination_and_gather_and_activation(act, T, H, top):
+    g = torch.Generator().manual_seed(H + top)
+    n = T * top
+    rows = torch.randn(n + 3, H, generator=g)
+    rop = torch.randperm(n + 3, generator=g)[:n].to(torch.int32).reshape(T, top)
+    rop[0, top - 1] = -1                                      # a pair without a row
+    weight, shared = torch.rand(T, top, generator=g), torch.randn(T, H, generator=g).to(act)
+    out = torch.empty(T, H, dtype=act, device=DEV)
+    ops.moe_combine(rows.to(DEV), rop.to(DEV), weight.to(DEV), shared.to(DEV), out)
+    w = torch.where(rop >= 0, weight, 0.).double()
+    terms = w[..., None] * rows.double()[rop.clamp(min=0).long()]
+    want, size = terms.sum(1) + shared.double(), terms.abs().sum(1) + shared.double().abs()
+    step = 2.0 ** -24 if act == torch.float32 else 2.0 ** -8  # half the spacing of 24- and 8-bit significands over their least value
+    assert ((out.cpu().double() - want).abs() <= (top + 2) * 2.0 ** -24 * size + step * want.abs()).all()
+    got = torch.empty(T, H, device=DEV)
+    both = torch.randn(T, 2 * H, generator=g)
+    ops.clamped_glu(both.to(DEV), got, 1.2, 1.702)
+    gate, up = both[:, :H].double().clamp(max=1.2), both[:, H:].double().clamp(-1.2, 1.2)
+    assert torch.allclose(got.cpu().double(), gate * torch.sigmoid(1.702 * gate) * (up + 1), rtol=2e-6, atol=1e-9)
+    if H % 4 == 0:
+        x = torch.randn(T, 2 * H, generator=g).bfloat16()     # rows of a multiple of 8
+        pair = torch.tensor([*range(n), -1], dtype=torch.int32)
+        xs = torch.empty(n + 1, 2 * H, dtype=torch.bfloat16, device=DEV)
+        ops.moe_gather_rows(x.to(DEV), pair.to(DEV), top, xs)
+        assert torch.equal(xs.cpu(), torch.cat([x.repeat_interleave(top, 0), torch.zeros(1, 2 * H).bfloat16()]))
