@@ -20,8 +20,6 @@
 //          A channel's sums do not depend on what else is in the step or on how the tokens were cut into steps.
 #include <math_constants.h>
 
-#include <type_traits>
-
 #include "common.cuh"
 
 namespace srlm {
@@ -164,6 +162,10 @@ __device__ __forceinline__ void scan_cp_async_4(float* dst, const float* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src));
 }
+__device__ __forceinline__ void scan_cp_async_16(float* dst, const float* src) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src));
+}
 __device__ __forceinline__ void scan_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void scan_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -195,21 +197,32 @@ __device__ __forceinline__ void scan_load_row(const float* src, float (&dst)[NPL
 }
 
 // A chunk of 16 tokens lies in shared memory while the block walks it: B and C of every token, zero behind N up to
-// the lanes' reach; per (token, channel) dt (raw, then its softplus), x, z; and the block's y ahead of the gate.
-// Places behind an entry's last token hold dt = 0, x = 0, B = 0: S <- fma(1, S, 0) leaves every state as it is, so
-// the walk has no branch.
+// the lanes' reach; per (token, channel) the raw dt, x and z, each a plane of its own; per (token, channel) the pair of
+// the step size and its product with x; and the block's y ahead of the gate.  Places behind an entry's last token hold
+// dt = 0, dt x = 0, B = 0: S <- fma(1, S, 0) leaves every state as it is, so the walk has no branch.
 //
 // The block's first four warps walk; its other four fetch, prepare and finish.  While the walkers are on chunk j the
-// helpers wait for chunk j + 1 (cp.async), turn its raw step sizes into softplus(dt + bias), gate and write the y of
-// chunk j - 1, and issue the fetch of chunk j + K - 1 into the buffer chunk j - 1 has left: K buffers of operands
-// (a fetch has K - 2 walks of a chunk to arrive: a chunk's walk is shorter than a trip to DRAM), two of y, one
-// barrier a chunk.  Every round commits one group of copies, an empty one behind the entry's end, so that "all but
-// the last K - 3 groups" always names chunk j + 1.  A helper prepares and finishes exactly the (token, channel)
-// places it fetched, so only the barrier orders helpers and walkers.
+// helpers turn the raw step sizes of chunk j + 1 into softplus(dt + bias) and its product with x, gate and write the y
+// of chunk j - 1, issue the fetch of chunk j + K - 2 into the buffer chunk j - 2 has left, and wait until their own
+// copies of chunk j + 2 have landed: K buffers of operands (a fetch has K - 4 walks of a chunk to arrive: a chunk's walk
+// is about as long as a trip to DRAM), two of the pairs and of y, one barrier a chunk.  Every round commits one group of
+// copies, an empty one behind the entry's end, so that "all but the last K - 4 groups" always names chunk j + 2.  A
+// helper reads what other helpers fetched, and overwrites what other helpers read, only with a barrier in between.
+//
+// Bound by the SM's instructions, walkers and helpers together: 2,048 tokens, 4,096 channels of 16 states 131 us (with
+// the helpers copying four bytes at a time, (token, channel) by (token, channel), and reading bias and D for each,
+// 227 us at 3,570 cycles a chunk).
 constexpr int kScanWalkers = kScanLanes * kScanChannels, kScanThreads = 2 * kScanWalkers;
-constexpr int scan_buffers(int npl) { return npl <= 2 ? 6 : npl <= 4 ? 5 : 4; }
+constexpr int scan_buffers(int npl) { return npl <= 2 ? 8 : npl <= 4 ? 7 : npl <= 8 ? 6 : 5; }
+constexpr int kScanPlane = kScanChunk * kScanChannels;
+// floats of shared memory: the buffers (B | C up to the lanes' reach, three planes), two of pairs, two of y
+constexpr int scan_floats(int npl) {
+  return scan_buffers(npl) * (kScanChunk * 2 * npl * kScanLanes + 3 * kScanPlane) + 2 * 2 * kScanPlane + 2 * kScanPlane;
+}
+__device__ __forceinline__ void scan_helpers_meet() { asm volatile("bar.sync 1, %0;" ::"n"(kScanWalkers) : "memory"); }
 
-template <typename TO, int NPL>
+// WIDE: channels, N, the rows and the pointers allow copies of 16 bytes
+template <typename TO, int NPL, bool WIDE>
 __global__ void __launch_bounds__(kScanThreads)
 selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz, long long ld_xz,
                       const float* __restrict__ dbc, long long ld_dbc, int b_off, const float* __restrict__ dt_raw,
@@ -218,13 +231,14 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
                       const int* __restrict__ slots, TO* __restrict__ out, int channels, int N, int taps) {
   constexpr int NP = NPL * kScanLanes;                      // states a channel's lanes reach, >= N
   constexpr int GROUP = NPL <= 2 ? 8 : NPL <= 4 ? 4 : 2;    // tokens whose independent work the compiler interleaves
-  constexpr int BC = kScanChunk * 2 * NP, TOK = kScanChunk * kScanChannels * 4, YS = kScanChunk * kScanChannels;
+  constexpr int BC = kScanChunk * 2 * NP, YS = kScanPlane;
   constexpr int K = scan_buffers(NPL);
   pdl_wait();
   extern __shared__ __align__(16) float scan_smem[];
   float* bc_s = scan_smem;                                  // [K][chunk][2 NP]: B, then C
-  float* tok_s = bc_s + K * BC;                             // [K][chunk][channels of the block][4]: dt, x, z, -
-  float* y_s = tok_s + K * TOK;                             // [2][chunk][channels of the block]
+  float* raw_s = bc_s + K * BC;                             // [K][3][chunk][channels of the block]: raw dt, x, z
+  float2* step_s = reinterpret_cast<float2*>(raw_s + K * 3 * YS);       // [2][chunk][channels of the block]: dt, dt x
+  float* y_s = reinterpret_cast<float*>(step_s + 2 * YS);   // [2][chunk][channels of the block]
   const int e = blockIdx.y, c0 = blockIdx.x * kScanChannels;
   const bool walker = threadIdx.x < kScanWalkers;
   const int tid = walker ? threadIdx.x : threadIdx.x - kScanWalkers;      // place among the walkers, or among the helpers
@@ -243,48 +257,60 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
     }
     const int base = j * kScanChunk, n_here = min(kScanChunk, q_len - base);
     float* bc = bc_s + (j % K) * BC;
-    float* tk = tok_s + (j % K) * TOK;
-    for (int idx = tid; idx < kScanChunk * 2 * NP; idx += kScanWalkers) {
-      const int i = idx / (2 * NP), r = idx - i * 2 * NP, half = r / NP, n = r - half * NP;
-      if (i < n_here && n < N) scan_cp_async_4(bc + idx, dbc + (size_t)(t0 + base + i) * ld_dbc + b_off + half * N + n);
-      else bc[idx] = 0.f;
-    }
-    for (int idx = tid; idx < kScanChunk * kScanChannels; idx += kScanWalkers) {
-      const int i = idx / kScanChannels, cc = idx - i * kScanChannels;
-      float* dst = tk + (size_t)idx * 4;
-      if (i < n_here && c0 + cc < channels) {
-        const size_t t = (size_t)(t0 + base + i);
-        scan_cp_async_4(dst, dt_raw + t * channels + c0 + cc);
-        scan_cp_async_4(dst + 1, x + t * channels + c0 + cc);
-        scan_cp_async_4(dst + 2, xz + t * ld_xz + channels + c0 + cc);
+    float* raw = raw_s + (j % K) * 3 * YS;
+    constexpr int V = WIDE ? 4 : 1;                         // floats a copy
+    for (int idx = tid; idx < BC / V; idx += kScanWalkers) {
+      const int i = idx / (2 * NP / V), r = idx % (2 * NP / V) * V, half = r / NP, n = r % NP;
+      float* dst = bc + idx * V;
+      if (i < n_here && n < N) {
+        const float* src = dbc + (size_t)(t0 + base + i) * ld_dbc + b_off + half * N + n;
+        if constexpr (WIDE) scan_cp_async_16(dst, src);
+        else scan_cp_async_4(dst, src);
       } else {
-        dst[0] = dst[1] = dst[2] = 0.f;
+#pragma unroll
+        for (int u = 0; u < V; ++u) dst[u] = 0.f;
       }
+    }
+    for (int idx = tid; idx < YS / V; idx += kScanWalkers) {
+      const int i = idx / (kScanChannels / V), cc = idx % (kScanChannels / V) * V;
+      if (i >= n_here || c0 + cc >= channels) continue;
+      const size_t t = (size_t)(t0 + base + i);
+      const float* from[3] = {dt_raw + t * channels + c0 + cc, x + t * channels + c0 + cc, xz + t * ld_xz + channels + c0 + cc};
+#pragma unroll
+      for (int p = 0; p < 3; ++p)
+        if constexpr (WIDE) scan_cp_async_16(raw + p * YS + idx * V, from[p]);
+        else scan_cp_async_4(raw + p * YS + idx * V, from[p]);
     }
     scan_cp_async_commit();
   };
-  // helpers: the step sizes of chunk j, once it has landed (a helper's own copies: no barrier between); `behind`
-  // groups were committed after the chunk's own
-  auto prepare = [&](int j, auto behind) {
+  // a helper's channel is the same at all its (token, channel) places
+  const int hc = c0 + tid % kScanChannels;
+  const float bias = !walker && dt_bias && hc < channels ? dt_bias[hc] : 0.f, skip = !walker && hc < channels ? D[hc] : 0.f;
+  // helpers: the step sizes of chunk j, all of whose copies have landed and were waited for ahead of a barrier
+  auto prepare = [&](int j) {
     const int n_here = min(kScanChunk, q_len - j * kScanChunk);
-    float* tk = tok_s + (j % K) * TOK;
-    scan_cp_async_wait<decltype(behind)::value>();
-    for (int idx = tid; idx < kScanChunk * kScanChannels; idx += kScanWalkers) {
-      const int i = idx / kScanChannels, cc = idx - i * kScanChannels;
-      if (i < n_here && c0 + cc < channels) tk[idx * 4] = softplus_f(tk[idx * 4] + (dt_bias ? dt_bias[c0 + cc] : 0.f));
+    const float* raw = raw_s + (j % K) * 3 * YS;
+    float2* step = step_s + (j & 1) * YS;
+#pragma unroll
+    for (int u = 0; u < YS / kScanWalkers; ++u) {
+      const int idx = tid + u * kScanWalkers;
+      const bool on = idx / kScanChannels < n_here && hc < channels;
+      const float dt = on ? softplus_f(raw[idx] + bias) : 0.f;
+      step[idx] = make_float2(dt, on ? dt * raw[YS + idx] : 0.f);
     }
   };
   // helpers: y of chunk j, gated and written: out = (y + D x) * silu(z)
   auto finish = [&](int j) {
     const int base = j * kScanChunk, n_here = min(kScanChunk, q_len - base);
-    const float* tk = tok_s + (j % K) * TOK;
+    const float* raw = raw_s + (j % K) * 3 * YS;
     const float* ys = y_s + (j & 1) * YS;
-    for (int idx = tid; idx < n_here * kScanChannels; idx += kScanWalkers) {
-      const int i = idx / kScanChannels, cc = idx - i * kScanChannels;
-      if (c0 + cc < channels) {
-        const float xv = tk[idx * 4 + 1], z = tk[idx * 4 + 2];
-        out[(size_t)(t0 + base + i) * channels + c0 + cc] = from_float<TO>((ys[idx] + D[c0 + cc] * xv) * silu_f(z));
-      }
+    if (hc >= channels) return;
+#pragma unroll
+    for (int u = 0; u < YS / kScanWalkers; ++u) {
+      const int idx = tid + u * kScanWalkers;
+      const int i = idx / kScanChannels;
+      if (i < n_here)
+        out[(size_t)(t0 + base + i) * channels + hc] = from_float<TO>((ys[idx] + skip * raw[YS + idx]) * silu_f(raw[2 * YS + idx]));
     }
   };
 
@@ -298,20 +324,23 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
       a[k] = on ? A[(size_t)c * N + n] * kLog2e : 0.f;      // exp(dt A) = 2^(dt A log2 e)
     }
   } else if (n_chunks > 0) {
-    for (int j = 0; j < K - 1; ++j) stage(j);
-    prepare(0, std::integral_constant<int, K - 2>());
+    for (int j = 0; j < K - 2; ++j) stage(j);
+    scan_cp_async_wait<K - 4>();                            // the helper's own copies of chunks 0 and 1
+    scan_helpers_meet();
+    prepare(0);
   }
   for (int j = 0; j < n_chunks; ++j) {
-    __syncthreads();       // chunk j lies prepared; the walk over chunk j - 1 is over and its y lies in its buffer
+    __syncthreads();       // chunk j lies prepared, chunk j + 1 has landed; the y of chunk j - 1 lies in its buffer
     if (!walker) {
-      if (j + 1 < n_chunks) prepare(j + 1, std::integral_constant<int, K - 3>());
+      stage(j + K - 2);                                     // into the buffer of chunk j - 2, which was finished in round j - 1
+      if (j + 1 < n_chunks) prepare(j + 1);
       if (j > 0) finish(j - 1);
-      stage(j + K - 1);                                     // into the buffer of chunk j - 1
+      scan_cp_async_wait<K - 4>();
       continue;
     }
     const int n_here = min(kScanChunk, q_len - j * kScanChunk);
     const float* bc = bc_s + (j % K) * BC;
-    const float* tk = tok_s + (j % K) * TOK;
+    const float2* step = step_s + (j & 1) * YS;
     float* ys = y_s + (j & 1) * YS;
 #pragma unroll 1
     for (int i0 = 0; i0 < n_here; i0 += GROUP) {
@@ -319,8 +348,8 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
 #pragma unroll
       for (int u = 0; u < GROUP; ++u) {
         const int i = i0 + u;
-        const float4 v = *reinterpret_cast<const float4*>(tk + (size_t)(i * kScanChannels + ch) * 4);
-        const float dt = v.x, dtx = v.x * v.y;
+        const float2 v = step[i * kScanChannels + ch];
+        const float dt = v.x, dtx = v.y;
         float Bv[NPL], Cv[NPL];
         scan_load_row<NPL>(bc + i * 2 * NP + lane * NPL, Bv);
         scan_load_row<NPL>(bc + i * 2 * NP + NP + lane * NPL, Cv);
@@ -506,17 +535,22 @@ extern "C" int srlm_selective_scan(const float* x, const float* xz, long long ld
   int npl = 1;
   while (npl * kScanLanes < N) npl <<= 1;
   const bool early = max_q_len <= 4 * kScanChunk;      // a long walk starts on an empty GPU, its blocks spread evenly
-  // some buffers of a chunk's operands (B | C up to the lanes' reach, four words per (token, channel)), two of the block's y
-  const size_t smem = (size_t)kScanChunk * (scan_buffers(npl) * (2 * npl * kScanLanes + 4 * kScanChannels) + 2 * kScanChannels) * sizeof(float);
-#define SRLM_SCAN(TO, NPL)                                                                                              \
+  // copies of 16 bytes: neither four channels nor four states straddle an edge
+  const bool wide = channels % 4 == 0 && N % 4 == 0 && b_off % 4 == 0 && ld_dbc % 4 == 0 && ld_xz % 4 == 0 &&
+                    ((uintptr_t)x | (uintptr_t)xz | (uintptr_t)dbc | (uintptr_t)dt_raw) % 16 == 0;
+  const size_t smem = (size_t)scan_floats(npl) * sizeof(float);
+#define SRLM_SCAN_AS(TO, NPL, W)                                                                                        \
   do {                                                                                                                  \
-    static bool sized = false;      /* the widest form asks for more shared memory than a kernel gets unasked */        \
-    if (!sized && smem > 48 * 1024) {                                                                                   \
-      cudaFuncSetAttribute(selective_scan_kernel<TO, NPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
-      sized = true;                                                                                                     \
-    }                                                                                                                   \
-    launch_pdl_if(early, selective_scan_kernel<TO, NPL>, grid, dim3(kScanThreads), smem, stream, x, xz, ld_xz, dbc,     \
-                  ld_dbc, b_off, dt_raw, dt_bias, A, D, state, state_stride, cu_q, slots, (TO*)out, channels, N, taps); \
+    auto kern = selective_scan_kernel<TO, NPL, W>;                                                                      \
+    const cudaError_t got = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
+    if (got != cudaSuccess) return refuse((int)got, "selective_scan: cannot get %zu bytes of shared memory", smem);     \
+    launch_pdl_if(early, kern, grid, dim3(kScanThreads), smem, stream, x, xz, ld_xz, dbc, ld_dbc, b_off, dt_raw,        \
+                  dt_bias, A, D, state, state_stride, cu_q, slots, (TO*)out, channels, N, taps);                        \
+  } while (0)
+#define SRLM_SCAN(TO, NPL)                    \
+  do {                                        \
+    if (wide) SRLM_SCAN_AS(TO, NPL, true);    \
+    else SRLM_SCAN_AS(TO, NPL, false);        \
   } while (0)
 #define SRLM_SCAN_N(TO)                                   \
   switch (npl) {                                          \
@@ -531,6 +565,7 @@ extern "C" int srlm_selective_scan(const float* x, const float* xz, long long ld
   else return refuse(ST_BAD_DTYPE, "selective_scan: output dtype %d", out_dtype);
 #undef SRLM_SCAN_N
 #undef SRLM_SCAN
+#undef SRLM_SCAN_AS
   return launched();
 }
 
