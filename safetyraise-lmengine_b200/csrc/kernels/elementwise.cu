@@ -41,6 +41,48 @@ __global__ void embed_gather_kernel(const int* __restrict__ ids, const TW* __res
   }
 }
 
+// The same, four columns a thread and four such pieces in flight (H a multiple of 4, rows aligned to four elements): 2,048
+// rows of 4,096 9.8 us, one row 2.1 (one column a thread: 21.5 and 4.8).
+__device__ __forceinline__ float4 embed_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 embed_load4(const bf16* p) {
+  const uint2 v = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.x));
+  const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+template <typename TW>
+__global__ void embed_gather_vec_kernel(const int* __restrict__ ids, const TW* __restrict__ table, float* __restrict__ out,
+                                        int H, int vocab, int* __restrict__ bad, float scale, int add) {
+  pdl_wait();
+  pdl_trigger();
+  constexpr int AHEAD = 4;
+  const int t = blockIdx.x, id = ids[t], pieces = H / 4;
+  const bool known = id >= 0 && id < vocab;
+  if (!known && threadIdx.x == 0) atomicExch(bad, 1);
+  if (!known && add) return;
+  const TW* row = table + (size_t)(known ? id : 0) * H;
+  float4* to = reinterpret_cast<float4*>(out + (size_t)t * H);
+  for (int p0 = threadIdx.x; p0 < pieces; p0 += AHEAD * blockDim.x) {
+    float4 v[AHEAD];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      const int p = p0 + i * blockDim.x;
+      v[i] = known && p < pieces ? embed_load4(row + 4 * p) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      const int p = p0 + i * blockDim.x;
+      if (p >= pieces) continue;
+      if (add) {
+        const float4 o = to[p];
+        to[p] = make_float4(o.x + v[i].x * scale, o.y + v[i].y * scale, o.z + v[i].z * scale, o.w + v[i].w * scale);
+      } else {
+        to[p] = known ? make_float4(v[i].x * scale, v[i].y * scale, v[i].z * scale, v[i].w * scale) : v[i];
+      }
+    }
+  }
+}
+
 // x = residual[src] (+ delta_scale * delta[src]); residual[src] = x when rows == nullptr;
 // out[r] = x * rsqrt(mean(x^2) + eps) * (w (+1)).  CENTER: the mean of the row is taken off x first (layer norm: the
 // residual keeps it), so that the second moment is the variance.
@@ -272,8 +314,14 @@ extern "C" int srlm_embed_gather(const int* ids, const void* table, int table_dt
   if (T <= 0) return ST_OK;
   if (H <= 0 || vocab <= 0) return refuse(ST_BAD_SIZE, "embed_gather: H=%d vocab=%d", H, vocab);
   const int block = H >= 1024 ? 256 : 128;
-  SRLM_DISPATCH_ACT(table_dtype, TW, launch_pdl(embed_gather_kernel<TW>, dim3(T), dim3(block), 0, stream,
-      ids, (const TW*)table, out, H, vocab, bad_flag, scale, add));
+  SRLM_DISPATCH_ACT(table_dtype, TW, {
+    if (H % 4 == 0 && (uintptr_t)table % (4 * sizeof(TW)) == 0 && (uintptr_t)out % 16 == 0)
+      launch_pdl(embed_gather_vec_kernel<TW>, dim3(T), dim3(block), 0, stream, ids, (const TW*)table, out, H, vocab, bad_flag,
+                 scale, add);
+    else
+      launch_pdl(embed_gather_kernel<TW>, dim3(T), dim3(block), 0, stream, ids, (const TW*)table, out, H, vocab, bad_flag,
+                 scale, add);
+  });
   return launched();
 }
 
