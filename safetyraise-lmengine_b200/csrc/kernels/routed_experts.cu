@@ -646,12 +646,9 @@ extern "C" int srlm_moe_look_up(const int* ids, const int* table, int vocab, int
 // start at a multiple of it; group_of_tile [max_tiles >= (n + E * (tile_rows - 1)) / tile_rows] names each tile's
 // expert (-1: none) and pair_of_row has rows_cap >= max_tiles * tile_rows entries (-1: no pair).
 // logits (float32 [n / top, ld >= E], with bias [E] or null) given: the kernel routes the tokens first and
-// writes choice and weight [n / top, top] itself; taken up to 512 tokens and 256 experts, and the better form up to 32
-// tokens (srlm_moe_sort_routes), which its one block of 32 warps routes at once.  Every 32 more cost it some 4 us, a kernel
-// of its own 4 us and a launch in all: a step of 33 tokens (top 4 of 16 experts) 79.7 us against 76.9, of 64 85.8 against
-// 81.0; the two kernels alone at 200 tokens 29 us against 16 + 7 (not waited for).
+// writes choice and weight [n / top, top] itself; offered for E <= 256 (srlm_moe_sort_routes).
 // table (int32 [vocab, top]) with ids (int32 [n / top]) given: likewise, by looking the ids up; every weight weight_scale.
-extern "C" int srlm_moe_sort_routes(int tokens, int E) { return tokens <= 32 && E <= 256; }
+extern "C" int srlm_moe_sort_routes(int tokens, int E) { return tokens <= 512 && E <= 256; }
 
 extern "C" int srlm_moe_sort(int* choice, int n, int E, int* offsets, int* tiles, int* pair_of_row,
                              int* row_of_pair, int tile_rows, int* group_of_tile, int max_tiles, int rows_cap,
@@ -665,7 +662,7 @@ extern "C" int srlm_moe_sort(int* choice, int n, int E, int* offsets, int* tiles
   if (logits)
     if (int r = routing_ok("moe_sort", E, top, scoring, groups, kept)) return r;
   if (correction && (!logits || scoring != 1)) return refuse(ST_BAD_SIZE, "moe_sort: corrected choices come with scoring 1");
-  if (logits && (top <= 0 || top > E || n % top || ld < E || !weight || n / top > 512 || E > 256))
+  if (logits && (top <= 0 || top > E || n % top || ld < E || !weight || !srlm_moe_sort_routes(n / top, E)))
     return refuse(ST_BAD_SIZE, "moe_sort: routing %d pairs, top=%d of %d experts, ld=%lld", n, top, E, ld);
   const int align = tile_rows > 0;
   if (align && (!group_of_tile || (long long)max_tiles < ((long long)n + (long long)E * (tile_rows - 1)) / tile_rows ||

@@ -166,7 +166,7 @@ class RoutedExperts(Part):
         if self.table is not None and pairs <= 4096:   # a small step: the block that orders the pairs looks them up too
             ops.moe_sort(choice, s.experts, offsets, tiles, pair_of_row, row_of_pair,
                          look_up=(ctx.token_ids, self.table, weight), weight_scale=s.weight_scale / s.top)
-        elif self.table is None and ops.moe_sort_routes(T, s.experts):   # likewise, and routes them
+        elif self.table is None and T <= ops.ROUTES_IN_SORT and ops.moe_sort_routes(T, s.experts):   # likewise, and routes them
             ops.moe_sort(choice, s.experts, offsets, tiles, pair_of_row, row_of_pair,
                          route=(first, self.router_column, self.router_bias, weight), **self.routing)
         else:
