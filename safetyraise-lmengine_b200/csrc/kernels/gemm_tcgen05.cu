@@ -224,7 +224,7 @@ struct GemmArgs {
                            //    the first sk_blocks blocks, or pairs of blocks (0: every block takes whole tiles only)
   int m_major;             // persistent kernel: tile t covers token tile t / (tiles along N); else t % (tiles along M)
   GemmFuse fuse;           // one-tile kernel only; all zero: none
-  // persistent kernel, one SM per tile: grouped products.  Token tile mt (128 rows) multiplies the weight rows
+  // persistent kernel, whole tiles: grouped products.  Token tile mt (of the kernel's BN rows) multiplies the weight rows
   // [group_of_mtile[mt] * N, + N) of W (N: weight rows per group); a tile whose entry is negative is skipped.
   const int* group_of_mtile = nullptr;
   // swiglu8 with glu_limit > 0: the output is g * logistic(glu_alpha * g) * (u + 1), g = min(gate, limit),
@@ -1666,9 +1666,15 @@ extern "C" int srlm_gemm_tn_tcgen05_grouped(const void* X, const void* W, void* 
   a.act = act;
   CUtensorMap mw_copy, mx_copy;
   const CUtensorMap *mw = &mw_copy, *mx = &mx_copy;
-  // (the pair form fetches the tokens of a tile in two boxes of 128 rows, one a block)
-  if (!cached_map(&mw_copy, W, (long long)groups * N, K, K, BM, true) || !cached_map(&mx_copy, X, M, K, ldx, 128, false))
+  // Tiles of 128 tokens go to pairs too where no half of a pair would stand idle: 256 weight rows x 128 tokens, 24 KB from
+  // the L2 into each SM a k-block in place of 32 for the same products (8,192 rows over 16 experts, 2,048 -> 2 x 1,024 ->
+  // 2,048, both products: 219 -> 207 us; the epilogue's four warps bound the rest, most of all at 1,024 k).
+  const bool pairs = tile_rows == 256 || N % (2 * BM) == 0;
+  // (the pair form fetches the tokens of a tile in two boxes, one a block)
+  if (!cached_map(&mw_copy, W, (long long)groups * N, K, K, BM, true) ||
+      !cached_map(&mx_copy, X, M, K, ldx, pairs ? tile_rows / 2 : 128, false))
     return refuse(ST_BAD_SIZE, "gemm_tcgen05_grouped: cuTensorMapEncodeTiled refused the operands");
   if (tile_rows == 256) return launch_pair<256, 6>(mw, mx, a, 0, stream);
+  if (pairs) return launch_pair<128, 8>(mw, mx, a, 0, stream);
   return launch_persistent<128, 5>(mw, mx, a, 0, stream);
 }
