@@ -451,8 +451,8 @@ __device__ void select_by_mass(const float* v, int V, Slice sl, const Kept& kept
 
 // The choice among few kept elements (top-k of at most kList): block 0 of the cluster collects them, orders them by key
 // descending and id ascending, and reads the cutoff and the draw off their running masses: the element that the searches
-// above would find.  -> its id in block 0's thread 0; the other blocks return at once.  lists: 3 * kList words of shared
-// memory, at the same place in every block.
+// above would find.  -> its id in block 0's thread 0, -1 where no kept element has a mass (the adjusted maximum is not a finite
+// number); the other blocks return at once.  lists: 3 * kList words of shared memory, at the same place in every block.
 constexpr int kList = 512;
 __device__ int select_from_list(const float* v, int V, Slice sl, const Kept& kept, float vmax, float tp, float uniform,
                                 Shared& sh, u64* lists) {
@@ -499,6 +499,7 @@ __device__ int select_from_list(const float* v, int V, Slice sl, const Kept& kep
     if (lane >= o) through += up;
   }
   const u64 total = __shfl_sync(0xffffffffu, through, 31);
+  if (total == 0) return -1;
   // the first element whose running mass reaches `target` (1 .. total), and that mass
   auto reach = [&](u64 target, u64* mass_through) {
     const int lane_of = __ffs(__ballot_sync(0xffffffffu, through >= target)) - 1;
@@ -602,7 +603,10 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
   }
   if (k > 0 && k < V && k <= kList) {
     const int id = select_from_list(v, V, sl, kept, bv, top_p[r], uniform[r], sh, reinterpret_cast<u64*>(copies));
-    if (writer) out_token[r] = id;
+    if (writer) {
+      if (id < 0) atomicExch(bad, 1);
+      out_token[r] = id < 0 ? bi : id;
+    }
     return;
   }
   // the kept set's masses by the top 8 bits of the key; their sum is the softmax denominator

@@ -334,6 +334,49 @@ def test_sampling_around_the_longest_collected_list(V, k):
         assert consistent_with_plain(got[i], logits[i], [], 1.0, k, p.top_p, 1.0, uniform_for(seeds[i], idx[i])), (i, got[i])
 
 
+@pytest.mark.parametrize("V", [600, 40004])
+@pytest.mark.parametrize("k", [0, 1, 50, 512, 513])
+@pytest.mark.parametrize("top_p", [0.9, 1.0])
+def test_values_that_overflow_raise_the_fault_word(V, k, top_p):
+    """Finite logits whose adjusted maximum is no finite number (a tiny temperature, a tiny or a huge penalty) have no masses to
+    draw from: the fault word is raised and the token is the argmax, however many are kept; a row beside them is not affected."""
+    from safetyraise_lmengine_b200.kernels import ops
+    from safetyraise_lmengine_b200.parts.base import FAULT_LOGITS
+    from safetyraise_lmengine_b200.sampling.params import SamplingParams
+    from safetyraise_lmengine_b200.sampling.sampler import Sampler
+    rng = np.random.default_rng(V + k)
+    logits = rng.normal(0, 8.0, size=(4, V)).astype(np.float32)
+    logits[2] = -20.0
+    history = [[], [int(np.argmax(logits[1])), 3], list(range(V)), []]
+    temperature, penalty = np.float32([1e-38, 1.0, 1.0, 1.0]), np.float32([1.0, 1e-38, 3e38, 1.0])
+    with np.errstate(over="ignore"):
+        adjusted = logits.copy()
+        for i, ids in enumerate(history):
+            for t in ids:
+                adjusted[i, t] = adjusted[i, t] / penalty[i] if adjusted[i, t] >= 0 else adjusted[i, t] * penalty[i]
+        adjusted /= temperature[:, None]
+    assert not np.isfinite(adjusted[:3].max(1)).any()
+    f32 = lambda v: torch.tensor(v, dtype=torch.float32, device=DEV)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=DEV)
+    offsets = np.cumsum([0] + [len(ids) for ids in history])
+    uniform, scratch = f32([0.3, 0.99, 0.0, 0.5]), torch.empty(4, V, device=DEV)
+    for rows, faulty in ((slice(0, 3), 1), (slice(3, 4), 0)):
+        n = rows.stop - rows.start
+        out, bad = torch.full((n,), -7, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+        ops.sample(f32(logits[rows]), f32(temperature[rows]), i32([k] * n), f32([top_p] * n), f32(penalty[rows]), uniform[rows],
+                   i32([t for ids in history for t in ids]), i32(offsets[rows.start:rows.stop + 1]), out, bad, scratch)
+        assert int(bad) == faulty
+        if faulty:
+            assert out.tolist() == [int(np.argmax(row)) for row in adjusted[rows]]
+        else:
+            assert 0 <= int(out) < V
+    sampler = Sampler(DEV, V, 4)
+    params = [SamplingParams(temperature=float(temperature[i]), top_p=top_p, top_k=k, repetition_penalty=float(penalty[i]))
+              for i in range(4)]
+    tokens = sampler.sample(f32(logits), params, [1, 2, 3, 4], [0] * 4, history)
+    assert sampler.last_words[FAULT_LOGITS] == 1 and tokens[:3] == [int(np.argmax(row)) for row in adjusted[:3]]
+
+
 def test_sampling_statistics():
     """Frequencies over many draws follow the truncated distribution."""
     from safetyraise_lmengine_b200.sampling.params import SamplingParams
