@@ -177,8 +177,10 @@ __device__ __forceinline__ float row_max(const Row& r, int k_lo, int k_hi) {
   part(r.d, 96);
   return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
 }
-// P = exp2(S * scale - base) as bfloat16 pairs over the first 64 columns of S; returns the row sum.
-template <bool MASKED>
+// P = exp2(S * scale - base) as bfloat16 pairs over the first 64 columns of S; returns the row sum, of the weights as they are
+// or (ROUNDED) as the product with V reads them: a row's weights then add up to one exactly, and the rounding of one that
+// outweighs the others cancels.
+template <bool MASKED, bool ROUNDED = false>
 __device__ __forceinline__ float row_exp(uint32_t s_addr, const Row& r, float scale, float base, int k_lo, int k_hi) {
   float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
   const float nb = -base;
@@ -197,9 +199,12 @@ __device__ __forceinline__ float row_exp(uint32_t s_addr, const Row& r, float sc
         p2 = (k + 2 >= k_lo && k + 2 < k_hi) ? p2 : 0.f;
         p3 = (k + 3 >= k_lo && k + 3 < k_hi) ? p3 : 0.f;
       }
+      const uint32_t lo = pk[j >> 1] = pack2(p0, p1), hi = pk[(j >> 1) + 1] = pack2(p2, p3);
+      if (ROUNDED) {
+        p0 = __uint_as_float(lo << 16), p1 = __uint_as_float(lo & 0xffff0000u);
+        p2 = __uint_as_float(hi << 16), p3 = __uint_as_float(hi & 0xffff0000u);
+      }
       s0 += p0; s1 += p1; s2 += p2; s3 += p3;
-      pk[j >> 1] = pack2(p0, p1);
-      pk[(j >> 1) + 1] = pack2(p2, p3);
     }
     tmem_st16(s_addr + (c >> 1), pk);
   };

@@ -101,6 +101,40 @@ def test_prompts_against_float64(page, window, heads, pairs, interleaved, gated)
     assert (got - ref).abs().max() <= 2.0 ** -8 * (1.0 + ref.abs().max())
 
 
+def test_a_weight_that_outweighs_the_others_loses_nothing():
+    """One key of every head has nearly all the weight and comes behind one that is e^4 to e^5.5 smaller: the output is its value
+    but for what the other key adds, rounded once.  A weight rounded to 8 bits beside a sum that is not, or measured from a
+    maximum that lags, would be off by up to 2^-8 of itself."""
+    from safetyraise_lmengine_b200.kernels import ops
+    g = torch.Generator().manual_seed(3)
+    heads, n, k, page = 8, 130, 400, 16
+    ctx = Ctx([n], [k])
+    q = torch.zeros(n, heads * (DIM + ROT))
+    q[:, ::DIM + ROT] = 1.0
+    rows = torch.randn(k, heads * (DIM + DV), generator=g).bfloat16()
+    rows[:, :heads * DIM:DIM] = -100.0
+    rows[5, :heads * DIM:DIM] = 0.0
+    rows[200, :heads * DIM:DIM] = (4.0 + 1.5 * torch.rand(heads, generator=g)).bfloat16()
+    pages = torch.zeros(k // page, 1, page, RANK + ROT, dtype=torch.bfloat16, device=DEV)
+    table = torch.arange(k // page, dtype=torch.int32, device=DEV)[None]
+    out = torch.empty(n, heads * DV, dtype=torch.bfloat16, device=DEV)
+    flag = torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.bind_error_flag(flag)
+    try:
+        ops.latent_prefill_tcgen05(ctx, q.to(DEV), None, pages, rows.to(DEV), torch.zeros(1, dtype=torch.int32, device=DEV), out, table,
+                                   heads, DIM, ROT, DV, RANK, heads * DIM, 1.0)
+        got = out.double().cpu().view(n, heads, DV)
+    finally:
+        ops.bind_error_flag(None)
+    assert int(flag) == 0
+    small = torch.exp(-rows[200, :heads * DIM:DIM].double())[:, None]
+    v = rows[:, heads * DIM:].double().view(k, heads, DV)
+    ref = (v[200] + small * v[5]) / (1 + small)
+    # half a step of the result's 8 bits, and 2^-8 of the small weight's part
+    half = 2.0 ** (torch.floor(torch.log2(ref.abs())) - 8)
+    assert ((got - ref).abs() <= half * 1.001 + 2.0 ** -8 * small * (v[5] - v[200]).abs() + 1e-6).all()
+
+
 @pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 40])
 @pytest.mark.parametrize("dim, rot, rank, dv", [(128, 64, 512, 128), (12, 6, 20, 9), (64, 0, 130, 33), (3, 2, 5, 1)])
 def test_the_per_head_products(T, dim, rot, rank, dv):
