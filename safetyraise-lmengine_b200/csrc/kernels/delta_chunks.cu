@@ -16,9 +16,10 @@
 // 2,000 tokens, 16 heads of 128 x 128, one entry: 72 + 152 us; the kernels that go token by token: 98 + 610 us.
 //
 // The products of the walk are mma.sync m16n8k8 on tf32 operands, each operand split into two tf32 numbers (high, and the rest)
-// and each product formed as high high + high low + low high, with float32 sums.  Relative error against float64 (2-norm; 100 to
-// 2,048 tokens, decays from fast to nearly one), outputs and state: 2.2e-7 to 5.8e-7 and 1e-8 to 4.9e-7; the kernels that go
-// token by token in float32 FMAs: 1.5e-7 to 2.4e-6 and 1e-8 to 2.1e-6.
+// and each product formed as high high + high low + low high.  Relative error against float64 (2-norm; 16 to 2,000 tokens, decays
+// from fast to nearly one), outputs and state: 1.3e-7 to 2.1e-7 and 5e-8 to 2.1e-7; the kernels that go token by token in float32
+// FMAs: 1.3e-7 to 3.7e-6 and 1.4e-7 to 5.2e-6, never below.  It takes the sums of their own in mma_split (one running sum in the
+// tensor core: up to 2.9 times the token walk's error) and the scalars of a token in 64 bits (up to 1.7 times without).
 #include "state_walk.cuh"
 
 namespace srlm {
@@ -57,8 +58,10 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
   pdl_wait();
   pdl_trigger();
   __shared__ __align__(16) float k_s[TOK][DK + 4], q_s[TOK][DK + 4];
-  __shared__ __align__(16) float x_s[TOK][TOK], m_s[TOK][TOK], n_s[TOK][TOK], d_s[TOK][TOK];
-  __shared__ float unit_k[TOK], unit_q[TOK], beta_s[TOK], g_s[TOK], pre_s[TOK];
+  __shared__ __align__(16) float x_s[TOK][TOK], m_s[TOK][TOK], n_s[TOK][TOK];
+  // what multiplies a whole token or a pair of tokens is formed in 64 bits and rounded once
+  __shared__ double d_s[TOK][TOK], unit_k[TOK], unit_q[TOK], g_s[TOK], pre_s[TOK];
+  __shared__ float beta_s[TOK], fade_k[TOK], fade_q[TOK], last_k[TOK];   // P_i / |k_i|, P_i / (|q_i| sqrt(DK)), R_i / |k_i|
   const Home home = home_of(cu_q, n_entries, blockIdx.x);
   if (home.entry < 0) return;
   const int h = blockIdx.y, kh = h / (z.H / z.G), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -100,11 +103,13 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
     for (int i = 0; i < TOK; ++i) (part ? k_s : q_s)[i][tid] = y[i];
   }
   if (tid < TOK) {
-    float b = 0.f, g = 1.f;
+    float b = 0.f;
+    double g = 1.;
     if (tid < home.n) {
       const float* row = proj + (size_t)(home.t0 + tid) * ldp + z.C;
-      b = logistic_f(row[h]);
-      g = expf(-expf(a_log[h]) * softplus_f(row[z.H + h] + dt_bias[h]));
+      const double a = (double)row[z.H + h] + dt_bias[h];
+      b = (float)(1. / (1. + exp(-(double)row[h])));
+      g = exp(-exp((double)a_log[h]) * (a > 20. ? a + log1p(exp(-a)) : log1p(exp(a))));
     }
     beta_s[tid] = b;
     g_s[tid] = g;
@@ -114,15 +119,15 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
     const int i = v % TOK;
     const float4 x = *reinterpret_cast<const float4*>((v < TOK ? k_s[i] : q_s[i]) + 4 * lane);
     const float ss = warp_sum((x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w));
-    if (lane == 0) (v < TOK ? unit_k : unit_q)[i] = (v < TOK ? 1.f : 1.f / sqrtf((float)DK)) / sqrtf(ss + unit_eps);
+    if (lane == 0) (v < TOK ? unit_k : unit_q)[i] = (v < TOK ? 1. : 1. / sqrt((double)DK)) / sqrt((double)ss + unit_eps);
   }
   if (tid < TOK) {                             // column tid of D, and P
-    float p = 1.f, d = 1.f;
+    double p = 1., d = 1.;
     for (int i = 0; i <= tid; ++i) p *= g_s[i];
     pre_s[tid] = p;
     for (int i = 0; i < TOK; ++i) {
       if (i > tid) d *= g_s[i];
-      d_s[i][tid] = i >= tid ? d : 0.f;
+      d_s[i][tid] = i >= tid ? d : 0.;
     }
   }
   // k_i . k_j (threads 0 .. 63) and q_i . k_j (64 .. 127): rows i, i + 8, columns j, j + 8
@@ -130,7 +135,7 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
     const int i = (tid & 63) >> 3, j = tid & 7;
     const float* a0 = tid < 64 ? k_s[i] : q_s[i];
     const float* a1 = tid < 64 ? k_s[i + 8] : q_s[i + 8];
-    float acc[2][2] = {};
+    float part[2][2][4] = {};
 #pragma unroll 4
     for (int c = 0; c < DK; c += 4) {
       const float4 a[2] = {*reinterpret_cast<const float4*>(a0 + c), *reinterpret_cast<const float4*>(a1 + c)};
@@ -139,10 +144,10 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
       for (int x = 0; x < 2; ++x)
 #pragma unroll
         for (int y = 0; y < 2; ++y) {
-          acc[x][y] = fmaf(a[x].x, b[y].x, acc[x][y]);
-          acc[x][y] = fmaf(a[x].y, b[y].y, acc[x][y]);
-          acc[x][y] = fmaf(a[x].z, b[y].z, acc[x][y]);
-          acc[x][y] = fmaf(a[x].w, b[y].w, acc[x][y]);
+          part[x][y][0] = fmaf(a[x].x, b[y].x, part[x][y][0]);
+          part[x][y][1] = fmaf(a[x].y, b[y].y, part[x][y][1]);
+          part[x][y][2] = fmaf(a[x].z, b[y].z, part[x][y][2]);
+          part[x][y][3] = fmaf(a[x].w, b[y].w, part[x][y][3]);
         }
     }
     __syncthreads();                           // the unit factors and D are here
@@ -151,10 +156,16 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
 #pragma unroll
       for (int y = 0; y < 2; ++y) {
         const int r = i + 8 * x, c = j + 8 * y;
-        const float s = acc[x][y] * unit_k[c] * d_s[r][c];       // D is 0 above the diagonal
-        if (tid < 64) n_s[r][c] = r > c ? s * unit_k[r] : 0.f;
-        else m_s[r][c] = s * unit_q[r];
+        const float sum = (part[x][y][0] + part[x][y][1]) + (part[x][y][2] + part[x][y][3]);
+        const double s = sum * unit_k[c] * d_s[r][c];            // D is 0 above the diagonal
+        if (tid < 64) n_s[r][c] = r > c ? (float)(s * unit_k[r]) : 0.f;
+        else m_s[r][c] = (float)(s * unit_q[r]);
       }
+  }
+  if (tid < TOK) {
+    fade_k[tid] = (float)(pre_s[tid] * unit_k[tid]);
+    fade_q[tid] = (float)(pre_s[tid] * unit_q[tid]);
+    last_k[tid] = (float)(d_s[TOK - 1][tid] * unit_k[tid]);
   }
   __syncthreads();
   if (tid < TOK) {                             // column tid of X, forward along the rows
@@ -193,9 +204,8 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
     if (c < 0) {
 #pragma unroll
       for (int i = 0; i < TOK; ++i) {
-        x[i] = unit_k[i] * k_s[i][tid];
-        rec[(2 * TOK + i) * DK + tid] = d_s[TOK - 1][i] * x[i];
-        x[i] *= pre_s[i];
+        rec[(2 * TOK + i) * DK + tid] = last_k[i] * k_s[i][tid];
+        x[i] = fade_k[i] * k_s[i][tid];
       }
     } else {
       convolve(2 * z.G * DK + h * z.dv + c, x);
@@ -207,9 +217,9 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
     for (int i = 0; i < TOK; ++i) out[i * ld] = x[i];
     lower(m_s, x);
 #pragma unroll
-    for (int i = 0; i < TOK; ++i) out[(TOK + i) * ld] = c < 0 ? pre_s[i] * unit_q[i] * q_s[i][tid] - x[i] : x[i];
+    for (int i = 0; i < TOK; ++i) out[(TOK + i) * ld] = c < 0 ? fmaf(fade_q[i], q_s[i][tid], -x[i]) : x[i];
   }
-  if (tid == 0) rec[3 * TOK * DK + 2 * TOK * z.dv] = pre_s[TOK - 1];
+  if (tid == 0) rec[3 * TOK * DK + 2 * TOK * z.dv] = (float)pre_s[TOK - 1];
 }
 
 // ---- the walk -----------------------------------------------------------------------------------------------------------
@@ -235,11 +245,13 @@ __device__ __forceinline__ void mma_tf32(float (&c)[4], uint32_t a0, uint32_t a1
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// c += a b in three products, the small ones first
-__device__ __forceinline__ void mma_split(float (&c)[4], const Split (&a)[4], const Split (&b)[2]) {
-  mma_tf32(c, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
-  mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
-  mma_tf32(c, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
+// A sum of a tensor-core product is cut off, not rounded, behind its 24th bit, each time that it is written.  So the products
+// of the high parts (`large`, one product a sum) and those with a rest (`small`, 2^-11 of it) have sums of their own, which
+// float32 additions join.
+__device__ __forceinline__ void mma_split(float (&small)[4], float (&large)[4], const Split (&a)[4], const Split (&b)[2]) {
+  mma_tf32(small, a[0].lo, a[1].lo, a[2].lo, a[3].lo, b[0].hi, b[1].hi);
+  mma_tf32(small, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].lo, b[1].lo);
+  mma_tf32(large, a[0].hi, a[1].hi, a[2].hi, a[3].hi, b[0].hi, b[1].hi);
 }
 
 // A warp holds 16 columns x 16 rows of S as two accumulator tiles [column][8 rows]: lane (g, t) = (lane / 4, lane % 4) has
@@ -306,14 +318,19 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
   };
   // kx . S or qm . S over the warp's rows, 16 tokens
   auto product = [&](const float* rows, const Split (&a)[2][4], float (&c)[2][4]) {
+    float large[2][2][4] = {};
 #pragma unroll
     for (int x = 0; x < 2; ++x)
 #pragma unroll
       for (int y = 0; y < 2; ++y) {
         const float2 r = *reinterpret_cast<const float2*>(rows + (8 * y + g) * LD + warp * ROWS + 8 * x + 2 * t);
         const Split b[2] = {split(r.x), split(r.y)};
-        mma_split(c[y], a[x], b);
+        mma_split(c[y], large[x][y], a[x], b);
       }
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) c[y][v] += large[0][y][v] + large[1][y][v];
   };
   float o0 = 0.f;
   auto finish = [&](int s) {                             // the thread's o of chunk s
@@ -341,11 +358,8 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
     product(st + TOK * LD, a, w);                        // does not wait for u: its sums are gathered a chunk later
     o0 = st[3 * TOK * LD + TOK * COLS + tid];
     const float whole = st[3 * TOK * LD + 2 * TOK * COLS];
-#pragma unroll
-    for (int x = 0; x < 2; ++x)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) S[x][v] *= whole;
     __syncthreads();
+    float small[2][4] = {}, large[2][2][4] = {};
 #pragma unroll
     for (int y = 0; y < 2; ++y) {                        // eight tokens
       const float* at = u_s + (8 * y + t) * U_LD + g;
@@ -354,9 +368,13 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
       for (int x = 0; x < 2; ++x) {
         const float* ke = st + (2 * TOK + 8 * y + t) * LD + warp * ROWS + 8 * x + g;
         const Split b[2] = {split(ke[0]), split(ke[4 * LD])};
-        mma_split(S[x], ua, b);
+        mma_split(small[x], large[x][y], ua, b);
       }
     }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) S[x][v] = fmaf(whole, S[x][v], (large[x][0][v] + large[x][1][v]) + small[x][v]);
     leave(q_sums, w);
   }
   __syncthreads();
