@@ -119,7 +119,8 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
     const int i = v % TOK;
     const float4 x = *reinterpret_cast<const float4*>((v < TOK ? k_s[i] : q_s[i]) + 4 * lane);
     const float ss = warp_sum((x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w));
-    if (lane == 0) (v < TOK ? unit_k : unit_q)[i] = (v < TOK ? 1. : 1. / sqrt((double)DK)) / sqrt((double)ss + unit_eps);
+    const double one = v < TOK ? 1. : 1. / sqrt((double)DK);
+    if (lane == 0) (v < TOK ? unit_k : unit_q)[i] = i < home.n ? one / sqrt((double)ss + unit_eps) : 0.;   // a place without a token
   }
   if (tid < TOK) {                             // column tid of D, and P
     double p = 1., d = 1.;

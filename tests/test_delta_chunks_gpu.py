@@ -26,7 +26,7 @@ class Ctx:
         self.workspace = Workspace(torch.device(DEV), cu[-1])
 
 
-def recurrence(proj, conv_w, a_log, dt_bias, state, H, G, dv, taps):
+def recurrence(proj, conv_w, a_log, dt_bias, state, H, G, dv, taps, eps=EPS):
     """One entry in float64 -> (o [n, H, dv], the state row behind it)."""
     n, C = proj.shape[0], 2 * G * DK + H * dv
     S = state[:H * DK * dv].view(H, dv, DK).transpose(1, 2).clone()
@@ -34,7 +34,7 @@ def recurrence(proj, conv_w, a_log, dt_bias, state, H, G, dv, taps):
     x = torch.cat([carry, proj[:, :C]])
     y = sum(x[j:j + n] * conv_w[:, j] for j in range(taps))
     y = y * torch.sigmoid(y)
-    unit = lambda a: a / torch.sqrt((a * a).sum(-1, keepdim=True) + EPS)
+    unit = lambda a: a / torch.sqrt((a * a).sum(-1, keepdim=True) + eps)
     q, k = unit(y[:, :G * DK].view(n, G, DK)) * DK ** -0.5, unit(y[:, G * DK:2 * G * DK].view(n, G, DK))
     q, k = q.repeat_interleave(H // G, 1), k.repeat_interleave(H // G, 1)
     v = y[:, 2 * G * DK:].view(n, H, dv)
@@ -51,7 +51,8 @@ def recurrence(proj, conv_w, a_log, dt_bias, state, H, G, dv, taps):
 
 @pytest.mark.parametrize("H, G, dv, taps", [(2, 2, 128, 4), (4, 2, 48, 4), (3, 1, 16, 2), (2, 1, 144, 1), (1, 1, 128, 3)])
 @pytest.mark.parametrize("lens", [[16], [1, 17, 2, 33], [15, 31, 48], [130]])
-def test_against_float64(H, G, dv, taps, lens):
+@pytest.mark.parametrize("eps", [EPS, 0.0])                  # 0: the places behind an entry's last token have no length
+def test_against_float64(H, G, dv, taps, lens, eps):
     from safetyraise_lmengine_b200.kernels import ops
     gen = torch.Generator(device=DEV).manual_seed(H + dv + taps + len(lens))
     rand = lambda *s: torch.randn(*s, generator=gen, device=DEV)
@@ -72,11 +73,11 @@ def test_against_float64(H, G, dv, taps, lens):
         assert n == 0
         return
     assert n == sum(-(-x // 16) for x in lens)
-    ops.delta_chunks(ctx, proj, conv_w, a_log, dt_bias, state, o, n, H, G, DK, dv, taps, EPS)
+    ops.delta_chunks(ctx, proj, conv_w, a_log, dt_bias, state, o, n, H, G, DK, dv, taps, eps)
     want_o, want_state, t = [], before.clone(), 0
     for x, slot in zip(lens, slots):
         used = H * DK * dv + C * (taps - 1)
-        a, b = recurrence(proj[t:t + x].double(), conv_w.double(), a_log.double(), dt_bias.double(), before[slot, :used], H, G, dv, taps)
+        a, b = recurrence(proj[t:t + x].double(), conv_w.double(), a_log.double(), dt_bias.double(), before[slot, :used], H, G, dv, taps, eps)
         want_o.append(a.reshape(x, -1))
         want_state[slot, :used] = b
         t += x
