@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(128, 5)
 delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* __restrict__ conv_w, int taps,
                     const float* __restrict__ a_log, const float* __restrict__ dt_bias, const float* __restrict__ state,
                     long long state_stride, const int* __restrict__ cu_q, int n_entries, const int* __restrict__ slots,
-                    float* __restrict__ records, Sizes z, float unit_eps) {
+                    float* __restrict__ records, int first_chunk, Sizes z, float unit_eps) {
   pdl_wait();
   pdl_trigger();
   __shared__ __align__(16) float k_s[TOK][DK + 4], q_s[TOK][DK + 4];
@@ -62,7 +62,7 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
   // what multiplies a whole token or a pair of tokens is formed in 64 bits and rounded once
   __shared__ double d_s[TOK][TOK], unit_k[TOK], unit_q[TOK], g_s[TOK], pre_s[TOK];
   __shared__ float beta_s[TOK], fade_k[TOK], fade_q[TOK], last_k[TOK];   // P_i / |k_i|, P_i / (|q_i| sqrt(DK)), R_i / |k_i|
-  const Home home = home_of(cu_q, n_entries, blockIdx.x);
+  const Home home = home_of(cu_q, n_entries, first_chunk + blockIdx.x);
   if (home.entry < 0) return;
   const int h = blockIdx.y, kh = h / (z.H / z.G), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* carry = state + (size_t)slots[home.entry] * state_stride + (size_t)z.H * DK * z.dv;   // [C][taps - 1]
@@ -260,23 +260,26 @@ __device__ __forceinline__ void mma_split(float (&small)[4], float (&large)[4], 
 // the product's k-th place t standing for row 2 t and t + 4 for row 2 t + 1 (on both sides).
 __global__ void __launch_bounds__(THREADS, 2)
 delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ state, long long state_stride,
-                        const int* __restrict__ cu_q, const int* __restrict__ slots, float* __restrict__ o_out, Sizes z) {
+                        const int* __restrict__ cu_q, const int* __restrict__ slots, float* __restrict__ o_out, int first_chunk,
+                        int n_chunks, Sizes z) {
   pdl_wait();
   pdl_trigger();
+  // the records are those of the step's chunks first_chunk .. first_chunk + n_chunks - 1, of the entry's those from..to - 1
   extern __shared__ __align__(16) float chunk_smem[];
   float* p_sums = chunk_smem + STAGES * STAGE;           // [warp][SUMS]: kx . S
   float* q_sums = p_sums + WARPS * SUMS;                 // qm . S
   float* u_s = q_sums + WARPS * SUMS;                    // [token][U_LD]
   const int e = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int first = cu_q[e], n = cu_q[e + 1] - first, steps = (n + TOK - 1) / TOK;
-  int base = 0;
+  const int first = cu_q[e], n = cu_q[e + 1] - first;
+  int base = -first_chunk;
   for (int x = 0; x < e; ++x) base += (cu_q[x + 1] - cu_q[x] + TOK - 1) / TOK;
+  const int from = max(0, -base), to = min((n + TOK - 1) / TOK, n_chunks - base);
+  if (from >= to) return;
   const int rec_floats = record_floats(z.dv);
-  const float* rec0 = records + ((size_t)base * z.H + h) * rec_floats;
   auto fetch = [&](int s) {
-    if (s < steps) {
-      const float* src = rec0 + (size_t)s * z.H * rec_floats;
+    if (s < to) {
+      const float* src = records + ((size_t)(base + s) * z.H + h) * rec_floats;
       float* dst = chunk_smem + (s % STAGES) * STAGE;
 #pragma unroll
       for (int i = 0; i < 3 * TOK * DK / 4 / THREADS; ++i) {
@@ -292,7 +295,7 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
     state_copy_commit();
   };
 #pragma unroll
-  for (int s = 0; s < STAGES - 1; ++s) fetch(s);
+  for (int s = from; s < from + STAGES - 1; ++s) fetch(s);
   float* S_head = state + (size_t)slots[e] * state_stride + (size_t)h * z.dv * DK;
   float S[2][4];
 #pragma unroll
@@ -337,10 +340,10 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
   auto finish = [&](int s) {                             // the thread's o of chunk s
     if (s * TOK + tok < n) o_out[((size_t)(first + s * TOK + tok) * z.H + h) * z.dv + c0 + col] = o0 + gather(q_sums);
   };
-  for (int s = 0; s < steps; ++s) {
+  for (int s = from; s < to; ++s) {
     state_copy_wait<STAGES - 2>();
     __syncthreads();                                     // chunk s is here for all; chunk s - 1 is read by all
-    if (s > 0) finish(s - 1);
+    if (s > from) finish(s - 1);
     fetch(s + STAGES - 1);
     const float* st = chunk_smem + (s % STAGES) * STAGE;
     Split a[2][4];
@@ -379,7 +382,7 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
     leave(q_sums, w);
   }
   __syncthreads();
-  if (steps > 0) finish(steps - 1);
+  finish(to - 1);
   state_copy_wait<0>();
 #pragma unroll
   for (int x = 0; x < 2; ++x)
@@ -400,16 +403,16 @@ extern "C" int srlm_delta_chunk_record(int dk, int dv, int taps) {
              ? chunks::record_floats(dv) : 0;
 }
 
-// proj float32 [T, ldp] and state as in delta_rule.cu; n_chunks: how many chunks of 16 tokens the step's entries have
-// together; records float32 [n_chunks, H, record]; o_out float32 [T, H dv].  Renews S; the carried inputs of the
-// convolution are read and stay.
+// proj float32 [T, ldp] and state as in delta_rule.cu.  Takes the chunks first_chunk .. first_chunk + n_chunks - 1 of those that
+// the step's entries have together, entry by entry: a step whose chunks do not all fit `records` (float32 [n_chunks, H, record])
+// is several calls, in order.  o_out float32 [T, H dv].  Renews S; the carried inputs of the convolution are read and stay.
 extern "C" int srlm_delta_chunks(const float* proj, long long ldp, const float* conv_w, const float* a_log, const float* dt_bias,
                                  float* state, long long state_stride, const int* cu_q, const int* slots, int n_entries,
-                                 float* records, int n_chunks, float* o_out, int H, int G, int dk, int dv, int taps,
+                                 float* records, int first_chunk, int n_chunks, float* o_out, int H, int G, int dk, int dv, int taps,
                                  float unit_eps, cudaStream_t stream) {
   if (n_entries <= 0 || n_chunks <= 0) return ST_OK;
   const long long C = 2LL * G * dk + (long long)H * dv;
-  if (!srlm_delta_chunk_record(dk, dv, taps) || H <= 0 || G <= 0 || H % G || H > 65535 || n_entries > 65535 ||
+  if (!srlm_delta_chunk_record(dk, dv, taps) || first_chunk < 0 || H <= 0 || G <= 0 || H % G || H > 65535 || n_entries > 65535 ||
       ldp < C + 2LL * H || C > 0x7fffffff || state_stride < (long long)H * dk * dv + C * (taps - 1))
     return refuse(ST_BAD_SIZE, "delta_chunks: H=%d G=%d dk=%d dv=%d taps=%d ldp=%lld state=%lld entries=%d", H, G, dk, dv, taps,
                   ldp, state_stride, n_entries);
@@ -417,12 +420,13 @@ extern "C" int srlm_delta_chunks(const float* proj, long long ldp, const float* 
     return refuse(ST_BAD_ALIGN, "delta_chunks: states start on 8 bytes, records on 16");
   const chunks::Sizes z{H, G, dv, (int)C};
   launch_pdl(chunks::delta_chunks_kernel, dim3(n_chunks, H), dim3(128), 0, stream, proj, ldp, conv_w, taps, a_log, dt_bias,
-             (const float*)state, state_stride, cu_q, n_entries, slots, records, z, unit_eps);
+             (const float*)state, state_stride, cu_q, n_entries, slots, records, first_chunk, z, unit_eps);
   const cudaError_t e = cudaFuncSetAttribute(chunks::delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              chunks::WALK_SMEM);
   if (e != cudaSuccess) return refuse((int)e, "delta_chunks: cannot get %d bytes of shared memory", chunks::WALK_SMEM);
   // (not ahead of time: blocks that start while the chunks' kernel drains would share the SMs that happen to be free)
   launch_pdl_if(false, chunks::delta_chunk_walk_kernel, dim3(dv / chunks::COLS, H, n_entries), dim3(chunks::THREADS),
-                chunks::WALK_SMEM, stream, (const float*)records, state, state_stride, cu_q, slots, o_out, z);
+                chunks::WALK_SMEM, stream, (const float*)records, state, state_stride, cu_q, slots, o_out,
+                first_chunk, n_chunks, z);
   return launched();
 }

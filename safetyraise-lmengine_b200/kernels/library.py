@@ -1548,6 +1548,15 @@ class KernelLibrary:
     DELTA_CHUNK = 16         # tokens of a chunk
     DELTA_CHUNKS_FROM = 16   # steps with an entry of at least this many tokens go by chunks
 
+    # Chunks whose records lie in memory at a time (41 KB a chunk and head of 128 x 128: 105 MB for 16 heads); a step that has more
+    # takes them by turns, S in its slot in between.  160: the chunks of 2,048 tokens in up to 32 requests.
+    DELTA_CHUNKS_HELD = 160
+
+    def delta_chunks_held(self, max_tokens: int) -> int:
+        """Chunks that a workspace for steps of ``max_tokens`` tokens keeps records of: all that such a step can make (two by every
+        17 tokens), up to DELTA_CHUNKS_HELD.  It does not depend on the step: the buffer is made once."""
+        return min(self.DELTA_CHUNKS_HELD, 2 * max_tokens // (self.DELTA_CHUNK + 1) + 1)
+
     def delta_by_chunks(self, ctx, state, dk, dv, taps) -> int:
         """How many chunks of 16 tokens the step's entries make, 0 where the step goes token by token: decode steps and
         short portions, sizes that the chunked kernels do not take, and the float32 path, whose results do not depend on
@@ -1567,13 +1576,15 @@ class KernelLibrary:
         if proj.dtype != torch.float32:
             raise ShapeError("delta_chunks: the projection is float32")
         record = int(self.lib.srlm_delta_chunk_record(C.c_int(dk), C.c_int(dv), C.c_int(taps)))
-        records = ctx.workspace.get("delta.records", n_chunks * H, max(record, 1), torch.float32, reserve=0)
-        self._check(self.lib.srlm_delta_chunks(
-            _ptr(proj), C.c_longlong(proj.stride(0)), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias), _ptr(state),
-            C.c_longlong(state.stride(0)), _ptr(ctx.cu_q), _ptr(ctx.slots), C.c_int(ctx.n_entries), _ptr(records),
-            C.c_int(n_chunks), _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps),
-            _stream()), "delta_chunks")
-        self.launches += 1
+        held = self.delta_chunks_held(ctx.workspace.max_tokens)
+        records = ctx.workspace.get("delta.records", held * H, max(record, 1), torch.float32, reserve=held * H)
+        for first in range(0, n_chunks, held):
+            self._check(self.lib.srlm_delta_chunks(
+                _ptr(proj), C.c_longlong(proj.stride(0)), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias), _ptr(state),
+                C.c_longlong(state.stride(0)), _ptr(ctx.cu_q), _ptr(ctx.slots), C.c_int(ctx.n_entries), _ptr(records),
+                C.c_int(first), C.c_int(min(held, n_chunks - first)), _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv),
+                C.c_int(taps), C.c_float(unit_eps), _stream()), "delta_chunks")
+            self.launches += 1
         if taps > 1:
             self._check(self.lib.srlm_delta_conv_carry(
                 _ptr(proj), dtype_code(proj.dtype), C.c_longlong(proj.stride(0)), _ptr(state), C.c_longlong(state.stride(0)),

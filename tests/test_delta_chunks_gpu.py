@@ -133,3 +133,58 @@ def test_the_float32_path_and_short_steps_go_token_by_token():
     assert ops.delta_by_chunks(Ctx([15, 4], [0, 0]), state, 128, 128, 4) == 0
     assert ops.delta_by_chunks(Ctx([64], [0]), state, 64, 128, 4) == 0
     assert ops.delta_by_chunks(Ctx([64], [0]), state[:, 1:], 128, 128, 4) == 0
+
+
+def walked(lens, held=None, max_tokens=None):
+    """(o, state, the workspace's generation) of a step of these entries, four heads of 128, inputs that depend on the entry alone."""
+    from safetyraise_lmengine_b200.kernels import ops
+    H, dv, taps = 4, 128, 4
+    C = 3 * H * DK
+    parts, states = [], []
+    for e, n in enumerate(lens):
+        g = torch.Generator(device=DEV).manual_seed(100 + e)
+        states.append(torch.randn(H * DK * dv + C * (taps - 1), generator=g, device=DEV))
+        parts.append(torch.randn(n, C + 2 * H + H * dv, generator=g, device=DEV))
+    g = torch.Generator(device=DEV).manual_seed(7)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    conv_w, dt_bias, a_log = rand(C, taps) * 0.5, rand(H) - 4.0, rand(H)
+    ctx, state = Ctx(lens, list(range(len(lens)))), torch.stack(states)
+    if max_tokens:
+        ctx.workspace.max_tokens = max_tokens
+    o = torch.empty(sum(lens), H * dv, device=DEV)
+    was = type(ops).DELTA_CHUNKS_HELD
+    try:
+        type(ops).DELTA_CHUNKS_HELD = held or was
+        n = ops.delta_by_chunks(ctx, state, DK, dv, taps)
+        ops.delta_chunks(ctx, torch.cat(parts), conv_w, a_log, dt_bias, state, o, n, H, H, DK, dv, taps, EPS)
+    finally:
+        type(ops).DELTA_CHUNKS_HELD = was
+    return o, state, ctx.workspace
+
+
+@pytest.mark.parametrize("held", [1, 3, 5, 8])
+def test_steps_whose_chunks_are_taken_by_turns(held):
+    """Records for fewer chunks than a step has: the same bits, whatever lies together."""
+    lens = [70, 16, 33, 100]
+    o, state, _ = walked(lens)
+    o2, state2, work = walked(lens, held)
+    assert torch.equal(o, o2) and torch.equal(state, state2)
+    assert max(b.shape[0] for (name, _, _), b in work._bufs.items() if name == "delta.records") == 4 * held
+
+
+def test_the_records_do_not_grow_with_the_portions():
+    """Portions of growing length leave the workspace where it is: a buffer that moves throws the recorded decode graphs away."""
+    from safetyraise_lmengine_b200.kernels import ops
+    H, dv, taps, most = 2, 128, 4, 4096
+    C = 3 * H * DK
+    work = None
+    for lens in ([16], [17] * 8, [400], [1000, 40], [4096], [17] * 240):
+        ctx = Ctx(lens, list(range(len(lens))))
+        work = ctx.workspace = work or type(ctx.workspace)(torch.device(DEV), most)
+        state = torch.zeros(len(lens), H * DK * dv + C * (taps - 1), device=DEV)
+        T = sum(lens)
+        ops.delta_chunks(ctx, torch.zeros(T, C + 2 * H + H * dv, device=DEV), torch.zeros(C, taps, device=DEV), torch.zeros(H, device=DEV),
+                         torch.zeros(H, device=DEV), state, torch.empty(T, H * dv, device=DEV),
+                         ops.delta_by_chunks(ctx, state, DK, dv, taps), H, H, DK, dv, taps, EPS)
+        assert work.generation == 0
+    assert sum(b.numel() * b.element_size() for (name, _, _), b in work._bufs.items() if name == "delta.records") <= 160 * H * 42000
