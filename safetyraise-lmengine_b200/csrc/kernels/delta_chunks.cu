@@ -33,10 +33,12 @@ __host__ __device__ inline int record_floats(int dv) { return 3 * TOK * DK + 2 *
 struct Home {
   int entry, t0, n, first;                     // first: the entry's first token in the step
 };
-__device__ __forceinline__ Home home_of(const int* __restrict__ cu_q, int n_entries, int index) {
+// Chunks of an entry of `len` tokens: none where it goes token by token (fewer than `least` tokens).
+__device__ __forceinline__ int chunks_of(int len, int least) { return len < least ? 0 : (len + TOK - 1) / TOK; }
+__device__ __forceinline__ Home home_of(const int* __restrict__ cu_q, int n_entries, int least, int index) {
   int base = 0;
   for (int e = 0; e < n_entries; ++e) {
-    const int a = cu_q[e], len = cu_q[e + 1] - a, mine = (len + TOK - 1) / TOK;
+    const int a = cu_q[e], len = cu_q[e + 1] - a, mine = chunks_of(len, least);
     if (index < base + mine) {
       const int at = (index - base) * TOK;
       return Home{e, a + at, min(TOK, len - at), a};
@@ -54,7 +56,7 @@ __global__ void __launch_bounds__(128, 5)
 delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* __restrict__ conv_w, int taps,
                     const float* __restrict__ a_log, const float* __restrict__ dt_bias, const float* __restrict__ state,
                     long long state_stride, const int* __restrict__ cu_q, int n_entries, const int* __restrict__ slots,
-                    float* __restrict__ records, int first_chunk, Sizes z, float unit_eps) {
+                    float* __restrict__ records, int least, int first_chunk, Sizes z, float unit_eps) {
   pdl_wait();
   pdl_trigger();
   __shared__ __align__(16) float k_s[TOK][DK + 4], q_s[TOK][DK + 4];
@@ -62,7 +64,7 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
   // what multiplies a whole token or a pair of tokens is formed in 64 bits and rounded once
   __shared__ double d_s[TOK][TOK], unit_k[TOK], unit_q[TOK], g_s[TOK], pre_s[TOK];
   __shared__ float beta_s[TOK], fade_k[TOK], fade_q[TOK], last_k[TOK];   // P_i / |k_i|, P_i / (|q_i| sqrt(DK)), R_i / |k_i|
-  const Home home = home_of(cu_q, n_entries, first_chunk + blockIdx.x);
+  const Home home = home_of(cu_q, n_entries, least, first_chunk + blockIdx.x);
   if (home.entry < 0) return;
   const int h = blockIdx.y, kh = h / (z.H / z.G), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float* carry = state + (size_t)slots[home.entry] * state_stride + (size_t)z.H * DK * z.dv;   // [C][taps - 1]
@@ -260,8 +262,8 @@ __device__ __forceinline__ void mma_split(float (&small)[4], float (&large)[4], 
 // the product's k-th place t standing for row 2 t and t + 4 for row 2 t + 1 (on both sides).
 __global__ void __launch_bounds__(THREADS, 2)
 delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ state, long long state_stride,
-                        const int* __restrict__ cu_q, const int* __restrict__ slots, float* __restrict__ o_out, int first_chunk,
-                        int n_chunks, Sizes z) {
+                        const int* __restrict__ cu_q, const int* __restrict__ slots, float* __restrict__ o_out, int least,
+                        int first_chunk, int n_chunks, Sizes z) {
   pdl_wait();
   pdl_trigger();
   // the records are those of the step's chunks first_chunk .. first_chunk + n_chunks - 1, of the entry's those from..to - 1
@@ -273,8 +275,8 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int first = cu_q[e], n = cu_q[e + 1] - first;
   int base = -first_chunk;
-  for (int x = 0; x < e; ++x) base += (cu_q[x + 1] - cu_q[x] + TOK - 1) / TOK;
-  const int from = max(0, -base), to = min((n + TOK - 1) / TOK, n_chunks - base);
+  for (int x = 0; x < e; ++x) base += chunks_of(cu_q[x + 1] - cu_q[x], least);
+  const int from = max(0, -base), to = min(chunks_of(n, least), n_chunks - base);
   if (from >= to) return;
   const int rec_floats = record_floats(z.dv);
   auto fetch = [&](int s) {
@@ -403,30 +405,31 @@ extern "C" int srlm_delta_chunk_record(int dk, int dv, int taps) {
              ? chunks::record_floats(dv) : 0;
 }
 
-// proj float32 [T, ldp] and state as in delta_rule.cu.  Takes the chunks first_chunk .. first_chunk + n_chunks - 1 of those that
-// the step's entries have together, entry by entry: a step whose chunks do not all fit `records` (float32 [n_chunks, H, record])
-// is several calls, in order.  o_out float32 [T, H dv].  Renews S; the carried inputs of the convolution are read and stay.
+// proj float32 [T, ldp] and state as in delta_rule.cu, whose limits hold for an entry of any length.  Serves the entries of
+// `least` tokens and more: the chunks first_chunk .. first_chunk + n_chunks - 1 of those that they have together, entry by entry;
+// a step whose chunks do not all fit `records` (float32 [n_chunks, H, record]) is several calls, in order.  o_out float32 [T, H dv].  Renews S; the carried inputs of the convolution
+// are read and stay.
 extern "C" int srlm_delta_chunks(const float* proj, long long ldp, const float* conv_w, const float* a_log, const float* dt_bias,
                                  float* state, long long state_stride, const int* cu_q, const int* slots, int n_entries,
-                                 float* records, int first_chunk, int n_chunks, float* o_out, int H, int G, int dk, int dv, int taps,
-                                 float unit_eps, cudaStream_t stream) {
+                                 float* records, int least, int first_chunk, int n_chunks, float* o_out, int H, int G, int dk, int dv,
+                                 int taps, float unit_eps, cudaStream_t stream) {
   if (n_entries <= 0 || n_chunks <= 0) return ST_OK;
   const long long C = 2LL * G * dk + (long long)H * dv;
   if (!srlm_delta_chunk_record(dk, dv, taps) || first_chunk < 0 || H <= 0 || G <= 0 || H % G || H > 65535 || n_entries > 65535 ||
-      ldp < C + 2LL * H || C > 0x7fffffff || state_stride < (long long)H * dk * dv + C * (taps - 1))
+      ldp < C + 2LL * H || C * 4 > 200 * 1024 || state_stride < (long long)H * dk * dv + C * (taps - 1))
     return refuse(ST_BAD_SIZE, "delta_chunks: H=%d G=%d dk=%d dv=%d taps=%d ldp=%lld state=%lld entries=%d", H, G, dk, dv, taps,
                   ldp, state_stride, n_entries);
   if ((uintptr_t)state % 8 || state_stride % 2 || (uintptr_t)records % 16)
     return refuse(ST_BAD_ALIGN, "delta_chunks: states start on 8 bytes, records on 16");
   const chunks::Sizes z{H, G, dv, (int)C};
   launch_pdl(chunks::delta_chunks_kernel, dim3(n_chunks, H), dim3(128), 0, stream, proj, ldp, conv_w, taps, a_log, dt_bias,
-             (const float*)state, state_stride, cu_q, n_entries, slots, records, first_chunk, z, unit_eps);
+             (const float*)state, state_stride, cu_q, n_entries, slots, records, least, first_chunk, z, unit_eps);
   const cudaError_t e = cudaFuncSetAttribute(chunks::delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              chunks::WALK_SMEM);
   if (e != cudaSuccess) return refuse((int)e, "delta_chunks: cannot get %d bytes of shared memory", chunks::WALK_SMEM);
   // (not ahead of time: blocks that start while the chunks' kernel drains would share the SMs that happen to be free)
   launch_pdl_if(false, chunks::delta_chunk_walk_kernel, dim3(dv / chunks::COLS, H, n_entries), dim3(chunks::THREADS),
-                chunks::WALK_SMEM, stream, (const float*)records, state, state_stride, cu_q, slots, o_out,
+                chunks::WALK_SMEM, stream, (const float*)records, state, state_stride, cu_q, slots, o_out, least,
                 first_chunk, n_chunks, z);
   return launched();
 }

@@ -13,7 +13,8 @@
 //   delta_conv_carry   -- the slot's last taps-1 inputs after this step;
 //   delta_recurrence   -- the recurrence, token by token within an entry, entries / heads / columns of S in parallel;
 //   delta_output       -- per head o / rms(o) * w * silu(gate) in the activation dtype.
-// Steps with longer portions in bfloat16 go by chunks of tokens instead of the first and the third (delta_chunks.cu).
+// Longer portions in bfloat16 go by chunks of tokens instead of the first and the third (delta_chunks.cu), entry by entry:
+// `below` > 0 leaves entries of that many tokens and more to them.
 // Projection row (proj, [T, ldp]): q (G dk) | k (G dk) | v (H dv) | b (H) | a (H) | gate (H dv).
 #include "common.cuh"
 
@@ -31,13 +32,14 @@ __global__ void delta_prepare_kernel(const TP* __restrict__ proj, long long ldp,
                                      const int* __restrict__ slots, float* __restrict__ qkv_out,
                                      float* __restrict__ beta_out, float* __restrict__ decay_out,
                                      float* __restrict__ qk_out, int H, int G, int dk, int dv, int taps,
-                                     float unit_eps) {
+                                     float unit_eps, int below) {
   pdl_wait();        // launched as a dependent of the kernel ahead: nothing is read before it has finished
   pdl_trigger();
   extern __shared__ float ch[];                              // [C] convolved and activated channels of this token
   const int t = blockIdx.x;
   const int C = 2 * G * dk + H * dv;
   const int e = entry_of_token[t];
+  if (below > 0 && cu_q[e + 1] - cu_q[e] >= below) return;
   const int local = t - cu_q[e];                             // index of the token among the entry's tokens of this step
   const float* carry = state + (size_t)slots[e] * state_stride + (size_t)H * dk * dv;   // [C][taps - 1]
   for (int c = threadIdx.x; c < C; c += blockDim.x) {
@@ -125,7 +127,7 @@ template <int RPL>
 __global__ void __launch_bounds__(kColumnsPerBlock* kLanesPerColumn)
 delta_recurrence_kernel(const float* __restrict__ qkv, const float* __restrict__ beta, const float* __restrict__ decay,
                         const float* __restrict__ qk, float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
-                        const int* __restrict__ slots, float* __restrict__ o_out, int H, int G, int dk, int dv) {
+                        const int* __restrict__ slots, float* __restrict__ o_out, int H, int G, int dk, int dv, int below) {
   pdl_wait();        // launched as a dependent of the kernel ahead: nothing is read before it has finished
   pdl_trigger();
   constexpr int DKP = RPL * kLanesPerColumn;                 // rows held in shared memory (zero beyond dk)
@@ -138,6 +140,7 @@ delta_recurrence_kernel(const float* __restrict__ qkv, const float* __restrict__
   const int kh = h / (H / G);
   const int C = 2 * G * dk + H * dv;
   const int t0 = cu_q[e], n_tok = cu_q[e + 1] - t0;
+  if (below > 0 && n_tok >= below) return;
   float* S_col = state + (size_t)slots[e] * state_stride + ((size_t)h * dv + (live ? col : 0)) * dk;
   float S[RPL];
 #pragma unroll
@@ -303,7 +306,7 @@ extern "C" int srlm_delta_prepare(const void* proj, int proj_dtype, long long ld
                                   const float* a_log, const float* dt_bias, float* state, long long state_stride,
                                   const int* entry_of_token, const int* cu_q, const int* slots, int n_entries,
                                   float* qkv_out, float* beta_out, float* decay_out, float* qk_out, int T, int H,
-                                  int G, int dk, int dv, int taps, float unit_eps, cudaStream_t stream) {
+                                  int G, int dk, int dv, int taps, float unit_eps, int below, cudaStream_t stream) {
   if (T <= 0) return ST_OK;
   const long long C = 2LL * G * dk + (long long)H * dv;
   if (!delta_sizes_ok(H, G, dk, dv, taps) || ldp < C + 2LL * H + (long long)H * dv || C * 4 > 200 * 1024 ||
@@ -316,7 +319,7 @@ extern "C" int srlm_delta_prepare(const void* proj, int proj_dtype, long long ld
       cudaFuncSetAttribute(delta_prepare_kernel<TP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     launch_pdl(delta_prepare_kernel<TP>, dim3(T), dim3(256), smem, stream, (const TP*)proj, ldp, conv_w, a_log, dt_bias, state, state_stride,
                                                        entry_of_token, cu_q, slots, qkv_out, beta_out, decay_out, qk_out,
-                                                       H, G, dk, dv, taps, unit_eps);
+                                                       H, G, dk, dv, taps, unit_eps, below);
   });
   if (int r = launched()) return r;
   return srlm_delta_conv_carry(proj, proj_dtype, ldp, state, state_stride, cu_q, slots, n_entries, H, G, dk, dv, taps, stream);
@@ -324,7 +327,7 @@ extern "C" int srlm_delta_prepare(const void* proj, int proj_dtype, long long ld
 
 extern "C" int srlm_delta_recurrence(const float* qkv, const float* beta, const float* decay, const float* qk, float* state,
                                      long long state_stride, const int* cu_q, const int* slots, int n_entries,
-                                     float* o_out, int H, int G, int dk, int dv, cudaStream_t stream) {
+                                     float* o_out, int H, int G, int dk, int dv, int below, cudaStream_t stream) {
   if (n_entries <= 0) return ST_OK;
   if (!delta_sizes_ok(H, G, dk, dv, 1) || n_entries > 65535 || H > 65535)
     return refuse(ST_BAD_SIZE, "delta_recurrence: H=%d G=%d dk=%d dv=%d entries=%d (dk <= 512)", H, G, dk, dv, n_entries);
@@ -337,7 +340,7 @@ extern "C" int srlm_delta_recurrence(const float* qkv, const float* beta, const 
     if (smem > 48 * 1024)                                                                                        \
       cudaFuncSetAttribute(delta_recurrence_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);  \
     launch_pdl(delta_recurrence_kernel<R>, dim3(grid), dim3(threads), smem, stream, qkv, beta, decay, qk, state, state_stride, cu_q, \
-                                                                slots, o_out, H, G, dk, dv);                     \
+                                                                slots, o_out, H, G, dk, dv, below);              \
   } while (0)
   if (rpl <= 4) SRLM_DELTA_CASE(4);
   else if (rpl <= 8) SRLM_DELTA_CASE(8);

@@ -1527,26 +1527,40 @@ class KernelLibrary:
 
     # ---- the gated delta rule ------------------------------------------------------------------
     def delta_prepare(self, ctx, proj, conv_w, a_log, dt_bias, state, qkv_out, beta_out, decay_out, qk_out, H, G, dk,
-                      dv, taps, unit_eps):
+                      dv, taps, unit_eps, below=0):
         """Convolution + SiLU of the q | k | v columns of proj (carrying each slot's last taps-1 inputs in its
-        state), unit vectors, beta, decay and q . k (float32 [T, G]) for every token; then the slots' carried inputs are renewed.
+        state), unit vectors, beta, decay and q . k (float32 [T, G]) for every token (below > 0: of the entries of fewer tokens
+        than that); then the slots' carried inputs are renewed, every entry's.
         state: float32 [slots, state_size], laid out as csrc/kernels/delta_rule.cu says."""
         self._check(self.lib.srlm_delta_prepare(
             _ptr(proj), dtype_code(proj.dtype), C.c_longlong(proj.stride(0)), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias),
             _ptr(state), C.c_longlong(state.stride(0)), _ptr(ctx.entry_of_token), _ptr(ctx.cu_q), _ptr(ctx.slots),
             C.c_int(ctx.n_entries), _ptr(qkv_out), _ptr(beta_out), _ptr(decay_out), _ptr(qk_out), C.c_int(proj.shape[0]),
-            C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps), _stream()), "delta_prepare")
+            C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps), C.c_int(below),
+            _stream()), "delta_prepare")
         if taps > 1:
             self.launches += 1
 
-    def delta_recurrence(self, ctx, qkv, beta, decay, qk, state, o_out, H, G, dk, dv):
+    def delta_recurrence(self, ctx, qkv, beta, decay, qk, state, o_out, H, G, dk, dv, below=0):
         self._check(self.lib.srlm_delta_recurrence(
             _ptr(qkv), _ptr(beta), _ptr(decay), _ptr(qk), _ptr(state), C.c_longlong(state.stride(0)), _ptr(ctx.cu_q),
             _ptr(ctx.slots), C.c_int(ctx.n_entries), _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv),
-            _stream()), "delta_recurrence")
+            C.c_int(below), _stream()), "delta_recurrence")
+
+    def delta_walk(self, ctx, proj, conv_w, a_log, dt_bias, state, o_out, H, G, dk, dv, taps, unit_eps, below=0):
+        """o_out float32 [T, H dv] = the gated delta rule of the step's tokens, token by token (below > 0: of the entries of
+        fewer tokens than that); S of those entries and the carried inputs of all are renewed."""
+        T, get = proj.shape[0], ctx.workspace.get
+        qkv = get("delta.qkv", T, 2 * G * dk + H * dv, torch.float32)
+        beta, decay = get("delta.beta", T, H, torch.float32), get("delta.decay", T, H, torch.float32)
+        qk = get("delta.qk", T, G, torch.float32)
+        self.delta_prepare(ctx, proj, conv_w, a_log, dt_bias, state, qkv, beta, decay, qk, H, G, dk, dv, taps, unit_eps, below)
+        self.delta_recurrence(ctx, qkv, beta, decay, qk, state, o_out, H, G, dk, dv, below)
 
     DELTA_CHUNK = 16         # tokens of a chunk
-    DELTA_CHUNKS_FROM = 16   # steps with an entry of at least this many tokens go by chunks
+    # Entries of at least this many tokens go by chunks.  A layer in us, by chunks | token by token (16 heads of 128 x 128): one
+    # portion of 16 tokens 60 | 59, of 32 60 | 68; 8 of 16 79 | 93; 64 of 16 290 | 284, of 32 407 | 487; 32 heads: one of 16 73 | 101.
+    DELTA_CHUNKS_FROM = 16
 
     # Chunks whose records lie in memory at a time (41 KB a chunk and head of 128 x 128: 105 MB for 16 heads); a step that has more
     # takes them by turns, S in its slot in between.  160: the chunks of 2,048 tokens in up to 32 requests.
@@ -1558,21 +1572,22 @@ class KernelLibrary:
         return min(self.DELTA_CHUNKS_HELD, 2 * max_tokens // (self.DELTA_CHUNK + 1) + 1)
 
     def delta_by_chunks(self, ctx, state, dk, dv, taps) -> int:
-        """How many chunks of 16 tokens the step's entries make, 0 where the step goes token by token: decode steps and
-        short portions, sizes that the chunked kernels do not take, and the float32 path, whose results do not depend on
-        where a request is cut."""
+        """How many chunks of 16 tokens the step's longer entries make together (those that go by chunks, whatever else is in
+        the step), 0 where every entry goes token by token: decode steps and short portions, sizes that the chunked kernels do
+        not take, and the float32 path, whose results do not depend on where a request is cut."""
         if ctx.dtype != torch.bfloat16 or ctx.max_q_len < self.DELTA_CHUNKS_FROM:
             return 0
         if not self.lib.srlm_delta_chunk_record(C.c_int(dk), C.c_int(dv), C.c_int(taps)):
             return 0
         if state.stride(0) % 2 or state.data_ptr() % 8:        # the walk moves two rows of a column at a time
             return 0
-        return sum(-(-n // self.DELTA_CHUNK) for n in ctx.host["q_lens"])
+        return sum(-(-n // self.DELTA_CHUNK) for n in ctx.host["q_lens"] if n >= self.DELTA_CHUNKS_FROM)
 
     def delta_chunks(self, ctx, proj, conv_w, a_log, dt_bias, state, o_out, n_chunks, H, G, dk, dv, taps, unit_eps):
         """o_out float32 [T, H dv] = the gated delta rule of the step's tokens from the projection (float32 rows: q | k | v |
-        beta | decay ..), by chunks of 16 tokens, as csrc/kernels/delta_chunks.cu says; S and the convolution's carried
-        inputs in ``state`` are renewed."""
+        beta | decay ..): the longer entries by chunks of 16 tokens, as csrc/kernels/delta_chunks.cu says (n_chunks: what
+        delta_by_chunks counted), the others token by token; S and the convolution's carried inputs in ``state`` are
+        renewed."""
         if proj.dtype != torch.float32:
             raise ShapeError("delta_chunks: the projection is float32")
         record = int(self.lib.srlm_delta_chunk_record(C.c_int(dk), C.c_int(dv), C.c_int(taps)))
@@ -1582,10 +1597,12 @@ class KernelLibrary:
             self._check(self.lib.srlm_delta_chunks(
                 _ptr(proj), C.c_longlong(proj.stride(0)), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias), _ptr(state),
                 C.c_longlong(state.stride(0)), _ptr(ctx.cu_q), _ptr(ctx.slots), C.c_int(ctx.n_entries), _ptr(records),
-                C.c_int(first), C.c_int(min(held, n_chunks - first)), _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv),
-                C.c_int(taps), C.c_float(unit_eps), _stream()), "delta_chunks")
+                C.c_int(self.DELTA_CHUNKS_FROM), C.c_int(first), C.c_int(min(held, n_chunks - first)), _ptr(o_out),
+                C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps), _stream()), "delta_chunks")
             self.launches += 1
-        if taps > 1:
+        if min(ctx.host["q_lens"]) < self.DELTA_CHUNKS_FROM:       # the carried inputs are renewed behind the last who reads them
+            self.delta_walk(ctx, proj, conv_w, a_log, dt_bias, state, o_out, H, G, dk, dv, taps, unit_eps, self.DELTA_CHUNKS_FROM)
+        elif taps > 1:
             self._check(self.lib.srlm_delta_conv_carry(
                 _ptr(proj), dtype_code(proj.dtype), C.c_longlong(proj.stride(0)), _ptr(state), C.c_longlong(state.stride(0)),
                 _ptr(ctx.cu_q), _ptr(ctx.slots), C.c_int(ctx.n_entries), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv),

@@ -61,7 +61,7 @@ def test_against_float64(H, G, dv, taps, lens, eps):
     row += row % 2
     state = rand(6, row)
     slots = [4, 1, 5, 2][:len(lens)]
-    proj = rand(T, C + 2 * H + 3)
+    proj = rand(T, C + 2 * H + H * dv + 3)
     proj[T // 2:, C + H:C + 2 * H] += 8.0            # decays that underflow within a chunk, behind decays of nearly one
     conv_w, dt_bias = rand(C, taps) * 0.5, rand(H) - 4.0
     a_log = torch.log(1.0 + 15.0 * torch.rand(H, generator=gen, device=DEV))
@@ -72,7 +72,7 @@ def test_against_float64(H, G, dv, taps, lens, eps):
     if max(lens) < ops.DELTA_CHUNKS_FROM:
         assert n == 0
         return
-    assert n == sum(-(-x // 16) for x in lens)
+    assert n == sum(-(-x // 16) for x in lens if x >= ops.DELTA_CHUNKS_FROM)
     ops.delta_chunks(ctx, proj, conv_w, a_log, dt_bias, state, o, n, H, G, DK, dv, taps, eps)
     want_o, want_state, t = [], before.clone(), 0
     for x, slot in zip(lens, slots):
@@ -170,6 +170,34 @@ def test_steps_whose_chunks_are_taken_by_turns(held):
     o2, state2, work = walked(lens, held)
     assert torch.equal(o, o2) and torch.equal(state, state2)
     assert max(b.shape[0] for (name, _, _), b in work._bufs.items() if name == "delta.records") == 4 * held
+
+
+def test_an_entry_does_not_depend_on_who_shares_the_step():
+    """A decoded token, a few tokens and a portion: the same bits beside others and alone (the walk, or the chunks)."""
+    from safetyraise_lmengine_b200.kernels import ops
+    lens, H, dv, taps = [1, 40, 3, 15, 16], 4, 128, 4
+    C = 3 * H * DK
+    g = torch.Generator(device=DEV).manual_seed(11)
+    rand = lambda *s: torch.randn(*s, generator=g, device=DEV)
+    proj, states = rand(sum(lens), C + 2 * H + H * dv), rand(len(lens), H * DK * dv + C * (taps - 1))
+    conv_w, dt_bias, a_log = rand(C, taps) * 0.5, rand(H) - 4.0, rand(H)
+
+    def go(lens, slots, rows):
+        ctx, state = Ctx(lens, slots), states.clone()
+        o = torch.full((sum(lens), H * dv), float("nan"), device=DEV)
+        n = ops.delta_by_chunks(ctx, state, DK, dv, taps)
+        if n:
+            ops.delta_chunks(ctx, rows, conv_w, a_log, dt_bias, state, o, n, H, H, DK, dv, taps, EPS)
+        else:
+            ops.delta_walk(ctx, rows, conv_w, a_log, dt_bias, state, o, H, H, DK, dv, taps, EPS)
+        return o, state
+
+    o, state = go(lens, list(range(len(lens))), proj)
+    t = 0
+    for e, n in enumerate(lens):
+        alone_o, alone_state = go([n], [e], proj[t:t + n].contiguous())
+        assert torch.equal(alone_o, o[t:t + n]) and torch.equal(alone_state[e], state[e])
+        t += n
 
 
 def test_the_records_do_not_grow_with_the_portions():
