@@ -104,10 +104,8 @@ __device__ unsigned long long cluster_best(const float* row, int V, Slice sl, un
   }
   cluster_sync();
   best = 0;
-  const uint32_t n = cluster_size();
-#pragma unroll
-  for (uint32_t r = 0; r < kMaxCluster; ++r) {
-    const unsigned long long other = r < n ? peer_u64(slot, r) : 0;
+  for (uint32_t r = 0; r < cluster_size(); ++r) {
+    const unsigned long long other = peer_u64(slot, r);
     best = other > best ? other : best;
   }
   cluster_sync();                       // nobody rewrites its slot while another block still reads it
