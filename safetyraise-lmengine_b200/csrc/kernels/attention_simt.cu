@@ -15,26 +15,32 @@
 // rows, a lane the dimensions lane + 32 i.  Bound by the FMA and shared-memory pipes for prompts (2,048 tokens, 32 heads of
 // 128: 2.8 ms; 34.2 with a warp a row that read its keys from global memory), by the chain of spans of the longest request
 // for decode steps (8 requests of 2,048: 0.19 ms; 2.75).
+//
+// Such a block fills an SM.  Where a step has many requests of few rows, or few keys, the small form takes 8 rows and spans of 32
+// keys without a second buffer: several blocks an SM hide the trips to memory that a short request consists of (64 requests of 16 keys, 32 heads of 64: 118 us
+// in the large form, which leaves such a request an SM, 15 in the small one, 19 with the warp a row; see simt_small).
 #include <math_constants.h>
 
 #include "common.cuh"
 
 namespace srlm {
 
-constexpr int SA_THREADS = 256, SA_WARPS = 8, SA_ROWS = 32, SA_OWN = SA_ROWS / SA_WARPS;
-
-template <int DIMS>                  // dimensions a lane owns: heads up to 32 * DIMS
-struct SimtSpan {
-  static constexpr int KEYS = DIMS <= 2 ? 128 : DIMS <= 4 ? 64 : 32;
+template <int DIMS, bool SMALL>      // DIMS: dimensions a lane owns, heads up to 32 * DIMS
+struct SimtForm {
+  static constexpr int KEYS = SMALL ? 32 : DIMS <= 2 ? 128 : DIMS <= 4 ? 64 : 32;
+  static constexpr int THREADS = SMALL ? 128 : 256, WARPS = THREADS / 32;
+  static constexpr int STAGES = SMALL ? 1 : 2, ROWS = SMALL ? 8 : 32, OWN = ROWS / WARPS;
+  static constexpr int BLOCKS = SMALL ? (DIMS <= 2 ? 8 : DIMS <= 4 ? 5 : 3) : 1;      // an SM
 };
 
 // Floats from a staged key to the next: an odd number of 16-byte pieces, so that lanes on neighbouring keys share no bank.
 __host__ __device__ __forceinline__ int simt_key_ld(int hd) { return 4 * (((hd + 3) / 4) | 1); }
 __host__ __device__ __forceinline__ int simt_row_ld(int hd) { return (hd + 3) / 4 * 4; }
 
-static size_t simt_smem(int hd, int keys) {
-  return sizeof(float) * (2ull * keys * (simt_key_ld(hd) + simt_row_ld(hd)) + (size_t)SA_ROWS * simt_row_ld(hd) +
-                          (size_t)SA_ROWS * keys) + sizeof(long long) * 2 * keys;
+template <typename F>
+static size_t simt_smem(int hd) {
+  return sizeof(float) * ((size_t)F::STAGES * F::KEYS * (simt_key_ld(hd) + simt_row_ld(hd)) + (size_t)F::ROWS * simt_row_ld(hd) +
+                          (size_t)F::ROWS * F::KEYS) + sizeof(long long) * 2 * F::KEYS;
 }
 
 // Scores of `NR` neighbouring rows against a lane's key.
@@ -61,20 +67,22 @@ struct SimtYes { static constexpr bool value = true; };
 struct SimtNo { static constexpr bool value = false; };
 
 // The rows of tokens t0 .. t0 + tokens - 1 (one request) and heads h_lo .. h_lo + heads - 1 of KV head kvh.
-template <typename TA, int DIMS, bool COPY>       // COPY: float32 rows of whole 16-byte pieces, fetched asynchronously
+template <typename TA, int DIMS, bool COPY, bool SMALL>       // COPY: float32 rows of whole 16-byte pieces, fetched asynchronously
 __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cache, const TA* __restrict__ v_cache,
                           TA* __restrict__ out, const int* __restrict__ table, const int* __restrict__ positions, int t0,
                           int tokens, int nq, int nkv, int kvh, int h_lo, int heads, int hd, int page_size, float scale,
                           int window) {
-  constexpr int KEYS = SimtSpan<DIMS>::KEYS;
+  typedef SimtForm<DIMS, SMALL> Form;
+  constexpr int KEYS = Form::KEYS, STAGES = Form::STAGES, SA_ROWS = Form::ROWS, SA_OWN = Form::OWN,
+                SA_THREADS = Form::THREADS, SA_WARPS = Form::WARPS;
   extern __shared__ __align__(16) float simt_sh[];
   const int g = nq / nkv;
   const int rows = tokens * heads;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ldk = simt_key_ld(hd), ldv = simt_row_ld(hd), pieces = ldv / 4;
-  float* k_sh = simt_sh;                                     // [2][KEYS][ldk]
-  float* v_sh = k_sh + 2 * KEYS * ldk;                       // [2][KEYS][ldv]
-  float* q_sh = v_sh + 2 * KEYS * ldv;                       // [SA_ROWS][ldv]
+  float* k_sh = simt_sh;                                     // [STAGES][KEYS][ldk]
+  float* v_sh = k_sh + STAGES * KEYS * ldk;                  // [STAGES][KEYS][ldv]
+  float* q_sh = v_sh + STAGES * KEYS * ldv;                  // [SA_ROWS][ldv]
   float* s_sh = q_sh + SA_ROWS * ldv;                        // [SA_ROWS][KEYS]: scores, then weights
   long long* at_sh = reinterpret_cast<long long*>(s_sh + SA_ROWS * KEYS);      // [2][KEYS]: cache row of a key, or -1
 
@@ -100,8 +108,8 @@ __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cac
   };
   auto fetch = [&](int span) {
     if (span < spans) {
-      float* kd = k_sh + (span & 1) * KEYS * ldk;
-      float* vd = v_sh + (span & 1) * KEYS * ldv;
+      float* kd = k_sh + span % STAGES * KEYS * ldk;
+      float* vd = v_sh + span % STAGES * KEYS * ldv;
       const long long* at = at_sh + (span & 1) * KEYS;
       for (int i = tid; i < KEYS * pieces; i += SA_THREADS) {
         const int key = i / pieces, c = (i % pieces) * 4;
@@ -141,26 +149,30 @@ __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cac
 
   locate(0);
   __syncthreads();
-  fetch(0);
-  locate(1);
-  __syncthreads();
+  if constexpr (STAGES == 2) {
+    fetch(0);
+    locate(1);
+    __syncthreads();
+  }
   for (int span = 0; span < spans; ++span) {
-    fetch(span + 1);
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    fetch(span + STAGES - 1);
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 1) : "memory");
     __syncthreads();                                         // the span has arrived, the places of the next are read
     const int j0 = first + span * KEYS;
+    const int here = min(KEYS / 32, (last - j0) / 32 + 1);   // blocks of 32 keys that somebody may see
     {
-      const float* ks = k_sh + (span & 1) * KEYS * ldk;
+      const float* ks = k_sh + span % STAGES * KEYS * ldk;
+      constexpr int EACH = SMALL ? 2 : 8;                    // rows a task: two where a span is one block of keys for four warps
       const bool few = rows <= 2;
-      const int groups = few ? 1 : (rows + 7) / 8;
-      for (int task = warp; task < groups * (KEYS / 32); task += SA_WARPS) {
-        const int kb = task % (KEYS / 32) * 32, r0 = task / (KEYS / 32) * 8;
+      const int groups = few ? 1 : (rows + EACH - 1) / EACH;
+      for (int task = warp; task < groups * here; task += SA_WARPS) {
+        const int kb = task % here * 32, r0 = task / here * EACH;
         const float* kp = ks + (kb + lane) * ldk;
-        if (few) {
+        if (SMALL || few) {
           float dot[2];
-          simt_scores<2>(kp, q_sh, ldv, pieces, dot);
+          simt_scores<2>(kp, q_sh + r0 * ldv, ldv, pieces, dot);
 #pragma unroll
-          for (int r = 0; r < 2; ++r) s_sh[r * KEYS + kb + lane] = dot[r] * scale;
+          for (int r = 0; r < 2; ++r) s_sh[(r0 + r) * KEYS + kb + lane] = dot[r] * scale;
         } else {
           float dot[8];
           simt_scores<8>(kp, q_sh + r0 * ldv, ldv, pieces, dot);
@@ -169,11 +181,11 @@ __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cac
         }
       }
     }
-    locate(span + 2);
+    locate(span + STAGES);
     __syncthreads();
-    const float* vs = v_sh + (span & 1) * KEYS * ldv;
+    const float* vs = v_sh + span % STAGES * KEYS * ldv;
 #pragma unroll 1
-    for (int kb = 0; kb < KEYS; kb += 32) {
+    for (int kb = 0; kb < 32 * here; kb += 32) {
       const int jb = j0 + kb, j = jb + lane;
       bool any = false, all = true;                          // (uniform over the warp)
 #pragma unroll
@@ -241,14 +253,15 @@ __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cac
 
 // Blocks (tile of tokens, KV head, z): of the runs of tokens of one request within the tile, the block serves the z-th and
 // every gridDim.z-th behind it.
-template <typename TA, int DIMS, bool COPY>
-__global__ void __launch_bounds__(SA_THREADS, 1)
+template <typename TA, int DIMS, bool COPY, bool SMALL>
+__global__ void __launch_bounds__((SimtForm<DIMS, SMALL>::THREADS), (SimtForm<DIMS, SMALL>::BLOCKS))
 paged_attention_simt_kernel(const TA* __restrict__ q, const TA* __restrict__ k_cache, const TA* __restrict__ v_cache,
                             TA* __restrict__ out, const int* __restrict__ block_table, int table_stride,
                             const int* __restrict__ entry_of_token, const int* __restrict__ positions, int T, int nq,
                             int nkv, int hd, int page_size, float scale, int window, int tile_tokens, int head_groups) {
-  const int g = nq / nkv, kvh = blockIdx.y / head_groups, h_lo = (blockIdx.y % head_groups) * SA_ROWS;
-  const int heads = min(g - h_lo, SA_ROWS);                  // (tile_tokens is 1 where a group has more heads than rows)
+  constexpr int ROWS = SimtForm<DIMS, SMALL>::ROWS;
+  const int g = nq / nkv, kvh = blockIdx.y / head_groups, h_lo = (blockIdx.y % head_groups) * ROWS;
+  const int heads = min(g - h_lo, ROWS);                  // (tile_tokens is 1 where a group has more heads than rows)
   const int t_end = min(((int)blockIdx.x + 1) * tile_tokens, T);
   int run = 0;
   for (int t = blockIdx.x * tile_tokens; t < t_end; ++run) {
@@ -256,27 +269,56 @@ paged_attention_simt_kernel(const TA* __restrict__ q, const TA* __restrict__ k_c
     int tokens = 1;
     while (t + tokens < t_end && entry_of_token[t + tokens] == entry) ++tokens;
     if (run % gridDim.z == blockIdx.z)
-      simt_rows<TA, DIMS, COPY>(q, k_cache, v_cache, out, block_table + (size_t)entry * table_stride, positions, t, tokens, nq,
+      simt_rows<TA, DIMS, COPY, SMALL>(q, k_cache, v_cache, out, block_table + (size_t)entry * table_stride, positions, t, tokens, nq,
                                 nkv, kvh, h_lo, heads, hd, page_size, scale, window);
     t += tokens;
   }
 }
 
-template <typename TA, int DIMS, bool COPY>
-static int run_simt(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
-                    int table_stride, const int* entry_of_token, const int* positions, int T, int nq, int nkv, int hd,
-                    int page_size, float scale, int window, int runs, cudaStream_t stream) {
-  const size_t smem = simt_smem(hd, SimtSpan<DIMS>::KEYS);
-  const auto kernel = paged_attention_simt_kernel<TA, DIMS, COPY>;
+// Which form.  Requests of up to 8 rows (decode): the small one once there are more of them than SMs (us, large | small: 16 heads
+// over 8 of 64, 64 requests of 700 keys 174 | 79, of 16 27 | 7; below that the long spans win, 4 requests of 700 43 | 76).
+// Prompts: the small one where they see few keys (16 over 8 heads of 64, 20 tokens 12.4 | 7.5), or where the heads are wide,
+// whose spans are short in both, and its finer blocks fill the GPU better (32 over 4 of 128, 40 tokens 19.9 | 14.5, behind 500
+// keys 103 | 74; 300 tokens of 16 over 8 of 64 54 | 62).
+static bool simt_small(int T, int nq, int nkv, int hd, int runs, int most_keys) {
+  const int g = nq / nkv, rows = 32, tile_tokens = g >= rows ? 1 : rows / g;
+  if (runs > T) runs = T;
+  const long long tiles = (T + tile_tokens - 1) / tile_tokens;
+  const long long blocks = (tiles > runs ? tiles : runs) * nkv * ((g + rows - 1) / rows);      // of the large form
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    sms = 148;
+  if ((long long)T * g <= 8ll * runs) return blocks > sms;
+  return (most_keys > 0 && most_keys <= 128) || (hd > 64 && blocks <= 2 * sms);
+}
+
+template <typename TA, int DIMS, bool COPY, bool SMALL>
+static int run_simt_form(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
+                         int table_stride, const int* entry_of_token, const int* positions, int T, int nq, int nkv, int hd,
+                         int page_size, float scale, int window, int runs, cudaStream_t stream) {
+  typedef SimtForm<DIMS, SMALL> Form;
+  const size_t smem = simt_smem<Form>(hd);
+  const auto kernel = paged_attention_simt_kernel<TA, DIMS, COPY, SMALL>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const int g = nq / nkv, head_groups = (g + SA_ROWS - 1) / SA_ROWS;
-  const int tile_tokens = g >= SA_ROWS ? 1 : SA_ROWS / g;
+  const int g = nq / nkv, head_groups = (g + Form::ROWS - 1) / Form::ROWS;
+  const int tile_tokens = g >= Form::ROWS ? 1 : Form::ROWS / g;
   const int z = runs < 1 ? 1 : runs < tile_tokens ? runs : tile_tokens;
-  kernel<<<dim3((T + tile_tokens - 1) / tile_tokens, nkv * head_groups, z), SA_THREADS, smem, stream>>>(
+  kernel<<<dim3((T + tile_tokens - 1) / tile_tokens, nkv * head_groups, z), Form::THREADS, smem, stream>>>(
       (const TA*)q, (const TA*)k_cache, (const TA*)v_cache, (TA*)out, block_table, table_stride, entry_of_token, positions, T,
       nq, nkv, hd, page_size, scale, window, tile_tokens, head_groups);
   return launched();
+}
+
+template <typename TA, int DIMS, bool COPY>
+static int run_simt(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
+                    int table_stride, const int* entry_of_token, const int* positions, int T, int nq, int nkv, int hd,
+                    int page_size, float scale, int window, int runs, int most_keys, cudaStream_t stream) {
+  if (simt_small(T, nq, nkv, hd, runs, most_keys))
+    return run_simt_form<TA, DIMS, COPY, true>(q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T,
+                                               nq, nkv, hd, page_size, scale, window, runs, stream);
+  return run_simt_form<TA, DIMS, COPY, false>(q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T, nq,
+                                              nkv, hd, page_size, scale, window, runs, stream);
 }
 
 template <typename TA, bool COPY, typename... Args>
@@ -290,16 +332,17 @@ static int run_simt_dims(int hd, Args... args) {
 
 using namespace srlm;
 
-// runs: how many requests' tokens may stand beside each other in a tile of tokens (a hint: it spreads them over blocks).
+// runs: how many requests' tokens may stand beside each other in a tile of tokens (a hint: it spreads them over blocks);
+// most_keys: no request of the step has more keys (a hint too; 0: not known).
 extern "C" int srlm_paged_attention_simt(const void* q, const void* k_cache, const void* v_cache,
                                          void* out, int act_dtype, int cache_dtype,
                                          const int* block_table, int table_stride,
                                          const int* entry_of_token, const int* positions, int T, int nq,
                                          int nkv, int hd, int page_size, float scale, int window, int runs,
-                                         cudaStream_t stream) {
+                                         int most_keys, cudaStream_t stream) {
   if (T <= 0) return ST_OK;
   if (nq <= 0 || nkv <= 0 || nq % nkv || hd <= 0 || hd > 256 || page_size <= 0 ||
-      nkv * ((nq / nkv + SA_ROWS - 1) / SA_ROWS) > 65535)
+      nkv * ((nq / nkv + 7) / 8) > 65535)
     return refuse(ST_BAD_SIZE,
                   "paged_attention_simt: nq=%d nkv=%d hd=%d page_size=%d (needs nq %% nkv == 0, hd <= %d)",
                   nq, nkv, hd, page_size, 256);
@@ -309,11 +352,11 @@ extern "C" int srlm_paged_attention_simt(const void* q, const void* k_cache, con
   if (act_dtype == DT_F32) {
     if (hd % 4 == 0 && ((uintptr_t)k_cache | (uintptr_t)v_cache) % 16 == 0)
       return run_simt_dims<float, true>(hd, q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T,
-                                        nq, nkv, hd, page_size, scale, window, runs, stream);
+                                        nq, nkv, hd, page_size, scale, window, runs, most_keys, stream);
     return run_simt_dims<float, false>(hd, q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T,
-                                       nq, nkv, hd, page_size, scale, window, runs, stream);
+                                       nq, nkv, hd, page_size, scale, window, runs, most_keys, stream);
   }
   if (act_dtype != DT_BF16) return refuse(ST_BAD_DTYPE, "dtype code %d is not known", act_dtype);
   return run_simt_dims<bf16, false>(hd, q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T, nq,
-                                    nkv, hd, page_size, scale, window, runs, stream);
+                                    nkv, hd, page_size, scale, window, runs, most_keys, stream);
 }

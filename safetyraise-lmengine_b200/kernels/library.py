@@ -252,7 +252,8 @@ class KernelLibrary:
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(out), dtype_code(q.dtype), dtype_code(k_cache.dtype),
             _ptr(block_table), C.c_int(block_table.stride(0)), _ptr(entry_of_token), _ptr(positions),
             C.c_int(T), C.c_int(nq), C.c_int(nkv), C.c_int(hd), C.c_int(page_size), C.c_float(scale),
-            C.c_int(window or 0), C.c_int(block_table.shape[0]), _stream()), "paged_attention_simt")
+            C.c_int(window or 0), C.c_int(block_table.shape[0]), C.c_int(block_table.shape[1] * page_size), _stream()),
+            "paged_attention_simt")
 
     # ---- matrix products ----------------------------------------------------
     def gemm_tn_simt(self, a, w, out):

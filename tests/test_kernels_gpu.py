@@ -292,6 +292,31 @@ def test_paged_attention_simt_spans_and_runs(nq, nkv, hd, ps, dt, window):
     assert torch.equal(mixed, out[order])
 
 
+@pytest.mark.parametrize("nq, nkv, hd, ps", [(4, 2, 64, 16), (3, 3, 20, 5), (16, 2, 128, 16), (40, 2, 130, 7), (4, 4, 256, 8), (9, 1, 80, 16)])
+@pytest.mark.parametrize("dt", ACT)
+@pytest.mark.parametrize("window", [0, 40])
+def test_paged_attention_simt_forms_agree_bit_for_bit(nq, nkv, hd, ps, dt, window):
+    """Many requests at once take the form with several blocks an SM, the same requests a few at a time the one with long spans;
+    a prompt of few keys the one or the other by the width of its table.  A row's result is the same in both."""
+    g = torch.Generator().manual_seed(nq + hd)
+    lens = torch.randint(1, 200, (330,), generator=g).tolist()
+    q, kc, vc, _, bt, eot, pos = make_paged_case(nq, nkv, hd, ps, dt, [1] * 330, lens, pages=sum(-(-n // ps) for n in lens) + 1)
+
+    def run(q, bt, eot, pos):
+        out = torch.empty_like(q)
+        ops().paged_attention_simt(q, kc, vc, out, bt, eot, pos, nq, nkv, hd, ps, 1 / math.sqrt(hd), window)
+        return out
+
+    whole = run(q, bt, eot, pos)
+    parts = [run(q[i:i + 6], bt[i:i + 6], eot[i:i + 6] - i, pos[i:i + 6]) for i in range(0, 330, 6)]
+    assert torch.isfinite(whole).all() and torch.equal(whole, torch.cat(parts))
+    for n in (1, 5, 31, 100):
+        q, kc, vc, _, bt, eot, pos = make_paged_case(nq, nkv, hd, ps, dt, [n], [n], pages=max(64, 200 // ps))
+        wide = torch.zeros(1, 600 // ps, dtype=torch.int32, device=DEV)
+        wide[:, :bt.shape[1]] = bt
+        assert torch.equal(run(q, bt, eot, pos), run(q, wide, eot, pos))
+
+
 def test_argmax_ties_go_to_the_lowest_id():
     logits = torch.zeros(4, 1000, device=DEV)
     logits[0, [5, 700]] = 3.0
