@@ -215,15 +215,15 @@ __device__ __forceinline__ void scan_load_row(const float* src, float (&dst)[NPL
 constexpr int kScanWalkers = kScanLanes * kScanChannels, kScanThreads = 2 * kScanWalkers;
 constexpr int scan_buffers(int npl) { return npl <= 2 ? 8 : npl <= 4 ? 7 : npl <= 8 ? 6 : 5; }
 constexpr int kScanPlane = kScanChunk * kScanChannels;
-// floats of shared memory: the buffers (B | C up to the lanes' reach, three planes), two of pairs, two of y
-constexpr int scan_floats(int npl) {
-  return scan_buffers(npl) * (kScanChunk * 2 * npl * kScanLanes + 3 * kScanPlane) + 2 * 2 * kScanPlane + 2 * kScanPlane;
+// floats of shared memory: two of pairs, two of y, `held` buffers (B | C up to the lanes' reach, three planes)
+constexpr int scan_floats(int npl, int held) {
+  return 2 * 2 * kScanPlane + 2 * kScanPlane + held * (kScanChunk * 2 * npl * kScanLanes + 3 * kScanPlane);
 }
 __device__ __forceinline__ void scan_helpers_meet() { asm volatile("bar.sync 1, %0;" ::"n"(kScanWalkers) : "memory"); }
 
 // WIDE: channels, N, the rows and the pointers allow copies of 16 bytes
 template <typename TO, int NPL, bool WIDE>
-__global__ void __launch_bounds__(kScanThreads)
+__global__ void __launch_bounds__(kScanThreads, NPL <= 4 ? 5 : NPL <= 8 ? 4 : 3)
 selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz, long long ld_xz,
                       const float* __restrict__ dbc, long long ld_dbc, int b_off, const float* __restrict__ dt_raw,
                       const float* __restrict__ dt_bias, const float* __restrict__ A, const float* __restrict__ D,
@@ -235,10 +235,13 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
   constexpr int K = scan_buffers(NPL);
   pdl_wait();
   extern __shared__ __align__(16) float scan_smem[];
-  float* bc_s = scan_smem;                                  // [K][chunk][2 NP]: B, then C
-  float* raw_s = bc_s + K * BC;                             // [K][3][chunk][channels of the block]: raw dt, x, z
-  float2* step_s = reinterpret_cast<float2*>(raw_s + K * 3 * YS);       // [2][chunk][channels of the block]: dt, dt x
-  float* y_s = reinterpret_cast<float*>(step_s + 2 * YS);   // [2][chunk][channels of the block]
+  float2* step_s = reinterpret_cast<float2*>(scan_smem);    // [2][chunk][channels of the block]: dt, dt x
+  float* y_s = scan_smem + 2 * 2 * YS;                      // [2][chunk][channels of the block]
+  // K buffers, of which a launch has those that its longest entry fills (chunk j lies in buffer j % K): [3][chunk][channels of the
+  // block], raw dt, x, z, then [chunk][2 NP], B and C
+  constexpr int BUF = 3 * YS + BC;
+  float* raw_s = y_s + 2 * YS;
+  float* bc_s = raw_s + 3 * YS;
   const int e = blockIdx.y, c0 = blockIdx.x * kScanChannels;
   const bool walker = threadIdx.x < kScanWalkers;
   const int tid = walker ? threadIdx.x : threadIdx.x - kScanWalkers;      // place among the walkers, or among the helpers
@@ -256,8 +259,8 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
       return;
     }
     const int base = j * kScanChunk, n_here = min(kScanChunk, q_len - base);
-    float* bc = bc_s + (j % K) * BC;
-    float* raw = raw_s + (j % K) * 3 * YS;
+    float* bc = bc_s + (j % K) * BUF;
+    float* raw = raw_s + (j % K) * BUF;
     constexpr int V = WIDE ? 4 : 1;                         // floats a copy
     for (int idx = tid; idx < BC / V; idx += kScanWalkers) {
       const int i = idx / (2 * NP / V), r = idx % (2 * NP / V) * V, half = r / NP, n = r % NP;
@@ -289,7 +292,7 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
   // helpers: the step sizes of chunk j, all of whose copies have landed and were waited for ahead of a barrier
   auto prepare = [&](int j) {
     const int n_here = min(kScanChunk, q_len - j * kScanChunk);
-    const float* raw = raw_s + (j % K) * 3 * YS;
+    const float* raw = raw_s + (j % K) * BUF;
     float2* step = step_s + (j & 1) * YS;
 #pragma unroll
     for (int u = 0; u < YS / kScanWalkers; ++u) {
@@ -302,7 +305,7 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
   // helpers: y of chunk j, gated and written: out = (y + D x) * silu(z)
   auto finish = [&](int j) {
     const int base = j * kScanChunk, n_here = min(kScanChunk, q_len - base);
-    const float* raw = raw_s + (j % K) * 3 * YS;
+    const float* raw = raw_s + (j % K) * BUF;
     const float* ys = y_s + (j & 1) * YS;
     if (hc >= channels) return;
 #pragma unroll
@@ -339,7 +342,7 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
       continue;
     }
     const int n_here = min(kScanChunk, q_len - j * kScanChunk);
-    const float* bc = bc_s + (j % K) * BC;
+    const float* bc = bc_s + (j % K) * BUF;
     const float2* step = step_s + (j & 1) * YS;
     float* ys = y_s + (j & 1) * YS;
 #pragma unroll 1
@@ -538,11 +541,17 @@ extern "C" int srlm_selective_scan(const float* x, const float* xz, long long ld
   // copies of 16 bytes: neither four channels nor four states straddle an edge
   const bool wide = channels % 4 == 0 && N % 4 == 0 && b_off % 4 == 0 && ld_dbc % 4 == 0 && ld_xz % 4 == 0 &&
                     ((uintptr_t)x | (uintptr_t)xz | (uintptr_t)dbc | (uintptr_t)dt_raw) % 16 == 0;
-  const size_t smem = (size_t)scan_floats(npl) * sizeof(float);
+  // a step of short portions (decode) needs no ring: with one, fewer of its many blocks share an SM (64 requests of
+  // one token, 8,192 channels of 16 states: the layer 237 us, without it and with the registers
+  // of five blocks an SM 206)
+  const int chunks = (max_q_len + kScanChunk - 1) / kScanChunk;
+  const int held = chunks < 1 ? 1 : chunks < scan_buffers(npl) ? chunks : scan_buffers(npl);
+  const size_t smem = (size_t)scan_floats(npl, held) * sizeof(float);
 #define SRLM_SCAN_AS(TO, NPL, W)                                                                                        \
   do {                                                                                                                  \
     auto kern = selective_scan_kernel<TO, NPL, W>;                                                                      \
-    const cudaError_t got = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);         \
+    const cudaError_t got =                                                                                             \
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                             \
     if (got != cudaSuccess) return refuse((int)got, "selective_scan: cannot get %zu bytes of shared memory", smem);     \
     launch_pdl_if(early, kern, grid, dim3(kScanThreads), smem, stream, x, xz, ld_xz, dbc, ld_dbc, b_off, dt_raw,        \
                   dt_bias, A, D, state, state_stride, cu_q, slots, (TO*)out, channels, N, taps);                        \

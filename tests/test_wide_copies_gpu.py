@@ -25,7 +25,7 @@ class _Entries:
 
 
 @pytest.mark.parametrize("channels,N", [(4, 4), (20, 8), (36, 12), (16, 16), (48, 20), (16, 64), (20, 128)])
-@pytest.mark.parametrize("lens", [(1,), (15, 16, 17), (33, 1, 160), (2, 530)])
+@pytest.mark.parametrize("lens", [(1,), (15, 16, 17), (40, 100, 7), (33, 1, 160), (2, 530)])
 def test_scan_and_its_convolution(channels, N, lens):
     g = torch.Generator().manual_seed(channels + N)
     rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
