@@ -1638,9 +1638,9 @@ extern "C" int srlm_gemm_tn_tcgen05_static(const void* X, const void* W, void* C
   return ST_OK;
 }
 
-// Grouped products on the persistent kernel: token tile mt of X (tile_rows = 128 rows, one SM a tile of 128 weight
-// rows, or 256 rows, a pair of SMs a tile of 256 weight rows; X and C hold every group's rows from a multiple of
-// tile_rows on) multiplies the N weight rows of group group_of_mtile[mt] (device, int32 [ceil(M / tile_rows)];
+// Grouped products on the persistent kernel: token tile mt of X (tile_rows = 128 or 256 rows: a pair of SMs a tile of 256
+// weight rows, or one SM a tile of 128 weight rows x 128 tokens, see below; X and C hold every group's rows from a multiple
+// of tile_rows on) multiplies the N weight rows of group group_of_mtile[mt] (device, int32 [ceil(M / tile_rows)];
 // negative: the tile is skipped and its rows of C are not written).  W: [groups * N, K], contiguous.  glu: the
 // weight rows of a group come in blocks of 16 (8 gate rows, then the 8 up rows of the same features) and
 // C [M, N / 2] gets g * logistic(alpha g) * (u + 1) with g = min(gate, limit), u = clamp(up, -limit, limit); with
@@ -1666,10 +1666,14 @@ extern "C" int srlm_gemm_tn_tcgen05_grouped(const void* X, const void* W, void* 
   a.act = act;
   CUtensorMap mw_copy, mx_copy;
   const CUtensorMap *mw = &mw_copy, *mx = &mx_copy;
-  // Tiles of 128 tokens go to pairs too where no half of a pair would stand idle: 256 weight rows x 128 tokens, 24 KB from
-  // the L2 into each SM a k-block in place of 32 for the same products (8,192 rows over 16 experts, 2,048 -> 2 x 1,024 ->
-  // 2,048, both products: 219 -> 207 us; the epilogue's four warps bound the rest, most of all at 1,024 k).
-  const bool pairs = tile_rows == 256 || N % (2 * BM) == 0;
+  // Tiles of 128 tokens go to pairs too where no half of a pair would stand idle: 256 weight rows x 128 tokens, 24 KB from the L2
+  // into each SM a k-block in place of 32 for the same products; and where a group has a tile's worth of rows on average (M
+  // counts up to a tile of padding a group).  A layer of 16 experts, top 4, in us, pairs | one SM: 4,096 wide, 1,024 tokens 491..555 |
+  // 585, 256 tokens (64 rows an expert) 288 | 269; 64 experts, top 8, 2,048 wide, 3,000 tokens 813..879 | 891..918.  Where the
+  // weights fit the L2 the two forms are within 2 % (2,048 wide, 1,500 tokens 295 | 293; 1,024 wide 170 | 167) but for sizes
+  // at which the skipped tiles, which lie between the others, fall on some SMs more than on others: 2,048 tokens 332 | 348 and
+  // 176 | 192, 900 tokens 1,024 wide 137 | 129.
+  const bool pairs = tile_rows == 256 || (N % (2 * BM) == 0 && M >= 256ll * groups);
   // (the pair form fetches the tokens of a tile in two boxes, one a block)
   if (!cached_map(&mw_copy, W, (long long)groups * N, K, K, BM, true) ||
       !cached_map(&mx_copy, X, M, K, ldx, pairs ? tile_rows / 2 : 128, false))

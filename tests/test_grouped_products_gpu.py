@@ -56,3 +56,43 @@ def test_combination_and_gather_and_activation(act, T, H, top):
         xs = torch.empty(n + 1, 2 * H, dtype=torch.bfloat16, device=DEV)
         ops.moe_gather_rows(x.to(DEV), pair.to(DEV), top, xs)
         assert torch.equal(xs.cpu(), torch.cat([x.repeat_interleave(top, 0), torch.zeros(1, 2 * H).bfloat16()]))
+
+
+@pytest.mark.parametrize("act, glu", [(None, False), ("gelu", False), ("relu_squared", False), (None, True)])
+@pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("tile, N, K, M", [(128, 256, 72, 800), (128, 512, 136, 768), (128, 768, 64, 1100), (256, 512, 72, 700),
+                                           (256, 256, 64, 1),
+                                           # one SM a tile: 384 is no multiple of 256, fewer rows than two tiles a group
+                                           (128, 384, 72, 800), (128, 256, 72, 767), (128, 512, 64, 1)])
+def test_tensor_memory_products_with_their_epilogues(act, glu, odt, tile, N, K, M):
+    """Tiles of 128 and 256 tokens on pairs of SMs, with every epilogue: groups in any order, tiles without rows, a ragged last
+    tile."""
+    g = torch.Generator().manual_seed(N + M)
+    E, tiles = 3, -(-M // tile)
+    group = torch.tensor([[2, -1, 0, 1][t % 4] if M > 1 else 1 for t in range(tiles)], dtype=torch.int32)
+    x = torch.randn(M, K, generator=g).bfloat16()
+    w = (torch.randn(E, N, K, generator=g) * K ** -0.5).bfloat16()
+    out = torch.full((M, N // 2 if glu else N), 7.0, dtype=odt, device=DEV)
+    ops.gemm_tn_tcgen05_grouped(x.to(DEV), w.to(DEV), out, group.to(DEV), glu=glu, limit=1.5, alpha=1.702, tile_rows=tile, act=act)
+    assert ops.gemm_error_flag(out.device) == 0
+    e = group.repeat_interleave(tile)[:M]
+    rows = e >= 0
+    assert (out[~rows] == 7.0).all()                          # tiles without a group are not written
+    z, size = torch.zeros(M, N, dtype=torch.float64), torch.zeros(M, N, dtype=torch.float64)
+    for k in range(E):
+        z[e == k], size[e == k] = x[e == k].double() @ w[k].double().T, x[e == k].double().abs() @ w[k].double().abs().T
+    err = K * 2.0 ** -23 * size                               # float32 sums of exact products
+    if glu:
+        z, err = z.view(M, N // 16, 2, 8), err.view(M, N // 16, 2, 8)
+        gate, up = z[:, :, 0].clamp(max=1.5), z[:, :, 1].clamp(-1.5, 1.5)
+        want = (gate * torch.sigmoid(1.702 * gate) * (up + 1)).reshape(M, -1)
+        # gate * logistic(1.702 gate) below 1.5 has a slope below 1.11 and a size below 1.4; up + 1 lies below 2.5
+        err = (2.8 * err[:, :, 0] + 1.4 * err[:, :, 1]).reshape(M, -1) + 2.0 ** -20
+    elif act == "gelu":
+        want, err = 0.5 * z * (1 + torch.erf(z / 2 ** 0.5)), 1.13 * err + z.abs() * 2.0 ** -21
+    elif act == "relu_squared":
+        want, err = z.clamp(min=0) ** 2, (2 * z.abs() + err) * err + z * z * 2.0 ** -23
+    else:
+        want = z
+    err = err + (2.0 ** -24 if odt == torch.float32 else 2.0 ** -8) * want.abs()      # the result's own rounding
+    assert ((out.cpu().double() - want).abs() <= err * 1.001)[rows].all()
