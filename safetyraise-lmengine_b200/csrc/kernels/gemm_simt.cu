@@ -8,9 +8,11 @@
 // Two forms, with the same sums:
 //  * tiles: a block forms BM x BN outputs from a ring of slabs of 32 k's that asynchronous copies fill two slabs ahead.
 //    Bound by the FMA pipes; the tile is chosen by size (see `pick_tile`).
-//  * few rows (M <= 16): a warp streams 8 weight rows through a ring of its own, a lane owns up to four outputs.  Bound by
+//  * few rows (M <= 16, see `few_rows`): a warp streams 8 weight rows through a ring of its own, a lane owns up to four outputs.  Bound by
 //    the chain of K dependent FMAs (4 cycles each) for small weights (8 x 4,096 x 4,096: 33 us, 195 in tiles), by memory for
 //    large ones (1 x 24,576 x 4,096: 85 us, 484 in tiles).
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace srlm {
@@ -258,20 +260,35 @@ static int device_sms() {
 // thread's shared-memory reads (TM + TN values a k) and FMAs (TM x TN) overlap only between blocks, so 8 x 8 outputs a
 // thread win where there are blocks enough (2,048 x 6,144 x 4,096: 2.26 ms in tiles of 64 x 128, 2.71 in tiles of 32 x 32,
 // 3.18 with the 64 x 64 tiles of 4 x 4 outputs that this replaces) and 32 x 32 tiles where larger ones leave SMs idle
-// (305 x 1,024 x 3,072: 195 and 83 us; 155 before).
-static int pick_tile(int M, int N) {
-  struct Tile { int bm, bn, cycles; };
-  static const Tile tiles[] = {{128, 128, 225}, {64, 128, 110}, {64, 64, 62}, {32, 64, 37}, {32, 32, 18}};
+// (305 x 1,024 x 3,072: 195 and 83 us; 155 before).  Rows that are no whole 16-byte pieces (not `vec`) are fetched number by
+// number, which blocks beside each other hide: `first` is the time of blocks that have an SM each, `each` what one more costs
+// (us at 1,001 k; 100 x 8,192: 115, 84, 74, 79, 81 in the five tiles; 300 x 8,192: 229, 188, 172, 173, 204).
+static int pick_tile(int M, int N, bool vec) {
+  struct Tile { int bm, bn, cycles, first, each; };
+  static const Tile tiles[] = {{128, 128, 225, 115, 176}, {64, 128, 110, 83, 80}, {64, 64, 62, 45, 39}, {32, 64, 37, 31, 21},
+                               {32, 32, 18, 21, 12}};
   const int sms = device_sms();
   int best = 0;
   long long least = 0;
   for (int i = 0; i < 5; ++i) {
     if (i && (M + tiles[i].bm - 1) / tiles[i].bm > 65535) continue;          // more tiles than a grid has rows
     const long long blocks = (long long)((M + tiles[i].bm - 1) / tiles[i].bm) * ((N + tiles[i].bn - 1) / tiles[i].bn);
-    const long long cost = (blocks + sms - 1) / sms * tiles[i].cycles;
+    const long long cost = vec ? (blocks + sms - 1) / sms * tiles[i].cycles
+                               : std::max((long long)tiles[i].first * sms, blocks * tiles[i].each);
     if (i == 0 || cost < least) best = i, least = cost;
   }
   return best;
+}
+
+// Whether few rows are streamed or taken in tiles.  A block of the streaming form is one warp with up to four outputs a lane: the
+// more rows and the more of them an SM holds, the more the tiles' reuse wins; with few k's the streaming form is all ramp.  us,
+// streamed | tiles: 4 x 8,192 x 128 6.5 | 4.8, x 512 10.6 | 12.2; 8 x 32,000 x 512 35 | 33, x 1,024 48 | 63; 16 x 2,048 x 1,024
+// 10.9 | 16.3; 16 x 4,096 x 1,024 17.1 | 16.3, x 2,048 27.6 | 30.4; 16 x 8,192 x 4,096 92 | 80.
+static bool few_rows(int M, int N, int K) {
+  if (M <= 2 || M > FEW_M) return M <= 2;
+  if (N >= 2048 && K < FEW_K) return false;
+  if (M <= 8) return K >= 512 ? M <= 4 || N < 16384 || K >= 1024 : N < 4096;
+  return N <= 2048 || (N <= 4096 && K >= 2048);
 }
 
 template <typename TA, typename TW, typename TO>
@@ -280,11 +297,13 @@ static int run(const void* A, const void* W, void* C, int M, int N, int K, long 
   const bool vec = sizeof(TA) == 4 && sizeof(TW) == 4 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 &&
                    ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
   if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4 && sizeof(TO) == 4) {
-    if (vec && M <= 4) return run_few<1>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    if (vec && M <= 8) return run_few<2>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    if (vec && M <= FEW_M) return run_few<4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    if (vec && few_rows(M, N, K)) {
+      if (M <= 4) return run_few<1>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+      if (M <= 8) return run_few<2>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+      return run_few<4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    }
   }
-  switch (pick_tile(M, N)) {
+  switch (pick_tile(M, N, vec)) {
     case 0: return run_tile<TA, TW, TO, 128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
     case 1: return run_tile<TA, TW, TO, 64, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
     case 2: return run_tile<TA, TW, TO, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
