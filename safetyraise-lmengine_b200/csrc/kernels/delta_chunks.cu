@@ -13,7 +13,7 @@
 //                      bound by instructions (silu, the products by X and M) at 20 warps an SM.
 //   delta_chunk_walk   a block per (entry, head, 16 columns of S) walks the records: three products a chunk on tensor cores,
 //                      S in the accumulators; bound by the latency of a chunk (two exchanges between the eight warps).
-// 2,000 tokens, 16 heads of 128 x 128, one entry: 72 + 152 us; the kernels that go token by token: 98 + 610 us.
+// 2,000 tokens, 16 heads of 128 x 128, one entry: 84 + 155 us; the kernels that go token by token: 98 + 610 us.
 //
 // The products of the walk are mma.sync m16n8k8 on tf32 operands, each operand split into two tf32 numbers (high, and the rest)
 // and each product formed as high high + high low + low high.  Relative error against float64 (2-norm; 16 to 2,000 tokens, decays
@@ -262,8 +262,8 @@ __device__ __forceinline__ void mma_split(float (&small)[4], float (&large)[4], 
 // the product's k-th place t standing for row 2 t and t + 4 for row 2 t + 1 (on both sides).
 __global__ void __launch_bounds__(THREADS, 2)
 delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ state, long long state_stride,
-                        const int* __restrict__ cu_q, const int* __restrict__ slots, float* __restrict__ o_out, int least,
-                        int first_chunk, int n_chunks, Sizes z) {
+                        const int* __restrict__ cu_q, int n_entries, const int* __restrict__ slots,
+                        float* __restrict__ o_out, int least, int first_chunk, int n_chunks, Sizes z) {
   pdl_wait();
   pdl_trigger();
   // the records are those of the step's chunks first_chunk .. first_chunk + n_chunks - 1, of the entry's those from..to - 1
@@ -271,11 +271,26 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
   float* p_sums = chunk_smem + STAGES * STAGE;           // [warp][SUMS]: kx . S
   float* q_sums = p_sums + WARPS * SUMS;                 // qm . S
   float* u_s = q_sums + WARPS * SUMS;                    // [token][U_LD]
-  const int e = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * COLS;
+  // the blockIdx.z-th of the entries that go by chunks, and the place of its first record
+  int e = blockIdx.z, base = -first_chunk;
+  if (gridDim.z == n_entries) {                          // all of them
+    for (int x = 0; x < e; ++x) base += chunks_of(cu_q[x + 1] - cu_q[x], least);
+  } else {
+    e = n_entries;
+#pragma unroll 8
+    for (int x = 0, seen = 0, before = -first_chunk; x < n_entries; ++x) {       // no way out: the loads do not wait for each other
+      const int mine = chunks_of(cu_q[x + 1] - cu_q[x], least);
+      const bool it = mine > 0 && seen == (int)blockIdx.z;
+      e = it ? x : e;
+      base = it ? before : base;
+      seen += mine > 0;
+      before += mine;
+    }
+  }
+  if (e == n_entries) return;
+  const int h = blockIdx.y, c0 = blockIdx.x * COLS;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int first = cu_q[e], n = cu_q[e + 1] - first;
-  int base = -first_chunk;
-  for (int x = 0; x < e; ++x) base += chunks_of(cu_q[x + 1] - cu_q[x], least);
   const int from = max(0, -base), to = min(chunks_of(n, least), n_chunks - base);
   if (from >= to) return;
   const int rec_floats = record_floats(z.dv);
@@ -407,16 +422,16 @@ extern "C" int srlm_delta_chunk_record(int dk, int dv, int taps) {
 
 // proj float32 [T, ldp] and state as in delta_rule.cu, whose limits hold for an entry of any length.  Serves the entries of
 // `least` tokens and more: the chunks first_chunk .. first_chunk + n_chunks - 1 of those that they have together, entry by entry;
-// a step whose chunks do not all fit `records` (float32 [n_chunks, H, record]) is several calls, in order.  o_out float32 [T, H dv].  Renews S; the carried inputs of the convolution
-// are read and stay.
+// a step whose chunks do not all fit `records` (float32 [n_chunks, H, record]) is several calls, in order.  n_long:
+// how many entries they are.  o_out float32 [T, H dv].  Renews S; the carried inputs of the convolution are read and stay.
 extern "C" int srlm_delta_chunks(const float* proj, long long ldp, const float* conv_w, const float* a_log, const float* dt_bias,
                                  float* state, long long state_stride, const int* cu_q, const int* slots, int n_entries,
-                                 float* records, int least, int first_chunk, int n_chunks, float* o_out, int H, int G, int dk, int dv,
-                                 int taps, float unit_eps, cudaStream_t stream) {
-  if (n_entries <= 0 || n_chunks <= 0) return ST_OK;
+                                 float* records, int least, int n_long, int first_chunk, int n_chunks, float* o_out, int H,
+                                 int G, int dk, int dv, int taps, float unit_eps, cudaStream_t stream) {
+  if (n_entries <= 0 || n_long <= 0 || n_chunks <= 0) return ST_OK;
   const long long C = 2LL * G * dk + (long long)H * dv;
   if (!srlm_delta_chunk_record(dk, dv, taps) || first_chunk < 0 || H <= 0 || G <= 0 || H % G || H > 65535 || n_entries > 65535 ||
-      ldp < C + 2LL * H || C * 4 > 200 * 1024 || state_stride < (long long)H * dk * dv + C * (taps - 1))
+      n_long > n_entries || ldp < C + 2LL * H || C * 4 > 200 * 1024 || state_stride < (long long)H * dk * dv + C * (taps - 1))
     return refuse(ST_BAD_SIZE, "delta_chunks: H=%d G=%d dk=%d dv=%d taps=%d ldp=%lld state=%lld entries=%d", H, G, dk, dv, taps,
                   ldp, state_stride, n_entries);
   if ((uintptr_t)state % 8 || state_stride % 2 || (uintptr_t)records % 16)
@@ -428,8 +443,8 @@ extern "C" int srlm_delta_chunks(const float* proj, long long ldp, const float* 
                                              chunks::WALK_SMEM);
   if (e != cudaSuccess) return refuse((int)e, "delta_chunks: cannot get %d bytes of shared memory", chunks::WALK_SMEM);
   // (not ahead of time: blocks that start while the chunks' kernel drains would share the SMs that happen to be free)
-  launch_pdl_if(false, chunks::delta_chunk_walk_kernel, dim3(dv / chunks::COLS, H, n_entries), dim3(chunks::THREADS),
-                chunks::WALK_SMEM, stream, (const float*)records, state, state_stride, cu_q, slots, o_out, least,
-                first_chunk, n_chunks, z);
+  launch_pdl_if(false, chunks::delta_chunk_walk_kernel, dim3(dv / chunks::COLS, H, n_long), dim3(chunks::THREADS),
+                chunks::WALK_SMEM, stream, (const float*)records, state, state_stride, cu_q, n_entries, slots, o_out,
+                least, first_chunk, n_chunks, z);
   return launched();
 }

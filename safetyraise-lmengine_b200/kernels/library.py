@@ -1559,8 +1559,10 @@ class KernelLibrary:
         self.delta_recurrence(ctx, qkv, beta, decay, qk, state, o_out, H, G, dk, dv, below)
 
     DELTA_CHUNK = 16         # tokens of a chunk
-    # Entries of at least this many tokens go by chunks.  A layer in us, by chunks | token by token (16 heads of 128 x 128): one
-    # portion of 16 tokens 60 | 59, of 32 60 | 68; 8 of 16 79 | 93; 64 of 16 290 | 284, of 32 407 | 487; 32 heads: one of 16 73 | 101.
+    # Entries of at least this many tokens go by chunks.  A layer of 16 heads of 128 x 128 in us, by chunks | token by token: one
+    # portion of 16 tokens 45 | 56, of 48 50 | 74; 8 heads: 16 tokens 40 | 37, 24 40 | 40; 32 heads: 16 tokens 65 | 95.  Beside decoding
+    # requests, which go token by token, the chunks' two launches come on top (16 tokens beside 8 80 | 63, 64 89 | 90, 128 112 | 153;
+    # beside 63 153 | 122, 160 | 155, 188 | 215), but an entry's road does not depend on who shares its step.
     DELTA_CHUNKS_FROM = 16
 
     # Chunks whose records lie in memory at a time (41 KB a chunk and head of 128 x 128: 105 MB for 16 heads); a step that has more
@@ -1594,12 +1596,13 @@ class KernelLibrary:
         record = int(self.lib.srlm_delta_chunk_record(C.c_int(dk), C.c_int(dv), C.c_int(taps)))
         held = self.delta_chunks_held(ctx.workspace.max_tokens)
         records = ctx.workspace.get("delta.records", held * H, max(record, 1), torch.float32, reserve=held * H)
+        n_long = sum(n >= self.DELTA_CHUNKS_FROM for n in ctx.host["q_lens"])
         for first in range(0, n_chunks, held):
             self._check(self.lib.srlm_delta_chunks(
                 _ptr(proj), C.c_longlong(proj.stride(0)), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias), _ptr(state),
                 C.c_longlong(state.stride(0)), _ptr(ctx.cu_q), _ptr(ctx.slots), C.c_int(ctx.n_entries), _ptr(records),
-                C.c_int(self.DELTA_CHUNKS_FROM), C.c_int(first), C.c_int(min(held, n_chunks - first)), _ptr(o_out),
-                C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps), _stream()), "delta_chunks")
+                C.c_int(self.DELTA_CHUNKS_FROM), C.c_int(n_long), C.c_int(first), C.c_int(min(held, n_chunks - first)),
+                _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps), _stream()), "delta_chunks")
             self.launches += 1
         if min(ctx.host["q_lens"]) < self.DELTA_CHUNKS_FROM:       # the carried inputs are renewed behind the last who reads them
             self.delta_walk(ctx, proj, conv_w, a_log, dt_bias, state, o_out, H, G, dk, dv, taps, unit_eps, self.DELTA_CHUNKS_FROM)
