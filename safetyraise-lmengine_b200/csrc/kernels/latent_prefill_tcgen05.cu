@@ -13,9 +13,9 @@
 // is applied to the float32 sums as they leave.
 //
 // Shared memory holds 96 KB of queries, two K tiles (96 KB) and one V tile (32 KB): a V tile is fetched under the S product
-// and the softmax that follow the product that freed it.  Bound by the softmax (one exponential and about eight other
-// instructions a score) and the MMA issue of the longest block: 2.1 us a tile of 128 keys for two row tiles, 10 us before and
-// after them.  1,800 tokens behind 200, 16 heads: 53 us (485 on mma.sync, plus 30 for the rotation and the gate by themselves).
+// and the softmax that follow the product that freed it.  Bound by the softmax (one exponential and about nine other
+// instructions a score), the rescaling and the MMA issue of the longest block.  1,800 tokens behind 200, 16 heads: 62 us (485 on
+// mma.sync, plus 30 for the rotation and the gate by themselves).
 #include "attention_tcgen05.cuh"
 
 namespace srlm {

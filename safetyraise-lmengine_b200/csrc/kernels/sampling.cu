@@ -153,7 +153,8 @@ static void launch_rows(void (*kernel)(KArgs...), int rows, int cluster, int blo
 // Blocks per row: a long row is shared by a cluster of up to 8 (the portable size), each block a slice,
 // as long as the clusters of all rows find room on the GPU at once.
 // whole_sms: a block fills an SM, and the GPU's clusters of SMs hold 15 clusters of 8 such blocks or 36 of 4 at a time
-// (16 rows: 128 us in clusters of 8, which take two rounds, 85 us in clusters of 4).
+// (16 rows: 128 us in clusters of 8, which take two rounds, 85 us in clusters of 4, although a quarter of 151,936 values no
+// longer fits a block's shared memory beside the bins).  The counts are those of the 148 SMs of a B200.
 static int blocks_per_row(int V, int rows, bool whole_sms = false) {
   int c = V >= 32768 ? 8 : V >= 8192 ? 2 : 1;
   while (c > 1 && (rows * c > 148 || (whole_sms && rows > (c == 8 ? 15 : c == 4 ? 36 : 74)))) c >>= 1;

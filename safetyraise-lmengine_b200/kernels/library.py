@@ -81,7 +81,7 @@ class KernelLibrary:
         self.split_mixed_heads = True                   # ... short prompts: the keys in slices
         self.retention_in_chunks = True                 # retention: portions in chunks of 64 tokens
         self.states_by_groups = True                    # channel-wise delta rule, state space: portions in groups of 8 tokens
-        self.grouped_pairs = True                       # ... whose largest steps run pairs of SMs on tiles of 256 tokens
+        self.grouped_pairs = True                       # ... whose largest steps have tiles of 256 tokens
 
     @property
     def lib(self):
@@ -1034,15 +1034,16 @@ class KernelLibrary:
         self._check(self.lib.srlm_moe_look_up(_ptr(ids), _ptr(table), C.c_int(table.shape[0]), C.c_int(T), C.c_int(experts),
                                               C.c_int(top), C.c_float(share), _ptr(choice), _ptr(weight), _stream()), "moe_look_up")
 
-    GROUPED_TILE = 128       # token rows of a tile of the grouped tensor-memory product (one SM a tile)
-    GROUPED_PAIR_TILE = 256  # ... of its pair form (two SMs on 256 weight rows x 256 tokens)
+    GROUPED_TILE = 128       # token rows of a tile of the grouped tensor-memory product (one SM or two, by the sizes)
+    GROUPED_PAIR_TILE = 256  # ... of its widest form (two SMs on 256 weight rows x 256 tokens)
 
     def grouped_tile_rows(self, pairs: int, experts: int, weight_elements: int) -> int:
         """The token tile of the grouped tensor-memory product for a step of ``pairs`` rows over ``experts`` groups
-        whose first weight matrix has ``weight_elements`` elements a group: 256 (pairs of SMs) once an expert has 512
-        rows on average (so that about an eighth of the tiles' rows is padding) and 16 Mi weight elements; else 128.
-        Measured at 8,192 rows over 16 experts: 2,048 x 2,048 a group 0.76 ms in pairs against 0.68 ms for the eight
-        products of four layers, 4,096 x 4,096 a group 1.32 against 1.85 ms."""
+        whose first weight matrix has ``weight_elements`` elements a group: 256 once an expert has 512 rows on average (so
+        that about an eighth of the tiles' rows is padding) and 16 Mi weight elements; else 128.  A layer of 16 experts in
+        us, tiles of 256 | of 128 (pairs of SMs both): 4,096 wide, 512 rows an expert 803..937 | 923..936, 1,024 rows
+        1,556..1,593 | 1,746..1,775; one product of 2,048 x 2,048 a group 83 | 84 and 153 | 166, with an eighth more rows
+        in the tiles of 256 when the experts' shares are uneven."""
         big = pairs >= 512 * experts and weight_elements >= 16 << 20
         return self.GROUPED_PAIR_TILE if self.grouped_pairs and big else self.GROUPED_TILE
 
@@ -1477,7 +1478,8 @@ class KernelLibrary:
     def latent_prefill_plan(self, q_lens, kv_lens, heads: int, sms: int) -> int:
         """Row tiles a block (1 or 2) of latent_prefill_tcgen05, by a model of its time in microseconds fitted to
         measurements on B200: a block of one row tile takes 10 + 1.9 a key tile, a block of two 13 + 2.1 a key tile;
-        blocks run in rounds of one per SM."""
+        blocks run in rounds of one per SM.  (Fitted before the rows were rescaled at every new maximum; its choice was
+        the faster one at all of 42 sizes with that: 1,024 to 4,096 wide, 5 to 2,048 tokens behind up to 3,000.)"""
         key_tiles = (max(kv_lens) + 127) // 128
         blocks = lambda rows: sum((n + rows - 1) // rows for n in q_lens) * heads
         rounds = lambda n: -(-n // max(1, sms))
