@@ -17,8 +17,9 @@
 // for decode steps (8 requests of 2,048: 0.19 ms; 2.75).
 //
 // Such a block fills an SM.  Where a step has many requests of few rows, or few keys, the small form takes 8 rows and spans of 32
-// keys without a second buffer: several blocks an SM hide the trips to memory that a short request consists of (64 requests of 16 keys, 32 heads of 64: 118 us
-// in the large form, which leaves such a request an SM, 15 in the small one, 19 with the warp a row; see simt_small).
+// keys without a second buffer: several blocks an SM hide the trips to memory that a short request consists of (64 requests of 16
+// keys, 32 heads of 64: 118 us in the large form, which leaves such a request an SM, 15 in the small one, 19 with the warp a row;
+// see simt_small).
 #include <math_constants.h>
 
 #include "common.cuh"

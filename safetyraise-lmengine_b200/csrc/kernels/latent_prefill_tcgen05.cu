@@ -5,12 +5,12 @@
 // The plan is attention_prefill_tcgen05.cu's, with a KV head per query head: a block takes up to 256 tokens of one entry and
 // one head as two tiles of 128 rows and walks the keys in tiles of 128; S = Q K^T and O += P V are tcgen05.mma with
 // accumulators in tensor memory, P is bfloat16 over the columns of S, one thread owns a row's softmax.  What differs: O is
-// rescaled whenever a row's maximum has grown, and a row's sum is that of the rounded weights (with sums of the unrounded ones
-// and a maximum that may lag by 2^8, so that the largest weight is rounded too, the layer's error against float64 was 0.5 % above
-// that of the kernel on mma.sync, 1.3 % at 300 tokens behind 1,000; so it is 0.1 % below; it costs 9 us of 166 in a layer of
-// 1,800 tokens); an operand row is three panels of 64 elements, two fetched from the step's matrix of keys and values (one box of 128 rows) and one from the pages (a box a page); the
-// queries arrive in float32 as projected and are rotated and rounded on their way into shared memory; a head's output gate
-// is applied to the float32 sums as they leave.
+// rescaled whenever a row's maximum has grown, and a row's sum is that of the rounded weights (with sums of the unrounded
+// ones and a maximum that may lag by 2^8, so that the largest weight is rounded too, the layer's error against float64 was
+// 0.5 % above that of the kernel on mma.sync, 1.3 % at 300 tokens behind 1,000; so it is 0.1 % below; it costs 9 us of 166
+// in a layer of 1,800 tokens); an operand row is three panels of 64 elements, two fetched from the step's matrix of keys and
+// values (one box of 128 rows) and one from the pages (a box a page); the queries arrive in float32 as projected and are
+// rotated and rounded on their way into shared memory; a head's output gate is applied to the float32 sums as they leave.
 //
 // Shared memory holds 96 KB of queries, two K tiles (96 KB) and one V tile (32 KB): a V tile is fetched under the S product
 // and the softmax that follow the product that freed it.  Bound by the softmax (one exponential and about nine other

@@ -1604,7 +1604,8 @@ class KernelLibrary:
                 _ptr(proj), C.c_longlong(proj.stride(0)), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias), _ptr(state),
                 C.c_longlong(state.stride(0)), _ptr(ctx.cu_q), _ptr(ctx.slots), C.c_int(ctx.n_entries), _ptr(records),
                 C.c_int(self.DELTA_CHUNKS_FROM), C.c_int(n_long), C.c_int(first), C.c_int(min(held, n_chunks - first)),
-                _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps), _stream()), "delta_chunks")
+                _ptr(o_out), C.c_int(H), C.c_int(G), C.c_int(dk), C.c_int(dv), C.c_int(taps), C.c_float(unit_eps), _stream()),
+                "delta_chunks")
             self.launches += 1
         if min(ctx.host["q_lens"]) < self.DELTA_CHUNKS_FROM:       # the carried inputs are renewed behind the last who reads them
             self.delta_walk(ctx, proj, conv_w, a_log, dt_bias, state, o_out, H, G, dk, dv, taps, unit_eps, self.DELTA_CHUNKS_FROM)
