@@ -182,6 +182,16 @@ __device__ __forceinline__ void tmem_load<32>(uint32_t taddr, uint32_t (&v)[32])
       : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// The same for values whose load was issued a while ago: none of them is touched in front of the wait.
+__device__ __forceinline__ void tmem_load_wait(uint32_t (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
+                 "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
+                 "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29])
+               :: "memory");
+  asm volatile("" : "+r"(v[30]), "+r"(v[31]) :: "memory");
+}
 
 // ---------------------------------------------------------------------------
 // the kernel
@@ -689,8 +699,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // The persistent variant for many tokens (prefill): one block per SM walks over output tiles.  The
 // accumulator is double-buffered in TMEM (2 x BN columns), so the epilogue of a tile runs while
 // the MMAs of the next one are issued, and the shared-memory ring never drains between tiles.
-// The epilogue transposes each 32-token slab through shared memory and writes whole rows of C
-// (256 contiguous bytes per token and tile) instead of one element per lane.
+// The epilogue's four warps store straight from the registers that tcgen05.ld fills: a lane has one weight
+// row, so a warp's store of one token is 32 neighbouring elements of C, whole sectors whatever the rows'
+// alignment, and the warps do not wait for each other.  Turned through shared memory (two barriers and a
+// division a 16-byte piece for every 32 tokens) a tile's epilogue took as long as 30 k-blocks, and the last
+// tile's is nobody's cover: 2,000 x 4,096 x 512 29.1 -> 15.9 us, 2,048 x 8,192 x 2,048 in float32 77.4 -> 53.7,
+// 512 x 7,168 x 5,120 45.1 -> 36.9, 2,048 x 4,096 x 4,096 54.8 -> 49.1.  Deeper rings in the shared memory that
+// this leaves (7 stages for 6) change nothing.
 //
 // Tiles seldom come in multiples of the SM count: 384 tiles leave 60 of 148 SMs idle in the third
 // round.  So the k-blocks of the tiles that do not fill a round (args.sk_tiles of them, the first;
@@ -778,6 +793,19 @@ __device__ __forceinline__ float clamped_glu_fast(float gate, float up, float li
   return g * __frcp_rn(1.f + exp2f(-alpha * 1.4426950408889634f * g)) * (u + 1.f);
 }
 
+// The first `tokens` of a lane's values, one below the other in C.
+template <typename TO, int COUNT>
+__device__ __forceinline__ void store_tokens(TO* at, long long ld, const float (&h)[COUNT], int tokens) {
+  if (tokens >= COUNT) {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j) at[j * ld] = from_float<TO>(h[j]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < COUNT; ++j)
+      if (j < tokens) at[j * ld] = from_float<TO>(h[j]);
+  }
+}
+
 template <int BN, int STAGES, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -791,10 +819,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
   constexpr int TILE_N = PAIR ? 2 * BM : BM;                 // weight rows of a tile
   constexpr int A_BYTES = BM * BK * 2, B_BYTES = B_ROWS * BK * 2, STAGE = A_BYTES + B_BYTES;
   constexpr int TMEM_COLS = 2 * BN;
-  constexpr int SLAB = 32;                                   // tokens per epilogue slab
-  constexpr int SLAB_ROW = BM * 4 + 16;                      // bytes per token row of the slab (padded)
-  uint8_t* slab = smem + STAGES * STAGE;                     // [2][SLAB][SLAB_ROW]
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(slab + 2 * SLAB * SLAB_ROW);
+  constexpr int SLAB = 32;                                   // tokens that the epilogue reads at a time
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* acc_full = empty_bar + STAGES;                   // [2]
   uint64_t* acc_empty = acc_full + 2;                        // [2]
@@ -911,10 +937,9 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
     const int ew = warp & 3;                               // TMEM lanes 32*ew .. 32*ew+31 belong to this warp
     const int lane_base = 32 * ew;
     const int tid_e = ew * 32 + lane;                      // 0..127 among the epilogue threads
-    const int out_cols = args.swiglu8 ? BM / 2 : BM;       // columns of C a tile produces
     const int esize = args.c_is_f32 ? 4 : 2;
     const bool vec_ok = (args.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(args.C) & 15) == 0);
-    int local = 0, slab_turn = 0;
+    int local = 0;
     bool ok = true;
     PieceWalk walk(args, num_kb, total_tiles, walker, walkers);
     int t, kb_lo, kb_hi;
@@ -1071,68 +1096,62 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
         }
         continue;
       }
+      // D[n, m] -> C[m][n]; the next 32 tokens leave TMEM while these are stored
+      uint32_t v[2][SLAB];
+      const uint32_t acc = tmem_base + ((uint32_t)lane_base << 16) + b * BN;
+      const int tokens = min(BN, args.M - m0);
+      static_assert(BN % (2 * SLAB) == 0, "slabs go two by two");
+      tmem_load<SLAB>(acc, v[0]);
 #pragma unroll 1
-      for (int c = 0; c < BN; c += SLAB, slab_turn ^= 1) {
-        uint32_t v[SLAB];
-        tmem_load<SLAB>(tmem_base + ((uint32_t)lane_base << 16) + b * BN + c, v);
-        tmem_load_wait();
-        if (c + SLAB >= BN) {                               // everything of this tile has left TMEM
-          tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) acc_drained<PAIR>(&acc_empty[b]);
-        }
-        if (m0 + c >= args.M) continue;                     // slab beyond the last token (same for all warps)
-        uint8_t* sl = slab + slab_turn * SLAB * SLAB_ROW;
-        // D[n, m] -> slab[m][column of C]
-        if (args.swiglu8) {
-          // lanes l and l^8 hold the gate and the up row of one feature; they share the work: the
-          // gate lane finishes the even token of a pair, the up lane the odd one
-          const bool gate_lane = (lane & 8) == 0;
-          const int col = (lane_base >> 1) + (lane >> 4) * 8 + (lane & 7);
+      for (int c = 0; c < BN;) {
 #pragma unroll
-          for (int j = 0; j < SLAB; j += 2) {
-            const float mine0 = __uint_as_float(v[j]), mine1 = __uint_as_float(v[j + 1]);
-            const float got = __shfl_xor_sync(0xffffffffu, gate_lane ? mine1 : mine0, 8);
-            const float gv = gate_lane ? mine0 : got, uv = gate_lane ? got : mine1;
-            const float hval = args.glu_limit > 0.f ? clamped_glu_fast(gv, uv, args.glu_limit, args.glu_alpha)
-                                                    : silu_stable(gv) * uv;
-            const int row = gate_lane ? j : j + 1;
-            if (args.c_is_f32) *reinterpret_cast<float*>(sl + row * SLAB_ROW + col * 4) = hval;
-            else *reinterpret_cast<bf16*>(sl + row * SLAB_ROW + col * 2) = __float2bfloat16_rn(hval);
+        for (int half = 0; half < 2; ++half, c += SLAB) {
+          uint32_t (&x)[SLAB] = v[half];
+          tmem_load_wait(x);
+          if (c + SLAB < BN) {
+            tmem_load<SLAB>(acc + c + SLAB, v[half ^ 1]);
+          } else {                                            // everything of this tile has left TMEM
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) acc_drained<PAIR>(&acc_empty[b]);
           }
-        } else {
+          if (args.swiglu8) {
+            // lanes l and l^8 hold the gate and the up row of one feature; they share the work: the
+            // gate lane finishes the even token of a pair, the up lane the odd one
+            const bool gate_lane = (lane & 8) == 0;
+            float h[SLAB / 2];
 #pragma unroll
-          for (int j = 0; j < SLAB; ++j) {
-            float x = __uint_as_float(v[j]);
-            if (args.act == 1) x = 0.5f * x * (1.f + erff(x * 0.70710678118654752440f));
-            else if (args.act == 2) x = x < 0.f ? 0.f : x * x;
-            const int col = lane_base + lane;
-            if (args.c_is_f32) *reinterpret_cast<float*>(sl + j * SLAB_ROW + col * 4) = x;
-            else *reinterpret_cast<bf16*>(sl + j * SLAB_ROW + col * 2) = __float2bfloat16_rn(x);
-          }
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        // rows of the slab -> C, 16 bytes per thread
-        const int row_bytes = out_cols * esize;
-        const int vec_per_row = row_bytes / 16;
-        const int n_limit = (args.swiglu8 ? args.N / 2 : args.N) - c0;     // valid columns in this tile
-        for (int idx = tid_e; idx < SLAB * vec_per_row; idx += 128) {
-          const int j = idx / vec_per_row, vcol = idx % vec_per_row;
-          const int m = m0 + c + j;
-          if (m >= args.M) continue;
-          const int col = vcol * (16 / esize);              // first column of this 16-byte piece
-          uint8_t* dst = reinterpret_cast<uint8_t*>(args.C) + ((size_t)m * args.ldc + c0 + col) * esize;
-          const uint8_t* src = sl + j * SLAB_ROW + vcol * 16;
-          if (vec_ok && col + 16 / esize <= n_limit) {
-            *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(src);
+            for (int j = 0; j < SLAB; j += 2) {
+              const float mine0 = __uint_as_float(x[j]), mine1 = __uint_as_float(x[j + 1]);
+              const float got = __shfl_xor_sync(0xffffffffu, gate_lane ? mine1 : mine0, 8);
+              const float gv = gate_lane ? mine0 : got, uv = gate_lane ? got : mine1;
+              h[j / 2] = args.glu_limit > 0.f ? clamped_glu_fast(gv, uv, args.glu_limit, args.glu_alpha) : silu_stable(gv) * uv;
+            }
+            const int col = c0 + (lane_base >> 1) + (lane >> 4) * 8 + (lane & 7), first = c + (gate_lane ? 0 : 1);
+            if (col < args.N / 2) {
+              const size_t at = (size_t)(m0 + first) * args.ldc + col;
+              if (args.c_is_f32) store_tokens(reinterpret_cast<float*>(args.C) + at, 2 * args.ldc, h, (tokens - first + 1) / 2);
+              else store_tokens(reinterpret_cast<bf16*>(args.C) + at, 2 * args.ldc, h, (tokens - first + 1) / 2);
+            }
           } else {
-            for (int e = 0; e < 16 / esize && col + e < n_limit; ++e) {
-              if (args.c_is_f32) reinterpret_cast<float*>(dst)[e] = reinterpret_cast<const float*>(src)[e];
-              else reinterpret_cast<bf16*>(dst)[e] = reinterpret_cast<const bf16*>(src)[e];
+            float h[SLAB];
+#pragma unroll
+            for (int j = 0; j < SLAB; ++j) h[j] = __uint_as_float(x[j]);
+            if (args.act == 1) {
+#pragma unroll
+              for (int j = 0; j < SLAB; ++j) h[j] = 0.5f * h[j] * (1.f + erff(h[j] * 0.70710678118654752440f));
+            } else if (args.act == 2) {
+#pragma unroll
+              for (int j = 0; j < SLAB; ++j) h[j] = h[j] < 0.f ? 0.f : h[j] * h[j];
+            }
+            const int col = n0 + lane_base + lane;
+            if (col < args.N) {
+              const size_t at = (size_t)(m0 + c) * args.ldc + col;
+              if (args.c_is_f32) store_tokens(reinterpret_cast<float*>(args.C) + at, args.ldc, h, tokens - c);
+              else store_tokens(reinterpret_cast<bf16*>(args.C) + at, args.ldc, h, tokens - c);
             }
           }
         }
-        // the other slab buffer is used next; this one is rewritten two slabs later, after another barrier
       }
     }
   }
@@ -1270,7 +1289,7 @@ static int dealt_tiles(int tiles, int num_kb, int walkers) {      // walkers: bl
 template <int BN, int STAGES>
 static int launch_persistent(const CUtensorMap* mw, const CUtensorMap* mx, const GemmArgs& a, long long ws_bytes,
                              cudaStream_t stream) {
-  constexpr int SMEM = STAGES * stage_bytes<BN>() + 2 * 32 * (BM * 4 + 16) + (2 * STAGES + 4) * 8 + 16 + 1024;
+  constexpr int SMEM = STAGES * stage_bytes<BN>() + (2 * STAGES + 4) * 8 + 16 + 1024;
   static bool configured = false;
   static int sm_count = 0;
   if (!configured) {
@@ -1318,7 +1337,7 @@ static int dealt_pair_tiles(int tiles, int num_kb, int pairs) {
 template <int BN, int STAGES>
 static int launch_pair(const CUtensorMap* mw, const CUtensorMap* mx, const GemmArgs& a, long long ws_bytes,
                        cudaStream_t stream) {
-  constexpr int SMEM = STAGES * (BM * BK * 2 + (BN / 2) * BK * 2) + 2 * 32 * (BM * 4 + 16) + (2 * STAGES + 4) * 8 + 16 + 1024;
+  constexpr int SMEM = STAGES * (BM * BK * 2 + (BN / 2) * BK * 2) + (2 * STAGES + 4) * 8 + 16 + 1024;
   static_assert(SMEM <= 232448, "shared memory of a block");
   static bool configured = false;
   static int sm_count = 0;

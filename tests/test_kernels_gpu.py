@@ -407,6 +407,32 @@ def test_gemm_tcgen05_persistent_forms(M, N, K, dealt, odt):
         assert torch.allclose(out3.float(), ref3, rtol=2e-2, atol=2e-2)
 
 
+# tokens at the edges of what the epilogue reads at a time (32) and of a tile, in tiles of one SM (128) and of two (256);
+# weight rows that end inside a warp's 32
+@pytest.mark.parametrize("M, N", [(129, 400), (160, 1001), (161, 144), (257, 12336), (287, 12401), (289, 24576), (512, 12303)])
+@pytest.mark.parametrize("glu", [False, True])
+@pytest.mark.parametrize("odt", [torch.bfloat16, torch.float32])
+def test_gemm_tcgen05_persistent_stores_stay_inside_the_result(M, N, glu, odt):
+    """Results that start on any element of a larger buffer: nothing in front of them and behind them is written."""
+    if glu:
+        N -= N % 16
+    g = torch.Generator(device=DEV).manual_seed(M + N)
+    K = 72
+    a = torch.randn(M, K, device=DEV, generator=g).to(torch.bfloat16)
+    w = (torch.randn(N, K, device=DEV, generator=g) / math.sqrt(K) * 2).to(torch.bfloat16)
+    width = N // 2 if glu else N
+    buffer = torch.full((M * width + 600,), 7.0, device=DEV, dtype=odt)
+    out = buffer[301:301 + M * width].view(M, width)
+    ops().gemm_tn_tcgen05(a, w, out, splits=1, swiglu8=glu)
+    assert ops().gemm_error_flag(a.device) == 0
+    ref = a.double() @ w.double().T
+    if glu:
+        full = ref.view(M, N // 16, 2, 8)
+        ref = (torch.nn.functional.silu(full[:, :, 0]) * full[:, :, 1]).reshape(M, width)
+    assert torch.allclose(out.double(), ref, rtol=2e-2 if odt == torch.bfloat16 else 1e-4, atol=2e-2 if odt == torch.bfloat16 else 1e-4)
+    assert (buffer[:301] == 7.0).all() and (buffer[301 + M * width:] == 7.0).all()
+
+
 @pytest.mark.parametrize("nq, nkv, hd, rd", [(4, 2, 16, 16), (3, 1, 48, 20), (2, 2, 128, 128), (6, 2, 64, 32)])
 @pytest.mark.parametrize("dt", ACT)
 def test_qk_norm_rope_append_interleaved_pairs(nq, nkv, hd, rd, dt):
