@@ -81,9 +81,17 @@ __device__ __forceinline__ unsigned long long best_word(float v, int i) {
 
 // The best (value, id) of the elements [sl.lo, sl.hi) over the block, then over the cluster; the same
 // word in every thread of every block.  `slot`: one 64-bit word of shared memory, `warp_best`: 32.
-template <typename F>
+// FLAG: `flag`, which `adjust` may set, becomes whether any thread of the cluster has set it.  It travels as the one bit that
+// a word leaves free.
+template <bool FLAG, typename F>
 __device__ unsigned long long cluster_best(const float* row, int V, Slice sl, unsigned long long* warp_best,
-                                           unsigned long long* slot, F adjust) {
+                                           unsigned long long* slot, bool& flag, F adjust) {
+  constexpr unsigned long long kFlag = 0x80000000ull;
+  auto join = [](unsigned long long a, unsigned long long b) {
+    if (!FLAG) return b > a ? b : a;
+    const unsigned long long x = a & ~kFlag, y = b & ~kFlag;
+    return (y > x ? y : x) | ((a | b) & kFlag);
+  };
   unsigned long long best = 0;
   for_each_of_row(row, V, sl, [&](int i, float x) {
     const unsigned long long w = best_word(adjust(i, x), i);
@@ -95,20 +103,22 @@ __device__ unsigned long long cluster_best(const float* row, int V, Slice sl, un
     best = other > best ? other : best;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (FLAG && __any_sync(0xffffffffu, flag)) best |= kFlag;
   if (lane == 0) warp_best[warp] = best;
   __syncthreads();
   if (threadIdx.x == 0) {
     unsigned long long b = 0;
-    for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) b = warp_best[w] > b ? warp_best[w] : b;
+    for (int w = 0; w < (int)((blockDim.x + 31) >> 5); ++w) b = join(b, warp_best[w]);
     *slot = b;
   }
   cluster_sync();
   best = 0;
-  for (uint32_t r = 0; r < cluster_size(); ++r) {
-    const unsigned long long other = peer_u64(slot, r);
-    best = other > best ? other : best;
-  }
+  for (uint32_t r = 0; r < cluster_size(); ++r) best = join(best, peer_u64(slot, r));
   cluster_sync();                       // nobody rewrites its slot while another block still reads it
+  if (FLAG) {
+    flag = (best & kFlag) != 0;
+    best &= ~kFlag;
+  }
   return best;
 }
 
@@ -120,7 +130,7 @@ __global__ void argmax_kernel(const float* __restrict__ logits, long long row_st
   const int r = blockIdx.x / cluster_size();
   const float* row = logits + (size_t)r * row_stride;
   bool nonfinite = false;
-  const unsigned long long best = cluster_best(row, V, slice_of(V), warp_best, &slot, [&](int, float x) {
+  const unsigned long long best = cluster_best<false>(row, V, slice_of(V), warp_best, &slot, nonfinite, [&](int, float x) {
     if (!isfinite(x)) nonfinite = true;
     return x;
   });
@@ -187,9 +197,12 @@ extern "C" int srlm_argmax(const float* logits, long long row_stride, int n, int
 // order of the additions: the same token on every run.  Elements with equal keys
 // are ordered by id; a tie on a boundary is resolved by a search over the ids.
 // About a dozen passes over the row instead of a hundred; a block's slice of the row lies in shared memory where it fits.
-// A top-k of a few hundred ends after the search for its boundary: the kept elements are collected and ordered.
+// A top-k of a few hundred ends its search for the boundary at the first digit down to which a list takes all elements: these
+// are collected and ordered.  Its first pass counts while the values are adjusted.
+// Bound by what a pass costs beside its elements: the bins' copies, their sums, the exchange in the cluster (3 to 4 us).
 // 8 rows of 151,936, top-k 50, top-p 0.9, penalty: 154 us with 64-bit additions and the bins scanned by one thread, 85 us
-// without either, 42 us with the collected list; without a top-k 114 -> 64 us.
+// without either, 40 us with the collected list behind all four digits, 27 us with the list behind the digit (two here) that
+// bounds it; without a top-k 114 -> 63 us.
 // ---------------------------------------------------------------------------
 namespace srlm {
 
@@ -300,10 +313,10 @@ __device__ __forceinline__ void scan_bins(const u64* bins, u64 above, u64 target
 // `target`, the sum above that digit, and the digit's own bin go to sh.found.  The keys of a row share
 // few leading digits, so every lane adds into a copy of the bins of its own (`copies`, in dynamic shared
 // memory); the copies are summed before the scan.  Integer additions: any order gives the same sums.
-// COUNT: every weight is 1.  turn: passes that fill alternate between 0 and 1.
+// COUNT: every weight is 1.  turn: passes that fill alternate between 0 and 1.  counted: the copies hold the slice's counts.
 template <bool COUNT, typename Match, typename Weight>
 __device__ __forceinline__ void radix_pass(const float* v, int V, Slice sl, int shift, u64 above, u64 target, int& turn,
-                                           Shared& sh, uint32_t* copies, Match match, Weight weight, bool fill) {
+                                           Shared& sh, uint32_t* copies, Match match, Weight weight, bool fill, bool counted = false) {
   if (fill) {
     u64* mine = sh.mine[turn];
     turn ^= 1;
@@ -311,9 +324,11 @@ __device__ __forceinline__ void radix_pass(const float* v, int V, Slice sl, int 
       for (int i = threadIdx.x; i < 256; i += blockDim.x) sh.low_id[i] = 0x7fffffffull;
     uint32_t* lane_copy = copies + (threadIdx.x & (REPLICAS - 1)) * REPLICA_STRIDE;
     for (int lo = sl.lo; lo == sl.lo || lo < sl.hi; lo += MAX_PART) {      // one part, for every vocabulary that there is
-      const Slice part{lo, min(sl.hi, lo + MAX_PART)};
-      for (int i = threadIdx.x; i < (COUNT ? 1 : 2) * COPY_WORDS; i += blockDim.x) copies[i] = 0;
-      __syncthreads();
+      const Slice part{counted ? sl.hi : lo, counted ? sl.hi : min(sl.hi, lo + MAX_PART)};
+      if (!counted) {
+        for (int i = threadIdx.x; i < (COUNT ? 1 : 2) * COPY_WORDS; i += blockDim.x) copies[i] = 0;
+        __syncthreads();
+      }
       for_each_of_row(v, V, part, [&](int i, float x) {
         const uint32_t key = order_key(x);
         if (match(key, i)) {
@@ -343,6 +358,7 @@ __device__ __forceinline__ void radix_pass(const float* v, int V, Slice sl, int 
       sum += __shfl_xor_sync(0xffffffffu, sum, 2);
       if (quarter == 0) mine[d] = lo == sl.lo ? sum : mine[d] + sum;
       __syncthreads();
+      if (counted) break;
     }
     cluster_sync();                       // every block's slice is in its `mine`
     const uint32_t n = cluster_size();
@@ -448,12 +464,12 @@ __device__ void select_by_mass(const float* v, int V, Slice sl, const Kept& kept
   *mass_through = above + need * w;
 }
 
-// The choice among few kept elements (top-k of at most kList): block 0 of the cluster collects them, orders them by key
-// descending and id ascending, and reads the cutoff and the draw off their running masses: the element that the searches
-// above would find.  -> its id in block 0's thread 0, -1 where no kept element has a mass (the adjusted maximum is not a finite
+// The choice among few elements (top-k of at most kList; `kept`: those k, or at most kList with them among these): block 0 of the
+// cluster collects them, orders them by key descending and id ascending, and reads the cutoff and the draw off the running
+// masses of the first k: the element that the searches above would find.  -> its id in block 0's thread 0, -1 where no kept element has a mass (the adjusted maximum is not a finite
 // number); the other blocks return at once.  lists: 3 * kList words of shared memory, at the same place in every block.
 constexpr int kList = 512;
-__device__ int select_from_list(const float* v, int V, Slice sl, const Kept& kept, float vmax, float tp, float uniform,
+__device__ int select_from_list(const float* v, int V, Slice sl, const Kept& kept, int k, float vmax, float tp, float uniform,
                                 Shared& sh, u64* lists) {
   u64 *own = lists, *all = lists + kList, *sorted = lists + 2 * kList;
   __syncthreads();
@@ -487,6 +503,7 @@ __device__ int select_from_list(const float* v, int V, Slice sl, const Kept& kep
   }
   __syncthreads();
   if (threadIdx.x >= 32) return 0;
+  n = min(n, k);
   const int lane = threadIdx.x, per = (n + 31) / 32, lo = min(n, lane * per), hi = min(n, lo + per);
   auto mass = [&](int i) { return (u64)mass_of(key_value((uint32_t)(sorted[i] >> 32)), vmax); };
   u64 own_mass = 0;
@@ -559,49 +576,60 @@ sample_kernel(const float* __restrict__ logits, long long row_stride, int V,
   }
   // the adjusted values, once (each block its slice); their argmax (ties to the lowest id) and the
   // non-finite check, over the whole row
+  // and, for a top-k, the counts of the first pass of its search
+  const int k = top_k ? top_k[r] : 0;
+  const bool cuts = k > 0 && k < V && temp > 0.f;
+  uint32_t* lane_copy = copies + (threadIdx.x & (REPLICAS - 1)) * REPLICA_STRIDE;
+  if (cuts) {
+    for (int i = threadIdx.x; i < COPY_WORDS; i += blockDim.x) copies[i] = 0;
+    __syncthreads();
+  }
   bool nonfinite = false;
-  const unsigned long long best = cluster_best(row, V, sl, sh.warp_best, &sh.word, [&](int i, float x) {
+  const unsigned long long best = cluster_best<true>(row, V, sl, sh.warp_best, &sh.word, nonfinite, [&](int i, float x) {
     if (!isfinite(x)) nonfinite = true;
     if (use_pen && (seen_bits[i >> 5] >> (i & 31) & 1u)) x = x < 0.f ? x * pen : x / pen;
     if (temp > 0.f) x = x / temp;
     v[i] = x;
+    if (cuts) atomicAdd(&lane_copy[order_key(x) >> 24], 1u);
     return x;
   });
-  if (nonfinite) atomicExch(bad, 1);
   const float bv = key_value((uint32_t)(best >> 32));
   const int bi = best ? 0x7fffffff - (int)(uint32_t)best : 0;
   const bool writer = cluster_rank() == 0 && threadIdx.x == 0;
-  // the decision must be the same in every block of the cluster: they meet again at every pass
-  const bool any_nonfinite = cluster_sum((u64)__syncthreads_or(nonfinite), sh) != 0;
-  if (any_nonfinite || !(temp > 0.f)) {
-    if (writer) out_token[r] = bi;
+  // the decision is the same in every block of the cluster: they meet again at every pass
+  if (nonfinite || !(temp > 0.f)) {
+    if (writer) {
+      if (nonfinite) atomicExch(bad, 1);
+      out_token[r] = bi;
+    }
     return;
   }
   // top-k: the k-th largest key, and the id cut among the elements equal to it
   Kept kept{0u, 0x7fffffff};
-  const int k = top_k ? top_k[r] : 0;
-  if (k > 0 && k < V) {
+  if (cuts) {
     uint32_t prefix = 0;
     u64 above = 0;
-    for (int level = 0; level < 4; ++level) {
+    bool few = false;                   // no more elements down to the boundary's digit than a list takes: it is ordered whole
+    for (int level = 0; level < 4 && !few; ++level) {
       const int shift = 24 - 8 * level;
       const uint32_t pre = prefix;
       radix_pass<true>(v, V, sl, shift, above, (u64)k, turn, sh, copies,
-                       [&](uint32_t key, int) { return level == 0 || (key >> (shift + 8)) == pre; },
-                       [](float) { return 1u; }, true);
+                       [&](uint32_t key, int) { return (key >> (shift + 8)) == pre; },
+                       [](float) { return 1u; }, true, level == 0);
       prefix = (prefix << 8) | (uint32_t)sh.found[0];
       above = sh.found[1];
+      few = k <= kList && above + sh.found[2] <= (u64)kList;
+      kept.kth = prefix << shift;
     }
     const u64 ties = sh.found[2];
     const int first_id = (int)sh.low_all[prefix & 255u];
     __syncthreads();
-    kept.kth = prefix;
-    if (above + ties > (u64)k)             // a tie on the boundary: keep the lowest ids among the equal
+    if (!few && above + ties > (u64)k)     // a tie on the boundary: keep the lowest ids among the equal
       kept.id_cut = nth_holder(v, V, sl, prefix, Kept{0u, 0x7fffffff}, (u64)k - above, ties,
                                first_id == 0x7fffffff ? -1 : first_id, sh);
   }
-  if (k > 0 && k < V && k <= kList) {
-    const int id = select_from_list(v, V, sl, kept, bv, top_p[r], uniform[r], sh, reinterpret_cast<u64*>(copies));
+  if (cuts && k <= kList) {
+    const int id = select_from_list(v, V, sl, kept, k, bv, top_p[r], uniform[r], sh, reinterpret_cast<u64*>(copies));
     if (writer) {
       if (id < 0) atomicExch(bad, 1);
       out_token[r] = id < 0 ? bi : id;

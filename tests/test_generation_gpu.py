@@ -334,6 +334,28 @@ def test_sampling_around_the_longest_collected_list(V, k):
         assert consistent_with_plain(got[i], logits[i], [], 1.0, k, p.top_p, 1.0, uniform_for(seeds[i], idx[i])), (i, got[i])
 
 
+@pytest.mark.parametrize("V", [1500, 40004, 151936])
+@pytest.mark.parametrize("spread", [8.0, 0.25, 2.0 ** -11, 2.0 ** -18])
+def test_a_top_k_whose_search_ends_at_any_digit(V, spread):
+    """The search for the boundary ends as soon as a list takes all elements down to its digit: after one digit for values far
+    apart, after two, three or four for neighbours; behind it elements that share the digit but are not among the first k."""
+    from safetyraise_lmengine_b200.sampling.params import SamplingParams
+    from safetyraise_lmengine_b200.sampling.sampler import Sampler, uniform_for
+    rng = np.random.default_rng(V)
+    ks = [1, 7, 200, 512, 700, 0]
+    logits = np.full((len(ks), V), -3.0, dtype=np.float32)
+    for row in logits:                                 # 600 elements within `spread` of the top, in any place, 100 of them twice
+        at = rng.permutation(V)[:600]
+        row[at] = 4.0 + spread * rng.random(600, dtype=np.float32)
+        row[at[:100]] = row[at[100:200]]
+    params = [SamplingParams(temperature=1.0, top_p=[1.0, 0.7][i % 2], top_k=k) for i, k in enumerate(ks)]
+    for turn in range(3):
+        seeds = [90 + i for i in range(len(ks))]
+        got = Sampler(DEV, V, len(ks)).sample(torch.tensor(logits, device=DEV), params, seeds, [turn] * len(ks), [[]] * len(ks))
+        for i, p in enumerate(params):
+            assert consistent_with_plain(got[i], logits[i], [], 1.0, p.top_k, p.top_p, 1.0, uniform_for(seeds[i], turn)), (i, got[i])
+
+
 @pytest.mark.parametrize("V", [600, 40004])
 @pytest.mark.parametrize("k", [0, 1, 50, 512, 513])
 @pytest.mark.parametrize("top_p", [0.9, 1.0])
