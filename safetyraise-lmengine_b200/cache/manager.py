@@ -92,6 +92,8 @@ def runtime():
         lib.srlm_lay_out_tokens.argtypes = [C.c_int, at, at, at, at, at, at]
         lib.srlm_lay_out_tokens.restype = None
         lib.srlm_cache_lay_out_pages.argtypes = [C.c_void_p, C.c_int, C.c_int, at, at, at, C.c_int, C.c_int, at, at]
+        lib.srlm_sampling_uniforms.argtypes = [C.c_int, at, at, at]
+        lib.srlm_sampling_uniforms.restype = None
         lib.srlm_cache_destroy.argtypes = [C.c_void_p]
         lib.srlm_cache_reuse_counts.argtypes = [C.c_void_p, C.POINTER(C.c_int64), C.POINTER(C.c_int64)]
         lib.srlm_sched_destroy.argtypes = [C.c_void_p]

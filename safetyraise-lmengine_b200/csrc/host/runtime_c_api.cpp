@@ -36,6 +36,18 @@ int srlm_cache_table(void* c, int group, int slot, int32_t* out, int cap) {
 }
 int srlm_cache_free_pages(void* c, int group) { return static_cast<CacheManager*>(c)->free_pages(group); }
 int srlm_cache_audit(void* c) { return static_cast<CacheManager*>(c)->audit(); }
+static uint64_t splitmix64(uint64_t x) {
+  x += 0x9E3779B97F4A7C15ull;
+  x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
+  x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
+  return x ^ (x >> 31);
+}
+void srlm_sampling_uniforms(int n, const uint64_t* seeds, const uint64_t* indices, float* out) {
+  for (int i = 0; i < n; ++i) {
+    const uint64_t bits = splitmix64(splitmix64(seeds[i]) ^ (indices[i] + 1) * 0xD1B54A32D192ED03ull);
+    out[i] = static_cast<float>(bits >> 40) * (1.0f / (1 << 24));
+  }
+}
 void srlm_cache_reuse_counts(void* c, int64_t* taken, int64_t* reused) {
   *taken = static_cast<CacheManager*>(c)->pages_taken_total();
   *reused = static_cast<CacheManager*>(c)->pages_reused_total();

@@ -36,6 +36,8 @@ void srlm_lay_out_tokens(int n, const int32_t* starts, const int32_t* q_lens, in
                          int32_t* cu_q, int32_t* kv_lens);
 int srlm_cache_lay_out_pages(void* cache, int group, int n, const int32_t* slots, const int32_t* starts,
                              const int32_t* q_lens, int page_size, int pages, int32_t* tables, int32_t* kv_slot);
+/* out[i]: the uniform number in [0, 1) of draw indices[i] of a request with seeds[i] (24 bits, a function of the two alone). */
+void srlm_sampling_uniforms(int n, const uint64_t* seeds, const uint64_t* indices, float* out);
 void srlm_cache_reuse_counts(void* cache, int64_t* taken, int64_t* reused);
 
 void* srlm_sched_create(void* cache, int max_active, int queue_capacity, int prefill_chunk,

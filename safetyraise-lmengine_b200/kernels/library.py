@@ -1704,12 +1704,30 @@ class KernelLibrary:
         self._check(self.lib.srlm_argmax(_ptr(logits), C.c_longlong(logits.stride(0)), C.c_int(n), C.c_int(V),
                                          _ptr(out_tokens), _ptr(bad_flag), _stream()), "argmax")
 
+    def _check_sample_scratch(self, n, V, scratch):
+        if scratch is None or scratch.dtype != torch.float32 or scratch.numel() < n * V:
+            raise ShapeError("sample: scratch must hold n x V float32 values")
+
+    def sample_packed(self, logits, words, ids, out_tokens, bad_flag, scratch):
+        """sample() of what lies in one buffer of 32-bit words: temperature, top-p, penalty, uniform number (float32) and top-k of
+        the n rows, each n words; where ids > 0 then the rows' n + 1 offsets and that many ids."""
+        n, V = logits.shape
+        self._check_sample_scratch(n, V, scratch)
+        if words.dtype != torch.int32 or words.numel() < 5 * n + (n + 1 + ids if ids else 0) or out_tokens.numel() < n:
+            raise ShapeError(f"sample: {words.numel()} words for {n} rows and {ids} ids")
+        _ptr(words)                                           # (on the device and contiguous)
+        at = words.data_ptr()
+        part = lambda j: C.c_void_p(at + 4 * n * j)
+        self._check(self.lib.srlm_sample(
+            _ptr(logits), C.c_longlong(logits.stride(0)), C.c_int(n), C.c_int(V), part(0), part(4), part(1), part(2), part(3),
+            C.c_void_p(at + 4 * (6 * n + 1) if ids else 0), C.c_void_p(at + 20 * n if ids else 0), _ptr(scratch),
+            _ptr(out_tokens), _ptr(bad_flag), _stream()), "sample")
+
     def sample(self, logits, temperature, top_k, top_p, penalty, uniform, history, hist_offsets, out_tokens,
                bad_flag, scratch):
         """scratch: float32 [n, V] that the kernel may overwrite (the adjusted values of each row)."""
         n, V = logits.shape
-        if scratch is None or scratch.dtype != torch.float32 or scratch.numel() < n * V:
-            raise ShapeError("sample: scratch must hold n x V float32 values")
+        self._check_sample_scratch(n, V, scratch)
         self._check(self.lib.srlm_sample(_ptr(logits), C.c_longlong(logits.stride(0)), C.c_int(n), C.c_int(V),
                                          _ptr(temperature), _ptr(top_k), _ptr(top_p), _ptr(penalty),
                                          _ptr(uniform), _ptr(history), _ptr(hist_offsets), _ptr(scratch),

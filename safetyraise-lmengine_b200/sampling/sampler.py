@@ -9,11 +9,13 @@ distribution and order of operations are.
 from __future__ import annotations
 
 import os
+from itertools import chain
 from typing import List, Sequence
 
 import numpy as np
 import torch
 
+from ..cache.manager import runtime
 from ..kernels import ops
 from ..parts.base import FAULT_LOGITS, FAULT_TOKEN, STATUS_WORDS
 from .params import SamplingParams
@@ -33,6 +35,16 @@ def uniform_for(seed: int, index: int) -> float:
     """A float32 in [0, 1) for the index-th draw of a request with this seed."""
     bits = _splitmix64(_splitmix64(seed & _MASK) ^ ((index + 1) * 0xD1B54A32D192ED03 & _MASK))
     return float(np.float32((bits >> 40) * (1.0 / (1 << 24))))
+
+
+def fill_uniforms(seeds: Sequence[int], indices: Sequence[int], out: np.ndarray) -> None:
+    """out[i] = uniform_for(seeds[i], indices[i]) (float32, contiguous) in one native call: two microseconds a pair in Python."""
+    n = len(out)
+    pairs = np.array([x & _MASK for x in chain(seeds, indices)], dtype=np.uint64)
+    if len(pairs) != 2 * n:
+        raise ValueError(f"{n} rows, {len(seeds)} seeds and {len(indices)} indices")
+    at = pairs.ctypes.data
+    runtime().srlm_sampling_uniforms(n, at, at + 8 * n, out.ctypes.data)
 
 
 def fresh_seed() -> int:
@@ -55,6 +67,7 @@ class Sampler:
         self.bad = self._status[FAULT_LOGITS:FAULT_LOGITS + 1]
         self.last_words = [0] * STATUS_WORDS      # the fault words as the last collect() read them
         self._cap = 0
+        self._hosts, self._host_turn, self._dev = [], 0, None
         self._grow(max_rows)
 
     def _grow(self, rows: int):
@@ -68,15 +81,21 @@ class Sampler:
             self._status[:self._words].copy_(old[:self._words])
             self.bad = self._status[FAULT_LOGITS:FAULT_LOGITS + 1]
         self._cap = rows
-        # the rows' parameters go through pinned buffers taken in turn: a launch may be queued while the copy
-        # of the launch before it has not run yet; each buffer waits for the event behind its last copy
-        self._hosts = [[torch.empty(5 * rows, dtype=torch.float32, pin_memory=True), None] for _ in range(3)]
-        self._host_turn = 0
-        self._dev = torch.empty(5 * rows, dtype=torch.float32, device=self.device)
         self._out = self._status[self._words:self._words + rows]
         self._scratch = None               # [rows, vocab] float32, made when a row is first sampled
-        if not hasattr(self, "_hist_host"):
-            self._hist_host = self._hist_dev = None
+
+    def _buffer(self, words: int):
+        """A pinned buffer of at least ``words`` 32-bit words, one of three taken in turn (a launch may be queued while the
+        copy of the launch before it has not run yet), once the event behind its last copy has passed."""
+        if not self._hosts or self._hosts[0][0].numel() < words:
+            cap = max(words, 4096, 2 * self._hosts[0][0].numel() if self._hosts else 0)
+            self._hosts = [[torch.empty(cap, dtype=torch.int32, pin_memory=True), torch.cuda.Event(), False] for _ in range(3)]
+            self._dev = torch.empty(cap, dtype=torch.int32, device=self.device)
+        self._host_turn = (self._host_turn + 1) % len(self._hosts)
+        turn = self._hosts[self._host_turn]
+        if turn[2]:
+            turn[1].synchronize()
+        return turn
 
     def sample(self, logits: torch.Tensor, params: Sequence[SamplingParams], seeds: Sequence[int],
                indices: Sequence[int], histories: Sequence[Sequence[int]]) -> List[int]:
@@ -131,69 +150,52 @@ class Sampler:
         if all(p.is_greedy for p in params):
             ops.argmax(logits, self._out[:n], self.bad)
             return n
-        self._host_turn = (self._host_turn + 1) % len(self._hosts)
-        pair = self._hosts[self._host_turn]
-        if pair[1] is not None:
-            pair[1].synchronize()
-        h = pair[0].numpy()
-        c = self._cap
-        for i, p in enumerate(params):
-            h[i] = p.temperature
-            h[c + i] = p.top_p
-            h[2 * c + i] = p.repetition_penalty
-            h[3 * c + i] = uniform_for(seeds[i], indices[i]) if p.temperature > 0 else 0.0
-        h[4 * c:4 * c + n].view(np.int32)[:] = [p.top_k for p in params]
-        self._dev.copy_(pair[0], non_blocking=True)
-        pair[1] = torch.cuda.Event()
-        pair[1].record()
-        d = self._dev
-        hist = offs = None
-        if any(p.repetition_penalty != 1.0 for p in params):
-            # ids and row offsets go through one pinned buffer and one asynchronous copy: a pageable
-            # copy would make the host wait for the forward that is still running on the device
-            late = [pending is not None and pending[i] is not None and p.repetition_penalty != 1.0
-                    for i, p in enumerate(params)]
-            lens = [len(hh) + late[i] if p.repetition_penalty != 1.0 else 0
-                    for i, (p, hh) in enumerate(zip(params, histories))]
+        # All that the rows bring goes through one pinned buffer and one asynchronous copy (a pageable copy would make the host
+        # wait for the forward that is still running on the device), as 32-bit words: five parameters a row, each n words;
+        # with a penalty the rows' offsets and ids, and the pairs of patch_words behind them.
+        penalised = [p.repetition_penalty != 1.0 for p in params]
+        words, late, total = 5 * n, [], 0
+        if any(penalised):
+            late = [on and pending is not None and pending[i] is not None for i, on in enumerate(penalised)]
+            lens = [len(ids) + behind if on else 0 for on, ids, behind in zip(penalised, histories, late)]
             total = sum(lens)
-            words = n + 1 + max(total, 1) + 2 * sum(late)            # (the pairs of patch_words ride behind)
-            if self._hist_host is None or self._hist_host[0][0].numel() < words:
-                cap = max(words, 2 * (self._hist_host[0][0].numel() if self._hist_host is not None else 4096))
-                # pinned buffers taken in turn, like the parameters' (a launch may be queued before the copy of
-                # the launch ahead of it has run)
-                self._hist_host = [[torch.empty(cap, dtype=torch.int32, pin_memory=True), None] for _ in range(3)]
-                self._hist_dev = torch.empty(cap, dtype=torch.int32, device=self.device)
-                self._hist_turn = 0
-            self._hist_turn = (self._hist_turn + 1) % len(self._hist_host)
-            hist_pair = self._hist_host[self._hist_turn]
-            if hist_pair[1] is not None:
-                hist_pair[1].synchronize()
-            hh_np = hist_pair[0].numpy()
-            hh_np[0] = 0
-            np.cumsum(lens, out=hh_np[1:n + 1])
-            at = n + 1
-            pairs = []
-            for i, (ln, hist_ids) in enumerate(zip(lens, histories)):
-                if ln:
-                    hh_np[at:at + ln - late[i]] = hist_ids
-                    if late[i]:
-                        hh_np[at + ln - 1] = -1                       # an id the kernel skips, until it is put in place
-                        pairs += [at + ln - 1, int(pending[i])]
-                    at += ln
+            words += n + 1 + max(total, 1) + 2 * sum(late)
+        turn = self._buffer(words)
+        host = turn[0].numpy()
+        h = host[:4 * n].view(np.float32)
+        h[:n] = [p.temperature for p in params]
+        h[n:2 * n] = [p.top_p for p in params]
+        h[2 * n:3 * n] = [p.repetition_penalty for p in params]
+        fill_uniforms(seeds, indices, h[3 * n:])              # (of a row without a temperature nothing is drawn)
+        host[4 * n:5 * n] = [p.top_k for p in params]
+        pairs = []
+        if late:
+            offsets, at = host[5 * n:6 * n + 1], 6 * n + 1
+            offsets[0] = 0
+            np.cumsum(lens, out=offsets[1:])
+            if True not in late:
+                host[at:at + total] = np.fromiter(chain.from_iterable(ids for on, ids in zip(penalised, histories) if on),
+                                                  np.int32, total)
+            else:
+                for i, (ln, ids) in enumerate(zip(lens, histories)):
+                    if ln:
+                        host[at:at + ln - late[i]] = ids
+                        if late[i]:
+                            host[at + ln - 1] = -1                # an id the kernel skips, until it is put in place
+                            pairs += [at + ln - 1 - 5 * n, int(pending[i])]
+                        at += ln
             if total == 0:
-                hh_np[n + 1] = 0
-            ids_end = n + 1 + max(total, 1)
-            hh_np[ids_end:ids_end + len(pairs)] = pairs
-            self._hist_dev[:words].copy_(hist_pair[0][:words], non_blocking=True)
-            hist_pair[1] = torch.cuda.Event()
-            hist_pair[1].record()
-            if pairs:
-                ops.patch_words(self._hist_dev, self._hist_dev[ids_end:ids_end + len(pairs)],
-                                self._status[self._words:], len(pairs) // 2, self._status[FAULT_TOKEN:FAULT_TOKEN + 1])
-            offs = self._hist_dev[:n + 1]
-            hist = self._hist_dev[n + 1:ids_end]
+                host[6 * n + 1] = 0
+            ids_end = 6 * n + 1 + max(total, 1)
+            host[ids_end:ids_end + len(pairs)] = pairs
+        dev = self._dev[:words]
+        dev.copy_(turn[0][:words], non_blocking=True)
+        turn[1].record()
+        turn[2] = True
+        if pairs:
+            ops.patch_words(dev[5 * n:], dev[ids_end:ids_end + len(pairs)], self._status[self._words:], len(pairs) // 2,
+                            self._status[FAULT_TOKEN:FAULT_TOKEN + 1])
         if self._scratch is None or self._scratch.shape[0] < self._cap:
             self._scratch = torch.empty(self._cap, self.vocab, dtype=torch.float32, device=self.device)
-        ops.sample(logits, d[:n], d[4 * c:4 * c + n].view(torch.int32), d[c:c + n], d[2 * c:2 * c + n],
-                   d[3 * c:3 * c + n], hist, offs, self._out[:n], self.bad, self._scratch)
+        ops.sample_packed(logits, dev, max(total, 1) if late else 0, self._out[:n], self.bad, self._scratch)
         return n

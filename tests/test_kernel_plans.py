@@ -53,3 +53,19 @@ def test_prefill_attention_plan():
         assert tiles in (1, 2) and 1 <= nsplit <= 16
         if nsplit > 1:
             assert tiles == 2 and chunk % 128 == 0 and nsplit * chunk >= max(kv) > (nsplit - 1) * chunk - 128
+
+
+def test_native_uniform_numbers_are_those_of_the_plain_function():
+    import random
+
+    import numpy as np
+    import pytest
+    from safetyraise_lmengine_b200.sampling.sampler import fill_uniforms, uniform_for
+    r = random.Random(5)
+    seeds = [r.randrange(-9, 1 << 64) for _ in range(300)] + [0, -1, (1 << 64) - 1]
+    indices = [r.randrange(1 << 31) for _ in seeds]
+    out = np.empty(len(seeds), dtype=np.float32)
+    fill_uniforms(seeds, indices, out)
+    assert out.tolist() == [uniform_for(s, i) for s, i in zip(seeds, indices)]
+    with pytest.raises(ValueError):
+        fill_uniforms(seeds, indices, out[1:])
