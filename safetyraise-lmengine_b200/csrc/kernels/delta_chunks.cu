@@ -12,8 +12,10 @@
 //   delta_chunks       a block per (chunk, head): convolution, silu, unit vectors, beta, decays, and the record of the chunk;
 //                      bound by instructions (silu, the products by X and M) at 20 warps an SM.
 //   delta_chunk_walk   a block per (entry, head, 16 columns of S) walks the records: three products a chunk on tensor cores,
-//                      S in the accumulators; bound by the latency of a chunk (two exchanges between the eight warps).
-// 2,000 tokens, 16 heads of 128 x 128, one entry: 84 + 155 us; the kernels that go token by token: 98 + 610 us.
+//                      S in the accumulators; bound by the latency of a chunk (two exchanges between the eight warps).  Blocks
+//                      start in the order of their entries' lengths, the longest first: entries of 486, 458 and 1,056 tokens
+//                      163 us in the step's order, where the longest waited for places, 126 so.
+// 2,000 tokens, 16 heads of 128 x 128, one entry: 77 + 153 us; the kernels that go token by token: 98 + 610 us.
 //
 // The products of the walk are mma.sync m16n8k8 on tf32 operands, each operand split into two tf32 numbers (high, and the rest)
 // and each product formed as high high + high low + low high.  Relative error against float64 (2-norm; 16 to 2,000 tokens, decays
@@ -104,33 +106,45 @@ delta_chunks_kernel(const float* __restrict__ proj, long long ldp, const float* 
 #pragma unroll
     for (int i = 0; i < TOK; ++i) (part ? k_s : q_s)[i][tid] = y[i];
   }
-  if (tid < TOK) {
+  // The scalars in 64 bits take long chains of instructions: side by side, in lanes and warps of their own.
+  if (warp == 1 && lane < TOK) {
     float b = 0.f;
-    double g = 1.;
-    if (tid < home.n) {
-      const float* row = proj + (size_t)(home.t0 + tid) * ldp + z.C;
-      const double a = (double)row[z.H + h] + dt_bias[h];
-      b = (float)(1. / (1. + exp(-(double)row[h])));
-      g = exp(-exp((double)a_log[h]) * (a > 20. ? a + log1p(exp(-a)) : log1p(exp(a))));
+    if (lane < home.n) b = (float)(1. / (1. + exp(-(double)proj[(size_t)(home.t0 + lane) * ldp + z.C + h])));
+    beta_s[lane] = b;
+  }
+  if (warp == 0) {                             // lane i: g_i; then column i of D, and P
+    const bool on = lane < min(home.n, TOK);
+    const double a = on ? (double)proj[(size_t)(home.t0 + lane) * ldp + z.C + z.H + h] + dt_bias[h] : 0.;
+    const bool far = a > 20.;
+    const double e = exp(lane < TOK ? (far ? -a : a) : (double)a_log[h]);        // the upper lanes: exp(a_log)
+    const double rate = __shfl_sync(0xffffffffu, e, TOK), l = log1p(e);
+    const double g = on ? exp(-rate * (far ? a + l : l)) : 1.;
+    if (lane < TOK) g_s[lane] = g;
+    __syncwarp();
+    if (lane < TOK) {
+      double p = 1., d = 1.;
+      for (int i = 0; i <= lane; ++i) p *= g_s[i];
+      pre_s[lane] = p;
+      for (int i = 0; i < TOK; ++i) {
+        if (i > lane) d *= g_s[i];
+        d_s[i][lane] = i >= lane ? d : 0.;
+      }
     }
-    beta_s[tid] = b;
-    g_s[tid] = g;
   }
   __syncthreads();
-  for (int v = warp; v < 2 * TOK; v += 4) {
-    const int i = v % TOK;
-    const float4 x = *reinterpret_cast<const float4*>((v < TOK ? k_s[i] : q_s[i]) + 4 * lane);
-    const float ss = warp_sum((x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w));
-    const double one = v < TOK ? 1. : 1. / sqrt((double)DK);
-    if (lane == 0) (v < TOK ? unit_k : unit_q)[i] = i < home.n ? one / sqrt((double)ss + unit_eps) : 0.;   // a place without a token
-  }
-  if (tid < TOK) {                             // column tid of D, and P
-    double p = 1., d = 1.;
-    for (int i = 0; i <= tid; ++i) p *= g_s[i];
-    pre_s[tid] = p;
-    for (int i = 0; i < TOK; ++i) {
-      if (i > tid) d *= g_s[i];
-      d_s[i][tid] = i >= tid ? d : 0.;
+  {
+    float mine = 0.f;                          // lane j: of the warp's j-th token of k, then of q
+#pragma unroll
+    for (int j = 0; j < 2 * TOK / 4; ++j) {
+      const int v = warp + 4 * j, i = v % TOK;
+      const float4 x = *reinterpret_cast<const float4*>((v < TOK ? k_s[i] : q_s[i]) + 4 * lane);
+      const float ss = warp_sum((x.x * x.x + x.y * x.y) + (x.z * x.z + x.w * x.w));
+      if (lane == j) mine = ss;
+    }
+    if (lane < 2 * TOK / 4) {
+      const int v = warp + 4 * lane, i = v % TOK;
+      const double one = v < TOK ? 1. : 1. / sqrt((double)DK);
+      (v < TOK ? unit_k : unit_q)[i] = i < home.n ? one / sqrt((double)mine + unit_eps) : 0.;      // a place without a token
     }
   }
   // k_i . k_j (threads 0 .. 63) and q_i . k_j (64 .. 127): rows i, i + 8, columns j, j + 8
@@ -271,12 +285,29 @@ delta_chunk_walk_kernel(const float* __restrict__ records, float* __restrict__ s
   float* p_sums = chunk_smem + STAGES * STAGE;           // [warp][SUMS]: kx . S
   float* q_sums = p_sums + WARPS * SUMS;                 // qm . S
   float* u_s = q_sums + WARPS * SUMS;                    // [token][U_LD]
-  // the blockIdx.z-th of the entries that go by chunks, and the place of its first record
-  int e = blockIdx.z, base = -first_chunk;
-  if (gridDim.z == n_entries) {                          // all of them
-    for (int x = 0; x < e; ++x) base += chunks_of(cu_q[x + 1] - cu_q[x], least);
-  } else {
-    e = n_entries;
+  // the blockIdx.z-th longest of the entries, and the place of its first record: the blocks of the longest entry start first
+  int e = n_entries, base = 0;
+  if (n_entries == 1) {
+    e = 0;
+    base = -first_chunk;
+  } else if (n_entries <= THREADS) {
+    __shared__ int found[2];
+    const int t = threadIdx.x;
+    if (t < n_entries) {
+      const int len = cu_q[t + 1] - cu_q[t];
+      int longer = 0, before = -first_chunk;
+#pragma unroll 4
+      for (int x = 0; x < n_entries; ++x) {
+        const int other = cu_q[x + 1] - cu_q[x];
+        longer += other > len || (other == len && x < t);
+        before += x < t ? chunks_of(other, least) : 0;
+      }
+      if (longer == (int)blockIdx.z) found[0] = t, found[1] = before;
+    }
+    __syncthreads();
+    e = __reduce_max_sync(0xffffffffu, found[0]);        // (the same in every lane, which the compiler can see)
+    base = __reduce_max_sync(0xffffffffu, found[1]);
+  } else {                                               // more than one a thread: in the step's order
 #pragma unroll 8
     for (int x = 0, seen = 0, before = -first_chunk; x < n_entries; ++x) {       // no way out: the loads do not wait for each other
       const int mine = chunks_of(cu_q[x + 1] - cu_q[x], least);

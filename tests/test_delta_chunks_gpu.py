@@ -151,7 +151,7 @@ def walked(lens, held=None, max_tokens=None):
     ctx, state = Ctx(lens, list(range(len(lens)))), torch.stack(states)
     if max_tokens:
         ctx.workspace.max_tokens = max_tokens
-    o = torch.empty(sum(lens), H * dv, device=DEV)
+    o = torch.full((sum(lens), H * dv), float("nan"), device=DEV)
     was = type(ops).DELTA_CHUNKS_HELD
     try:
         type(ops).DELTA_CHUNKS_HELD = held or was
@@ -170,6 +170,19 @@ def test_steps_whose_chunks_are_taken_by_turns(held):
     o2, state2, work = walked(lens, held)
     assert torch.equal(o, o2) and torch.equal(state, state2)
     assert max(b.shape[0] for (name, _, _), b in work._bufs.items() if name == "delta.records") == 4 * held
+
+
+@pytest.mark.parametrize("lens", [[16, 40, 40, 100, 17], [100, 1, 16, 16, 300, 3, 16], [17, 1, 20] * 85, [17, 1, 20, 33] * 64, [20, 1, 17] * 86])
+def test_entries_in_the_order_of_their_length(lens):
+    """Equal lengths, short ones between them, as many entries as a block has threads (256) and more: the blocks take the longest
+    first, and every entry's bits are those of a step of the first few alone."""
+    o, state, _ = walked(lens)
+    for first in (1, 5):
+        alone, alone_state, _ = walked(lens[:first])
+        assert torch.equal(o[:sum(lens[:first])].isnan(), alone.isnan())
+        long = [t for t, n in zip(torch.arange(sum(lens[:first])).split(lens[:first]), lens) if n >= 16]
+        rows = torch.cat(long).to(DEV)
+        assert torch.equal(o[rows], alone[rows]) and torch.equal(state[:first], alone_state)
 
 
 def test_an_entry_does_not_depend_on_who_shares_the_step():
