@@ -12,11 +12,11 @@
 //
 //   conv   one thread per (token, four neighbouring channels; one where rows do not allow 16-byte accesses): reads
 //          the step's inputs, and the slot's carried inputs for the first taps - 1 tokens of an entry
-//   scan   one block per (entry, 16 channels): four warps walk the entry's tokens in order, 8 lanes sharing a channel's
-//          N states, through chunks of 16 tokens in shared memory; the lanes' partial sums of 8 tokens are added in
-//          one exchange of 7 shuffles.  Four more warps fetch the chunks several ahead (cp.async), form the step
-//          sizes, and gate and write a finished chunk's y as a block; at the end the walkers renew the slot's S and
-//          carried inputs.
+//   scan   one block per (entry, 16 channels): two or four warps walk the entry's tokens in order, 4 lanes (8 from 17
+//          states on) sharing a channel's N states, through chunks of 16 tokens in shared memory; the lanes' partial sums
+//          of 8 tokens are added in one exchange of 6 shuffles (7).  Four more warps fetch the chunks several ahead
+//          (cp.async), form the step sizes, and gate and write a finished chunk's y as a block; at the end the walkers
+//          renew the slot's S and carried inputs.
 //          A channel's sums do not depend on what else is in the step or on how the tokens were cut into steps.
 #include <math_constants.h>
 
@@ -156,7 +156,8 @@ __global__ void scan_conv_rows_kernel(const float* __restrict__ xz, long long ld
   }
 }
 
-constexpr int kScanLanes = 8, kScanChannels = 16, kScanChunk = 16;
+constexpr int kScanChannels = 16, kScanChunk = 16;
+constexpr int scan_helpers(bool lengthy) { return lengthy ? 256 : 128; }
 
 __device__ __forceinline__ void scan_cp_async_4(float* dst, const float* src) {
   const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
@@ -171,6 +172,7 @@ template <int N>
 __device__ __forceinline__ void scan_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kScanStates = 128;                           // most states of a channel
 
 // 2^x for x <= 0 (a decay): the hardware's approximation, 2 ulp, zero below 2^-126
 __device__ __forceinline__ float scan_exp2(float x) {
@@ -179,19 +181,43 @@ __device__ __forceinline__ float scan_exp2(float x) {
   return y;
 }
 
-// n neighbouring floats of shared memory (n a power of two; the address a multiple of min(n, 4) floats)
-template <int NPL>
-__device__ __forceinline__ void scan_load_row(const float* src, float (&dst)[NPL]) {
-  if constexpr (NPL == 1) {
-    dst[0] = src[0];
-  } else if constexpr (NPL == 2) {
-    const float2 f = *reinterpret_cast<const float2*>(src);
-    dst[0] = f.x, dst[1] = f.y;
+// Two neighbouring floats as one operand: an instruction of the FMA pipe for both, each rounded as alone.
+typedef unsigned long long Pair;
+__device__ __forceinline__ Pair pair_of(float lo, float hi) {
+  Pair p;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(p) : "f"(lo), "f"(hi));
+  return p;
+}
+__device__ __forceinline__ float2 halves_of(Pair p) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(p));
+  return f;
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  Pair p;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(a), "l"(b));
+  return p;
+}
+__device__ __forceinline__ Pair fma2(Pair a, Pair b, Pair c) {
+  Pair p;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(p) : "l"(a), "l"(b), "l"(c));
+  return p;
+}
+__device__ __forceinline__ Pair scan_exp2(Pair p) {
+  const float2 f = halves_of(p);
+  return pair_of(scan_exp2(f.x), scan_exp2(f.y));
+}
+
+// n neighbouring pairs of shared memory (n a power of two; the address a multiple of min(n, 2) pairs)
+template <int PAIRS>
+__device__ __forceinline__ void scan_load_row(const float* src, Pair (&dst)[PAIRS]) {
+  if constexpr (PAIRS == 1) {
+    dst[0] = *reinterpret_cast<const Pair*>(src);
   } else {
 #pragma unroll
-    for (int k = 0; k < NPL; k += 4) {
-      const float4 f = *reinterpret_cast<const float4*>(src + k);
-      dst[k] = f.x, dst[k + 1] = f.y, dst[k + 2] = f.z, dst[k + 3] = f.w;
+    for (int k = 0; k < PAIRS; k += 2) {
+      const ulonglong2 f = *reinterpret_cast<const ulonglong2*>(src + 2 * k);
+      dst[k] = f.x, dst[k + 1] = f.y;
     }
   }
 }
@@ -201,7 +227,7 @@ __device__ __forceinline__ void scan_load_row(const float* src, float (&dst)[NPL
 // the step size and its product with x; and the block's y ahead of the gate.  Places behind an entry's last token hold
 // dt = 0, dt x = 0, B = 0: S <- fma(1, S, 0) leaves every state as it is, so the walk has no branch.
 //
-// The block's first four warps walk; its other four fetch, prepare and finish.  While the walkers are on chunk j the
+// The block's last four warps fetch, prepare and finish; the others walk.  While the walkers are on chunk j the
 // helpers turn the raw step sizes of chunk j + 1 into softplus(dt + bias) and its product with x, gate and write the y
 // of chunk j - 1, issue the fetch of chunk j + K - 2 into the buffer chunk j - 2 has left, and wait until their own
 // copies of chunk j + 2 have landed: K buffers of operands (a fetch has K - 4 walks of a chunk to arrive: a chunk's walk
@@ -209,49 +235,62 @@ __device__ __forceinline__ void scan_load_row(const float* src, float (&dst)[NPL
 // copies, an empty one behind the entry's end, so that "all but the last K - 4 groups" always names chunk j + 2.  A
 // helper reads what other helpers fetched, and overwrites what other helpers read, only with a barrier in between.
 //
-// Bound by the SM's instructions, walkers and helpers together: 2,048 tokens, 4,096 channels of 16 states 131 us (with
-// the helpers copying four bytes at a time, (token, channel) by (token, channel), and reading bias and D for each,
-// 227 us at 3,570 cycles a chunk).
-constexpr int kScanWalkers = kScanLanes * kScanChannels, kScanThreads = 2 * kScanWalkers;
-constexpr int scan_buffers(int npl) { return npl <= 2 ? 8 : npl <= 4 ? 7 : npl <= 8 ? 6 : 5; }
+// Bound by a chunk's dependent instructions, of the walkers (75 cycles a token in the form for two blocks an SM) and of the
+// helpers alike, and with several blocks an SM by their number: 2,048 tokens, 4,096 channels of 16 states 107 us (2,048
+// channels 88).  With 8 lanes a channel and a state an instruction 132 (105); pairs of states in 4 lanes 133, with both groups
+// of a chunk and 96 registers in flight 111, with a copy a helper 107.  8 lanes of a pair each: 74 us at 2,048 channels, where
+// an SM has one block, and 119 at 4,096.
+constexpr int scan_buffers(int np) { return np <= 16 ? 8 : np <= 32 ? 7 : np <= 64 ? 6 : 5; }
 constexpr int kScanPlane = kScanChunk * kScanChannels;
-// floats of shared memory: two of pairs, two of y, `held` buffers (B | C up to the lanes' reach, three planes)
-constexpr int scan_floats(int npl, int held) {
-  return 2 * 2 * kScanPlane + 2 * kScanPlane + held * (kScanChunk * 2 * npl * kScanLanes + 3 * kScanPlane);
+constexpr int kScanYRow = kScanChannels + 4;               // floats from a token's y to the next: a channel's lanes share no bank
+// floats of shared memory: two of steps, two of y, `held` buffers (B | C up to the lanes' reach, three planes)
+constexpr int scan_floats(int np, int held) {
+  return 2 * 2 * kScanPlane + 2 * kScanChunk * kScanYRow + held * (kScanChunk * 2 * np + 3 * kScanPlane);
 }
-__device__ __forceinline__ void scan_helpers_meet() { asm volatile("bar.sync 1, %0;" ::"n"(kScanWalkers) : "memory"); }
+template <int HELPERS>
+__device__ __forceinline__ void scan_helpers_meet() { asm volatile("bar.sync 1, %0;" ::"n"(HELPERS) : "memory"); }
 
-// WIDE: channels, N, the rows and the pointers allow copies of 16 bytes
-template <typename TO, int NPL, bool WIDE>
-__global__ void __launch_bounds__(kScanThreads, NPL <= 4 ? 5 : NPL <= 8 ? 4 : 3)
+// WIDE: channels, N, the rows and the pointers allow copies of 16 bytes.  LENGTHY (with WIDE): a long walk of few blocks
+// LANES of a channel hold NPL states each, neighbours
+template <typename TO, int LANES, int NPL, bool WIDE, bool LENGTHY>
+__global__ void __launch_bounds__(LANES * kScanChannels + scan_helpers(LENGTHY), LENGTHY ? 2 : NPL <= 4 ? 5 : NPL <= 8 ? 4 : 3)
 selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz, long long ld_xz,
                       const float* __restrict__ dbc, long long ld_dbc, int b_off, const float* __restrict__ dt_raw,
                       const float* __restrict__ dt_bias, const float* __restrict__ A, const float* __restrict__ D,
                       float* __restrict__ state, long long state_stride, const int* __restrict__ cu_q,
                       const int* __restrict__ slots, TO* __restrict__ out, int channels, int N, int taps) {
-  constexpr int NP = NPL * kScanLanes;                      // states a channel's lanes reach, >= N
-  constexpr int GROUP = NPL <= 2 ? 8 : NPL <= 4 ? 4 : 2;    // tokens whose independent work the compiler interleaves
-  constexpr int BC = kScanChunk * 2 * NP, YS = kScanPlane;
-  constexpr int K = scan_buffers(NPL);
+  constexpr int NP = NPL * LANES;                           // states a channel's lanes reach, >= N
+  constexpr int GROUP = LANES == 4 ? 8 : NPL <= 4 ? 4 : 2;  // tokens whose independent work the compiler interleaves
+  constexpr int BC = kScanChunk * 2 * NP, YS = kScanPlane, WALKERS = LANES * kScanChannels, PAIRS = NPL / 2;
+  constexpr int HELPERS = scan_helpers(LENGTHY), UNROLL = LENGTHY && NPL <= 4 ? kScanChunk / GROUP : 1;
+  constexpr int K = scan_buffers(NP);
   pdl_wait();
   extern __shared__ __align__(16) float scan_smem[];
   float2* step_s = reinterpret_cast<float2*>(scan_smem);    // [2][chunk][channels of the block]: dt, dt x
-  float* y_s = scan_smem + 2 * 2 * YS;                      // [2][chunk][channels of the block]
+  float* y_s = scan_smem + 2 * 2 * YS;                      // [2][chunk][kScanYRow]
   // K buffers, of which a launch has those that its longest entry fills (chunk j lies in buffer j % K): [3][chunk][channels of the
   // block], raw dt, x, z, then [chunk][2 NP], B and C
   constexpr int BUF = 3 * YS + BC;
-  float* raw_s = y_s + 2 * YS;
+  float* raw_s = y_s + 2 * kScanChunk * kScanYRow;
   float* bc_s = raw_s + 3 * YS;
   const int e = blockIdx.y, c0 = blockIdx.x * kScanChannels;
-  const bool walker = threadIdx.x < kScanWalkers;
-  const int tid = walker ? threadIdx.x : threadIdx.x - kScanWalkers;      // place among the walkers, or among the helpers
-  const int lane = tid % kScanLanes, ch = tid / kScanLanes;
+  const bool walker = threadIdx.x < WALKERS;
+  const int tid = walker ? threadIdx.x : threadIdx.x - WALKERS;           // place among the walkers, or among the helpers
+  const int lane = tid % LANES, ch = tid / LANES;
   const int c = c0 + ch;
   const bool live = c < channels;
   const int t0 = cu_q[e], q_len = cu_q[e + 1] - t0;
   float* slot = state + (size_t)slots[e] * state_stride;
   const int n_chunks = (q_len + kScanChunk - 1) / kScanChunk;
 
+  // what a helper copies of every chunk where there are more helpers than copies of either kind: a piece of B or C, a piece of a
+  // plane (raw dt, x, z: 64 pieces each)
+  const int bc_i = tid / 8, raw_p = (tid - 64) / 64, raw_i = (tid - 64) % 64 / 4, raw_c = c0 + (tid - 64) % 4 * 4;
+  const int bc_n = tid % 4 * 4;
+  const float* bc_from = dbc + (size_t)(t0 + bc_i) * ld_dbc + b_off + (tid % 8 / 4) * N + bc_n;
+  const bool raw_on = raw_c < channels;
+  const long long raw_ld = raw_p == 2 ? ld_xz : channels;
+  const float* raw_from = (raw_p == 0 ? dt_raw : raw_p == 1 ? x : xz + channels) + (size_t)(t0 + raw_i) * raw_ld + raw_c;
   // helpers: the fetch of chunk j, one group of copies (an empty one behind the last chunk)
   auto stage = [&](int j) {
     if (j >= n_chunks) {
@@ -261,8 +300,15 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
     const int base = j * kScanChunk, n_here = min(kScanChunk, q_len - base);
     float* bc = bc_s + (j % K) * BUF;
     float* raw = raw_s + (j % K) * BUF;
+    if constexpr (LENGTHY && NP == 16) {                    // 128 pieces of B and C, 192 of the planes
+      if (tid < 128 && bc_i < n_here && bc_n < N) scan_cp_async_16(bc + 4 * tid, bc_from + (size_t)j * kScanChunk * ld_dbc);
+      if (tid < 128 && (bc_i >= n_here || bc_n >= N)) *reinterpret_cast<float4*>(bc + 4 * tid) = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (tid >= 64 && raw_on && raw_i < n_here) scan_cp_async_16(raw + 4 * (tid - 64), raw_from + (size_t)j * kScanChunk * raw_ld);
+      scan_cp_async_commit();
+      return;
+    }
     constexpr int V = WIDE ? 4 : 1;                         // floats a copy
-    for (int idx = tid; idx < BC / V; idx += kScanWalkers) {
+    for (int idx = tid; idx < BC / V; idx += HELPERS) {
       const int i = idx / (2 * NP / V), r = idx % (2 * NP / V) * V, half = r / NP, n = r % NP;
       float* dst = bc + idx * V;
       if (i < n_here && n < N) {
@@ -274,7 +320,7 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
         for (int u = 0; u < V; ++u) dst[u] = 0.f;
       }
     }
-    for (int idx = tid; idx < YS / V; idx += kScanWalkers) {
+    for (int idx = tid; idx < YS / V; idx += HELPERS) {
       const int i = idx / (kScanChannels / V), cc = idx % (kScanChannels / V) * V;
       if (i >= n_here || c0 + cc >= channels) continue;
       const size_t t = (size_t)(t0 + base + i);
@@ -295,8 +341,8 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
     const float* raw = raw_s + (j % K) * BUF;
     float2* step = step_s + (j & 1) * YS;
 #pragma unroll
-    for (int u = 0; u < YS / kScanWalkers; ++u) {
-      const int idx = tid + u * kScanWalkers;
+    for (int u = 0; u < YS / HELPERS; ++u) {
+      const int idx = tid + u * HELPERS;
       const bool on = idx / kScanChannels < n_here && hc < channels;
       const float dt = on ? softplus_f(raw[idx] + bias) : 0.f;
       step[idx] = make_float2(dt, on ? dt * raw[YS + idx] : 0.f);
@@ -306,30 +352,31 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
   auto finish = [&](int j) {
     const int base = j * kScanChunk, n_here = min(kScanChunk, q_len - base);
     const float* raw = raw_s + (j % K) * BUF;
-    const float* ys = y_s + (j & 1) * YS;
+    const float* ys = y_s + (j & 1) * kScanChunk * kScanYRow;
     if (hc >= channels) return;
 #pragma unroll
-    for (int u = 0; u < YS / kScanWalkers; ++u) {
-      const int idx = tid + u * kScanWalkers;
+    for (int u = 0; u < YS / HELPERS; ++u) {
+      const int idx = tid + u * HELPERS;
       const int i = idx / kScanChannels;
       if (i < n_here)
-        out[(size_t)(t0 + base + i) * channels + hc] = from_float<TO>((ys[idx] + skip * raw[YS + idx]) * silu_f(raw[2 * YS + idx]));
+        out[(size_t)(t0 + base + i) * channels + hc] = from_float<TO>((ys[i * kScanYRow + idx % kScanChannels] + skip * raw[YS + idx]) * silu_f(raw[2 * YS + idx]));
     }
   };
 
-  float S[NPL], a[NPL];                                     // a lane's states are neighbours: n = lane * NPL + k
+  Pair S[PAIRS], a[PAIRS];                                  // a lane's states are neighbours: n = lane * NPL + k
   if (walker) {
 #pragma unroll
-    for (int k = 0; k < NPL; ++k) {
-      const int n = lane * NPL + k;
-      const bool on = live && n < N;
-      S[k] = on ? slot[(size_t)c * N + n] : 0.f;
-      a[k] = on ? A[(size_t)c * N + n] * kLog2e : 0.f;      // exp(dt A) = 2^(dt A log2 e)
+    for (int k = 0; k < PAIRS; ++k) {
+      const int n = lane * NPL + 2 * k;
+      const bool on = live && n < N, two = live && n + 1 < N;
+      const float *s_at = slot + (size_t)c * N + n, *a_at = A + (size_t)c * N + n;
+      S[k] = pair_of(on ? s_at[0] : 0.f, two ? s_at[1] : 0.f);
+      a[k] = pair_of(on ? a_at[0] * kLog2e : 0.f, two ? a_at[1] * kLog2e : 0.f);      // exp(dt A) = 2^(dt A log2 e)
     }
   } else if (n_chunks > 0) {
     for (int j = 0; j < K - 2; ++j) stage(j);
     scan_cp_async_wait<K - 4>();                            // the helper's own copies of chunks 0 and 1
-    scan_helpers_meet();
+    scan_helpers_meet<HELPERS>();
     prepare(0);
   }
   for (int j = 0; j < n_chunks; ++j) {
@@ -344,31 +391,32 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
     const int n_here = min(kScanChunk, q_len - j * kScanChunk);
     const float* bc = bc_s + (j % K) * BUF;
     const float2* step = step_s + (j & 1) * YS;
-    float* ys = y_s + (j & 1) * YS;
-#pragma unroll 1
-    for (int i0 = 0; i0 < n_here; i0 += GROUP) {
+    float* ys = y_s + (j & 1) * kScanChunk * kScanYRow;
+#pragma unroll UNROLL
+    for (int i0 = 0; i0 < (UNROLL > 1 ? kScanChunk : n_here); i0 += GROUP) {
       float y[GROUP];
 #pragma unroll
       for (int u = 0; u < GROUP; ++u) {
         const int i = i0 + u;
         const float2 v = step[i * kScanChannels + ch];
-        const float dt = v.x, dtx = v.y;
-        float Bv[NPL], Cv[NPL];
-        scan_load_row<NPL>(bc + i * 2 * NP + lane * NPL, Bv);
-        scan_load_row<NPL>(bc + i * 2 * NP + NP + lane * NPL, Cv);
-        y[u] = 0.f;
+        const Pair dt = pair_of(v.x, v.x), dtx = pair_of(v.y, v.y);
+        Pair Bv[PAIRS], Cv[PAIRS], sum;
+        scan_load_row<PAIRS>(bc + i * 2 * NP + lane * NPL, Bv);
+        scan_load_row<PAIRS>(bc + i * 2 * NP + NP + lane * NPL, Cv);
 #pragma unroll
-        for (int k = 0; k < NPL; ++k) {
-          S[k] = fmaf(scan_exp2(dt * a[k]), S[k], dtx * Bv[k]);
-          y[u] = fmaf(S[k], Cv[k], y[u]);
+        for (int k = 0; k < PAIRS; ++k) {
+          S[k] = fma2(scan_exp2(mul2(dt, a[k])), S[k], mul2(dtx, Bv[k]));
+          sum = k ? fma2(S[k], Cv[k], sum) : mul2(S[k], Cv[k]);
         }
+        const float2 f = halves_of(sum);
+        y[u] = f.x + f.y;
       }
-      // the lanes' partial sums of GROUP tokens, added across the 8 lanes: each round a lane hands half of what it
-      // holds to its partner and keeps the other half, so 8 tokens cost 4 + 2 + 1 exchanges, and lane l ends with
-      // token l's sum; a group of fewer tokens ends with plain rounds (both partners then hold the sum)
+      // the lanes' partial sums of GROUP tokens, added across the lanes: each round a lane hands half of what it
+      // holds to its partner and keeps the other half, so 8 tokens cost 4 + 2 exchanges among 4 lanes, and lane l ends with
+      // two tokens' sums; a group of fewer tokens than lanes ends with plain rounds (both partners then hold the sum)
       int held = GROUP, tok = 0;
 #pragma unroll
-      for (int o = kScanLanes / 2; o > 0; o >>= 1) {
+      for (int o = LANES / 2; o > 0; o >>= 1) {
         if (held > 1) {
           const int h = held / 2;
           const bool upper = (lane & o) != 0;
@@ -384,7 +432,10 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
           y[0] += __shfl_xor_sync(0xffffffffu, y[0], o);
         }
       }
-      if ((lane & (kScanLanes / GROUP - 1)) == 0) ys[(i0 + tok) * kScanChannels + ch] = y[0];
+      if (GROUP >= LANES || (lane & (LANES / GROUP - 1)) == 0) {
+#pragma unroll
+        for (int u = 0; u < (GROUP > LANES ? GROUP / LANES : 1); ++u) ys[(i0 + tok + u) * kScanYRow + ch] = y[u];
+      }
     }
   }
   pdl_trigger();             // a long walk: the kernel behind would only sit on the SMs meanwhile
@@ -394,9 +445,11 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
     return;
   }
 #pragma unroll
-  for (int k = 0; k < NPL; ++k) {
-    const int n = lane * NPL + k;
-    if (live && n < N) slot[(size_t)c * N + n] = S[k];
+  for (int k = 0; k < PAIRS; ++k) {
+    const int n = lane * NPL + 2 * k;
+    const float2 f = halves_of(S[k]);
+    if (live && n < N) slot[(size_t)c * N + n] = f.x;
+    if (live && n + 1 < N) slot[(size_t)c * N + n + 1] = f.y;
   }
   // the carried inputs: the last taps - 1 inputs of the channel, of this step or, for a short one, shifted up
   if (live && lane == 0 && taps > 1) {
@@ -530,14 +583,19 @@ extern "C" int srlm_selective_scan(const float* x, const float* xz, long long ld
                                    int out_dtype, int n_entries, int max_q_len, int channels, int N, int taps,
                                    cudaStream_t stream) {
   if (n_entries <= 0) return ST_OK;
-  if (channels <= 0 || N <= 0 || N > 16 * kScanLanes || taps <= 0 || ld_xz < 2ll * channels || b_off < 0 ||
+  if (channels <= 0 || N <= 0 || N > kScanStates || taps <= 0 || ld_xz < 2ll * channels || b_off < 0 ||
       ld_dbc < b_off + 2ll * N || state_stride < (long long)channels * (N + taps - 1) || n_entries > 65535)
     return refuse(ST_BAD_SIZE, "selective_scan: channels=%d N=%d (at most %d) taps=%d ld_xz=%lld ld_dbc=%lld b_off=%d "
-                  "state_stride=%lld", channels, N, 16 * kScanLanes, taps, ld_xz, ld_dbc, b_off, state_stride);
+                  "state_stride=%lld", channels, N, kScanStates, taps, ld_xz, ld_dbc, b_off, state_stride);
   const dim3 grid((channels + kScanChannels - 1) / kScanChannels, n_entries);
-  int npl = 1;
-  while (npl * kScanLanes < N) npl <<= 1;
+  // four lanes a channel up to 16 states, eight beyond (64 states: 8 a lane, half the registers)
+  const int lanes = N <= 16 ? 4 : 8;
+  int npl = 2;
+  while (npl * lanes < N) npl <<= 1;
   const bool early = max_q_len <= 4 * kScanChunk;      // a long walk starts on an empty GPU, its blocks spread evenly
+  // at most two blocks an SM: more registers and helpers for each (2,048 tokens, 4,096 channels 107 us, 133 without;
+  // 8,192 channels 218, 204 without)
+  const bool roomy = !early && (long long)grid.x * grid.y <= 2 * 148;
   // copies of 16 bytes: neither four channels nor four states straddle an edge
   const bool wide = channels % 4 == 0 && N % 4 == 0 && b_off % 4 == 0 && ld_dbc % 4 == 0 && ld_xz % 4 == 0 &&
                     ((uintptr_t)x | (uintptr_t)xz | (uintptr_t)dbc | (uintptr_t)dt_raw) % 16 == 0;
@@ -545,29 +603,30 @@ extern "C" int srlm_selective_scan(const float* x, const float* xz, long long ld
   // one token, 8,192 channels of 16 states: the layer 237 us, without it and with the registers
   // of five blocks an SM 206)
   const int chunks = (max_q_len + kScanChunk - 1) / kScanChunk;
-  const int held = chunks < 1 ? 1 : chunks < scan_buffers(npl) ? chunks : scan_buffers(npl);
-  const size_t smem = (size_t)scan_floats(npl, held) * sizeof(float);
-#define SRLM_SCAN_AS(TO, NPL, W)                                                                                        \
+  const int held = chunks < 1 ? 1 : chunks < scan_buffers(npl * lanes) ? chunks : scan_buffers(npl * lanes);
+  const size_t smem = (size_t)scan_floats(npl * lanes, held) * sizeof(float);
+#define SRLM_SCAN_AS(TO, LANES, NPL, W, LONG)                                                                           \
   do {                                                                                                                  \
-    auto kern = selective_scan_kernel<TO, NPL, W>;                                                                      \
+    auto kern = selective_scan_kernel<TO, LANES, NPL, W, LONG>;                                                         \
     const cudaError_t got =                                                                                             \
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                             \
     if (got != cudaSuccess) return refuse((int)got, "selective_scan: cannot get %zu bytes of shared memory", smem);     \
-    launch_pdl_if(early, kern, grid, dim3(kScanThreads), smem, stream, x, xz, ld_xz, dbc, ld_dbc, b_off, dt_raw,        \
-                  dt_bias, A, D, state, state_stride, cu_q, slots, (TO*)out, channels, N, taps);                        \
+    launch_pdl_if(early, kern, grid, dim3(LANES * kScanChannels + scan_helpers(LONG)), smem, stream, x, xz, ld_xz, dbc, \
+                  ld_dbc, b_off, dt_raw, dt_bias, A, D, state, state_stride, cu_q, slots, (TO*)out, channels, N, taps); \
   } while (0)
-#define SRLM_SCAN(TO, NPL)                    \
-  do {                                        \
-    if (wide) SRLM_SCAN_AS(TO, NPL, true);    \
-    else SRLM_SCAN_AS(TO, NPL, false);        \
+#define SRLM_SCAN(TO, LANES, NPL)                                   \
+  do {                                                              \
+    if (wide && roomy) SRLM_SCAN_AS(TO, LANES, NPL, true, true);   \
+    else if (wide) SRLM_SCAN_AS(TO, LANES, NPL, true, false);       \
+    else SRLM_SCAN_AS(TO, LANES, NPL, false, false);                \
   } while (0)
 #define SRLM_SCAN_N(TO)                                   \
-  switch (npl) {                                          \
-    case 1: SRLM_SCAN(TO, 1); break;                      \
-    case 2: SRLM_SCAN(TO, 2); break;                      \
-    case 4: SRLM_SCAN(TO, 4); break;                      \
-    case 8: SRLM_SCAN(TO, 8); break;                      \
-    default: SRLM_SCAN(TO, 16);                           \
+  switch (lanes * 100 + npl) {                            \
+    case 402: SRLM_SCAN(TO, 4, 2); break;                 \
+    case 404: SRLM_SCAN(TO, 4, 4); break;                 \
+    case 804: SRLM_SCAN(TO, 8, 4); break;                 \
+    case 808: SRLM_SCAN(TO, 8, 8); break;                 \
+    default: SRLM_SCAN(TO, 8, 16);                        \
   }
   if (out_dtype == DT_F32) { SRLM_SCAN_N(float) }
   else if (out_dtype == DT_BF16) { SRLM_SCAN_N(bf16) }

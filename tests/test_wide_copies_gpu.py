@@ -24,7 +24,8 @@ class _Entries:
         self.entry_of_token = torch.tensor(sum(([e] * n for e, n in enumerate(lens)), []), dtype=torch.int32, device=DEV)
 
 
-@pytest.mark.parametrize("channels,N", [(4, 4), (20, 8), (36, 12), (16, 16), (48, 20), (16, 64), (20, 128)])
+# (1,600 channels and three entries: more blocks than the form for two blocks an SM takes)
+@pytest.mark.parametrize("channels,N", [(4, 4), (20, 8), (36, 12), (16, 16), (48, 20), (16, 64), (20, 128), (1600, 16), (1600, 4)])
 @pytest.mark.parametrize("lens", [(1,), (15, 16, 17), (40, 100, 7), (33, 1, 160), (2, 530)])
 def test_scan_and_its_convolution(channels, N, lens):
     g = torch.Generator().manual_seed(channels + N)
