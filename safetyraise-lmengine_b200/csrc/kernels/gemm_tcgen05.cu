@@ -793,6 +793,15 @@ __device__ __forceinline__ float clamped_glu_fast(float gate, float up, float li
   return g * __frcp_rn(1.f + exp2f(-alpha * 1.4426950408889634f * g)) * (u + 1.f);
 }
 
+// By a warp: the token tiles up to the last one that belongs to a group.  The rows of the groups take fewer tiles than are
+// reserved for them; numbered with the tiles behind them, those in use fell on some walkers more than on others.
+__device__ __forceinline__ int tiles_in_use(const int* group_of_mtile, int tiles, int lane) {
+  int used = 0;
+  for (int t = lane; t < tiles; t += 32)
+    if (group_of_mtile[t] >= 0) used = t + 1;
+  return __reduce_max_sync(0xffffffffu, used);
+}
+
 // The first `tokens` of a lane's values, one below the other in C.
 template <typename TO, int COUNT>
 __device__ __forceinline__ void store_tokens(TO* at, long long ld, const float (&h)[COUNT], int tokens) {
@@ -832,8 +841,8 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
   uint32_t rank = 0;                                         // of this block in its pair
   if (PAIR) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const int walker = PAIR ? blockIdx.x / 2 : blockIdx.x, walkers = PAIR ? gridDim.x / 2 : gridDim.x;
-  const int tiles_m = (args.M + BN - 1) / BN, tiles_n = (args.N + TILE_N - 1) / TILE_N;
-  const int total_tiles = tiles_m * tiles_n;
+  const int tiles_n = (args.N + TILE_N - 1) / TILE_N;
+  int tiles_m = (args.M + BN - 1) / BN;
   const int num_kb = (args.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
@@ -861,6 +870,11 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
   if (PAIR) cluster_sync_all();        // both blocks' barriers exist before either signals the other's
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (args.group_of_mtile) {           // the table is written by a kernel of the same step
+    pdl_wait();
+    tiles_m = tiles_in_use(args.group_of_mtile, tiles_m, lane);
+  }
+  const int total_tiles = tiles_m * tiles_n;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -904,7 +918,6 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
       bool ok = true;
       PieceWalk walk(args, num_kb, total_tiles, walker, walkers);
       int t, kb_lo, kb_hi;
-      if (args.group_of_mtile) pdl_wait();                 // the table is written by a kernel of the same step
       for (; ok && walk.next(t, kb_lo, kb_hi); ++local) {
         if (args.group_of_mtile && args.group_of_mtile[args.m_major ? t / tiles_n : t % tiles_m] < 0) {
           --local;
@@ -1685,14 +1698,12 @@ extern "C" int srlm_gemm_tn_tcgen05_grouped(const void* X, const void* W, void* 
   a.act = act;
   CUtensorMap mw_copy, mx_copy;
   const CUtensorMap *mw = &mw_copy, *mx = &mx_copy;
-  // Tiles of 128 tokens go to pairs too where no half of a pair would stand idle: 256 weight rows x 128 tokens, 24 KB from the L2
-  // into each SM a k-block in place of 32 for the same products; and where a group has a tile's worth of rows on average (M
-  // counts up to a tile of padding a group).  A layer of 16 experts, top 4, in us, pairs | one SM: 4,096 wide, 1,024 tokens 491..555 |
-  // 585, 256 tokens (64 rows an expert) 288 | 269; 64 experts, top 8, 2,048 wide, 3,000 tokens 813..879 | 891..918.  Where the
-  // weights fit the L2 the two forms are within 2 % (2,048 wide, 1,500 tokens 295 | 293; 1,024 wide 170 | 167) but for sizes
-  // at which the skipped tiles, which lie between the others, fall on some SMs more than on others: 2,048 tokens 332 | 348 and
-  // 176 | 192, 900 tokens 1,024 wide 137 | 129.
-  const bool pairs = tile_rows == 256 || (N % (2 * BM) == 0 && M >= 256ll * groups);
+  // Tiles of 128 tokens go to pairs too where the weights of all groups exceed the L2 and a group has half a tile's rows or more
+  // (M counts up to a tile of padding a group): 24 KB from the L2 into each SM a k-block in place of 32 for the same products.
+  // A layer in us, pairs | one SM: 16 experts, top 4, 4,096 wide, 128 rows an expert 284 | 296, 512 rows 731 | 782; 64 experts,
+  // top 8, 2,048 wide, 150 rows 376 | 406, 256 rows 488 | 555, 50 rows 272 | 267.  Where the L2 holds them one SM a tile splits the
+  // work finer: 16 experts 1,024 wide, 225 rows 102 | 97, 256 rows 113 | 106; 2,048 wide 165.0 | 164.2 and 176.9 | 176.3.
+  const bool pairs = tile_rows == 256 || (N % (2 * BM) == 0 && (long long)groups * N * K >= 64ll << 20 && M >= 192ll * groups);
   // (the pair form fetches the tokens of a tile in two boxes, one a block)
   if (!cached_map(&mw_copy, W, (long long)groups * N, K, K, BM, true) ||
       !cached_map(&mx_copy, X, M, K, ldx, pairs ? tile_rows / 2 : 128, false))

@@ -1037,14 +1037,23 @@ class KernelLibrary:
     GROUPED_TILE = 128       # token rows of a tile of the grouped tensor-memory product (one SM or two, by the sizes)
     GROUPED_PAIR_TILE = 256  # ... of its widest form (two SMs on 256 weight rows x 256 tokens)
 
+    def grouped_takes_tiles(self, pairs: int, experts: int, weight_elements: int) -> bool:
+        """Whether a step's ``pairs`` rows over ``experts`` groups, whose first weight matrix has ``weight_elements`` elements a
+        group, go through the grouped product in tensor memory (whole tiles, however few rows an expert has) rather than the
+        one of mma.sync (tiles of 32 or 64 rows).  A layer in us, mma.sync | tiles, at 25, 37.5 and 50 rows an expert: 16 experts
+        1,024 wide (1 Mi elements) 58 | 64, 62 | 66, 73 | 68; 2,048 wide (4 Mi) 88 | 99, 103 | 103, 141 | 105; 4,096 wide (16 Mi)
+        230 | 230, 289 | 239, 351 | 243; 64 experts 1,024 wide 104 | 130, 112 | 132, 143 | 136; 2,048 wide 243 | 254, 267 |
+        254, 326 | 267."""
+        return pairs >= (36 if weight_elements >= 4 << 20 else 44) * experts
+
     def grouped_tile_rows(self, pairs: int, experts: int, weight_elements: int) -> int:
         """The token tile of the grouped tensor-memory product for a step of ``pairs`` rows over ``experts`` groups
-        whose first weight matrix has ``weight_elements`` elements a group: 256 once an expert has 512 rows on average (so
-        that about an eighth of the tiles' rows is padding) and 16 Mi weight elements; else 128.  A layer of 16 experts in
-        us, tiles of 256 | of 128 (pairs of SMs both): 4,096 wide, 512 rows an expert 803..937 | 923..936, 1,024 rows
-        1,556..1,593 | 1,746..1,775; one product of 2,048 x 2,048 a group 83 | 84 and 153 | 166, with an eighth more rows
-        in the tiles of 256 when the experts' shares are uneven."""
-        big = pairs >= 512 * experts and weight_elements >= 16 << 20
+        whose first weight matrix has ``weight_elements`` elements a group: 256 once an expert has 144 rows on average and
+        16 Mi weight elements; else 128.  A layer in us, tiles of 256 | of 128: 16 experts 4,096 wide, 128 rows an expert
+        298 | 284, 160 rows 329 | 354, 512 rows 660 | 733; 8 experts 4,096 wide, 75 rows 188 | 169, 150 rows 223 | 252;
+        16 experts 2,048 wide, 160 rows 149 | 154, 225 rows 180 | 164, 512 rows 257 | 256; 64 experts 2,048 wide, 256 rows
+        526 | 488."""
+        big = pairs >= 144 * experts and weight_elements >= 16 << 20
         return self.GROUPED_PAIR_TILE if self.grouped_pairs and big else self.GROUPED_TILE
 
     def moe_gather_rows(self, x, pair_of_row, pairs_per_token, out, pair_scale=None):

@@ -153,10 +153,10 @@ class RoutedExperts(Part):
         first = self.first(ctx, x, "moe.first", out_dtype=torch.float32) if self.table is None else None
         choice = ws.get("moe.choice", T, s.top, torch.int32)
         weight = ws.get("moe.weight", T, s.top, torch.float32)
-        # steps of many tokens (64 rows an expert on average): the experts' products on the persistent tensor-memory
-        # kernel, every expert's rows in whole tiles of 128 of a gathered copy of the input
-        if (self.in_tiles and ops.grouped_products_in_tensor_memory and pairs >= 64 * s.experts
-                and s.intermediate_size % 8 == 0):
+        # steps of many tokens: the experts' products on the persistent tensor-memory kernel, every expert's rows in whole
+        # tiles of a gathered copy of the input
+        if (self.in_tiles and ops.grouped_products_in_tensor_memory and s.intermediate_size % 8 == 0
+                and ops.grouped_takes_tiles(pairs, s.experts, (2 if s.gated else 1) * s.intermediate_size * H)):
             self._route(ctx, first, choice, weight)
             return self._forward_tiles(ctx, x, first, choice, weight, add)
         heads = ws.get("moe.heads", 2, s.experts + 1, torch.int32, reserve=2)

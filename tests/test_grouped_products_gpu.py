@@ -96,3 +96,23 @@ def test_tensor_memory_products_with_their_epilogues(act, glu, odt, tile, N, K, 
         want = z
     err = err + (2.0 ** -24 if odt == torch.float32 else 2.0 ** -8) * want.abs()      # the result's own rounding
     assert ((out.cpu().double() - want).abs() <= err * 1.001)[rows].all()
+
+
+@pytest.mark.parametrize("tile, N, K", [(128, 128, 64), (128, 512, 72), (256, 256, 136)])
+@pytest.mark.parametrize("table", [[-1], [-1, -1, -1], [0] + [-1] * 40, [-1] * 33 + [1], [1, -1, 0] + [-1] * 70])
+def test_tiles_behind_the_last_one_in_use(tile, N, K, table):
+    """Tables with no group at all, with groups at their start or end, longer than a warp: the tiles of the groups are computed,
+    the others' rows stay as they are."""
+    g = torch.Generator().manual_seed(N + len(table))
+    M = tile * len(table) - 5
+    x, w = torch.randn(M, K, generator=g).bfloat16(), (torch.randn(2, N, K, generator=g) * K ** -0.5).bfloat16()
+    out = torch.full((M, N), 7.0, device=DEV)
+    ops.gemm_tn_tcgen05_grouped(x.to(DEV), w.to(DEV), out, torch.tensor(table, dtype=torch.int32, device=DEV), tile_rows=tile)
+    assert ops.gemm_error_flag(out.device) == 0
+    for t, group in enumerate(table):
+        rows = slice(t * tile, min(M, (t + 1) * tile))
+        got, a = out[rows].cpu(), x[rows].double()
+        if group < 0:
+            assert (got == 7.0).all()
+        else:      # float32 sums of exact products, cut off or rounded K times
+            assert ((got - a @ w[group].double().T).abs() <= K * 2.0 ** -23 * (a.abs() @ w[group].double().abs().T) + 1e-9).all()
