@@ -118,6 +118,137 @@ __device__ __forceinline__ void head_product(const float* __restrict__ in_s, int
   }
 }
 
+// The same sums for wider blocks: 16 tokens x 128 columns, a lane owns four neighbouring columns.  A read of a token's four k's
+// serves 16 products in place of four, and a warp's weights come 8 bytes a lane.  Bound by the exchange of the warps' sums
+// (128 KB of shared memory written and read) and the FMAs alike.  64 tokens, 32 heads, 16 tokens x 32 columns a block | these:
+// absorb (128 x 512) 64 | 20 us, expand (512 x 128) 34 | 11.
+constexpr int kWideTokens = 16, kWideCols = 128;
+static size_t wide_smem(int K) {
+  return ((size_t)kWideTokens * product_ld(K) + (size_t)kProductWarps * kWideTokens * kWideCols) * sizeof(float);
+}
+template <typename TW> struct FourWeights;
+template <> struct FourWeights<float> {
+  float4 v;
+  __device__ __forceinline__ void load(const float* w) { v = *reinterpret_cast<const float4*>(w); }
+  __device__ __forceinline__ void none() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ float4 get() const { return v; }
+};
+template <> struct FourWeights<bf16> {
+  uint2 v;
+  __device__ __forceinline__ void load(const bf16* w) { v = *reinterpret_cast<const uint2*>(w); }
+  __device__ __forceinline__ void none() { v = make_uint2(0u, 0u); }
+  __device__ __forceinline__ float4 get() const {
+    return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16),
+                       __uint_as_float(v.y & 0xffff0000u));
+  }
+};
+// -> the sums of token `warp`, columns col .. col + 3 (col: the lane's first, a multiple of 4 below cols, or beyond it)
+template <typename TW>
+__device__ __forceinline__ float4 wide_product(const float* __restrict__ in_s, int K, const TW* __restrict__ w, int cols, int col,
+                                               float* __restrict__ red) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, ld = product_ld(K);
+  const int per = ((K + kProductWarps - 1) / kProductWarps + 3) / 4 * 4, k0 = min(K, warp * per), k1 = min(K, k0 + per);
+  float acc[kWideTokens][4] = {};
+  constexpr int AHEAD = 8;
+  const bool on = col < cols;
+  for (int k = k0; k < k1; k += AHEAD) {
+    FourWeights<TW> y[AHEAD];
+#pragma unroll
+    for (int x = 0; x < AHEAD; ++x) {
+      if (on && k + x < k1) y[x].load(w + (size_t)(k + x) * cols + col);
+      else y[x].none();
+    }
+#pragma unroll
+    for (int x = 0; x < AHEAD; x += 4) {
+      if (k + x >= k1) break;                             // (the inputs behind K are zero)
+      const float4 a = y[x].get(), b = y[x + 1].get(), c = y[x + 2].get(), d = y[x + 3].get();
+#pragma unroll
+      for (int tt = 0; tt < kWideTokens; ++tt) {
+        const float4 v = *reinterpret_cast<const float4*>(in_s + tt * ld + k + x);
+        acc[tt][0] = fmaf(v.w, d.x, fmaf(v.z, c.x, fmaf(v.y, b.x, fmaf(v.x, a.x, acc[tt][0]))));
+        acc[tt][1] = fmaf(v.w, d.y, fmaf(v.z, c.y, fmaf(v.y, b.y, fmaf(v.x, a.y, acc[tt][1]))));
+        acc[tt][2] = fmaf(v.w, d.z, fmaf(v.z, c.z, fmaf(v.y, b.z, fmaf(v.x, a.z, acc[tt][2]))));
+        acc[tt][3] = fmaf(v.w, d.w, fmaf(v.z, c.w, fmaf(v.y, b.w, fmaf(v.x, a.w, acc[tt][3]))));
+      }
+    }
+  }
+#pragma unroll
+  for (int tt = 0; tt < kWideTokens; ++tt)
+    *reinterpret_cast<float4*>(red + (warp * kWideTokens + tt) * kWideCols + 4 * lane) =
+        make_float4(acc[tt][0], acc[tt][1], acc[tt][2], acc[tt][3]);
+  __syncthreads();
+  static_assert(kWideTokens == kProductWarps, "a warp finishes a token");
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+  for (int ww = 0; ww < kProductWarps; ++ww) {
+    const float4 v = *reinterpret_cast<const float4*>(red + (ww * kWideTokens + warp) * kWideCols + 4 * lane);
+    sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+  }
+  return sum;
+}
+
+template <typename TP, typename TW>
+__global__ void __launch_bounds__(kProductWarps * 32)
+latent_absorb_wide_kernel(const TP* __restrict__ proj, long long ldp, const TW* __restrict__ uk,
+                          const float* __restrict__ cos_t, const float* __restrict__ sin_t, int pairs, int halves,
+                          float* __restrict__ q_out, int T, int heads, int dim, int rot, int rank) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) float sh[];                // [16][ld] | [warps][16][128]
+  const int ld = product_ld(dim), t0 = blockIdx.x * kWideTokens, h = blockIdx.y, n = min(kWideTokens, T - t0), qd = rank + rot;
+  for (int idx = threadIdx.x; idx < kWideTokens * ld; idx += blockDim.x) {
+    const int tt = idx / ld, d = idx - tt * ld;
+    sh[idx] = tt < n && d < dim ? to_float(proj[(size_t)(t0 + tt) * ldp + (size_t)h * (dim + rot) + d]) : 0.f;
+  }
+  __syncthreads();
+  const int col = blockIdx.z * kWideCols + 4 * (threadIdx.x & 31), warp = threadIdx.x >> 5;
+  const float4 sum = wide_product(sh, dim, uk + (size_t)h * dim * rank, rank, col, sh + kWideTokens * ld);
+  if (warp < n && col < rank) {
+    float* at = q_out + ((size_t)(t0 + warp) * heads + h) * qd + col;
+    at[0] = sum.x, at[1] = sum.y, at[2] = sum.z, at[3] = sum.w;
+  }
+  if (blockIdx.z != 0) return;
+  for (int idx = threadIdx.x; idx < n * rot; idx += blockDim.x) {
+    const int tt = idx / rot, i = idx - tt * rot, t = t0 + tt;
+    const TP* src = proj + (size_t)t * ldp + (size_t)h * (dim + rot) + dim;
+    q_out[((size_t)t * heads + h) * qd + rank + i] =
+        i < 2 * pairs ? rotated_element(src, i, (size_t)t, pairs, halves, cos_t, sin_t) : to_float(src[i]);
+  }
+}
+
+template <typename TP, typename TW, typename TA>
+__global__ void __launch_bounds__(kProductWarps * 32)
+latent_expand_wide_kernel(const float* __restrict__ o_lat, const TW* __restrict__ uv_t, const TP* __restrict__ proj,
+                          long long ldp, int g_off, TA* __restrict__ out, int T, int heads, int rank, int dv) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) float sh[];                // [16][ld] | [warps][16][128]
+  const int ld = product_ld(rank), t0 = blockIdx.x * kWideTokens, h = blockIdx.y, n = min(kWideTokens, T - t0);
+  if (rank % 4 == 0) {
+    const int r4 = rank / 4;
+    for (int idx = threadIdx.x; idx < kWideTokens * r4; idx += blockDim.x) {
+      const int tt = idx / r4, r = (idx - tt * r4) * 4;
+      const float4 v = tt < n ? *reinterpret_cast<const float4*>(o_lat + ((size_t)(t0 + tt) * heads + h) * rank + r)
+                              : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(sh + tt * ld + r) = v;
+    }
+  } else {
+    for (int idx = threadIdx.x; idx < kWideTokens * ld; idx += blockDim.x) {
+      const int tt = idx / ld, r = idx - tt * ld;
+      sh[idx] = tt < n && r < rank ? o_lat[((size_t)(t0 + tt) * heads + h) * rank + r] : 0.f;
+    }
+  }
+  __syncthreads();
+  const int col = blockIdx.z * kWideCols + 4 * (threadIdx.x & 31), warp = threadIdx.x >> 5;
+  const float4 sum = wide_product(sh, rank, uv_t + (size_t)h * rank * dv, dv, col, sh + kWideTokens * ld);
+  if (warp >= n || col >= dv) return;
+  const size_t t = t0 + warp;
+  const float g = g_off >= 0 ? 1.f / (1.f + expf(-to_float(proj[t * ldp + g_off + h]))) : 1.f;
+  TA* at = out + (t * heads + h) * dv + col;
+  at[0] = from_float<TA>(sum.x * g), at[1] = from_float<TA>(sum.y * g);
+  at[2] = from_float<TA>(sum.z * g), at[3] = from_float<TA>(sum.w * g);
+}
+
 // Block (token tile, head, 32 columns of the latent).  q row: heads x [dim unrotated | rot rotated].
 // uk: [heads, dim, rank].  q_out: float32 [T, heads, rank + rot]; the blocks of the first columns also rotate.
 template <int TOK, typename TP, typename TW>
@@ -301,6 +432,16 @@ extern "C" int srlm_latent_append(const void* proj, int proj_dtype, long long ld
   return launched();
 }
 
+// Whether a product goes to the wide form: where the blocks of 32 columns are more than the SMs of a B200, which then run them
+// two by two and in rounds, and the sizes allow it: columns in pieces of four, the tile's inputs and the warps' sums in shared
+// memory.  us, 32 columns a block | wide: absorb 128 x 512, 8 heads, 16 tokens (128 blocks) 6.0 | 6.1, 17 tokens (256) 9.7 |
+// 6.1, 32 heads, 8 tokens (512) 10.6 | 5.3; expand 512 x 128, 32 heads, 16 tokens (128) 9.6 | 11.2, 17 tokens (256) 17.8 | 11.3.
+static bool takes_wide(int T, int heads, int K, int cols, const void* w, int w_dtype) {
+  const int tok = T <= 8 ? 8 : 16;
+  const long long blocks = (long long)((T + tok - 1) / tok) * heads * ((cols + kColTile - 1) / kColTile);
+  return blocks > 148 && cols % 4 == 0 && (uintptr_t)w % (w_dtype == DT_F32 ? 16 : 8) == 0 && wide_smem(K) <= 227 * 1024;
+}
+
 extern "C" int srlm_latent_absorb(const void* proj, int proj_dtype, long long ldp, const void* uk, int w_dtype,
                                   const float* cos_t, const float* sin_t, int pairs, int halves, float* q_out, int T, int heads,
                                   int dim, int rot, int rank, cudaStream_t stream) {
@@ -309,6 +450,21 @@ extern "C" int srlm_latent_absorb(const void* proj, int proj_dtype, long long ld
       ldp < (long long)heads * (dim + rot) || (pairs > 0 && (!cos_t || !sin_t)))
     return refuse(ST_BAD_SIZE, "latent_absorb: heads=%d dim=%d rot=%d rank=%d pairs=%d ldp=%lld", heads, dim, rot, rank,
                   pairs, ldp);
+  if (takes_wide(T, heads, dim, rank, uk, w_dtype)) {
+    const size_t room = wide_smem(dim);
+    const dim3 tiles((T + kWideTokens - 1) / kWideTokens, heads, (rank + kWideCols - 1) / kWideCols);
+#define SRLM_ABSORB_WIDE                                                                                         \
+  do {                                                                                                           \
+    auto kern = latent_absorb_wide_kernel<TP, TW>;                                                               \
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);    \
+    if (e != cudaSuccess) return refuse((int)e, "latent_absorb: cannot get %zu bytes of shared memory", room);   \
+    launch_pdl(kern, tiles, dim3(kProductWarps * 32), room, stream, (const TP*)proj, ldp, (const TW*)uk, cos_t,  \
+               sin_t, pairs, halves, q_out, T, heads, dim, rot, rank);                                           \
+  } while (0)
+    SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_ABSORB_WIDE);
+#undef SRLM_ABSORB_WIDE
+    return launched();
+  }
   const int tok = T <= 8 ? 8 : 16;
   const size_t smem = product_smem(tok, dim);
   dim3 grid((T + tok - 1) / tok, heads, (rank + kColTile - 1) / kColTile);
@@ -331,6 +487,23 @@ extern "C" int srlm_latent_expand(const float* o_lat, const void* uv_t, int w_dt
   if (T <= 0) return ST_OK;
   if (heads <= 0 || heads > 65535 || rank <= 0 || rank > 3072 || dv <= 0 || (g_off >= 0 && ldp < g_off + heads))
     return refuse(ST_BAD_SIZE, "latent_expand: heads=%d rank=%d dv=%d g_off=%d ldp=%lld", heads, rank, dv, g_off, ldp);
+  if (takes_wide(T, heads, rank, dv, uv_t, w_dtype)) {
+    const size_t room = wide_smem(rank);
+    const dim3 tiles((T + kWideTokens - 1) / kWideTokens, heads, (dv + kWideCols - 1) / kWideCols);
+#define SRLM_EXPAND_WIDE(TA)                                                                                     \
+  do {                                                                                                           \
+    auto kern = latent_expand_wide_kernel<TP, TW, TA>;                                                           \
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);    \
+    if (e != cudaSuccess) return refuse((int)e, "latent_expand: cannot get %zu bytes of shared memory", room);   \
+    launch_pdl(kern, tiles, dim3(kProductWarps * 32), room, stream, o_lat, (const TW*)uv_t, (const TP*)proj,     \
+               ldp, g_off, (TA*)out, T, heads, rank, dv);                                                        \
+  } while (0)
+    if (out_dtype == DT_F32) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_EXPAND_WIDE(float));
+    else if (out_dtype == DT_BF16) SRLM_LATENT_TYPES(proj_dtype, w_dtype, SRLM_EXPAND_WIDE(bf16));
+    else return refuse(ST_BAD_DTYPE, "latent_expand: output dtype %d", out_dtype);
+#undef SRLM_EXPAND_WIDE
+    return launched();
+  }
   const int tok = T <= 8 ? 8 : 16;
   const size_t smem = product_smem(tok, rank);
   dim3 grid((T + tok - 1) / tok, heads, (dv + kColTile - 1) / kColTile);

@@ -135,14 +135,15 @@ def test_a_weight_that_outweighs_the_others_loses_nothing():
     assert ((got - ref).abs() <= half * 1.001 + 2.0 ** -8 * small * (v[5] - v[200]).abs() + 1e-6).all()
 
 
+# (3 heads in blocks of 32 columns; 40 heads of 130 or 516 columns and up in the wide form, 148 blocks of 32 and more)
+@pytest.mark.parametrize("heads", [3, 40])
 @pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 40])
-@pytest.mark.parametrize("dim, rot, rank, dv", [(128, 64, 512, 128), (12, 6, 20, 9), (64, 0, 130, 33), (3, 2, 5, 1)])
-def test_the_per_head_products(T, dim, rot, rank, dv):
+@pytest.mark.parametrize("dim, rot, rank, dv", [(128, 64, 512, 128), (12, 6, 20, 9), (64, 0, 130, 33), (3, 2, 5, 1), (30, 4, 516, 132)])
+def test_the_per_head_products(heads, T, dim, rot, rank, dv):
     """The up projections folded into the queries and applied behind the attention: token tiles of 8 and 16, sizes that are no
     whole pieces, columns beyond a block's 32; a token's result does not depend on its neighbours."""
     from safetyraise_lmengine_b200.kernels import ops
     g = torch.Generator().manual_seed(T + dim)
-    heads = 3
     q = torch.randn(T, heads * (dim + rot) + heads, generator=g)
     uk, uv = torch.randn(heads, dim, rank, generator=g).bfloat16(), torch.randn(heads, rank, dv, generator=g).bfloat16()
     out = torch.empty(T, heads * (rank + rot), device=DEV)
@@ -158,3 +159,6 @@ def test_the_per_head_products(T, dim, rot, rank, dv):
     one = torch.empty(1, heads * dv, device=DEV)
     ops.latent_expand(o[T - 1:].contiguous().to(DEV), uv.to(DEV), q[T - 1:].contiguous().to(DEV), heads * (dim + rot), one, heads, rank, dv)
     assert torch.equal(one[0], got[T - 1])
+    folded = torch.empty(1, heads * (rank + rot), device=DEV)
+    ops.latent_absorb(q[T - 1:].contiguous().to(DEV), uk.to(DEV), None, folded, heads, dim, rot, rank)
+    assert torch.equal(folded[0], out[T - 1])
