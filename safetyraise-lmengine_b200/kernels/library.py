@@ -647,6 +647,20 @@ class KernelLibrary:
         nsplit = -(-tiles * 64 // chunk)
         return nsplit, chunk
 
+    @staticmethod
+    def latent_split(n_entries: int, blocks: int, max_kv: int):
+        """(nsplit, kv_chunk) for the decode form of a cached latent, whose blocks have an SM each: one round of them; three
+        where a slice would have 1,024 keys or more, since contexts of unlike length then even out (64 requests, us, one round |
+        three: up to 4,000 keys, 32 heads 226 | 206; 2,048 keys, 16 heads 122 | 114; 200 keys 93 | 100; 20 requests of 3,000
+        keys 98 | 106)."""
+        tiles = max(1, (max_kv + 63) // 64)
+        for rounds in (1, 3):
+            nsplit = max(1, min(tiles, rounds * KernelLibrary.SMS // max(1, n_entries * blocks), 64))
+            chunk = -(-tiles // nsplit) * 64
+            if chunk < 1024:
+                break
+        return -(-tiles * 64 // chunk), chunk
+
     def _decode_plan(self, ctx, nkv, hd, n_entries=None, kv_bound=None):
         """(nsplit, kv_chunk, cluster, part_o, part_ml) for the TMA decode kernel on the batch of ctx, or on
         ``n_entries`` of its entries whose keys number at most ``kv_bound``."""
@@ -875,7 +889,11 @@ class KernelLibrary:
             rows_padded = (ctx.max_q_len * g + 15) // 16 * 16
             # with a window the slices lie over the keys a row tile can see, not over the whole context
             span = min(ctx.kv_bound, window + ctx.max_q_len + 64) if window else ctx.kv_bound
-            nsplit, chunk = self.attention_split(n, nkv * (rows_padded // 16), span, max_slices=64)
+            block_rows = self.lib.srlm_attention_latent_decode_rows(C.c_int(dk), C.c_int(dv), from_keys, C.c_int(ctx.max_q_len * g))
+            if block_rows:
+                nsplit, chunk = self.latent_split(n, nkv * -(-rows_padded // block_rows), span)
+            else:
+                nsplit, chunk = self.attention_split(n, nkv * (rows_padded // 16), span, max_slices=64)
             if not self.split_general_attention:
                 nsplit, chunk = 1, 0
             part_o = part_ml = None
@@ -889,7 +907,7 @@ class KernelLibrary:
                 C.c_int(block_table.stride(0)), _ptr(ctx.cu_q), _ptr(ctx.kv_lens), _ptr(sinks), C.c_int(n),
                 C.c_int(ctx.max_q_len), C.c_int(nq), C.c_int(nkv), C.c_int(dk), C.c_int(dv), C.c_int(k_cache.shape[2]),
                 C.c_float(scale), C.c_int(window or 0), C.c_int(nsplit), C.c_int(chunk), _ptr(part_o), _ptr(part_ml),
-                *mods, *gate_args, _stream()), "paged_attention_general_decode")
+                *mods, *gate_args, _ptr(self._gemm_state(q.device)[1]), _stream()), "paged_attention_general_decode")
             if nsplit > 1:
                 self._check(self.lib.srlm_attention_general_merge(
                     _ptr(part_o), _ptr(part_ml), _ptr(out), dtype_code(out.dtype), _ptr(ctx.cu_q), C.c_int(n),

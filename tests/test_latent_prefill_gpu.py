@@ -162,3 +162,70 @@ def test_the_per_head_products(heads, T, dim, rot, rank, dv):
     folded = torch.empty(1, heads * (rank + rot), device=DEV)
     ops.latent_absorb(q[T - 1:].contiguous().to(DEV), uk.to(DEV), None, folded, heads, dim, rot, rank)
     assert torch.equal(folded[0], out[T - 1])
+
+
+@pytest.mark.parametrize("heads, most", [(1, 1), (8, 2), (16, 1), (16, 4), (17, 1), (33, 1)])     # 1 to 64 rows an entry
+@pytest.mark.parametrize("rot, page", [(0, 16), (16, 8), (64, 256), (64, 3)])
+@pytest.mark.parametrize("window", [0, 100])
+@pytest.mark.parametrize("extras", [False, True])
+def test_decoding_over_a_latent_of_512(heads, most, rot, page, window, extras):
+    """Row tiles of 16 and 32, contexts at the edges of tiles of 64 keys, slices and none, pages given back behind a window, no
+    number behind a context's last key; with sinks, score changes and a gate: against float64 over the rounded queries."""
+    from safetyraise_lmengine_b200.kernels import ops
+    rank, g = 512, torch.Generator().manual_seed(heads + rot + page)
+    dk = rank + rot
+    kv_lens = [64, 4, 65, 700, 129, 1]
+    q_lens = [min(most, k) for k in kv_lens[:-1]] + [1]
+    T, scale = sum(q_lens), 0.2
+    ctx = Ctx(q_lens, kv_lens)
+    from safetyraise_lmengine_b200.parts.base import Workspace
+    ctx.n_entries, ctx.max_q_len, ctx.kv_bound, ctx.workspace = len(q_lens), max(q_lens), max(kv_lens), Workspace(torch.device(DEV), T)
+    q = torch.randn(T, heads, dk, generator=g)
+    keys = [torch.randn(k, dk, generator=g).bfloat16() for k in kv_lens]
+    n_pages = sum(-(-k // page) for k in kv_lens)
+    order, at = torch.randperm(n_pages, generator=g).tolist(), 0
+    pool = torch.full((n_pages, 1, page, dk), float("nan"), dtype=torch.bfloat16)
+    table = torch.full((len(kv_lens), max(-(-k // page) for k in kv_lens)), -1, dtype=torch.int32)
+    for e, k in enumerate(kv_lens):
+        first = max(0, k - q_lens[e] - window + 1) if window else 0
+        for b in range(-(-k // page)):
+            if (b + 1) * page <= first:
+                continue                                                                # behind the window: given back
+            table[e, b] = order[at]
+            pool[order[at], 0, :min(page, k - b * page)] = keys[e][b * page:(b + 1) * page]
+            at += 1
+    sinks = torch.randn(heads, generator=g) if extras else None
+    factor, weight, rate = torch.rand(heads, generator=g) + 0.5, torch.rand(heads, generator=g), torch.rand(heads, generator=g)
+    logits = torch.randn(T, 3 + heads, generator=g)
+    dev = lambda t: None if t is None else t.to(DEV)
+    more = dict(head_scale=dev(factor), penalty=(dev(weight), dev(rate)), softcap=30.0, gate=(dev(logits), 3)) if extras else {}
+    got = []
+    for split in (True, False):
+        out = torch.full((T, heads * rank), float("nan"), device=DEV)
+        try:
+            ops.split_general_attention = split
+            ops.paged_attention_general(ctx, q.view(T, -1).to(DEV), pool.to(DEV), None, out, table.to(DEV), dev(sinks), heads, 1, dk, rank,
+                                        scale, window, **more)
+        finally:
+            ops.split_general_attention = True
+        got.append(out.cpu().double().view(T, heads, rank))
+    assert ops.gemm_error_flag(out.device) == 0
+    t = 0
+    for e, (n, k) in enumerate(zip(q_lens, kv_lens)):
+        x, c = q[t:t + n].bfloat16().double(), keys[e].double()
+        i, j = torch.arange(k - n, k)[:, None], torch.arange(k)[None]
+        s = torch.einsum("ihd,jd->hij", x, c) * scale
+        if extras:
+            s = 30.0 * torch.tanh(s * factor.double()[:, None, None] / 30.0)
+            s = s - weight.double()[:, None, None] * torch.log1p(rate.double()[:, None, None] * (i - j).clamp(min=0))
+        s = s.masked_fill((j > i) | ((window > 0) & (j <= i - window)), -math.inf)
+        if extras:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(heads, n, 1)], -1)
+        p = torch.softmax(s, -1)[..., :k]
+        want, size = torch.einsum("hij,jd->ihd", p, c[:, :rank]), torch.einsum("hij,jd->ihd", p, c[:, :rank].abs())
+        if extras:
+            gate = torch.sigmoid(logits[t:t + n, 3:].double())[:, :, None]
+            want, size = want * gate, size * gate
+        for out in got:      # weights of 16 bits; scores of some 20 with float32 sums cut off a few dozen times
+            assert ((out[t:t + n] - want).abs() <= 1e-4 * size + 1e-6).all(), e
+        t += n
