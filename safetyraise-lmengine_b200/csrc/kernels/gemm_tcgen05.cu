@@ -38,6 +38,7 @@
 #include <tuple>
 
 #include "common.cuh"
+#include "expert_activations.cuh"
 
 namespace srlm {
 
@@ -1182,6 +1183,150 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
 }
 
 // ---------------------------------------------------------------------------
+// Routed experts of a step of a few tokens: a block streams 128 weight rows of one expert past all tokens of the step (BN of
+// them, no gather: what the expert does not take is not stored), or past the expert's rows of a packed matrix.  Bound by
+// memory, and on the way there by the tokens' bytes, which every block fetches (16 KB of weights and 2, 4 or 8 KB of tokens a
+// k-block).  The ring's loads are one thread's; where eight warps issue a slab's copies and meet over it (moe_grouped_mma_kernel) a
+// slab takes 0.8 us whatever its bytes.  8 tokens, top 4 of 16 experts, 2,048 -> 2 x 1,024 -> 2,048 (some 120 and 60 MB): 29 + 16 us
+// there, 23 + 13 here; weights asked for ahead of the wait for the kernel in front where nearly every expert has rows.
+// ---------------------------------------------------------------------------
+struct ExpertsArgs {
+  void* C;
+  int c_is_f32;
+  long long ldc;
+  int N, K;                  // weight rows an expert (twice the features with glu), elements of a row
+  const int* offsets;        // [experts + 1]: an expert's rows of the sorted pairs
+  const int* pair_of_row;    // token tt is column tt, row r its pair pair_of_row[r]; null: the expert's i-th row is column i
+  int pairs_per_token;
+  int glu, act;
+  float limit, alpha;
+  const float* pair_scale;   // with glu and pair_of_row: both sums of a row are multiplied by its pair's number; null: not
+  int ahead;                 // 1: the first weights are asked for before it is known whether the expert has rows
+  int* err_flag;
+};
+
+template <int BN, int STAGES>
+__global__ void __launch_bounds__(GEMM_THREADS)
+experts_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, const ExpertsArgs args) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  constexpr int A_BYTES = BM * BK * 2, STAGE = stage_bytes<BN>(), TMEM_COLS = BN < 32 ? 32 : BN;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE);
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* accum_bar = empty_bar + STAGES;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum_bar + 1);
+  int* row_of_col = reinterpret_cast<int*>(tmem_slot + 2);           // [BN]
+  pdl_trigger();
+  const int expert = blockIdx.y, n0 = blockIdx.x * BM, w_row = expert * args.N + n0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, num_kb = (args.K + BK - 1) / BK;
+  const int ahead = args.ahead && blockIdx.z == 0 ? min(num_kb, STAGES) : 0;
+  auto ask_weights = [&](int i) {
+    mbar_expect_tx(&full_bar[i % STAGES], STAGE);
+    tma_load_2d_hint(smem + i % STAGES * STAGE, &map_w, &full_bar[i % STAGES], i * BK, w_row, l2_policy_evict_first());
+  };
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    mbar_init(accum_bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int i = 0; i < ahead; ++i) ask_weights(i);
+  }
+  pdl_wait();
+  // (behind the first `rows` tokens of an expert's rows the next ones are another block's)
+  const int part = args.pair_of_row ? 0 : (int)blockIdx.z * BN;
+  const int row0 = args.offsets[expert] + part, count = min(args.offsets[expert + 1] - row0, args.pair_of_row ? INT32_MAX : BN);
+  const int x_row = args.pair_of_row ? 0 : row0;
+  if (count <= 0) {                                        // nothing to do but to see what was asked for arrive
+    if (threadIdx.x == 0) {
+      for (int i = 0; i < ahead; ++i) tma_load_2d(smem + i * STAGE + A_BYTES, &map_x, &full_bar[i], i * BK, 0);
+      for (int i = 0; i < ahead; ++i) mbar_wait(&full_bar[i], 0, args.err_flag, 44);
+    }
+    return;
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  if (warp == 0) {
+    if (lane == 0) {
+      for (int i = 0; i < num_kb; ++i) {
+        const int s = i % STAGES, j = i / STAGES;
+        if (j > 0 && !mbar_wait(&empty_bar[s], (j - 1) & 1, args.err_flag, 41)) break;
+        if (i >= ahead) ask_weights(i);
+        tma_load_2d(smem + s * STAGE + A_BYTES, &map_x, &full_bar[s], i * BK, x_row);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t idesc = umma_idesc_bf16_f32(BN);
+      for (int i = 0; i < num_kb; ++i) {
+        const int s = i % STAGES, j = i / STAGES;
+        if (!mbar_wait(&full_bar[s], j & 1, args.err_flag, 42)) break;
+        tcgen05_fence_after();
+        const uint32_t a_addr = smem_u32(smem + s * STAGE);
+        const uint64_t adesc = umma_desc_k_sw128(a_addr), bdesc = umma_desc_k_sw128(a_addr + A_BYTES);
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          tcgen05_mma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, (i | k) != 0 ? 1u : 0u);
+        tcgen05_commit(&empty_bar[s]);
+      }
+      tcgen05_commit(accum_bar);
+    }
+    __syncwarp();
+  } else {
+    const int tid_e = threadIdx.x - 64, lane_base = 32 * (warp & 3);
+    if (tid_e < BN) row_of_col[tid_e] = -1;
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    for (int r = tid_e; r < count; r += 128) {
+      const int col = args.pair_of_row ? args.pair_of_row[row0 + r] / args.pairs_per_token : r;
+      if (col < BN) row_of_col[col] = row0 + r;            // (always, by the caller's promise)
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (mbar_wait(accum_bar, 0, args.err_flag, 43)) {
+      tcgen05_fence_after();
+      // a lane has one weight row; with glu lane l + 8 has the up row of lane l's gate row
+      const int n = n0 + lane_base + lane, f = (n >> 4) * 8 + (n & 7);
+      constexpr int CH = BN < 32 ? 16 : 32;
+#pragma unroll 1
+      for (int c = 0; c < BN; c += CH) {
+        uint32_t v[CH];
+        tmem_load<CH>(tmem_base + ((uint32_t)lane_base << 16) + c, v);
+        tmem_load_wait();
+#pragma unroll
+        for (int j = 0; j < CH; ++j) {
+          const int row = row_of_col[c + j];               // the same in every lane
+          if (row < 0) continue;
+          float x = __uint_as_float(v[j]);
+          size_t at = (size_t)row * args.ldc + n;
+          bool mine = n < args.N;
+          if (args.glu) {
+            const float ws = args.pair_scale ? args.pair_scale[args.pair_of_row[row]] : 1.f;
+            const float up = __shfl_xor_sync(0xffffffffu, x, 8);
+            x = clamped_glu(x * ws, up * ws, args.limit, args.alpha);
+            at = (size_t)row * args.ldc + f;
+            mine = mine && (n & 8) == 0;
+          } else if (args.act) {
+            x = plain_activation(x, args.act);
+          }
+          if (mine) {
+            if (args.c_is_f32) reinterpret_cast<float*>(args.C)[at] = x;
+            else reinterpret_cast<bf16*>(args.C)[at] = __float2bfloat16_rn(x);
+          }
+        }
+      }
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+}
+
+// ---------------------------------------------------------------------------
 // host side: tensor maps and launch
 // ---------------------------------------------------------------------------
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -1711,4 +1856,49 @@ extern "C" int srlm_gemm_tn_tcgen05_grouped(const void* X, const void* W, void* 
   if (tile_rows == 256) return launch_pair<256, 6>(mw, mx, a, 0, stream);
   if (pairs) return launch_pair<128, 8>(mw, mx, a, 0, stream);
   return launch_persistent<128, 5>(mw, mx, a, 0, stream);
+}
+
+namespace srlm {
+template <int BN, int STAGES>
+static int launch_experts(const CUtensorMap* mw, const CUtensorMap* mx, const ExpertsArgs& a, dim3 grid, cudaStream_t stream) {
+  constexpr int SMEM = STAGES * stage_bytes<BN>() + (2 * STAGES + 1) * 8 + 16 + BN * 4 + 1024;
+  const cudaError_t e = cudaFuncSetAttribute(experts_stream_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  if (e != cudaSuccess) return refuse((int)e, "experts_stream: cannot get %d bytes of shared memory", SMEM);
+  launch_pdl(experts_stream_kernel<BN, STAGES>, grid, dim3(GEMM_THREADS), SMEM, stream, *mw, *mx, a);
+  return launched();
+}
+}  // namespace srlm
+
+// The experts' products of a step of at most 64 tokens, each token's experts distinct: out[r] = a[r's token] . W[r's expert]^T
+// for the rows r of the sorted pairs (offsets int32 [experts + 1]).  pair_of_row: A [rows, K] are the tokens, row r's token
+// pair_of_row[r] / pairs_per_token; null: A's row r belongs to row r, and no expert has more than `tokens` rows.  glu: the weight
+// rows of an expert (N of them) in blocks of 8 gate and 8 up rows, C [pairs, N / 2].
+extern "C" int srlm_moe_experts_stream(const void* A, int rows, long long lda, const int* pair_of_row, int pairs_per_token,
+                                       const void* W, void* C, int c_dtype, long long ldc, const int* offsets, int pairs,
+                                       int tokens, int experts, int N, int K, int glu, float limit, float alpha,
+                                       const float* pair_scale, int act, int* err_flag, cudaStream_t stream) {
+  if (pairs <= 0) return ST_OK;
+  if (tokens <= 0 || tokens > 64 || (pair_of_row && (rows > tokens || pairs_per_token <= 0)) || experts <= 0 || experts > 65535 ||
+      N <= 0 || K <= 0 || K % 8 || lda < K || lda % 8 || (glu && N % 16) || ldc < (glu ? N / 2 : N) || act < 0 || act > 2 ||
+      (act && glu) || (pair_scale && !(glu && pair_of_row)) || !err_flag || (long long)experts * N > INT32_MAX)
+    return refuse(ST_BAD_SIZE, "moe_experts_stream: tokens=%d rows=%d experts=%d N=%d K=%d lda=%lld ldc=%lld glu=%d act=%d",
+                  tokens, rows, experts, N, K, lda, ldc, glu, act);
+  if (((uintptr_t)A | (uintptr_t)W) & 15) return refuse(ST_BAD_ALIGN, "moe_experts_stream: operands must be 16-byte aligned");
+  if (c_dtype != DT_F32 && c_dtype != DT_BF16) return refuse(ST_BAD_DTYPE, "moe_experts_stream: output dtype %d", c_dtype);
+  // all tokens, or a tile of an expert's rows: 16, an expert having fewer than the step has tokens; 32 from 33 tokens on
+  const int bn = pair_of_row ? (tokens <= 16 ? 16 : tokens <= 32 ? 32 : 64) : (tokens <= 32 ? 16 : 32);
+  CUtensorMap mw, mx;
+  if (!cached_map(&mw, W, (long long)experts * N, K, K, BM, true) || !cached_map(&mx, A, rows, K, lda, bn, false))
+    return refuse(ST_BAD_SIZE, "moe_experts_stream: cuTensorMapEncodeTiled refused the operands");
+  // an expert that a pair in two or fewer per expert leaves without rows is the exception: its first weights are not waited for
+  const ExpertsArgs a{C, c_dtype == DT_F32, ldc, N, K, offsets, pair_of_row, pairs_per_token, glu ? 1 : 0, act, limit, alpha,
+                      pair_scale, pairs >= 2 * experts ? 1 : 0, err_flag};
+  const dim3 grid((N + BM - 1) / BM, experts, pair_of_row ? 1 : (tokens + bn - 1) / bn);
+  // at most a block an SM: a deep ring for each; else three blocks an SM
+  const bool deep = (long long)grid.x * (pairs < experts ? pairs : experts) <= 148;
+  switch (bn) {
+    case 16: return deep ? launch_experts<16, 10>(&mw, &mx, a, grid, stream) : launch_experts<16, 4>(&mw, &mx, a, grid, stream);
+    case 32: return deep ? launch_experts<32, 9>(&mw, &mx, a, grid, stream) : launch_experts<32, 3>(&mw, &mx, a, grid, stream);
+    default: return deep ? launch_experts<64, 8>(&mw, &mx, a, grid, stream) : launch_experts<64, 3>(&mw, &mx, a, grid, stream);
+  }
 }

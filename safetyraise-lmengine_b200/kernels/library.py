@@ -1098,21 +1098,41 @@ class KernelLibrary:
             C.c_float(limit), C.c_float(alpha), C.c_int(self.PLAIN_ACTIVATIONS[act]), _ptr(err), _stream()),
             "gemm_tn_tcgen05_grouped")
 
+    @staticmethod
+    def experts_stream(tokens: int, weight_elements: int) -> bool:
+        """Whether the experts' products of a step of ``tokens`` tokens (0: not known) whose weight matrix has
+        ``weight_elements`` elements an expert stream the weights past all tokens (up to 64) on tcgen05 tensor cores, rather than
+        past the expert's gathered rows on mma.sync ones.  A layer in us, gathered | streamed, at 8, 24 and 64 tokens: 16
+        experts, top 4, 1,024 wide (1 and 0.5 Mi elements) 44 | 37, 48 | 48, 52 | 60; 2,048 wide (4 and 2 Mi) 70 | 61, 74 | 67,
+        79 | 77; 4,096 wide 199 | 167, 204 | 182, 218 | 206; 64 experts, top 8, at 16, 32 and 64 tokens: 1,024 wide 79 | 64, 85 | 79,
+        85 | 91; 2,048 wide 177 | 141, 201 | 165, 204 | 184."""
+        return 0 < tokens <= (64 if weight_elements >= 2 << 20 else 16)
+
     PLAIN_ACTIVATIONS = {None: 0, "gelu": 1, "relu_squared": 2}
 
     def moe_grouped(self, a, pair_of_row, pairs_per_token, w, out, offsets, tiles, glu=False, interleaved=False,
-                    limit=0.0, alpha=0.0, pair_scale=None, act=None):
+                    limit=0.0, alpha=0.0, pair_scale=None, act=None, tokens=0):
         """out[row] = a[row's token] . w[row's expert]^T for every row of the sorted pairs (pair_of_row None: row r
         of ``a`` is row r of ``out``).  w [experts, N, K]; glu: w [experts, 2 N, K] and out gets the clamped GLU of
         the gate and up halves (interleaved: in blocks of 8 gate rows and 8 up rows, else all gate rows first);
         limit 0: the plain GLU, gate * logistic(gate) * up.  pair_scale (float32, one number a pair; with glu): the
         gate and up sums of a row are multiplied by its pair's number ahead of the activation, which for experts
         without biases is the activation of the scaled input.  act "gelu" / "relu_squared" (without glu): out gets that
-        activation of the product."""
+        activation of the product.  tokens > 0: the step has that many tokens and each token's experts are distinct, so
+        that no expert has more rows (see experts_stream)."""
         E, rows, K = w.shape
         n, N = out.shape
         if a.shape[1] != K or rows != (2 * N if glu else N):
             raise ShapeError(f"moe_grouped: a {tuple(a.shape)}, w {tuple(w.shape)}, out {tuple(out.shape)}")
+        if (self.experts_stream(tokens, rows * K) and a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and K % 8 == 0
+                and (interleaved or not glu) and rows % (16 if glu else 1) == 0 and a.stride(0) % 8 == 0
+                and (a.data_ptr() | w.data_ptr()) % 16 == 0 and self.grouped_products_on_tensor_cores):
+            self._check(self.lib.srlm_moe_experts_stream(
+                _ptr(a), C.c_int(a.shape[0]), C.c_longlong(a.stride(0)), _ptr(pair_of_row), C.c_int(pairs_per_token), _ptr(w),
+                _ptr(out), dtype_code(out.dtype), C.c_longlong(out.stride(0)), _ptr(offsets), C.c_int(n), C.c_int(tokens),
+                C.c_int(E), C.c_int(rows), C.c_int(K), C.c_int(int(glu)), C.c_float(limit), C.c_float(alpha), _ptr(pair_scale),
+                C.c_int(self.PLAIN_ACTIVATIONS[act]), _ptr(self._gemm_state(a.device)[1]), _stream()), "moe_experts_stream")
+            return
         if (a.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and (interleaved or not glu) and a.stride(0) % 8 == 0
                 and self.grouped_products_on_tensor_cores
                 and self.lib.srlm_moe_grouped_mma_takes(C.c_int(N), C.c_int(K), C.c_int(int(glu)))):

@@ -175,11 +175,11 @@ class RoutedExperts(Part):
         y = ws.get("moe.y", pairs, s.intermediate_size, ctx.dtype, reserve=ws.max_tokens * s.top)
         if s.gated:
             ops.moe_grouped(x, pair_of_row, s.top, self.gate_up, y, offsets, tiles, glu=True, interleaved=self.interleaved,
-                            limit=self.limit, alpha=s.glu_alpha, pair_scale=weight if s.weight_on_input else None)
+                            limit=self.limit, alpha=s.glu_alpha, pair_scale=weight if s.weight_on_input else None, tokens=T)
         else:
-            ops.moe_grouped(x, pair_of_row, s.top, self.gate_up, y, offsets, tiles, act=s.activation)
+            ops.moe_grouped(x, pair_of_row, s.top, self.gate_up, y, offsets, tiles, act=s.activation, tokens=T)
         rows = ws.get("moe.rows", pairs, H, torch.float32, reserve=ws.max_tokens * s.top)
-        ops.moe_grouped(y, None, 1, self.down, rows, offsets, tiles)
+        ops.moe_grouped(y, None, 1, self.down, rows, offsets, tiles, tokens=T)
         out = ws.get("moe.out", T, H, ctx.dtype)
         ops.moe_combine(rows, row_of_pair.view(T, s.top), None if s.weight_on_input else weight,
                         add if add is not None else self._shared(ctx, first), out)

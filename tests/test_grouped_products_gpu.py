@@ -116,3 +116,47 @@ def test_tiles_behind_the_last_one_in_use(tile, N, K, table):
             assert (got == 7.0).all()
         else:      # float32 sums of exact products, cut off or rounded K times
             assert ((got - a @ w[group].double().T).abs() <= K * 2.0 ** -23 * (a.abs() @ w[group].double().abs().T) + 1e-9).all()
+
+
+@pytest.mark.parametrize("T, E, top", [(1, 3, 2), (16, 5, 3), (17, 4, 4), (32, 40, 2), (33, 2, 2), (64, 7, 3)])
+@pytest.mark.parametrize("F, K", [(8, 72), (72, 640), (128, 64), (136, 1032)])
+@pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
+def test_experts_that_stream_their_weights(T, E, top, F, K, odt, monkeypatch):
+    """Token tiles of 16, 32 and 64, experts without rows and with all tokens, features and k's that end inside a tile, rings of
+    one block an SM and of three; rows by their tokens and packed, with every epilogue."""
+    monkeypatch.setattr(type(ops), "experts_stream", staticmethod(lambda tokens, weight_elements: tokens > 0))
+    g = torch.Generator().manual_seed(T + F)
+    choice = torch.stack([torch.randperm(E - (E > 4), generator=g)[:top] for _ in range(T)])         # the last expert may have none
+    flat = choice.flatten()
+    order = torch.sort(flat, stable=True).indices.to(torch.int32)                                    # pair of row
+    e = flat[order.long()]
+    offsets = torch.tensor([int((e < k).sum()) for k in range(E + 1)], dtype=torch.int32)
+    n, x = T * top, torch.randn(T, K, generator=g).bfloat16()
+    packed = torch.randn(n, K, generator=g).bfloat16()
+    scale = torch.rand(n, generator=g) + 0.5
+    for glu, act, pairs, own in ((True, None, True, None), (True, None, True, scale), (False, None, False, None), (False, "gelu", True, None),
+                                 (False, "relu_squared", False, None), (True, None, False, None)):
+        w = (torch.randn(E, 2 * F if glu else F, K, generator=g) * K ** -0.5).bfloat16()
+        out = torch.full((n, F), 7.0, dtype=odt, device=DEV)
+        ops.moe_grouped((x if pairs else packed).to(DEV), order.to(DEV) if pairs else None, top if pairs else 1, w.to(DEV), out,
+                        offsets.to(DEV), offsets.to(DEV), glu=glu, interleaved=glu, limit=1.5 if glu else 0.0, alpha=1.702 if glu else 0.0,
+                        pair_scale=None if own is None else own.to(DEV), act=act, tokens=T)
+        assert ops.gemm_error_flag(out.device) == 0
+        rows = (x[order.long() // top] if pairs else packed).double()
+        z = torch.einsum("rk,rnk->rn", rows, w[e].double())
+        err = K * 2.0 ** -23 * torch.einsum("rk,rnk->rn", rows.abs(), w[e].double().abs())           # float32 sums of exact products
+        if own is not None:
+            z, err = z * own[order.long()].double()[:, None], err * own[order.long()].double()[:, None] + z.abs() * 2.0 ** -22
+        if glu:
+            z, err = z.view(n, F // 8, 2, 8), err.view(n, F // 8, 2, 8)
+            gate, up = z[:, :, 0].clamp(max=1.5), z[:, :, 1].clamp(-1.5, 1.5)
+            want = (gate * torch.sigmoid(1.702 * gate) * (up + 1)).reshape(n, -1)
+            err = (2.8 * err[:, :, 0] + 1.4 * err[:, :, 1]).reshape(n, -1) + 2.0 ** -20              # slopes and sizes as above
+        elif act == "gelu":
+            want, err = 0.5 * z * (1 + torch.erf(z / 2 ** 0.5)), 1.13 * err + z.abs() * 2.0 ** -21
+        elif act == "relu_squared":
+            want, err = z.clamp(min=0) ** 2, (2 * z.abs() + err) * err + z * z * 2.0 ** -23
+        else:
+            want = z
+        err = err + (2.0 ** -24 if odt == torch.float32 else 2.0 ** -8) * want.abs()
+        assert ((out.cpu().double() - want).abs() <= err * 1.001).all(), (glu, act, pairs)
