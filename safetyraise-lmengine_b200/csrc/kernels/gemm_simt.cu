@@ -6,7 +6,7 @@
 // src/artifact/mod.rs:377-405.
 //
 // Two forms, with the same sums:
-//  * tiles: a block forms BM x BN outputs from a ring of slabs of 32 k's that asynchronous copies fill two slabs ahead.
+//  * tiles: a block forms BM x BN outputs from slabs of 32 k's, small tiles and large ones each in a form of their own.
 //    Bound by the FMA pipes; the tile is chosen by size (see `pick_tile`).
 //  * few rows (M <= 16, see `few_rows`): a warp streams 8 weight rows through a ring of its own, a lane owns up to four outputs.  Bound by
 //    the chain of K dependent FMAs (4 cycles each) for small weights (8 x 4,096 x 4,096: 33 us, 195 in tiles), by memory for
@@ -69,6 +69,8 @@ struct Slab {
 __device__ __forceinline__ int lane_row(int lane) { return (lane & 1) | (lane >> 2 & 2); }
 __device__ __forceinline__ int lane_col(int lane) { return (lane >> 1 & 3) | (lane >> 2 & 4); }
 
+// Small tiles, for sizes whose large tiles leave SMs idle: slabs lie row by row, as asynchronous copies bring them, and four to eight
+// warps an SM quarter hide the reads.  (32 x 32 outputs in the layout above: 305 x 1,024 x 3,072 in 124 us, 83 here.)
 // A thread forms TM x TN outputs, rows BM / TM and columns BN / TN apart.  VEC: float32 rows of whole 16-byte pieces.
 template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN, bool VEC>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
@@ -142,6 +144,139 @@ gemm_tn_simt_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TO* __re
     for (int j = 0; j < TN; ++j) {
       const int n = n0 + tn + j * DN;
       if (n < N) C[(size_t)m * ldc + n] = from_float<TO>(acc[i][j]);
+    }
+  }
+}
+
+// ROWS x BK elements of a matrix on their way to shared memory, where they lie k by k: four rows a 16-byte piece, four floats of
+// padding behind four k's, so that a warp's stores (4 rows by 32 k's) and reads (neighbouring fours of one k) share no bank.
+// What lies outside the matrix is zero.
+template <typename T, int ROWS, int THREADS, bool VEC>
+struct KSlab {
+  static constexpr int PIECES = ROWS * (BK / 4) / THREADS, GROUP = 4 * ROWS + 4, FLOATS = BK / 4 * GROUP;
+  static_assert(ROWS * (BK / 4) % THREADS == 0, "");
+  float4 v[PIECES];
+  __device__ __forceinline__ void load(const T* __restrict__ src, long long ld, int row0, int rows, int k0, int K, int tid) {
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      const int idx = tid + p * THREADS, r = row0 + idx / (BK / 4), k = k0 + (idx % (BK / 4)) * 4;
+      v[p] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < rows && k < K) {
+        const T* at = src + (size_t)r * ld + k;
+        if constexpr (VEC) {
+          v[p] = *reinterpret_cast<const float4*>(at);
+        } else {
+          v[p].x = to_float(at[0]);
+          if (k + 1 < K) v[p].y = to_float(at[1]);
+          if (k + 2 < K) v[p].z = to_float(at[2]);
+          if (k + 3 < K) v[p].w = to_float(at[3]);
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ void store(float* dst, int tid) const {
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      const int idx = tid + p * THREADS, r = idx / (BK / 4), c = idx % (BK / 4);
+      float* at = dst + c * GROUP + r;
+      at[0] = v[p].x;
+      at[ROWS] = v[p].y;
+      at[2 * ROWS] = v[p].z;
+      at[3 * ROWS] = v[p].w;
+    }
+  }
+};
+
+// Large tiles.  Slabs lie k by k, so that a read brings four rows of one k and two columns are one packed FMA (the same two sums,
+// half the instructions: a warp an SM quarter then issues its reads between the FMAs instead of before them).  Bound by
+// the FMA pipes, 70 % busy for 2,048 x 6,144 x 4,096: 1.99 ms where a tile of the form below took 2.26; with single FMAs 2.32.
+// A thread forms TM x TN outputs: rows in fours BM / TM fours apart, columns in fours BN / TN fours apart.  VEC: float32 rows of
+// whole 16-byte pieces.
+template <typename TA, typename TW, typename TO, int BM, int BN, int TM, int TN, bool VEC>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN))
+gemm_tn_pairs_kernel(const TA* __restrict__ A, const TW* __restrict__ W, TO* __restrict__ C, int M, int N,
+                    int K, long long lda, long long ldw, long long ldc) {
+  constexpr int THREADS = (BM / TM) * (BN / TN), DM = BM / TM, DN = BN / TN, PIECES = BK / 4;
+  extern __shared__ __align__(16) float slabs[];             // 2 x (a slab of A, one of W)
+  static_assert(DM % 4 == 0 && DN % 8 == 0 && TM % 4 == 0 && TN % 4 == 0, "");
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  const int tm = warp / (DN / 8) * 4 + lane_row(lane), tn = warp % (DN / 8) * 8 + lane_col(lane);
+  float2 acc[TM][TN / 2] = {};
+  typedef KSlab<TA, BM, THREADS, VEC> SlabA;
+  typedef KSlab<TW, BN, THREADS, VEC> SlabW;
+  SlabA a_slab;
+  SlabW w_slab;
+  const int steps = (K + BK - 1) / BK;
+  auto place = [&](int s) { return slabs + (s & 1) * (SlabA::FLOATS + SlabW::FLOATS); };
+  auto load = [&](int s) {
+    a_slab.load(A, lda, m0, M, s * BK, K, tid);
+    w_slab.load(W, ldw, n0, N, s * BK, K, tid);
+  };
+  auto store = [&](int s) {
+    a_slab.store(place(s), tid);
+    w_slab.store(place(s) + SlabA::FLOATS, tid);
+  };
+  float4 a[2][TM / 4], w[2][TN / 4];
+  auto read = [&](int set, const float* ap, const float* wp, int k) {
+#pragma unroll
+    for (int i = 0; i < TM / 4; ++i) a[set][i] = *reinterpret_cast<const float4*>(ap + k * BM + 4 * i * DM);
+#pragma unroll
+    for (int j = 0; j < TN / 4; ++j) w[set][j] = *reinterpret_cast<const float4*>(wp + k * BN + 4 * j * DN);
+  };
+  auto multiply = [&](int set) {
+#pragma unroll
+    for (int i = 0; i < TM; ++i) {
+      const float4 x = a[set][i / 4];
+      const float xi = i % 4 == 0 ? x.x : i % 4 == 1 ? x.y : i % 4 == 2 ? x.z : x.w;
+      const float2 xx = make_float2(xi, xi);
+#pragma unroll
+      for (int j = 0; j < TN / 2; ++j) {
+        const float4 y = w[set][j / 2];
+        acc[i][j] = fma2(xx, j % 2 ? make_float2(y.z, y.w) : make_float2(y.x, y.y), acc[i][j]);
+      }
+    }
+  };
+  load(0);
+  store(0);
+  if (steps > 1) load(1);
+  __syncthreads();
+  auto a_at = [&](int s) { return place(s) + 4 * tm; };
+  auto w_at = [&](int s) { return place(s) + SlabA::FLOATS + 4 * tn; };
+  const float *ap = a_at(0), *wp = w_at(0);
+  read(0, ap, wp, 0);
+  for (int s = 0; s < steps; ++s) {
+#pragma unroll 1
+    for (int c = 0; c < PIECES; ++c) {
+      read(1, ap, wp, 1);
+      multiply(0);
+      read(0, ap, wp, 2);
+      multiply(1);
+      read(1, ap, wp, 3);
+      multiply(0);
+      ap += SlabA::GROUP;
+      wp += SlabW::GROUP;
+      if (c == PIECES / 2 && s + 1 < steps) {                // (everyone has left slab s - 1, which lay there)
+        store(s + 1);
+        if (s + 2 < steps) load(s + 2);
+      }
+      if (c == PIECES - 1) {
+        __syncthreads();                                     // slab s + 1 is here; everyone has read slab s
+        ap = a_at(s + 1);
+        wp = w_at(s + 1);
+      }
+      read(0, ap, wp, 0);                                    // (behind the last slab: numbers that nobody uses)
+      multiply(1);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + 4 * (tm + i / 4 * DM) + i % 4;
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int n = n0 + 4 * (tn + j / 4 * DN) + j % 4;
+      if (n < N) C[(size_t)m * ldc + n] = from_float<TO>(j % 2 ? acc[i][j / 2].y : acc[i][j / 2].x);
     }
   }
 }
@@ -237,17 +372,27 @@ static int run_tile(const void* A, const void* W, void* C, int M, int N, int K, 
                     long long ldc, bool vec, cudaStream_t stream) {
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
   constexpr int threads = (BM / TM) * (BN / TN);
-  auto go = [&](auto kernel, int ring) {
-    const int smem = (int)sizeof(float) * ring * (BM + BN) * KLD;
+  auto go = [&](auto kernel, int floats) {
+    const int smem = (int)sizeof(float) * floats;
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     kernel<<<grid, threads, smem, stream>>>((const TA*)A, (const TW*)W, (TO*)C, M, N, K, lda, ldw, ldc);
     return launched();
   };
-  if constexpr (sizeof(TA) == 4 && sizeof(TW) == 4) {
-    if (vec) return go(gemm_tn_simt_kernel<TA, TW, TO, BM, BN, TM, TN, true>, STAGES);
+  constexpr bool f32 = sizeof(TA) == 4 && sizeof(TW) == 4;
+  if constexpr (BM >= 64) {
+    constexpr int floats = 2 * (KSlab<TA, BM, threads, false>::FLOATS + KSlab<TW, BN, threads, false>::FLOATS);
+    if constexpr (f32) {
+      if (vec) return go(gemm_tn_pairs_kernel<TA, TW, TO, BM, BN, TM, TN, true>, floats);
+    }
+    if constexpr (BN > 64) return refuse(ST_BAD_SIZE, "gemm_tn_simt: a tile of %d columns takes whole pieces", BN);
+    else return go(gemm_tn_pairs_kernel<TA, TW, TO, BM, BN, TM, TN, false>, floats);
+  } else {
+    if constexpr (f32) {
+      if (vec) return go(gemm_tn_simt_kernel<TA, TW, TO, BM, BN, TM, TN, true>, STAGES * (BM + BN) * KLD);
+    }
+    return go(gemm_tn_simt_kernel<TA, TW, TO, BM, BN, TM, TN, false>, 2 * (BM + BN) * KLD);
   }
-  return go(gemm_tn_simt_kernel<TA, TW, TO, BM, BN, TM, TN, false>, 2);
 }
 
 static int device_sms() {
@@ -256,26 +401,25 @@ static int device_sms() {
   return n > 0 ? n : 148;
 }
 
-// The tile whose blocks cost least.  `cycles`: what an SM spends on a k of one block where few blocks share it, measured.  A
-// thread's shared-memory reads (TM + TN values a k) and FMAs (TM x TN) overlap only between blocks, so 8 x 8 outputs a
-// thread win where there are blocks enough (2,048 x 6,144 x 4,096: 2.26 ms in tiles of 64 x 128, 2.71 in tiles of 32 x 32,
-// 3.18 with the 64 x 64 tiles of 4 x 4 outputs that this replaces) and 32 x 32 tiles where larger ones leave SMs idle
-// (305 x 1,024 x 3,072: 195 and 83 us; 155 before).  Rows that are no whole 16-byte pieces (not `vec`) are fetched number by
-// number, which blocks beside each other hide: `first` is the time of blocks that have an SM each, `each` what one more costs
-// (us at 1,001 k; 100 x 8,192: 115, 84, 74, 79, 81 in the five tiles; 300 x 8,192: 229, 188, 172, 173, 204).
+// The tile whose blocks cost least.  `cycles`: what an SM spends on a k of one block where few blocks share it, measured; large
+// tiles reuse what they read, small ones leave no SM idle (a block of 64 x 128 alone on its SM takes 112).  us in tiles of
+// 64 x 128, 64 x 64, 32 x 64, 32 x 32: 2,048 x 6,144 x 4,096 1,984, 2,101, 2,537, 2,710; 305 x 6,144 x 1,024 98.7, 110, 114,
+// 111; 500 x 1,024 x 2,048 108, 73.8, 78.9, 71.0; 305 x 1,024 x 3,072 160, 109, 116, 82.  Rows that are no whole 16-byte pieces
+// (not `vec`) are fetched number by number, which blocks beside each other hide: `first` is the time of blocks that have an SM
+// each, `each` what one more costs (us at 1,001 k; 300 x 8,192 in the last three tiles: 149, 173, 204; 24 x 8,192: 47, 34, 31;
+// in 64 x 128, which is then not taken, 160 and 65).
 static int pick_tile(int M, int N, bool vec) {
   struct Tile { int bm, bn, cycles, first, each; };
-  static const Tile tiles[] = {{128, 128, 225, 115, 176}, {64, 128, 110, 83, 80}, {64, 64, 62, 45, 39}, {32, 64, 37, 31, 21},
-                               {32, 32, 18, 21, 12}};
+  static const Tile tiles[] = {{64, 128, 100, 0, 0}, {64, 64, 62, 46, 34}, {32, 64, 37, 31, 21}, {32, 32, 18, 21, 12}};
   const int sms = device_sms();
-  int best = 0;
+  int best = -1;
   long long least = 0;
-  for (int i = 0; i < 5; ++i) {
-    if (i && (M + tiles[i].bm - 1) / tiles[i].bm > 65535) continue;          // more tiles than a grid has rows
+  for (int i = vec ? 0 : 1; i < 4; ++i) {
+    if ((M + tiles[i].bm - 1) / tiles[i].bm > 65535) continue;          // more tiles than a grid has rows
     const long long blocks = (long long)((M + tiles[i].bm - 1) / tiles[i].bm) * ((N + tiles[i].bn - 1) / tiles[i].bn);
-    const long long cost = vec ? (blocks + sms - 1) / sms * tiles[i].cycles
+    const long long cost = vec ? (blocks + sms - 1) / sms * tiles[i].cycles + (i == 0 ? 12 : 0)
                                : std::max((long long)tiles[i].first * sms, blocks * tiles[i].each);
-    if (i == 0 || cost < least) best = i, least = cost;
+    if (best < 0 || cost < least) best = i, least = cost;
   }
   return best;
 }
@@ -304,10 +448,9 @@ static int run(const void* A, const void* W, void* C, int M, int N, int K, long 
     }
   }
   switch (pick_tile(M, N, vec)) {
-    case 0: return run_tile<TA, TW, TO, 128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
-    case 1: return run_tile<TA, TW, TO, 64, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
-    case 2: return run_tile<TA, TW, TO, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
-    case 3: return run_tile<TA, TW, TO, 32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
+    case 0: return run_tile<TA, TW, TO, 64, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
+    case 1: return run_tile<TA, TW, TO, 64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
+    case 2: return run_tile<TA, TW, TO, 32, 64, 4, 4>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
     default: return run_tile<TA, TW, TO, 32, 32, 4, 2>(A, W, C, M, N, K, lda, ldw, ldc, vec, stream);
   }
 }

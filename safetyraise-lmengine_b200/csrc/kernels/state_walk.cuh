@@ -12,15 +12,6 @@ namespace srlm {
 constexpr int kStateLanes = 8;        // lanes that share a column of the state
 constexpr int kStateGroup = 8;        // tokens that a grouped walk takes at a time: lane l finishes token l
 
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;"
-      : "=l"(d)
-      : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-        "l"(*reinterpret_cast<unsigned long long*>(&c)));
-  return *reinterpret_cast<float2*>(&d);
-}
-
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 __device__ __forceinline__ float logistic_f(float z) { return 1.f / (1.f + expf(-z)); }
 

@@ -270,6 +270,22 @@ def test_gemm_simt_forms_agree_bit_for_bit(N, K):
     assert torch.equal(some, full[:5])
 
 
+@pytest.mark.parametrize("M, N, K", [(305, 6144, 36), (305, 6100, 1000), (500, 1024, 64), (451, 1021, 100), (300, 8191, 33), (257, 8250, 1)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_gemm_simt_large_tiles_agree_bit_for_bit(M, N, K, dt):
+    """Tiles of 64 x 128 and 64 x 64 (packed FMAs) form the sums of the small ones, at edges of tiles and slabs too."""
+    g = torch.Generator(device=DEV).manual_seed(12)
+    a = torch.randn(M, K, device=DEV, generator=g).to(dt)
+    w = torch.randn(N, K, device=DEV, generator=g).to(dt)
+    full = torch.full((M, N), 7.0, device=DEV, dtype=dt)
+    ops().gemm_tn_simt(a, w, full)
+    for m in range(0, M, 31):
+        some = torch.empty(min(31, M - m), 96, device=DEV, dtype=dt)
+        for n in (0, 61, N - 96):
+            ops().gemm_tn_simt(a[m:m + 31].contiguous(), w[n:n + 96].contiguous(), some)
+            assert torch.equal(some, full[m:m + 31, n:n + 96]), (m, n)
+
+
 @pytest.mark.parametrize("nq, nkv, hd, ps", [(40, 1, 64, 16), (33, 1, 20, 3), (3, 1, 18, 5), (2, 2, 7, 16), (64, 8, 128, 16),
                                              (8, 1, 130, 7)])
 @pytest.mark.parametrize("dt", ACT)
