@@ -10,28 +10,32 @@
 // KV head h / (nq/nkv), online softmax).
 //
 // A block serves up to 32 rows that read the same KV head: the query heads of a run of tokens of one request.  Keys and
-// values of a span of 128 / 64 / 32 keys (heads up to 64 / 128 / 256) are copied to shared memory once for all rows, the
-// next span in flight under the current one.  Eight warps form the scores, a lane a key; then each warp owns up to four
-// rows, a lane the dimensions lane + 32 i.  Bound by the FMA and shared-memory pipes for prompts (2,048 tokens, 32 heads of
-// 128: 2.8 ms; 34.2 with a warp a row that read its keys from global memory), by the chain of spans of the longest request
-// for decode steps (8 requests of 2,048: 0.19 ms; 2.75).
-//
-// Such a block fills an SM.  Where a step has many requests of few rows, or few keys, the small form takes 8 rows and spans of 32
-// keys without a second buffer: several blocks an SM hide the trips to memory that a short request consists of (64 requests of 16
-// keys, 32 heads of 64: 118 us in the large form, which leaves such a request an SM, 15 in the small one, 19 with the warp a row;
-// see simt_small).
+// values of a span of keys are copied to shared memory once for all rows, the next span in flight under the current one.  Eight
+// warps form the scores, a lane a key; then each warp owns up to four rows, a lane the dimensions lane + 32 i.  Bound by the
+// warps' waits for one another and for shared memory between two barriers, which a second block on the SM fills.  Three shapes with
+// the same sums (pick_shape):
+//  * paired: spans of 64 keys (32 for heads above 64), two blocks an SM.  Prompts: 2,048 tokens, 32 heads of 128 in 2.05 ms, of 64
+//    in 16 heads 0.69 (2.79 and 1.06 with one block an SM and spans twice as long, 34.2 with a warp a row that read its keys
+//    from global memory).
+//  * long: spans of 128 / 64 / 32 keys (heads up to 64 / 128 / 256), one block an SM, where the blocks are fewer than the SMs and
+//    the chain of spans of the longest request is the time (8 requests of 2,048, 32 heads of 128: 0.19 ms, 0.31 paired).
+//  * small: 8 rows and spans of 32 keys without a second buffer, several blocks an SM, for many requests of few rows, or few keys:
+//    they hide the trips to memory that a short request consists of (64 requests of 16 keys, 32 heads of 64: 118 us in the long
+//    shape, which leaves such a request an SM, 15 in the small one, 19 with the warp a row).
 #include <math_constants.h>
 
 #include "common.cuh"
 
 namespace srlm {
 
-template <int DIMS, bool SMALL>      // DIMS: dimensions a lane owns, heads up to 32 * DIMS
+enum SimtShape { SMALL, PAIRED, LONG };      // (see pick_shape)
+
+template <int DIMS, SimtShape SHAPE>          // DIMS: dimensions a lane owns, heads up to 32 * DIMS
 struct SimtForm {
-  static constexpr int KEYS = SMALL ? 32 : DIMS <= 2 ? 128 : DIMS <= 4 ? 64 : 32;
-  static constexpr int THREADS = SMALL ? 128 : 256, WARPS = THREADS / 32;
-  static constexpr int STAGES = SMALL ? 1 : 2, ROWS = SMALL ? 8 : 32, OWN = ROWS / WARPS;
-  static constexpr int BLOCKS = SMALL ? (DIMS <= 2 ? 8 : DIMS <= 4 ? 5 : 3) : 1;      // an SM
+  static constexpr int KEYS = SHAPE == SMALL ? 32 : SHAPE == PAIRED ? (DIMS <= 2 ? 64 : 32) : DIMS <= 2 ? 128 : DIMS <= 4 ? 64 : 32;
+  static constexpr int THREADS = SHAPE == SMALL ? 128 : 256, WARPS = THREADS / 32;
+  static constexpr int STAGES = SHAPE == SMALL ? 1 : 2, ROWS = SHAPE == SMALL ? 8 : 32, OWN = ROWS / WARPS;
+  static constexpr int BLOCKS = SHAPE == SMALL ? (DIMS <= 2 ? 8 : DIMS <= 4 ? 5 : 3) : SHAPE == PAIRED ? 2 : 1;      // an SM
 };
 
 // Floats from a staged key to the next: an odd number of 16-byte pieces, so that lanes on neighbouring keys share no bank.
@@ -68,12 +72,12 @@ struct SimtYes { static constexpr bool value = true; };
 struct SimtNo { static constexpr bool value = false; };
 
 // The rows of tokens t0 .. t0 + tokens - 1 (one request) and heads h_lo .. h_lo + heads - 1 of KV head kvh.
-template <typename TA, int DIMS, bool COPY, bool SMALL>       // COPY: float32 rows of whole 16-byte pieces, fetched asynchronously
+template <typename TA, int DIMS, bool COPY, SimtShape SHAPE>       // COPY: float32 rows of whole 16-byte pieces, fetched asynchronously
 __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cache, const TA* __restrict__ v_cache,
                           TA* __restrict__ out, const int* __restrict__ table, const int* __restrict__ positions, int t0,
                           int tokens, int nq, int nkv, int kvh, int h_lo, int heads, int hd, int page_size, float scale,
                           int window) {
-  typedef SimtForm<DIMS, SMALL> Form;
+  typedef SimtForm<DIMS, SHAPE> Form;
   constexpr int KEYS = Form::KEYS, STAGES = Form::STAGES, SA_ROWS = Form::ROWS, SA_OWN = Form::OWN,
                 SA_THREADS = Form::THREADS, SA_WARPS = Form::WARPS;
   extern __shared__ __align__(16) float simt_sh[];
@@ -163,13 +167,13 @@ __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cac
     const int here = min(KEYS / 32, (last - j0) / 32 + 1);   // blocks of 32 keys that somebody may see
     {
       const float* ks = k_sh + span % STAGES * KEYS * ldk;
-      constexpr int EACH = SMALL ? 2 : 8;                    // rows a task: two where a span is one block of keys for four warps
+      constexpr int EACH = SHAPE == SMALL ? 2 : 8;           // rows a task: two where a span is one block of keys for four warps
       const bool few = rows <= 2;
       const int groups = few ? 1 : (rows + EACH - 1) / EACH;
       for (int task = warp; task < groups * here; task += SA_WARPS) {
         const int kb = task % here * 32, r0 = task / here * EACH;
         const float* kp = ks + (kb + lane) * ldk;
-        if (SMALL || few) {
+        if (SHAPE == SMALL || few) {
           float dot[2];
           simt_scores<2>(kp, q_sh + r0 * ldv, ldv, pieces, dot);
 #pragma unroll
@@ -252,36 +256,50 @@ __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cac
   }
 }
 
-// Blocks (tile of tokens, KV head, z): of the runs of tokens of one request within the tile, the block serves the z-th and
-// every gridDim.z-th behind it.
-template <typename TA, int DIMS, bool COPY, bool SMALL>
-__global__ void __launch_bounds__((SimtForm<DIMS, SMALL>::THREADS), (SimtForm<DIMS, SMALL>::BLOCKS))
+// A block is (tile of tokens, KV head, lane of runs): of the runs of tokens of one request within the tile, it serves the
+// of_lane-th and every lanes-th behind it.  Where an SM holds one block or two, those with most keys should not come last: the
+// tiles are taken from both ends, the requests of a step's front (its decoding ones) and the end of its prompts first (300 tokens
+// beside 5 requests of up to 700 keys, 16 heads of 64: 68 us where the runs behind a tile's first came last, 56 now).
+template <typename TA, int DIMS, bool COPY, SimtShape SHAPE>
+__global__ void __launch_bounds__((SimtForm<DIMS, SHAPE>::THREADS), (SimtForm<DIMS, SHAPE>::BLOCKS))
 paged_attention_simt_kernel(const TA* __restrict__ q, const TA* __restrict__ k_cache, const TA* __restrict__ v_cache,
                             TA* __restrict__ out, const int* __restrict__ block_table, int table_stride,
                             const int* __restrict__ entry_of_token, const int* __restrict__ positions, int T, int nq,
                             int nkv, int hd, int page_size, float scale, int window, int tile_tokens, int head_groups) {
-  constexpr int ROWS = SimtForm<DIMS, SMALL>::ROWS;
-  const int g = nq / nkv, kvh = blockIdx.y / head_groups, h_lo = (blockIdx.y % head_groups) * ROWS;
+  constexpr int ROWS = SimtForm<DIMS, SHAPE>::ROWS;
+  const int g = nq / nkv, tiles = (T + tile_tokens - 1) / tile_tokens;
+  int tile, place, of_lane, lanes;
+  if constexpr (SHAPE == SMALL) {
+    tile = blockIdx.x, place = blockIdx.y, of_lane = blockIdx.z, lanes = gridDim.z;
+  } else {
+    const int turn = blockIdx.z * gridDim.y + blockIdx.y;
+    if (turn >= tiles) return;
+    tile = turn & 1 ? tiles - 1 - turn / 2 : turn / 2;
+    lanes = gridDim.x / (nkv * head_groups), place = blockIdx.x / lanes, of_lane = blockIdx.x % lanes;
+  }
+  const int kvh = place / head_groups, h_lo = place % head_groups * ROWS;
   const int heads = min(g - h_lo, ROWS);                  // (tile_tokens is 1 where a group has more heads than rows)
-  const int t_end = min(((int)blockIdx.x + 1) * tile_tokens, T);
+  const int t_end = min((tile + 1) * tile_tokens, T);
   int run = 0;
-  for (int t = blockIdx.x * tile_tokens; t < t_end; ++run) {
+  for (int t = tile * tile_tokens; t < t_end; ++run) {
     const int entry = entry_of_token[t];
     int tokens = 1;
     while (t + tokens < t_end && entry_of_token[t + tokens] == entry) ++tokens;
-    if (run % gridDim.z == blockIdx.z)
-      simt_rows<TA, DIMS, COPY, SMALL>(q, k_cache, v_cache, out, block_table + (size_t)entry * table_stride, positions, t, tokens, nq,
+    if (run % lanes == of_lane)
+      simt_rows<TA, DIMS, COPY, SHAPE>(q, k_cache, v_cache, out, block_table + (size_t)entry * table_stride, positions, t, tokens, nq,
                                 nkv, kvh, h_lo, heads, hd, page_size, scale, window);
     t += tokens;
   }
 }
 
-// Which form.  Requests of up to 8 rows (decode): the small one once there are more of them than SMs (us, large | small: 16 heads
+// Which shape.  Requests of up to 8 rows (decode): the small one once there are more of them than SMs (us, long | small: 16 heads
 // over 8 of 64, 64 requests of 700 keys 174 | 79, of 16 27 | 7; below that the long spans win, 4 requests of 700 43 | 76).
 // Prompts: the small one where they see few keys (16 over 8 heads of 64, 20 tokens 12.4 | 7.5), or where the heads are wide,
-// whose spans are short in both, and its finer blocks fill the GPU better (32 over 4 of 128, 40 tokens 19.9 | 14.5, behind 500
-// keys 103 | 74; 300 tokens of 16 over 8 of 64 54 | 62).
-static bool simt_small(int T, int nq, int nkv, int hd, int runs, int most_keys) {
+// whose spans are short in all, and its finer blocks fill the GPU better (us, paired | small, 16 over 8 of 128: 300 tokens
+// 69 | 63, 500 tokens 133 | 125; 32 over 4 of 128, 40 tokens behind 500 keys 103 long | 74).  Else two blocks an SM once there are
+// more blocks than SMs (16 over 8 of 64, us, long | paired: 1,000 tokens 280 | 206; 256 tokens behind 1,500 keys, 128 blocks,
+// 222 | 233).
+static SimtShape pick_shape(int T, int nq, int nkv, int hd, int runs, int most_keys) {
   const int g = nq / nkv, rows = 32, tile_tokens = g >= rows ? 1 : rows / g;
   if (runs > T) runs = T;
   const long long tiles = (T + tile_tokens - 1) / tile_tokens;
@@ -289,23 +307,26 @@ static bool simt_small(int T, int nq, int nkv, int hd, int runs, int most_keys) 
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
     sms = 148;
-  if ((long long)T * g <= 8ll * runs) return blocks > sms;
-  return (most_keys > 0 && most_keys <= 128) || (hd > 64 && blocks <= 2 * sms);
+  if ((long long)T * g <= 8ll * runs) return blocks > sms ? SMALL : LONG;
+  if ((most_keys > 0 && most_keys <= 128) || (hd > 64 && blocks <= 2 * sms)) return SMALL;
+  return blocks > sms && hd <= 128 ? PAIRED : LONG;
 }
 
-template <typename TA, int DIMS, bool COPY, bool SMALL>
+template <typename TA, int DIMS, bool COPY, SimtShape SHAPE>
 static int run_simt_form(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
                          int table_stride, const int* entry_of_token, const int* positions, int T, int nq, int nkv, int hd,
                          int page_size, float scale, int window, int runs, cudaStream_t stream) {
-  typedef SimtForm<DIMS, SMALL> Form;
+  typedef SimtForm<DIMS, SHAPE> Form;
   const size_t smem = simt_smem<Form>(hd);
-  const auto kernel = paged_attention_simt_kernel<TA, DIMS, COPY, SMALL>;
+  const auto kernel = paged_attention_simt_kernel<TA, DIMS, COPY, SHAPE>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int g = nq / nkv, head_groups = (g + Form::ROWS - 1) / Form::ROWS;
   const int tile_tokens = g >= Form::ROWS ? 1 : Form::ROWS / g;
   const int z = runs < 1 ? 1 : runs < tile_tokens ? runs : tile_tokens;
-  kernel<<<dim3((T + tile_tokens - 1) / tile_tokens, nkv * head_groups, z), Form::THREADS, smem, stream>>>(
+  const int tiles = (T + tile_tokens - 1) / tile_tokens, most = 65535, places = nkv * head_groups;
+  const dim3 grid = SHAPE == SMALL ? dim3(tiles, places, z) : dim3(places * z, tiles < most ? tiles : most, (tiles + most - 1) / most);
+  kernel<<<grid, Form::THREADS, smem, stream>>>(
       (const TA*)q, (const TA*)k_cache, (const TA*)v_cache, (TA*)out, block_table, table_stride, entry_of_token, positions, T,
       nq, nkv, hd, page_size, scale, window, tile_tokens, head_groups);
   return launched();
@@ -315,11 +336,16 @@ template <typename TA, int DIMS, bool COPY>
 static int run_simt(const void* q, const void* k_cache, const void* v_cache, void* out, const int* block_table,
                     int table_stride, const int* entry_of_token, const int* positions, int T, int nq, int nkv, int hd,
                     int page_size, float scale, int window, int runs, int most_keys, cudaStream_t stream) {
-  if (simt_small(T, nq, nkv, hd, runs, most_keys))
-    return run_simt_form<TA, DIMS, COPY, true>(q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T,
-                                               nq, nkv, hd, page_size, scale, window, runs, stream);
-  return run_simt_form<TA, DIMS, COPY, false>(q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T, nq,
-                                              nkv, hd, page_size, scale, window, runs, stream);
+  const auto go = [&](auto run_form) {
+    return run_form(q, k_cache, v_cache, out, block_table, table_stride, entry_of_token, positions, T, nq, nkv, hd, page_size, scale,
+                    window, runs, stream);
+  };
+  const SimtShape shape = pick_shape(T, nq, nkv, hd, runs, most_keys);
+  if (shape == SMALL) return go(run_simt_form<TA, DIMS, COPY, SMALL>);
+  if constexpr (DIMS <= 4) {
+    if (shape == PAIRED) return go(run_simt_form<TA, DIMS, COPY, PAIRED>);
+  }
+  return go(run_simt_form<TA, DIMS, COPY, LONG>);
 }
 
 template <typename TA, bool COPY, typename... Args>

@@ -333,6 +333,25 @@ def test_paged_attention_simt_forms_agree_bit_for_bit(nq, nkv, hd, ps, dt, windo
         assert torch.equal(run(q, bt, eot, pos), run(q, wide, eot, pos))
 
 
+@pytest.mark.parametrize("nq, nkv, hd, ps", [(16, 8, 64, 16), (32, 32, 128, 16), (40, 40, 18, 5), (64, 32, 100, 8)])
+@pytest.mark.parametrize("dt", ACT)
+@pytest.mark.parametrize("window", [0, 70])
+def test_paged_attention_simt_two_blocks_an_sm_agree_bit_for_bit(nq, nkv, hd, ps, dt, window):
+    """Prompts of more blocks than SMs beside single tokens take two blocks an SM, from both ends of the step; the same tokens
+    a few at a time take another shape.  A row's result is the same."""
+    lens_q, lens_kv = [1, 1, 210, 129], [200, 65, 210, 161]
+    q, kc, vc, _, bt, eot, pos = make_paged_case(nq, nkv, hd, ps, dt, lens_q, lens_kv, pages=640 // ps + 8)
+
+    def run(q, eot, pos):
+        out = torch.full_like(q, 7.0)
+        ops().paged_attention_simt(q, kc, vc, out, bt, eot, pos, nq, nkv, hd, ps, 1 / math.sqrt(hd), window)
+        return out
+
+    whole = run(q, eot, pos)
+    parts = [run(q[i:i + 7], eot[i:i + 7], pos[i:i + 7]) for i in range(0, q.shape[0], 7)]
+    assert torch.isfinite(whole).all() and torch.equal(whole, torch.cat(parts))
+
+
 def test_argmax_ties_go_to_the_lowest_id():
     logits = torch.zeros(4, 1000, device=DEV)
     logits[0, [5, 700]] = 3.0
