@@ -1231,7 +1231,7 @@ experts_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
     for (int i = 0; i < ahead; ++i) ask_weights(i);
   }
   pdl_wait();
-  // (behind the first `rows` tokens of an expert's rows the next ones are another block's)
+  // all tokens of the step, or the blockIdx.z-th BN of the expert's rows
   const int part = args.pair_of_row ? 0 : (int)blockIdx.z * BN;
   const int row0 = args.offsets[expert] + part, count = min(args.offsets[expert + 1] - row0, args.pair_of_row ? INT32_MAX : BN);
   const int x_row = args.pair_of_row ? 0 : row0;
@@ -1890,7 +1890,7 @@ extern "C" int srlm_moe_experts_stream(const void* A, int rows, long long lda, c
   CUtensorMap mw, mx;
   if (!cached_map(&mw, W, (long long)experts * N, K, K, BM, true) || !cached_map(&mx, A, rows, K, lda, bn, false))
     return refuse(ST_BAD_SIZE, "moe_experts_stream: cuTensorMapEncodeTiled refused the operands");
-  // an expert that a pair in two or fewer per expert leaves without rows is the exception: its first weights are not waited for
+  // first weights asked for ahead of the kernel in front: with two pairs an expert or more, few experts have no rows
   const ExpertsArgs a{C, c_dtype == DT_F32, ldc, N, K, offsets, pair_of_row, pairs_per_token, glu ? 1 : 0, act, limit, alpha,
                       pair_scale, pairs >= 2 * experts ? 1 : 0, err_flag};
   const dim3 grid((N + BM - 1) / BM, experts, pair_of_row ? 1 : (tokens + bn - 1) / bn);
