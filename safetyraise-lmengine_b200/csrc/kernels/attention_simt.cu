@@ -18,7 +18,8 @@
 //    in 16 heads 0.69 (2.79 and 1.06 with one block an SM and spans twice as long, 34.2 with a warp a row that read its keys
 //    from global memory).
 //  * long: spans of 128 / 64 / 32 keys (heads up to 64 / 128 / 256), one block an SM, where the blocks are fewer than the SMs and
-//    the chain of spans of the longest request is the time (8 requests of 2,048, 32 heads of 128: 0.19 ms, 0.31 paired).
+//    the chain of spans of the longest request is the time (8 requests of 2,048, 32 heads of 128: 0.14 ms; paired, 0.31
+//    where it was 0.19).
 //  * small: 8 rows and spans of 32 keys without a second buffer, several blocks an SM, for many requests of few rows, or few keys:
 //    they hide the trips to memory that a short request consists of (64 requests of 16 keys, 32 heads of 64: 118 us in the long
 //    shape, which leaves such a request an SM, 15 in the small one, 19 with the warp a row).
@@ -70,6 +71,7 @@ __device__ __forceinline__ void simt_scores(const float* __restrict__ kp, const 
 
 struct SimtYes { static constexpr bool value = true; };
 struct SimtNo { static constexpr bool value = false; };
+template <int N> struct SimtOwn { static constexpr int value = N; };
 
 // The rows of tokens t0 .. t0 + tokens - 1 (one request) and heads h_lo .. h_lo + heads - 1 of KV head kvh.
 template <typename TA, int DIMS, bool COPY, SimtShape SHAPE>       // COPY: float32 rows of whole 16-byte pieces, fetched asynchronously
@@ -189,57 +191,62 @@ __device__ void simt_rows(const TA* __restrict__ q, const TA* __restrict__ k_cac
     locate(span + STAGES);
     __syncthreads();
     const float* vs = v_sh + span % STAGES * KEYS * ldv;
+    auto values = [&](auto own) {                            // own: rows a warp owns, at most; with one nothing branches by row
+                                                             // (a request of 700 keys, 16 heads over 8 of 64: 42 -> 27 us)
 #pragma unroll 1
-    for (int kb = 0; kb < 32 * here; kb += 32) {
-      const int jb = j0 + kb, j = jb + lane;
-      bool any = false, all = true;                          // (uniform over the warp)
+      for (int kb = 0; kb < 32 * here; kb += 32) {
+        const int jb = j0 + kb, j = jb + lane;
+        bool any = false, all = true;                        // (uniform over the warp)
 #pragma unroll
-      for (int o = 0; o < SA_OWN; ++o) {
-        if (warp + o * SA_WARPS >= rows) continue;
-        float* sp = s_sh + (warp + o * SA_WARPS) * KEYS + kb + lane;
-        const bool valid = j >= low[o] && j <= high[o];
-        float p = 0.f;
-        if (__any_sync(0xffffffffu, valid)) {                // else the row does not see this block: nothing changes
-          const float s = valid ? *sp : -CUDART_INF_F;
-          const float m_new = fmaxf(m[o], warp_max(s));
-          const float alpha = expf(m[o] - m_new);            // m = -inf at first: exp(-inf) = 0
-          p = valid ? expf(s - m_new) : 0.f;
-          z[o] = z[o] * alpha + warp_sum(p);
-          m[o] = m_new;
+        for (int o = 0; o < decltype(own)::value; ++o) {
+          if (decltype(own)::value > 1 && warp + o * SA_WARPS >= rows) continue;
+          float* sp = s_sh + (warp + o * SA_WARPS) * KEYS + kb + lane;
+          const bool valid = j >= low[o] && j <= high[o];
+          float p = 0.f;
+          if (__any_sync(0xffffffffu, valid)) {              // else the row does not see this block: nothing changes
+            const float s = valid ? *sp : -CUDART_INF_F;
+            const float m_new = fmaxf(m[o], warp_max(s));
+            const float alpha = expf(m[o] - m_new);          // m = -inf at first: exp(-inf) = 0
+            p = valid ? expf(s - m_new) : 0.f;
+            z[o] = z[o] * alpha + warp_sum(p);
+            m[o] = m_new;
 #pragma unroll
-          for (int i = 0; i < DIMS; ++i) acc[o][i] *= alpha;
-          any = true;
+            for (int i = 0; i < DIMS; ++i) acc[o][i] *= alpha;
+            any = true;
+          }
+          all &= __all_sync(0xffffffffu, p != 0.f);
+          *sp = p;
         }
-        all &= __all_sync(0xffffffffu, p != 0.f);
-        *sp = p;
-      }
-      if (!any) continue;
-      __syncwarp();
-      const float* vp = vs + (size_t)kb * ldv + lane;
-      // a weight of zero (a key out of the row's sight, or one far below the maximum) leaves its value unread
-      auto add = [&](auto tested) {
+        if (!any) continue;
+        __syncwarp();
+        const float* vp = vs + (size_t)kb * ldv + lane;
+        // a weight of zero (a key out of the row's sight, or one far below the maximum) leaves its value unread
+        auto add = [&](auto tested) {
 #pragma unroll 2
-        for (int jj = 0; jj < 32; jj += 4) {
-          float v[4][DIMS];
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int i = 0; i < DIMS; ++i) v[e][i] = lane + 32 * i < ldv ? vp[(jj + e) * ldv + 32 * i] : 0.f;
-#pragma unroll
-          for (int o = 0; o < SA_OWN; ++o) {
-            if (warp + o * SA_WARPS >= rows) continue;
-            const float4 w = *reinterpret_cast<const float4*>(s_sh + (warp + o * SA_WARPS) * KEYS + kb + jj);
-            const float ws[4] = {w.x, w.y, w.z, w.w};
+          for (int jj = 0; jj < 32; jj += 4) {
+            float v[4][DIMS];
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-              if (!decltype(tested)::value || ws[e] != 0.f)
 #pragma unroll
-                for (int i = 0; i < DIMS; ++i) acc[o][i] = fmaf(ws[e], v[e][i], acc[o][i]);
+              for (int i = 0; i < DIMS; ++i) v[e][i] = lane + 32 * i < ldv ? vp[(jj + e) * ldv + 32 * i] : 0.f;
+#pragma unroll
+            for (int o = 0; o < decltype(own)::value; ++o) {
+              if (decltype(own)::value > 1 && warp + o * SA_WARPS >= rows) continue;
+              const float4 w = *reinterpret_cast<const float4*>(s_sh + (warp + o * SA_WARPS) * KEYS + kb + jj);
+              const float ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (!decltype(tested)::value || ws[e] != 0.f)
+#pragma unroll
+                  for (int i = 0; i < DIMS; ++i) acc[o][i] = fmaf(ws[e], v[e][i], acc[o][i]);
+            }
           }
-        }
-      };
-      if (all) add(SimtNo{}); else add(SimtYes{});
-    }
+        };
+        if (all) add(SimtNo{}); else add(SimtYes{});
+      }
+    };
+    if (rows > SA_WARPS) values(SimtOwn<SA_OWN>{});
+    else if (warp < rows) values(SimtOwn<1>{});
     __syncthreads();                                         // the span's buffers and scores are free
   }
 #pragma unroll
@@ -293,7 +300,8 @@ paged_attention_simt_kernel(const TA* __restrict__ q, const TA* __restrict__ k_c
 }
 
 // Which shape.  Requests of up to 8 rows (decode): the small one once there are more of them than SMs (us, long | small: 16 heads
-// over 8 of 64, 64 requests of 700 keys 174 | 79, of 16 27 | 7; below that the long spans win, 4 requests of 700 43 | 76).
+// over 8 of 64, 64 requests of 700 keys 174 | 79, of 16 27 | 7; below that the long spans win, 4 requests of 700 43 | 76; with a warp's one row unrolled by itself the small one
+// takes 69 for the 64 requests of 700, the long one 27 for the 4).
 // Prompts: the small one where they see few keys (16 over 8 heads of 64, 20 tokens 12.4 | 7.5), or where the heads are wide,
 // whose spans are short in all, and its finer blocks fill the GPU better (us, paired | small, 16 over 8 of 128: 300 tokens
 // 69 | 63, 500 tokens 133 | 125; 32 over 4 of 128, 40 tokens behind 500 keys 103 long | 74).  Else two blocks an SM once there are
