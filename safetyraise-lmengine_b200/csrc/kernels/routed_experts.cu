@@ -32,7 +32,7 @@ namespace srlm {
 constexpr int kTile = 64;        // rows (token, choice pairs) of a tile of the grouped products
 
 // One warp routes a token.  The row of logits sits in shared memory (z: E floats of the warp's own); `top` times
-// the warp takes the largest value left (ties: the lowest index) and strikes it out.  weights = softmax over the
+// the warp takes the largest value left (ties: the lowest index) and strikes it out: no expert twice, whatever the values.  weights = softmax over the
 // chosen values; scoring 1: weight = logistic of the chosen value itself, the choice by that logistic plus the
 // expert's `correction` when there is one (the weight does not see it).  Every weight is multiplied by wscale.
 __device__ __forceinline__ void route_token(const float* __restrict__ logits, long long ld, const float* __restrict__ bias,
@@ -87,7 +87,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, lo
     int at = E;
     for (int e = lane; e < E; e += 32) {
       const float v = z[e];
-      if (v > best || (v == best && e < at)) { best = v; at = e; }     // NaN never wins: a struck-out slot is -inf
+      if (v > best || (v == best && e < at)) { best = v; at = e; }     // NaN never wins, and a struck-out slot is NaN
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -95,7 +95,11 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, lo
       const int oa = __shfl_xor_sync(0xffffffffu, at, o);
       if (ob > best || (ob == best && oa < at)) { best = ob; at = oa; }
     }
-    if (at >= E) at = c < E ? c : 0;            // a row of NaN: any valid expert; the step's finite check reports it
+    if (at >= E) {                              // nothing but NaN is left: the first expert that is not chosen yet
+      at = 0;
+      for (int x = 0; x < c;)
+        if (choice[(size_t)t * top + x] == at) ++at, x = 0; else ++x;
+    }
     if (c == 0) first = best;
     if (correction) best = logits[(size_t)t * ld + at] + (bias ? bias[at] : 0.f);      // the weight is the score without it
     const float p = scoring == 1 ? wscale / (1.f + expf(-best)) : scoring == 2 ? expf(best - z_max) / z_den : expf(best - first);
@@ -103,7 +107,7 @@ __device__ __forceinline__ void route_token(const float* __restrict__ logits, lo
     if (lane == 0) {
       choice[(size_t)t * top + c] = at;
       weight[(size_t)t * top + c] = p;
-      z[at] = -CUDART_INF_F;
+      z[at] = CUDART_NAN_F;
     }
     __syncwarp();
   }

@@ -58,6 +58,8 @@ class RoutedExperts(Part):
             if spec.shared_size or not spec.gated or spec.weight_on_input:
                 raise Unsupported("experts named by a table are gated, weigh their outputs and come without a shared one")
             self.table = tensors[prefix + spec.expert_names.table]
+        # whether no token names an expert twice (a router's choice never does): its products may then count on it
+        self.distinct = self.table is None or self._names_each_once(self.table, spec.experts)
         self.routing = dict(scoring=spec.scoring, groups=(spec.groups, spec.groups_kept), weight_scale=spec.weight_scale,
                             correction=tensors[prefix + spec.expert_names.correction] if spec.correction else None)
         if not spec.gated:
@@ -92,6 +94,11 @@ class RoutedExperts(Part):
             self.shared_down = Linear(tensors[sp + nm.down], sp + nm.down)
         self.first = Linear(torch.cat(first, dim=0).contiguous(), p + "shared_gate_up_router")
         self.router_column = 2 * spec.shared_size
+
+    @staticmethod
+    def _names_each_once(table, experts) -> bool:
+        rows = table.sort(dim=1).values                 # (entries outside the experts all become expert 0)
+        return bool((rows >= 0).all() & (rows < experts).all() & (rows[:, 1:] != rows[:, :-1]).all())
 
     def _init_plain(self, spec, prefix, tensors, mctx):
         """Experts without a gate: [experts, ff, hidden] and [experts, hidden, ff]; the first product of the layer's input
@@ -173,13 +180,14 @@ class RoutedExperts(Part):
             self._route(ctx, first, choice, weight)
             ops.moe_sort(choice, s.experts, offsets, tiles, pair_of_row, row_of_pair)
         y = ws.get("moe.y", pairs, s.intermediate_size, ctx.dtype, reserve=ws.max_tokens * s.top)
+        tokens = T if self.distinct else 0
         if s.gated:
             ops.moe_grouped(x, pair_of_row, s.top, self.gate_up, y, offsets, tiles, glu=True, interleaved=self.interleaved,
-                            limit=self.limit, alpha=s.glu_alpha, pair_scale=weight if s.weight_on_input else None, tokens=T)
+                            limit=self.limit, alpha=s.glu_alpha, pair_scale=weight if s.weight_on_input else None, tokens=tokens)
         else:
-            ops.moe_grouped(x, pair_of_row, s.top, self.gate_up, y, offsets, tiles, act=s.activation, tokens=T)
+            ops.moe_grouped(x, pair_of_row, s.top, self.gate_up, y, offsets, tiles, act=s.activation, tokens=tokens)
         rows = ws.get("moe.rows", pairs, H, torch.float32, reserve=ws.max_tokens * s.top)
-        ops.moe_grouped(y, None, 1, self.down, rows, offsets, tiles, tokens=T)
+        ops.moe_grouped(y, None, 1, self.down, rows, offsets, tiles, tokens=tokens)
         out = ws.get("moe.out", T, H, ctx.dtype)
         ops.moe_combine(rows, row_of_pair.view(T, s.top), None if s.weight_on_input else weight,
                         add if add is not None else self._shared(ctx, first), out)
