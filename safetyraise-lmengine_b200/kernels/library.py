@@ -1055,13 +1055,19 @@ class KernelLibrary:
     GROUPED_TILE = 128       # token rows of a tile of the grouped tensor-memory product (one SM or two, by the sizes)
     GROUPED_PAIR_TILE = 256  # ... of its widest form (two SMs on 256 weight rows x 256 tokens)
 
-    def grouped_takes_tiles(self, pairs: int, experts: int, weight_elements: int) -> bool:
+    def grouped_takes_tiles(self, pairs: int, experts: int, weight_elements: int, weight_on_input: bool = False) -> bool:
         """Whether a step's ``pairs`` rows over ``experts`` groups, whose first weight matrix has ``weight_elements`` elements a
         group, go through the grouped product in tensor memory (whole tiles, however few rows an expert has) rather than the
         one of mma.sync (tiles of 32 or 64 rows).  A layer in us, mma.sync | tiles, at 25, 37.5 and 50 rows an expert: 16 experts
         1,024 wide (1 Mi elements) 58 | 64, 62 | 66, 73 | 68; 2,048 wide (4 Mi) 88 | 99, 103 | 103, 141 | 105; 4,096 wide (16 Mi)
         230 | 230, 289 | 239, 351 | 243; 64 experts 1,024 wide 104 | 130, 112 | 132, 143 | 136; 2,048 wide 243 | 254, 267 |
-        254, 326 | 267."""
+        254, 326 | 267.
+
+        weight_on_input: from 64 rows an expert on, whatever the time, since the tiles' gathered rows are multiplied by their
+        weight and rounded to bfloat16, where the products below multiply their float32 sums (outputs of a layer 256 wide
+        against float64, 45 to 63 rows an expert: 0.0034 rounded, 0.0024 so)."""
+        if weight_on_input:
+            return pairs >= 64 * experts
         return pairs >= (36 if weight_elements >= 4 << 20 else 44) * experts
 
     def grouped_tile_rows(self, pairs: int, experts: int, weight_elements: int) -> int:

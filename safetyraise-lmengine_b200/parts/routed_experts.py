@@ -163,7 +163,7 @@ class RoutedExperts(Part):
         # steps of many tokens: the experts' products on the persistent tensor-memory kernel, every expert's rows in whole
         # tiles of a gathered copy of the input
         if (self.in_tiles and ops.grouped_products_in_tensor_memory and s.intermediate_size % 8 == 0
-                and ops.grouped_takes_tiles(pairs, s.experts, (2 if s.gated else 1) * s.intermediate_size * H)):
+                and ops.grouped_takes_tiles(pairs, s.experts, (2 if s.gated else 1) * s.intermediate_size * H, s.weight_on_input)):
             self._route(ctx, first, choice, weight)
             return self._forward_tiles(ctx, x, first, choice, weight, add)
         heads = ws.get("moe.heads", 2, s.experts + 1, torch.int32, reserve=2)

@@ -95,3 +95,19 @@ def test_experts_whose_choice_is_masked_out_or_named_twice():
     ids = torch.tensor([0, 1, 2, 2, 2, 2, 2, 3, 0], dtype=torch.int32)
     want, err = layer.exact(x, table[ids.long()], torch.full((T, top), 1 / top, dtype=torch.float64))
     assert ((layer.run(x, ids) - want).abs() <= err).all()
+
+
+@pytest.mark.parametrize("T", [60, 90, 100, 127, 128, 200])
+def test_a_weight_on_the_input_costs_no_bits_below_whole_tiles(T):
+    """Below 64 rows an expert the weight multiplies float32 sums, so that only the products' inner result and the output are
+    rounded to 8 bits (each by 2^-9 of an element at most, independently of each other); from there on the input is, too."""
+    g = torch.Generator().manual_seed(T)
+    E, H, I = 2, 256, 256
+    layer = Layer(5, E, 1, H, I, scoring="logistic", weight_on_input=True)
+    x = torch.randn(T, H, generator=g).bfloat16()
+    z = x.double() @ layer.w["mlp.router"].double().T
+    weight, choice = torch.sigmoid(z).max(1, keepdim=True)
+    want, _ = layer.exact(x, choice, weight)
+    off = float((layer.run(x) - want).norm() / want.norm())
+    print("rows an expert", T / E, "error", off)
+    assert off <= 2 ** -9 * (2 ** 0.5 if T < 64 * E else 3)
