@@ -161,37 +161,31 @@ __device__ __forceinline__ uint32_t umma_idesc_bf16_f32(int n) {
          | ((uint32_t)(BM >> 4) << 24);  // M = 128; both operands K-major (bits 15, 16 zero)
 }
 
+// Registers that a load is still to fill have no name outside it: the wait is part of it.
 template <int COLS>
 __device__ __forceinline__ void tmem_load(uint32_t taddr, uint32_t (&v)[COLS]);
 template <>
 __device__ __forceinline__ void tmem_load<16>(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
         "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
+      : "r"(taddr)
+      : "memory");
 }
 template <>
 __device__ __forceinline__ void tmem_load<32>(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n\t"
+      "tcgen05.wait::ld.sync.aligned;"
       : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
         "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
         "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
         "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_load_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-// The same for values whose load was issued a while ago: none of them is touched in front of the wait.
-__device__ __forceinline__ void tmem_load_wait(uint32_t (&v)[32]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
-                 "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
-                 "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29])
-               :: "memory");
-  asm volatile("" : "+r"(v[30]), "+r"(v[31]) :: "memory");
+      : "r"(taddr)
+      : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -455,7 +449,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
       for (int c = 0; c < BN; c += CH) {
         uint32_t v[CH];
         tmem_load<CH>(tmem_base + ((uint32_t)lane_base << 16) + c, v);
-        tmem_load_wait();
 #pragma unroll
         for (int j = 0; j < CH; ++j) slab[(c + j) * SROW + lane_base + lane] = __uint_as_float(v[j]);
       }
@@ -701,12 +694,13 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
 // accumulator is double-buffered in TMEM (2 x BN columns), so the epilogue of a tile runs while
 // the MMAs of the next one are issued, and the shared-memory ring never drains between tiles.
 // The epilogue's four warps store straight from the registers that tcgen05.ld fills: a lane has one weight
-// row, so a warp's store of one token is 32 neighbouring elements of C, whole sectors whatever the rows'
-// alignment, and the warps do not wait for each other.  Turned through shared memory (two barriers and a
+// row, so a warp's store of one token is 32 neighbouring elements of C (whole sectors where C's rows start on
+// one), and the warps do not wait for each other.  Turned through shared memory (two barriers and a
 // division a 16-byte piece for every 32 tokens) a tile's epilogue took as long as 30 k-blocks, and the last
-// tile's is nobody's cover: 2,000 x 4,096 x 512 29.1 -> 15.9 us, 2,048 x 8,192 x 2,048 in float32 77.4 -> 53.7,
-// 512 x 7,168 x 5,120 45.1 -> 36.9, 2,048 x 4,096 x 4,096 54.8 -> 49.1.  Deeper rings in the shared memory that
-// this leaves (7 stages for 6) change nothing.
+// tile's is nobody's cover: 2,000 x 4,096 x 512 28.7 -> 12.9 us, 2,048 x 8,192 x 2,048 in float32 77.1 -> 54.3,
+// 512 x 7,168 x 5,120 40.3 -> 31.7, 2,048 x 4,096 x 4,096 54.1 -> 48.2.  A read of the next 32 tokens under the
+// stores of these costs more than it hides (15.0 for 12.9), as registers of a load in flight also must not be
+// moved; deeper rings in the shared memory that this leaves (7 stages for 6) change nothing.
 //
 // Tiles seldom come in multiples of the SM count: 384 tiles leave 60 of 148 SMs idle in the third
 // round.  So the k-blocks of the tiles that do not fill a round (args.sk_tiles of them, the first;
@@ -987,8 +981,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
         for (int c = 0; c < BN; c += SLAB) {
           uint32_t v[SLAB];
           tmem_load<SLAB>(tmem_base + ((uint32_t)lane_base << 16) + b * BN + c, v);
-          tmem_load_wait();
-          if (c + SLAB >= BN) {
+            if (c + SLAB >= BN) {
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) acc_drained<PAIR>(&acc_empty[b]);
@@ -1110,60 +1103,52 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
         }
         continue;
       }
-      // D[n, m] -> C[m][n]; the next 32 tokens leave TMEM while these are stored
-      uint32_t v[2][SLAB];
+      // D[n, m] -> C[m][n]
       const uint32_t acc = tmem_base + ((uint32_t)lane_base << 16) + b * BN;
       const int tokens = min(BN, args.M - m0);
-      static_assert(BN % (2 * SLAB) == 0, "slabs go two by two");
-      tmem_load<SLAB>(acc, v[0]);
 #pragma unroll 1
-      for (int c = 0; c < BN;) {
+      for (int c = 0; c < BN; c += SLAB) {
+        uint32_t x[SLAB];
+        tmem_load<SLAB>(acc + c, x);
+        if (c + SLAB >= BN) {                                 // everything of this tile has left TMEM
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) acc_drained<PAIR>(&acc_empty[b]);
+        }
+        if (args.swiglu8) {
+          // lanes l and l^8 hold the gate and the up row of one feature; they share the work: the
+          // gate lane finishes the even token of a pair, the up lane the odd one
+          const bool gate_lane = (lane & 8) == 0;
+          float h[SLAB / 2];
 #pragma unroll
-        for (int half = 0; half < 2; ++half, c += SLAB) {
-          uint32_t (&x)[SLAB] = v[half];
-          tmem_load_wait(x);
-          if (c + SLAB < BN) {
-            tmem_load<SLAB>(acc + c + SLAB, v[half ^ 1]);
-          } else {                                            // everything of this tile has left TMEM
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) acc_drained<PAIR>(&acc_empty[b]);
+          for (int j = 0; j < SLAB; j += 2) {
+            const float mine0 = __uint_as_float(x[j]), mine1 = __uint_as_float(x[j + 1]);
+            const float got = __shfl_xor_sync(0xffffffffu, gate_lane ? mine1 : mine0, 8);
+            const float gv = gate_lane ? mine0 : got, uv = gate_lane ? got : mine1;
+            h[j / 2] = args.glu_limit > 0.f ? clamped_glu_fast(gv, uv, args.glu_limit, args.glu_alpha) : silu_stable(gv) * uv;
           }
-          if (args.swiglu8) {
-            // lanes l and l^8 hold the gate and the up row of one feature; they share the work: the
-            // gate lane finishes the even token of a pair, the up lane the odd one
-            const bool gate_lane = (lane & 8) == 0;
-            float h[SLAB / 2];
+          const int col = c0 + (lane_base >> 1) + (lane >> 4) * 8 + (lane & 7), first = c + (gate_lane ? 0 : 1);
+          if (col < args.N / 2) {
+            const size_t at = (size_t)(m0 + first) * args.ldc + col;
+            if (args.c_is_f32) store_tokens(reinterpret_cast<float*>(args.C) + at, 2 * args.ldc, h, (tokens - first + 1) / 2);
+            else store_tokens(reinterpret_cast<bf16*>(args.C) + at, 2 * args.ldc, h, (tokens - first + 1) / 2);
+          }
+        } else {
+          float h[SLAB];
 #pragma unroll
-            for (int j = 0; j < SLAB; j += 2) {
-              const float mine0 = __uint_as_float(x[j]), mine1 = __uint_as_float(x[j + 1]);
-              const float got = __shfl_xor_sync(0xffffffffu, gate_lane ? mine1 : mine0, 8);
-              const float gv = gate_lane ? mine0 : got, uv = gate_lane ? got : mine1;
-              h[j / 2] = args.glu_limit > 0.f ? clamped_glu_fast(gv, uv, args.glu_limit, args.glu_alpha) : silu_stable(gv) * uv;
-            }
-            const int col = c0 + (lane_base >> 1) + (lane >> 4) * 8 + (lane & 7), first = c + (gate_lane ? 0 : 1);
-            if (col < args.N / 2) {
-              const size_t at = (size_t)(m0 + first) * args.ldc + col;
-              if (args.c_is_f32) store_tokens(reinterpret_cast<float*>(args.C) + at, 2 * args.ldc, h, (tokens - first + 1) / 2);
-              else store_tokens(reinterpret_cast<bf16*>(args.C) + at, 2 * args.ldc, h, (tokens - first + 1) / 2);
-            }
-          } else {
-            float h[SLAB];
+          for (int j = 0; j < SLAB; ++j) h[j] = __uint_as_float(x[j]);
+          if (args.act == 1) {
 #pragma unroll
-            for (int j = 0; j < SLAB; ++j) h[j] = __uint_as_float(x[j]);
-            if (args.act == 1) {
+            for (int j = 0; j < SLAB; ++j) h[j] = 0.5f * h[j] * (1.f + erff(h[j] * 0.70710678118654752440f));
+          } else if (args.act == 2) {
 #pragma unroll
-              for (int j = 0; j < SLAB; ++j) h[j] = 0.5f * h[j] * (1.f + erff(h[j] * 0.70710678118654752440f));
-            } else if (args.act == 2) {
-#pragma unroll
-              for (int j = 0; j < SLAB; ++j) h[j] = h[j] < 0.f ? 0.f : h[j] * h[j];
-            }
-            const int col = n0 + lane_base + lane;
-            if (col < args.N) {
-              const size_t at = (size_t)(m0 + c) * args.ldc + col;
-              if (args.c_is_f32) store_tokens(reinterpret_cast<float*>(args.C) + at, args.ldc, h, tokens - c);
-              else store_tokens(reinterpret_cast<bf16*>(args.C) + at, args.ldc, h, tokens - c);
-            }
+            for (int j = 0; j < SLAB; ++j) h[j] = h[j] < 0.f ? 0.f : h[j] * h[j];
+          }
+          const int col = n0 + lane_base + lane;
+          if (col < args.N) {
+            const size_t at = (size_t)(m0 + c) * args.ldc + col;
+            if (args.c_is_f32) store_tokens(reinterpret_cast<float*>(args.C) + at, args.ldc, h, tokens - c);
+            else store_tokens(reinterpret_cast<bf16*>(args.C) + at, args.ldc, h, tokens - c);
           }
         }
       }
@@ -1295,7 +1280,6 @@ experts_stream_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_co
       for (int c = 0; c < BN; c += CH) {
         uint32_t v[CH];
         tmem_load<CH>(tmem_base + ((uint32_t)lane_base << 16) + c, v);
-        tmem_load_wait();
 #pragma unroll
         for (int j = 0; j < CH; ++j) {
           const int row = row_of_col[c + j];               // the same in every lane
