@@ -981,7 +981,7 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
         for (int c = 0; c < BN; c += SLAB) {
           uint32_t v[SLAB];
           tmem_load<SLAB>(tmem_base + ((uint32_t)lane_base << 16) + b * BN + c, v);
-            if (c + SLAB >= BN) {
+          if (c + SLAB >= BN) {
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) acc_drained<PAIR>(&acc_empty[b]);
@@ -1107,10 +1107,10 @@ gemm_tcgen05_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const 
       const uint32_t acc = tmem_base + ((uint32_t)lane_base << 16) + b * BN;
       const int tokens = min(BN, args.M - m0);
 #pragma unroll 1
-      for (int c = 0; c < BN; c += SLAB) {
+      for (int c = 0; c < tokens; c += SLAB) {                // (no more: 147 x 34,816 x 5,120 with the GLU 75.6 -> 72.7 us)
         uint32_t x[SLAB];
         tmem_load<SLAB>(acc + c, x);
-        if (c + SLAB >= BN) {                                 // everything of this tile has left TMEM
+        if (c + SLAB >= tokens) {                             // everything of this tile has left TMEM
           tcgen05_fence_before();
           __syncwarp();
           if (lane == 0) acc_drained<PAIR>(&acc_empty[b]);
