@@ -1080,6 +1080,16 @@ class KernelLibrary:
         big = pairs >= 144 * experts and weight_elements >= 16 << 20
         return self.GROUPED_PAIR_TILE if self.grouped_pairs and big else self.GROUPED_TILE
 
+    def dense_tile_rows(self, tokens: int, features: int) -> int:
+        """The token tile of that product with one group: 256 where a round of pairs of SMs on 256 x 256, at 1.2 times the time
+        of a round of single SMs on 128 x 128, comes out ahead.  With the exact gelu in us, tiles of 256 | of 128: 256 tokens
+        x 8,192 x 2,048 (1 round | 1) 23.3 | 19.1, 300 tokens (1 | 2) 24.1 | 29.0; 256 x 12,288 x 3,072 (1 | 2) 31.1 | 39.6, 300
+        (2 | 2) 46.2 | 40.5, 500 (2 | 3) 48.0 | 57.5; 500 x 4,096 x 1,024 (1 | 1) 18.2 | 14.0, 640 (1 | 2) 17.9 | 18.9;
+        300 x 16,384 x 4,096 (2 | 3) 57.7 | 70.8."""
+        rounds = lambda tile, sms: -(-(-(-tokens // tile) * -(-features // tile)) // (self.SMS // sms))
+        wide = 6 * rounds(self.GROUPED_PAIR_TILE, 2) < 5 * rounds(self.GROUPED_TILE, 1)
+        return self.GROUPED_PAIR_TILE if self.grouped_pairs and wide else self.GROUPED_TILE
+
     def moe_gather_rows(self, x, pair_of_row, pairs_per_token, out, pair_scale=None):
         """out[row] = x[pair_of_row[row] // pairs_per_token] (bfloat16 rows; zeros where pair_of_row is -1), times
         pair_scale[pair] (float32, one number a pair) when given."""

@@ -92,7 +92,7 @@ class Dense(Part):
     def forward(self, ctx, x: torch.Tensor) -> torch.Tensor:
         T, (I, H) = x.shape[0], self.up.weight.shape
         h = ctx.workspace.get("dense.h", T, I, ctx.dtype)
-        tile = ops.grouped_tile_rows(T, 1, I * H)
+        tile = ops.dense_tile_rows(T, I)
         if (self.fused and ops.grouped_products_in_tensor_memory and T >= self.FUSED_TOKENS
                 and self.one_group.numel() * tile >= T):
             ops.gemm_tn_tcgen05_grouped(x, self.up.weight.view(1, I, H), h, self.one_group, act=self.spec.activation,

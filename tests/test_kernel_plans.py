@@ -37,6 +37,16 @@ def test_gemm_splits_keeps_its_bounds(M, N, K):
         assert 65536 + sp * tiles * 128 * bn * 4 <= KernelLibrary.GEMM_WS_BYTES
 
 
+# us of the dense product with its activation in tiles of 256 and of 128 tokens, as measured
+@pytest.mark.parametrize("tokens, features, us_256, us_128", [
+    (256, 4096, 17.3, 13.0), (500, 4096, 18.2, 14.0), (640, 4096, 17.9, 18.9), (2048, 4096, 28.1, 32.9),
+    (256, 8192, 23.3, 19.1), (300, 8192, 24.1, 29.0), (640, 8192, 35.6, 40.0), (256, 12288, 31.1, 39.6), (300, 12288, 46.2, 40.5),
+    (384, 12288, 46.7, 40.8), (500, 12288, 48.0, 57.5), (256, 16384, 39.3, 51.6), (300, 16384, 57.7, 70.8), (300, 20480, 92.3, 107.8)])
+def test_dense_tiles_are_the_faster_ones(tokens, features, us_256, us_128):
+    from safetyraise_lmengine_b200.kernels import ops
+    assert ops.dense_tile_rows(tokens, features) == (256 if us_256 < us_128 else 128)
+
+
 def test_prefill_attention_plan():
     plan = KernelLibrary.prefill_attention_plan
     # a whole prompt of 2,048 tokens, 4 heads per KV head, 8 KV heads: enough blocks of two row tiles, no slices
