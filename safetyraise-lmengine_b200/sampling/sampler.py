@@ -40,9 +40,9 @@ def uniform_for(seed: int, index: int) -> float:
 def fill_uniforms(seeds: Sequence[int], indices: Sequence[int], out: np.ndarray) -> None:
     """out[i] = uniform_for(seeds[i], indices[i]) (float32, contiguous) in one native call: two microseconds a pair in Python."""
     n = len(out)
-    pairs = np.array([x & _MASK for x in chain(seeds, indices)], dtype=np.uint64)
-    if len(pairs) != 2 * n:
+    if len(seeds) != n or len(indices) != n:
         raise ValueError(f"{n} rows, {len(seeds)} seeds and {len(indices)} indices")
+    pairs = np.array([x & _MASK for x in chain(seeds, indices)], dtype=np.uint64)
     at = pairs.ctypes.data
     runtime().srlm_sampling_uniforms(n, at, at + 8 * n, out.ctypes.data)
 
@@ -163,10 +163,19 @@ class Sampler:
         turn = self._buffer(words)
         host = turn[0].numpy()
         h = host[:4 * n].view(np.float32)
-        h[:n] = [p.temperature for p in params]
+        temperatures = [p.temperature for p in params]
+        h[:n] = temperatures
         h[n:2 * n] = [p.top_p for p in params]
         h[2 * n:3 * n] = [p.repetition_penalty for p in params]
-        fill_uniforms(seeds, indices, h[3 * n:])              # (of a row without a temperature nothing is drawn)
+        uniforms = h[3 * n:]
+        if min(temperatures) > 0 and len(seeds) == n == len(indices):
+            fill_uniforms(seeds, indices, uniforms)
+        else:                                                 # the seeds of rows without a temperature are not read
+            drawn = [i for i, t in enumerate(temperatures) if t > 0]
+            of_drawn = np.empty(len(drawn), dtype=np.float32)
+            fill_uniforms([seeds[i] for i in drawn], [indices[i] for i in drawn], of_drawn)
+            uniforms[:] = 0.0
+            uniforms[drawn] = of_drawn
         host[4 * n:5 * n] = [p.top_k for p in params]
         pairs = []
         if late:

@@ -399,6 +399,20 @@ def test_values_that_overflow_raise_the_fault_word(V, k, top_p):
     assert sampler.last_words[FAULT_LOGITS] == 1 and tokens[:3] == [int(np.argmax(row)) for row in adjusted[:3]]
 
 
+def test_rows_that_draw_nothing_need_no_seed():
+    """Seeds and draws of rows without a temperature are not read, nor what the sequences hold behind the rows."""
+    from safetyraise_lmengine_b200.sampling.sampler import Sampler
+    V, n = 700, 5
+    logits = torch.randn(n, V, device=DEV, generator=torch.Generator(device=DEV).manual_seed(9)) * 3
+    params = [SamplingParamsOf(1.0, 0.0), SamplingParamsOf(1.0, 0.9), SamplingParamsOf(1.4, 0.0), SamplingParamsOf(1.2, 1.3), SamplingParamsOf(1.0, 0.0)]
+    hist = [[], [], [5, 6, 7], [8], []]
+    want = Sampler(DEV, V, n).sample(logits, params, [1, 2, 3, 4, 5], [6, 7, 8, 9, 10], hist)
+    got = Sampler(DEV, V, n).sample(logits, params, [None, 2, None, 4, None, 77], [None, 7, None, 9, None, None, 3], hist)
+    assert got == want
+    assert Sampler(DEV, V, n).sample(logits, [params[1]] * n, range(20), range(30, 40), hist) == \
+        Sampler(DEV, V, n).sample(logits, [params[1]] * n, list(range(5)), list(range(30, 35)), hist)
+
+
 def test_sampling_statistics():
     """Frequencies over many draws follow the truncated distribution."""
     from safetyraise_lmengine_b200.sampling.params import SamplingParams

@@ -77,5 +77,6 @@ def test_native_uniform_numbers_are_those_of_the_plain_function():
     out = np.empty(len(seeds), dtype=np.float32)
     fill_uniforms(seeds, indices, out)
     assert out.tolist() == [uniform_for(s, i) for s, i in zip(seeds, indices)]
-    with pytest.raises(ValueError):
-        fill_uniforms(seeds, indices, out[1:])
+    for args in ((seeds, indices, out[1:]), (seeds[1:], indices, out[1:]), (seeds[2:], indices, out[1:])):
+        with pytest.raises(ValueError):
+            fill_uniforms(*args)
