@@ -182,7 +182,9 @@ class Sampler:
             offsets, at = host[5 * n:6 * n + 1], 6 * n + 1
             offsets[0] = 0
             np.cumsum(lens, out=offsets[1:])
-            if True not in late:
+            # lists in one run over all ids; an array's or a tensor's ids are copied as one piece (80,000 of them 33 us, one by
+            # one 9 ms)
+            if True not in late and all(isinstance(ids, (list, tuple)) for on, ids in zip(penalised, histories) if on):
                 host[at:at + total] = np.fromiter(chain.from_iterable(ids for on, ids in zip(penalised, histories) if on),
                                                   np.int32, total)
             else:

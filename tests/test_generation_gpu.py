@@ -413,6 +413,28 @@ def test_rows_that_draw_nothing_need_no_seed():
         Sampler(DEV, V, n).sample(logits, [params[1]] * n, list(range(5)), list(range(30, 35)), hist)
 
 
+def test_histories_in_arrays_and_tensors():
+    """Ids of a penalty as lists, arrays and tensors give the same tokens; an array's are copied as one piece, not id by id."""
+    from safetyraise_lmengine_b200.sampling.sampler import Sampler
+
+    class Counted(np.ndarray):
+        read = 0
+
+        def __iter__(self):
+            Counted.read += 1
+            return super().__iter__()
+
+    V, n = 700, 3
+    logits = torch.randn(n, V, device=DEV, generator=torch.Generator(device=DEV).manual_seed(9)) * 3
+    ids = [[int(t) for t in row.topk(40).indices] for row in logits]
+    params = [SamplingParamsOf(2.0, 0.9)] * n
+    want = Sampler(DEV, V, n).sample(logits, params, [1, 2, 3], [0] * n, ids)
+    for form in (tuple, np.array, torch.tensor, lambda x: np.array(x, dtype=np.int16), lambda x: np.array(x).view(Counted)):
+        assert Sampler(DEV, V, n).sample(logits, params, [1, 2, 3], [0] * n, [form(x) for x in ids]) == want
+    assert Sampler(DEV, V, n).sample(logits, params, [1, 2, 3], [0] * n, [ids[0], np.array(ids[1]), ids[2]]) == want
+    assert Counted.read == 0
+
+
 def test_sampling_statistics():
     """Frequencies over many draws follow the truncated distribution."""
     from safetyraise_lmengine_b200.sampling.params import SamplingParams
