@@ -58,28 +58,44 @@ def test_combination_and_gather_and_activation(act, T, H, top):
         assert torch.equal(xs.cpu(), torch.cat([x.repeat_interleave(top, 0), torch.zeros(1, 2 * H).bfloat16()]))
 
 
-@pytest.mark.parametrize("act, glu", [(None, False), ("gelu", False), ("relu_squared", False), (None, True)])
-@pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
+EPILOGUES = pytest.mark.parametrize("act, glu", [(None, False), ("gelu", False), ("relu_squared", False), (None, True)])
+OUT_TYPES = pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
+
+
+@EPILOGUES
+@OUT_TYPES
 @pytest.mark.parametrize("tile, N, K, M", [(128, 256, 72, 800), (128, 512, 136, 768), (128, 768, 64, 1100), (256, 512, 72, 700),
-                                           (256, 256, 64, 1),
-                                           # one SM a tile: 384 is no multiple of 256, fewer rows than two tiles a group
-                                           (128, 384, 72, 800), (128, 256, 72, 767), (128, 512, 64, 1)])
+                                           (256, 256, 64, 1), (128, 384, 72, 800), (128, 256, 72, 767), (128, 512, 64, 1)])
 def test_tensor_memory_products_with_their_epilogues(act, glu, odt, tile, N, K, M):
-    """Tiles of 128 and 256 tokens on pairs of SMs, with every epilogue: groups in any order, tiles without rows, a ragged last
-    tile."""
-    g = torch.Generator().manual_seed(N + M)
-    E, tiles = 3, -(-M // tile)
-    group = torch.tensor([[2, -1, 0, 1][t % 4] if M > 1 else 1 for t in range(tiles)], dtype=torch.int32)
-    x = torch.randn(M, K, generator=g).bfloat16()
-    w = (torch.randn(E, N, K, generator=g) * K ** -0.5).bfloat16()
+    """Tiles of 256 tokens on pairs of SMs and of 128 on one (the weights fit the L2), with every epilogue: groups in any order,
+    tiles without rows, a ragged last tile."""
+    check_grouped(3, act, glu, odt, tile, N, K, M)
+
+
+@EPILOGUES
+@OUT_TYPES
+@pytest.mark.parametrize("K, M", [(2056, 3109), (2048, 3072)])
+def test_pairs_of_sms_on_tiles_of_128_tokens(act, glu, odt, K, M):
+    """Weights of 64 Mi elements over all groups, and 192 rows a group (with its padding): tiles of 128 tokens on two SMs."""
+    E, N = 16, 2048
+    assert E * N * K >= 64 << 20 and M >= 192 * E
+    check_grouped(E, act, glu, odt, 128, N, K, M)
+
+
+def check_grouped(E, act, glu, odt, tile, N, K, M):
+    tiles = -(-M // tile)
+    g = torch.Generator(device=DEV).manual_seed(N + M)
+    group = torch.tensor([[E - 1, -1, 0, 1][t % 4] if M > 1 else 1 for t in range(tiles)], dtype=torch.int32, device=DEV)
+    x = torch.randn(M, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(E, N, K, generator=g, device=DEV) * K ** -0.5).bfloat16()
     out = torch.full((M, N // 2 if glu else N), 7.0, dtype=odt, device=DEV)
-    ops.gemm_tn_tcgen05_grouped(x.to(DEV), w.to(DEV), out, group.to(DEV), glu=glu, limit=1.5, alpha=1.702, tile_rows=tile, act=act)
+    ops.gemm_tn_tcgen05_grouped(x, w, out, group, glu=glu, limit=1.5, alpha=1.702, tile_rows=tile, act=act)
     assert ops.gemm_error_flag(out.device) == 0
     e = group.repeat_interleave(tile)[:M]
     rows = e >= 0
     assert (out[~rows] == 7.0).all()                          # tiles without a group are not written
-    z, size = torch.zeros(M, N, dtype=torch.float64), torch.zeros(M, N, dtype=torch.float64)
-    for k in range(E):
+    z, size = (torch.zeros(M, N, dtype=torch.float64, device=DEV) for _ in range(2))
+    for k in e[rows].unique().tolist():
         z[e == k], size[e == k] = x[e == k].double() @ w[k].double().T, x[e == k].double().abs() @ w[k].double().abs().T
     err = K * 2.0 ** -23 * size                               # float32 sums of exact products
     if glu:
@@ -95,7 +111,7 @@ def test_tensor_memory_products_with_their_epilogues(act, glu, odt, tile, N, K, 
     else:
         want = z
     err = err + (2.0 ** -24 if odt == torch.float32 else 2.0 ** -8) * want.abs()      # the result's own rounding
-    assert ((out.cpu().double() - want).abs() <= err * 1.001)[rows].all()
+    assert ((out.double() - want).abs() <= err * 1.001)[rows].all()
 
 
 @pytest.mark.parametrize("tile, N, K", [(128, 128, 64), (128, 512, 72), (256, 256, 136)])
@@ -118,8 +134,10 @@ def test_tiles_behind_the_last_one_in_use(tile, N, K, table):
             assert ((got - a @ w[group].double().T).abs() <= K * 2.0 ** -23 * (a.abs() @ w[group].double().abs().T) + 1e-9).all()
 
 
-@pytest.mark.parametrize("T, E, top", [(1, 3, 2), (16, 5, 3), (17, 4, 4), (32, 40, 2), (33, 2, 2), (64, 7, 3)])
-@pytest.mark.parametrize("F, K", [(8, 72), (72, 640), (128, 64), (136, 1032)])
+# (the last three: more than 148 blocks with rows, whose rings are the short ones)
+@pytest.mark.parametrize("T, E, top, F, K", [(*step, *size) for step in [(1, 3, 2), (16, 5, 3), (17, 4, 4), (32, 40, 2), (33, 2, 2), (64, 7, 3)]
+                                             for size in [(8, 72), (72, 640), (128, 64), (136, 1032)]]
+                         + [(16, 40, 3, 512, 328), (17, 40, 3, 512, 328), (33, 40, 2, 512, 328)])
 @pytest.mark.parametrize("odt", [torch.float32, torch.bfloat16])
 def test_experts_that_stream_their_weights(T, E, top, F, K, odt, monkeypatch):
     """Token tiles of 16, 32 and 64, experts without rows and with all tokens, features and k's that end inside a tile, rings of

@@ -139,13 +139,14 @@ def test_a_weight_that_outweighs_the_others_loses_nothing():
 @pytest.mark.parametrize("heads", [3, 40])
 @pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 40])
 @pytest.mark.parametrize("dim, rot, rank, dv", [(128, 64, 512, 128), (12, 6, 20, 9), (64, 0, 130, 33), (3, 2, 5, 1), (30, 4, 516, 132)])
-def test_the_per_head_products(heads, T, dim, rot, rank, dv):
+@pytest.mark.parametrize("wdt", [torch.bfloat16, torch.float32])
+def test_the_per_head_products(heads, T, dim, rot, rank, dv, wdt):
     """The up projections folded into the queries and applied behind the attention: token tiles of 8 and 16, sizes that are no
     whole pieces, columns beyond a block's 32; a token's result does not depend on its neighbours."""
     from safetyraise_lmengine_b200.kernels import ops
     g = torch.Generator().manual_seed(T + dim)
     q = torch.randn(T, heads * (dim + rot) + heads, generator=g)
-    uk, uv = torch.randn(heads, dim, rank, generator=g).bfloat16(), torch.randn(heads, rank, dv, generator=g).bfloat16()
+    uk, uv = torch.randn(heads, dim, rank, generator=g).to(wdt), torch.randn(heads, rank, dv, generator=g).to(wdt)
     out = torch.empty(T, heads * (rank + rot), device=DEV)
     ops.latent_absorb(q.to(DEV), uk.to(DEV), None, out, heads, dim, rot, rank)
     x = q[:, :heads * (dim + rot)].view(T, heads, dim + rot).double()

@@ -111,3 +111,20 @@ def test_a_weight_on_the_input_costs_no_bits_below_whole_tiles(T):
     off = float((layer.run(x) - want).norm() / want.norm())
     print("rows an expert", T / E, "error", off)
     assert off <= 2 ** -9 * (2 ** 0.5 if T < 64 * E else 3)
+
+
+# 16 and 64 tokens: the experts' weights are streamed past all tokens up to there (64: from 2 Mi elements a matrix on, here the first
+# product alone); 36 and 44 rows an expert: whole tiles from there on
+@pytest.mark.parametrize("H, I, lines", [(256, 256, (16, 88)), (1024, 1024, (16, 64, 88)), (1024, 2048, (16, 64, 72))])
+def test_a_token_on_either_side_of_the_lines_between_the_forms(H, I, lines):
+    """The forms of the experts' products round at the same places: below and above each line a token's output is within the
+    roundings' bound of float64."""
+    E, top = 4, 2
+    layer = Layer(7, E, top, H, I)
+    x = torch.randn(max(lines) + 1, H, generator=torch.Generator().manual_seed(H + I)).bfloat16()
+    value, choice = (x.double() @ layer.w["mlp.router"].double().T).topk(top, 1)
+    want, err = layer.exact(x, choice, torch.softmax(value, 1))
+    assert [ops.experts_stream(t, 2 * I * H) for t in (16, 17, 64, 65)] == [True, I * H >= 1 << 20, I * H >= 1 << 20, False]
+    assert [ops.grouped_takes_tiles(top * t, E, 2 * I * H) for t in (max(lines) - 1, max(lines))] == [False, True]
+    for T in sorted({t + d for t in lines for d in (-1, 0, 1)}):
+        assert ((layer.run(x[:T]) - want[:T]).abs() <= err[:T]).all(), T
