@@ -21,6 +21,7 @@ from ..parts.base import FAULT_LOGITS, FAULT_TOKEN, STATUS_WORDS
 from .params import SamplingParams
 
 _MASK = (1 << 64) - 1
+_LISTS = frozenset((list, tuple))
 
 
 def _splitmix64(x: int) -> int:
@@ -153,7 +154,8 @@ class Sampler:
         # All that the rows bring goes through one pinned buffer and one asynchronous copy (a pageable copy would make the host
         # wait for the forward that is still running on the device), as 32-bit words: five parameters a row, each n words;
         # with a penalty the rows' offsets and ids, and the pairs of patch_words behind them.
-        penalised = [p.repetition_penalty != 1.0 for p in params]
+        temperatures, penalties = [p.temperature for p in params], [p.repetition_penalty for p in params]
+        penalised = [x != 1.0 for x in penalties]
         words, late, total = 5 * n, [], 0
         if any(penalised):
             late = [on and pending is not None and pending[i] is not None for i, on in enumerate(penalised)]
@@ -163,10 +165,7 @@ class Sampler:
         turn = self._buffer(words)
         host = turn[0].numpy()
         h = host[:4 * n].view(np.float32)
-        temperatures = [p.temperature for p in params]
-        h[:n] = temperatures
-        h[n:2 * n] = [p.top_p for p in params]
-        h[2 * n:3 * n] = [p.repetition_penalty for p in params]
+        h[:3 * n] = temperatures + [p.top_p for p in params] + penalties
         uniforms = h[3 * n:]
         if min(temperatures) > 0 and len(seeds) == n == len(indices):
             fill_uniforms(seeds, indices, uniforms)
@@ -184,7 +183,7 @@ class Sampler:
             np.cumsum(lens, out=offsets[1:])
             # lists in one run over all ids; an array's or a tensor's ids are copied as one piece (80,000 of them 33 us, one by
             # one 9 ms)
-            if True not in late and all(isinstance(ids, (list, tuple)) for on, ids in zip(penalised, histories) if on):
+            if True not in late and _LISTS.issuperset(map(type, histories)):
                 host[at:at + total] = np.fromiter(chain.from_iterable(ids for on, ids in zip(penalised, histories) if on),
                                                   np.int32, total)
             else:
