@@ -300,8 +300,8 @@ paged_attention_simt_kernel(const TA* __restrict__ q, const TA* __restrict__ k_c
 }
 
 // Which shape.  Requests of up to 8 rows (decode): the small one once there are more of them than SMs (us, long | small: 16 heads
-// over 8 of 64, 64 requests of 700 keys 174 | 79, of 16 27 | 7; below that the long spans win, 4 requests of 700 43 | 76; with a warp's one row unrolled by itself the small one
-// takes 69 for the 64 requests of 700, the long one 27 for the 4).
+// over 8 of 64, 64 requests of 700 keys 174 | 79, of 16 27 | 7; below that the long spans win, 4 requests of 700 43 | 76; with
+// a warp's one row unrolled by itself the small one takes 69 for the 64 requests of 700, the long one 27 for the 4).
 // Prompts: the small one where they see few keys (16 over 8 heads of 64, 20 tokens 12.4 | 7.5), or where the heads are wide,
 // whose spans are short in all, and its finer blocks fill the GPU better (us, paired | small, 16 over 8 of 128: 300 tokens
 // 69 | 63, 500 tokens 133 | 125; 32 over 4 of 128, 40 tokens behind 500 keys 103 long | 74).  Else two blocks an SM once there are

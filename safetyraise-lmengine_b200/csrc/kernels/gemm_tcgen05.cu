@@ -1829,9 +1829,9 @@ extern "C" int srlm_gemm_tn_tcgen05_grouped(const void* X, const void* W, void* 
   const CUtensorMap *mw = &mw_copy, *mx = &mx_copy;
   // Tiles of 128 tokens go to pairs too where the weights of all groups exceed the L2 and a group has half a tile's rows or more
   // (M counts up to a tile of padding a group): 24 KB from the L2 into each SM a k-block in place of 32 for the same products.
-  // A layer in us, pairs | one SM: 16 experts, top 4, 4,096 wide, 128 rows an expert 284 | 296, 512 rows 731 | 782; 64 experts,
-  // top 8, 2,048 wide, 150 rows 376 | 406, 256 rows 488 | 555, 50 rows 272 | 267.  Where the L2 holds them one SM a tile splits the
-  // work finer: 16 experts 1,024 wide, 225 rows 102 | 97, 256 rows 113 | 106; 2,048 wide 165.0 | 164.2 and 176.9 | 176.3.
+  // A layer in us, pairs | one SM: 16 experts, top 4, 4,096 wide, 128 rows an expert 272 | 283, 512 rows 755 | 837; 64 experts,
+  // top 8, 2,048 wide, 150 rows 386 | 420, 256 rows 480 | 549, 50 rows 271 | 267.  Where the L2 holds them one SM a tile splits the
+  // work finer: 16 experts 1,024 wide, 225 rows 94 | 88, 256 rows 103 | 100; 2,048 wide 153.6 | 155.5 and 169.6 | 170.5.
   const bool pairs = tile_rows == 256 || (N % (2 * BM) == 0 && (long long)groups * N * K >= 64ll << 20 && M >= 192ll * groups);
   // (the pair form fetches the tokens of a tile in two boxes, one a block)
   if (!cached_map(&mw_copy, W, (long long)groups * N, K, K, BM, true) ||

@@ -15,8 +15,9 @@
 //   combine  out[token] = sum over its choices, in the order of the choices, of weight * row (+ the
 //            output of the expert that every token runs)
 //
-// Nothing here depends on what else is in the batch: a row's sums run over k in index order whatever
-// tile the row landed in, and the combination adds a token's rows in the order of its choices.
+// Nothing in this file depends on what else is in the batch: a row's sums run over k in index order whatever
+// tile the row landed in, and the combination adds a token's rows in the order of its choices.  (bfloat16 steps of a few
+// tokens or of many rows an expert run their products in gemm_tcgen05.cu, which adds in another order.)
 // Everything is sized on the host by upper bounds (pairs / kTile + experts tiles), so a step's launches
 // depend on its token count alone and can be replayed from a CUDA graph.
 //

@@ -1059,9 +1059,9 @@ class KernelLibrary:
         """Whether a step's ``pairs`` rows over ``experts`` groups, whose first weight matrix has ``weight_elements`` elements a
         group, go through the grouped product in tensor memory (whole tiles, however few rows an expert has) rather than the
         one of mma.sync (tiles of 32 or 64 rows).  A layer in us, mma.sync | tiles, at 25, 37.5 and 50 rows an expert: 16 experts
-        1,024 wide (1 Mi elements) 58 | 64, 62 | 66, 73 | 68; 2,048 wide (4 Mi) 88 | 99, 103 | 103, 141 | 105; 4,096 wide (16 Mi)
-        230 | 230, 289 | 239, 351 | 243; 64 experts 1,024 wide 104 | 130, 112 | 132, 143 | 136; 2,048 wide 243 | 254, 267 |
-        254, 326 | 267.
+        1,024 wide (1 Mi elements) 58 | 63, 62 | 65, 74 | 66; 2,048 wide (4 Mi) 91 | 96, 104 | 101, 138 | 103; 4,096 wide (16 Mi)
+        256 | 231, 284 | 237, 359 | 241; 64 experts 1,024 wide 104 | 122, 112 | 124, 142 | 128; 2,048 wide 244 | 253, 272 |
+        256, 319 | 263.
 
         weight_on_input: from 64 rows an expert on, whatever the time, since the tiles' gathered rows are multiplied by their
         weight and rounded to bfloat16, where the products below multiply their float32 sums (outputs of a layer 256 wide
@@ -1074,9 +1074,9 @@ class KernelLibrary:
         """The token tile of the grouped tensor-memory product for a step of ``pairs`` rows over ``experts`` groups
         whose first weight matrix has ``weight_elements`` elements a group: 256 once an expert has 144 rows on average and
         16 Mi weight elements; else 128.  A layer in us, tiles of 256 | of 128: 16 experts 4,096 wide, 128 rows an expert
-        298 | 284, 160 rows 329 | 354, 512 rows 660 | 733; 8 experts 4,096 wide, 75 rows 188 | 169, 150 rows 223 | 252;
-        16 experts 2,048 wide, 160 rows 149 | 154, 225 rows 180 | 164, 512 rows 257 | 256; 64 experts 2,048 wide, 256 rows
-        526 | 488."""
+        295 | 274, 160 rows 321 | 350, 512 rows 658 | 755; 8 experts 4,096 wide, 75 rows 174 | 155, 150 rows 183 | 212;
+        16 experts 2,048 wide, 160 rows 136 | 145, 225 rows 147 | 157, 512 rows 252 | 252; 64 experts 2,048 wide, 256 rows
+        512 | 486."""
         big = pairs >= 144 * experts and weight_elements >= 16 << 20
         return self.GROUPED_PAIR_TILE if self.grouped_pairs and big else self.GROUPED_TILE
 

@@ -20,8 +20,12 @@ weights are the chosen scores over their sum.
 ``scoring`` "table": no router; a table gives each token id its experts, each with the weight 1 / top.
 
 The pairs (token, chosen expert) are ordered by expert on the device and every expert's rows run through
-one grouped product per projection; a token's result does not depend on what else is in the step, and
-nothing is planned on the host, so decode steps replay from CUDA graphs.
+one grouped product per projection.  Nothing is planned on the host, so decode steps replay from CUDA graphs.
+In float32 a token's result does not depend on what else is in the step.  In bfloat16 the products have three
+forms, chosen by the step's tokens and its rows an expert (``experts_stream``, ``grouped_takes_tiles`` and
+``grouped_tile_rows`` of the kernel library): within a form the result does not depend on the others either, but
+a step that crosses a line between two adds the products in another order and takes the activation's
+exponential another way, and a token may round to a neighbouring number.
 """
 from __future__ import annotations
 
