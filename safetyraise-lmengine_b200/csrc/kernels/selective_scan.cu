@@ -364,14 +364,28 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
   };
 
   Pair S[PAIRS], a[PAIRS];                                  // a lane's states are neighbours: n = lane * NPL + k
-  if (walker) {
+  // Many states of short walks: pairs of S and A by one access each, N being even with WIDE (a step of 64 requests of one token, by
+  // single numbers | by pairs: 4,096 channels of 64 states 112 | 91 us, 1,024 of 128 84 | 58; with fewer states a lane, or a
+  // walk that hides its ends, the registers of both forms cost up to 8 % more than this gives).
+  const bool whole = WIDE && !LENGTHY && NPL >= 8 && (((uintptr_t)slot | (uintptr_t)A) & 7) == 0;
+  if (walker && whole) {
+#pragma unroll
+    for (int k = 0; k < PAIRS; ++k) {
+      const int n = lane * NPL + 2 * k;
+      const size_t at = (size_t)c * N + n;
+      float2 s = make_float2(0.f, 0.f), f = s;
+      if (live && n < N) s = *reinterpret_cast<const float2*>(slot + at), f = *reinterpret_cast<const float2*>(A + at);
+      S[k] = pair_of(s.x, s.y);
+      a[k] = pair_of(f.x * kLog2e, f.y * kLog2e);           // exp(dt A) = 2^(dt A log2 e)
+    }
+  } else if (walker) {
 #pragma unroll
     for (int k = 0; k < PAIRS; ++k) {
       const int n = lane * NPL + 2 * k;
       const bool on = live && n < N, two = live && n + 1 < N;
       const float *s_at = slot + (size_t)c * N + n, *a_at = A + (size_t)c * N + n;
       S[k] = pair_of(on ? s_at[0] : 0.f, two ? s_at[1] : 0.f);
-      a[k] = pair_of(on ? a_at[0] * kLog2e : 0.f, two ? a_at[1] * kLog2e : 0.f);      // exp(dt A) = 2^(dt A log2 e)
+      a[k] = pair_of(on ? a_at[0] * kLog2e : 0.f, two ? a_at[1] * kLog2e : 0.f);
     }
   } else if (n_chunks > 0) {
     for (int j = 0; j < K - 2; ++j) stage(j);
@@ -448,6 +462,10 @@ selective_scan_kernel(const float* __restrict__ x, const float* __restrict__ xz,
   for (int k = 0; k < PAIRS; ++k) {
     const int n = lane * NPL + 2 * k;
     const float2 f = halves_of(S[k]);
+    if (whole) {
+      if (live && n < N) *reinterpret_cast<float2*>(slot + (size_t)c * N + n) = f;
+      continue;
+    }
     if (live && n < N) slot[(size_t)c * N + n] = f.x;
     if (live && n + 1 < N) slot[(size_t)c * N + n + 1] = f.y;
   }

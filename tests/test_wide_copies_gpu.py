@@ -46,6 +46,29 @@ def test_scan_and_its_convolution(channels, N, lens):
     assert all(torch.equal(a, b) for a, b in zip(*got))
 
 
+@pytest.mark.parametrize("channels,N", [(16, 16), (20, 36), (16, 64), (20, 100), (20, 128)])
+@pytest.mark.parametrize("lens", [(1,), (1, 5, 64), (3, 70)])
+def test_states_of_the_scan_at_any_address(channels, N, lens):
+    """Pairs of states and decays by one access each, and number by number where an address or the slots' stride forbids it."""
+    g = torch.Generator().manual_seed(channels + N)
+    rnd = lambda *s: torch.randn(*s, generator=g).to(DEV)
+    ctx, T, taps = _Entries(lens), sum(lens), 4
+    x, xz, dbc, dt = rnd(T, channels), rnd(T, 2 * channels), rnd(T, 4 + 2 * N), rnd(T, channels)
+    A, D, bias = -torch.rand(channels, N, generator=g).to(DEV), rnd(channels), rnd(channels)
+    size = channels * (N + taps - 1)
+    start = rnd(len(lens), size)
+    got = []
+    for a, state in ((A, start.clone()), (_shifted(A), start.clone()), (A, _shifted(start)), (A, torch.full((len(lens), size + 1), 7.0, device=DEV))):
+        state[:, :size] = start
+        out = torch.empty(T, channels, device=DEV)
+        ops.selective_scan(ctx, x, xz, dbc, 4, dt, bias, a, D, state, out, channels, N, taps)
+        assert (state[:, size:] == 7.0).all()
+        got.append((out, state[:, :size]))
+    assert torch.isfinite(got[0][0]).all()
+    for other in got[1:]:
+        assert all(torch.equal(p, q) for p, q in zip(got[0], other))
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("H", [4, 508, 1020, 1024, 4100])
 @pytest.mark.parametrize("add", [False, True])
