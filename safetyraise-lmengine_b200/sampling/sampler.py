@@ -9,6 +9,7 @@ distribution and order of operations are.
 from __future__ import annotations
 
 import os
+from array import array
 from itertools import chain
 from typing import List, Sequence
 
@@ -43,8 +44,11 @@ def fill_uniforms(seeds: Sequence[int], indices: Sequence[int], out: np.ndarray)
     n = len(out)
     if len(seeds) != n or len(indices) != n:
         raise ValueError(f"{n} rows, {len(seeds)} seeds and {len(indices)} indices")
-    pairs = np.array([x & _MASK for x in chain(seeds, indices)], dtype=np.uint64)
-    at = pairs.ctypes.data
+    try:
+        pairs = array("Q", chain(seeds, indices))
+    except OverflowError:                                     # negative, or more than 64 bits
+        pairs = array("Q", [x & _MASK for x in chain(seeds, indices)])
+    at = pairs.buffer_info()[0]
     runtime().srlm_sampling_uniforms(n, at, at + 8 * n, out.ctypes.data)
 
 
